@@ -162,6 +162,45 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, in
     return !s_bad;
 }
 
+// The same barrier for kernels that cross it hundreds of times, with a vote:
+// *word counts arrivals in its lower half and arrivals with a true vote in its
+// upper half, both only ever up (the k-th crossing waits for k * nblocks, so
+// nothing is reset and no generation word follows the last arrival), and the
+// wait polls without sleeping.  *any: somebody voted true in this crossing
+// (votes: the thread 0's count of true votes so far, 0 at the first).  Only
+// when nobody did may the CTAs leave the loop, so a CTA that reads the word
+// late cannot miss a vote of this crossing.  *word starts at zero; *err as
+// above, looked at every 64 polls.
+__device__ __forceinline__ bool grid_vote(unsigned long long *word, unsigned target, bool vote,
+                                          unsigned *votes, bool *any, int *err) {
+    __shared__ int s_go;
+    const int v = __syncthreads_or(vote);
+    if (threadIdx.x == 0) {
+        int go = 1;
+        __threadfence();
+        const unsigned long long one = v ? 0x100000001ull : 1ull;
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(one) : "memory");
+        unsigned long long w;
+        for (unsigned spin = 0;; ++spin) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(word) : "memory");
+            if ((int)((unsigned)w - target) >= 0) break;
+            if ((spin & 63u) == 63u && *(volatile int *)err) { go = -1; break; }
+            if (spin > GRID_SPIN_LIMIT) {
+                atomicExch(err, 1);
+                go = -1;
+                break;
+            }
+        }
+        const unsigned now = (unsigned)(w >> 32);
+        if (go > 0 && now == *votes) go = 0;
+        *votes = now;
+        s_go = go;
+    }
+    __syncthreads();
+    *any = s_go > 0;
+    return s_go >= 0;
+}
+
 // consecutive level sets [first, last) of up to max_set rows each in one
 // cooperative launch with a bounded grid barrier between sets (bar: 2
 // device words, zero at first use; err: raised if a barrier wait ran out)

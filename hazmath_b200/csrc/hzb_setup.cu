@@ -2,6 +2,7 @@
 // Compiled with -fmad=false like the cycle kernels: the Galerkin sums are
 // rounded in the reference's order.
 #include "hzb_setup.cuh"
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -271,108 +272,29 @@ k_hem_seq(int n, const int *__restrict__ ia, const int *__restrict__ ja,
     if (lane == 0) { out[0] = nc; out[1] = status; }
 }
 
-// --- the same matching with the pass-1 state in shared memory -------------
-// Pass 1 only asks "is j already matched?".  While every neighbour index is
-// within B of its row (B = the graph's bandwidth), the vertices in play at
-// step k lie in [k - B, k + B], so one bit per vertex in a ring of RING bits
-// (RING > 2B) indexed by v mod RING holds that state; the slot of vertex
-// k + B is cleared when step k begins (its previous owner, k + B - RING,
-// finished long ago).  Pass 2 then visits only the vertices left unmatched.
-constexpr int HEM_RING_BITS = 1 << 20;                 // 128 KB of shared memory
-constexpr int HEM_RING_WORDS = HEM_RING_BITS / 32;
-
-// bw[0] = max |j - i| over the stored entries, bw[1] = longest row
-__global__ void k_graph_bandwidth(int n, const int *__restrict__ ia,
-                                  const int *__restrict__ ja, int *bw) {
+// longest row, for the ranking's limit
+__global__ void k_longest_row(int n, const int *__restrict__ ia, int *longest) {
     __shared__ int sh[32];
-    int b = 0, len = 0;
+    int len = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        for (int k = ia[i]; k < ia[i + 1]; ++k) b = max(b, abs(ja[k] - i));
+         i += gridDim.x * blockDim.x)
         len = max(len, ia[i + 1] - ia[i]);
-    }
-    b = block_max(b, sh);
     len = block_max(len, sh);
-    if (threadIdx.x == 0) { atomicMax(bw, b); atomicMax(bw + 1, len); }
+    if (threadIdx.x == 0) atomicMax(longest, len);
 }
 
-__global__ void k_hem_init(int n, const int *__restrict__ ia, int *mask, int *cnt) {
+__global__ void k_hem_init(int n, const int *__restrict__ ia, int *state) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x) {
-        mask[k] = (ia[k + 1] - ia[k] > 1) ? -1 : -2;   // pass 0
-        cnt[k] = 0;
-    }
+         k += gridDim.x * blockDim.x)
+        state[k] = (ia[k + 1] - ia[k] > 1) ? -1 : -2;   // pass 0
 }
 
-__global__ void __launch_bounds__(32)
-k_hem_pass1_ring(int n, int bw, const int *__restrict__ ia, const int *__restrict__ ja,
-                 const double *__restrict__ a, int *mask, int *cnt, int *out) {
-    extern __shared__ unsigned ring[];
-    const int lane = threadIdx.x;
-    for (int w = lane; w < HEM_RING_WORDS; w += 32) ring[w] = 0u;
-    __syncwarp();
-    constexpr unsigned RM = HEM_RING_BITS - 1;
-    int nc = 0;
-    for (int k = 0; k < n; ++k) {
-        if (lane == 0) {
-            const unsigned v = (unsigned)(k + bw) & RM;   // entering the window
-            ring[v >> 5] &= ~(1u << (v & 31));
-        }
-        __syncwarp();
-        const unsigned vk = (unsigned)k & RM;
-        const bool matched = (ring[vk >> 5] >> (vk & 31)) & 1u;
-        const int b0 = __ldg(ia + k), b1 = __ldg(ia + k + 1);
-        if (matched || b1 - b0 <= 1) continue;   // already paired / pass-0 isolated
-        double bwgt = 0.0;
-        int bp = -1;
-        for (int p = b0 + lane; p < b1; p += 32) {
-            const int j = __ldg(ja + p);
-            const unsigned vj = (unsigned)j & RM;
-            const bool mj = (ring[vj >> 5] >> (vj & 31)) & 1u;
-            if (j != k && !mj) better_last(bwgt, bp, fabs(__ldg(a + p)), p);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double w2 = __shfl_xor_sync(0xffffffffu, bwgt, o);
-            int p2 = __shfl_xor_sync(0xffffffffu, bp, o);
-            better_last(bwgt, bp, w2, p2);
-        }
-        if (bp >= 0) {
-            if (lane == 0) {
-                const int pick = __ldg(ja + bp);
-                const unsigned vp = (unsigned)pick & RM;
-                ring[vk >> 5] |= 1u << (vk & 31);
-                ring[vp >> 5] |= 1u << (vp & 31);
-                mask[k] = nc;
-                mask[pick] = nc;
-                cnt[nc] = 2;
-            }
-            ++nc;
-        }
-        __syncwarp();
-    }
-    if (lane == 0) out[0] = nc;
-}
-
-// --- pass 1 with pre-ranked candidate lists ---------------------------------
+// --- pass 1 in rounds over all SMs -------------------------------------------
 // Pass 1 of vertex k takes, among the unmatched neighbours j != k, the entry
 // of largest |a_kj|, ties to the later position.  That order does not depend
 // on the matching state, so a parallel kernel first writes every row's
-// neighbours in that order (self entries as -1 at the end), and the
-// sequential walk only looks for the first unmatched entry of the list.
-// The walk streams the lists through shared memory in tiles of 32 rows with
-// cp.async, HEM_PIPE tiles ahead of the tile it works on, so no global load
-// latency sits on its critical path.
-constexpr int HEM_PIPE = 4;                 // tiles in flight ahead of the walk
-constexpr int HEM_TILE_CAP = 3072;          // staged candidates per tile
+// neighbours in that order (self entries as -1 at the end).
 constexpr int HEM_RANK_MAXLEN = 4096;       // longest row the ranking accepts
-// slots: the tiles in flight plus the one being walked
-constexpr int HEM_IA_SLOTS = 2 * HEM_PIPE + 2, HEM_IA_STRIDE = 36;
-constexpr int HEM_C_SLOTS = HEM_PIPE + 2;
-constexpr int HEM_MISC_WORDS = 32 * 2 + 32 + 2 * 32 + 2;   // info, Pm, picks, accepted
-constexpr size_t HEM_STAGED_SMEM =
-    (size_t)HEM_RING_WORDS * 4 + (size_t)HEM_C_SLOTS * HEM_TILE_CAP * 4 +
-    (size_t)HEM_IA_SLOTS * HEM_IA_STRIDE * 4 + (size_t)HEM_MISC_WORDS * 4;
 
 // one warp per row: rank of entry p = number of entries that come before it
 __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restrict__ ja,
@@ -404,202 +326,156 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
     }
 }
 
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
+// The walk's outcome without the walk.  A row u that is still undecided
+// (neither matched nor visited) threatens a vertex v when it might take v at
+// its visit: v is u itself, or a free candidate of u not ranked below a
+// candidate that is certain to be free for u (one that no undecided row
+// before u threatens).  Row u can be decided as soon as no earlier row
+// threatens u, and it takes its best free candidate if no earlier row
+// threatens that one either: then the walk would find the same state at its
+// visit.  Threats only ever shrink, so what held a round ago is a safe bound,
+// and one barrier per round is enough: in round r a thread decides its row,
+// or posts the row's threats, by the smallest threatening row per vertex that
+// round r - 1 posted.  The posts carry the round in their upper half
+// (downwards, so a 64-bit minimum prefers the newer round), two arrays in
+// turn, and nothing has to be cleared.
+//
+// The rows in play are a window: a thread that finishes its row takes the
+// next one in ascending order, so every row below a row in play is decided or
+// in play itself.  A row that has just entered cannot use the previous
+// round's posts, which miss the rows that entered with it, and threatens all
+// its candidates.  The smallest undecided row is always decided within three
+// rounds, so the loop ends.
+//
+// Bound by the latency of a round (row state, previous posts, barrier: 3 to
+// 4 us over the grid), not by bytes: a walk of one CTA took 83 ns per row
+// (167 ms for the 2,048,383 rows of the 128^3 log-normal system, 318 ms for
+// its hierarchy; 11.8 and 37 ms now).
+//
+// CLUSTER: the CTAs are one cluster of at most 8, whose barrier and votes (in
+// every member's shared memory) cost half as much.  Its window of 8192 rows
+// can lengthen the dependency chain, which holds with half of the rows in
+// play (16,256 rows of a 2D 5-point hierarchy: 0.7 ms against 0.9) but not on
+// larger levels (32,512 rows: 584 rounds with 4096 in play, 254 with all),
+// hence HEM_CLUSTER_ROWS.
+constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = 16384;
 
-// The matched state of the vertices in play lives in a ring of shared memory:
-// one byte per vertex (BYTES, 2^17 vertices, plain stores) while the window
-// fits, else one bit per vertex (2^20 vertices, atomicOr).  Both rings take
-// 128 KB.  Ring size > 2 bw + 64: the 32 slots entering the window are
-// cleared when a tile begins (vertices >= r0 + bw cannot be matched before
-// tile r0 starts, and the slot's previous owner lies below r0 - bw).
-template <bool BYTES>
-struct HemRing {
-    static constexpr unsigned SIZE = BYTES ? (1u << 17) : (1u << 20);
-    static constexpr unsigned RM = SIZE - 1;
-    void *mem;
-    __device__ __forceinline__ bool get(int v) const {
-        const unsigned u = (unsigned)v & RM;
-        if (BYTES) return ((const volatile unsigned char *)mem)[u] != 0;
-        return (((const volatile unsigned *)mem)[u >> 5] >> (u & 31)) & 1u;
-    }
-    __device__ __forceinline__ void set(int v) {
-        const unsigned u = (unsigned)v & RM;
-        if (BYTES) ((volatile unsigned char *)mem)[u] = 1;
-        else atomicOr((unsigned *)mem + (u >> 5), 1u << (u & 31));
-    }
-    // vertices v0 .. v0 + 31, by the whole warp
-    __device__ __forceinline__ void clear32(int v0, int lane) {
-        if (BYTES) {
-            ((unsigned char *)mem)[((unsigned)v0 + lane) & RM] = 0;
-        } else {
-            const unsigned u = (unsigned)v0 & RM, sh = u & 31u, w0 = u >> 5;
-            unsigned *w = (unsigned *)mem;
-            if (lane == 0) w[w0] &= ~(0xffffffffu << sh);
-            if (lane == 1 && sh) w[(w0 + 1) & (SIZE / 32 - 1)] &= ~((1u << sh) - 1u);
-        }
-    }
-};
-
-// Two warps.  Warp 1 streams row pointers and ranked lists into shared
-// memory (cp.async, HEM_PIPE tiles ahead) and writes the pairs of finished
-// tiles to mask/cnt; warp 0 walks the tiles.  Within a tile of 32 rows every
-// row first takes its best candidate unmatched when the tile starts; rows are
-// then settled in order.  A row keeps that choice unless an earlier row of
-// the tile took it or matched the row's choice (vertices only ever become
-// matched, so the entries ranked above it stay ineligible); such a row scans
-// its list again.  For a row that keeps its choice the effect on the rows
-// after it is known in advance: the row it picks leaves the walk (rm) and the
-// rows that wanted the same vertex or this row go stale (st).
-template <bool BYTES>
-__global__ void __launch_bounds__(64)
-k_hem_pass1_staged(int n, int bw, const int *__restrict__ ia, const int *__restrict__ cand,
-                   int *mask, int *cnt, int *out) {
-    extern __shared__ unsigned hem_smem[];
-    HemRing<BYTES> ring{hem_smem};
-    int *cbuf = (int *)(hem_smem + HEM_RING_WORDS);
-    int *iabuf = cbuf + HEM_C_SLOTS * HEM_TILE_CAP;
-    uint2 *info = (uint2 *)(iabuf + HEM_IA_SLOTS * HEM_IA_STRIDE);
-    unsigned *pm = (unsigned *)(info + 32);
-    int *picks = (int *)(pm + 32);              // [2][32], by tile parity
-    unsigned *accepted = (unsigned *)(picks + 64);   // [2]
+template <bool CLUSTER>
+__global__ void __launch_bounds__(HEM_BLOCK)
+k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, int *state,
+             unsigned long long *post, int *next, unsigned long long *bar, int *err) {
     const int lane = threadIdx.x & 31;
-    const int ntiles = (n + 31) >> 5;
-
-    if (threadIdx.x >= 32) {   // ---- warp 1: staging and output
-        int nc = 0;
-        auto emit = [&](int u) {
-            const unsigned acc = accepted[u & 1];
-            if ((acc >> lane) & 1u) {
-                const int id = nc + __popc(acc & ((1u << lane) - 1u));
-                const int q = picks[(u & 1) * 32 + lane];
-                mask[(u << 5) + lane] = id;
-                mask[q] = id;
-                cnt[id] = 2;
-            }
-            nc += __popc(acc);
-        };
-        for (int j = -2 * HEM_PIPE; j < ntiles; ++j) {
-            if (j >= 2) emit(j - 2);
-            const int ui = j + 2 * HEM_PIPE;   // row pointers of tile j + 2 PIPE
-            if (ui < ntiles) {
-                const int r0 = ui << 5, rows = min(32, n - r0);
-                int *dst = iabuf + (ui % HEM_IA_SLOTS) * HEM_IA_STRIDE;
-                cp_async4(dst + lane, ia + r0 + min(lane, rows));
-                if (lane == 0) cp_async4(dst + 32, ia + r0 + rows);
-            }
-            cp_async_wait<HEM_PIPE - 1>();   // ia(j + PIPE) and cand(j) have landed
-            __syncwarp();
-            const int uc = j + HEM_PIPE;     // ranked lists of tile j + PIPE
-            if (uc >= 0 && uc < ntiles) {
-                const int *iu = iabuf + (uc % HEM_IA_SLOTS) * HEM_IA_STRIDE;
-                const int rows = min(32, n - (uc << 5));
-                const int e0 = iu[0], m = iu[rows] - e0;
-                if (m <= HEM_TILE_CAP) {
-                    int *dst = cbuf + (uc % HEM_C_SLOTS) * HEM_TILE_CAP;
-                    for (int e = lane; e < m; e += 32) cp_async4(dst + e, cand + e0 + e);
+    constexpr int B = 4;             // candidates examined at a time
+    __shared__ int s_vote[2][HEM_CLUSTER];
+    int u = -1, p0 = 0, p1 = 0;      // the row in play, its candidates left
+    int pending = blockIdx.x * blockDim.x + threadIdx.x;   // enters next round
+    bool more = true;                // rows may be left to take
+    unsigned votes = 0;
+    const unsigned max_round = 3u * (unsigned)n + 16u;
+    for (unsigned r = 1;; ++r) {
+        const unsigned long long *prev = post + (size_t)((r - 1) & 1u) * n;
+        unsigned long long *cur = post + (size_t)(r & 1u) * n;
+        const unsigned long long mark = (unsigned long long)(0xffffffffu - r) << 32;
+        const unsigned was = 0xffffffffu - (r - 1);
+        const bool fresh = u < 0;
+        if (u < 0 && pending < n) {
+            u = pending;
+            p0 = ia[u];
+            p1 = ia[u + 1];
+        }
+        if (u >= 0) {
+            // smallest row that threatened v in the previous round
+            auto threat = [&](unsigned long long t) {
+                return (unsigned)(t >> 32) == was ? (int)(unsigned)t : 0x7fffffff;
+            };
+            const int su = __ldcg(state + u);
+            const unsigned long long tu = __ldcg(prev + u);
+            bool done = su != -1;                  // an earlier row took it
+            const bool mine = !fresh && threat(tu) == u;
+            int best = -1;
+            bool open = true;
+            for (int p = p0; open && p < p1; p += B) {
+                int c[B], sc[B];
+                unsigned long long t[B];
+#pragma unroll
+                for (int q = 0; q < B; ++q) c[q] = p + q < p1 ? cand[p + q] : -1;
+#pragma unroll
+                for (int q = 0; q < B; ++q) {
+                    sc[q] = c[q] >= 0 ? __ldcg(state + c[q]) : 0;
+                    t[q] = c[q] >= 0 ? __ldcg(prev + c[q]) : 0ull;
                 }
-            }
-            cp_async_commit();
-            if (j >= 0) __syncthreads();   // tile j is ready; tile j - 1 is walked
-        }
-        cp_async_wait<0>();
-        __syncthreads();                    // the last tile is walked
-        if (ntiles >= 2) emit(ntiles - 2);
-        if (ntiles >= 1) emit(ntiles - 1);
-        if (lane == 0) out[0] = nc;
-        return;
-    }
-
-    // ---- warp 0: the walk
-    for (int w = lane; w < HEM_RING_WORDS; w += 32) hem_smem[w] = 0u;
-    __syncthreads();
-    for (int t = 0; t < ntiles; ++t) {
-        const int r0 = t << 5, rows = min(32, n - r0);
-        ring.clear32(r0 + bw, lane);
-        __syncwarp();
-        const int *it = iabuf + (t % HEM_IA_SLOTS) * HEM_IA_STRIDE;
-        const int e0 = it[0];
-        const bool staged = it[rows] - e0 <= HEM_TILE_CAP;
-        const int *ct = staged ? cbuf + (t % HEM_C_SLOTS) * HEM_TILE_CAP : cand;
-        const int off = staged ? e0 : 0;
-        int *pk = picks + (t & 1) * 32;
-        // rows of the tile still unmatched and not isolated (pass 0)
-        const bool act = lane < rows && it[lane + 1] - it[lane] > 1 && !ring.get(r0 + lane);
-        unsigned todo = __ballot_sync(0xffffffffu, act);
-        int p = -1;
-        if (act) {
-            const int b1 = it[lane + 1];
-            for (int e = it[lane]; e < b1; e += 2) {
-                const int c0 = ct[e - off];
-                const int c1 = e + 1 < b1 ? ct[e + 1 - off] : -1;
-                const bool ok0 = c0 >= 0 && !ring.get(c0);
-                const bool ok1 = c1 >= 0 && !ring.get(c1);
-                if (ok0) { p = c0; break; }
-                if (ok1) { p = c1; break; }
-            }
-        }
-        const unsigned tl = (unsigned)(p - r0);   // < 32: the pick is a row of this tile
-        pm[lane] = 0u;
-        __syncwarp();
-        if (p >= 0 && tl < 32u) atomicOr(pm + tl, 1u << lane);
-        const unsigned same = __match_any_sync(0xffffffffu, p);
-        const unsigned has = __ballot_sync(0xffffffffu, p >= 0);
-        __syncwarp();
-        if (p >= 0) info[lane] = make_uint2(tl < 32u ? 1u << tl : 0u, same | pm[lane]);
-        else info[lane] = make_uint2(0u, 0u);
-        pk[lane] = p;
-        __syncwarp();
-        unsigned stale = 0u, done = 0u, racc = 0u, written = 0u;
-        while (todo) {
-            const int i = __ffs(todo) - 1;
-            todo &= todo - 1u;
-            if ((stale >> i) & 1u) {
-                // the ring takes every pick of the tile so far, then row i scans again
-                const unsigned w = done & has & ~written;
-                if ((w >> lane) & 1u) { ring.set(r0 + lane); ring.set(p); }
-                written |= w;
-                __syncwarp();
-                const int b0 = it[i], b1 = it[i + 1];
-                int q = -1;
-                for (int e = b0; e < b1; e += 32) {
-                    const int c = e + lane < b1 ? ct[e + lane - off] : -1;
-                    const bool ok = c >= 0 && !ring.get(c);
-                    const unsigned bal = __ballot_sync(0xffffffffu, ok);
-                    if (bal) {
-                        q = __shfl_sync(0xffffffffu, c, __ffs(bal) - 1);
-                        break;
+                if (done) break;
+#pragma unroll
+                for (int q = 0; q < B; ++q) {
+                    if (!open) continue;
+                    if (c[q] < 0) { open = false; continue; }   // end of the list
+                    if (sc[q] >= 0) continue;                   // matched
+                    const int tv = threat(t[q]);
+                    if (best < 0) {
+                        best = c[q];
+                        p0 = p + q;           // what precedes it stays matched
+                        if (mine && tv == u) {
+                            __stcg(state + u, u);
+                            __stcg(state + best, u);
+                            done = true;
+                            open = false;
+                            continue;
+                        }
                     }
+                    atomicMin(cur + c[q], mark | (unsigned)u);
+                    if (!fresh && tv >= u) open = false;        // free for u for certain
                 }
-                if (q >= 0) {
-                    if (lane == 0) { ring.set(r0 + i); ring.set(q); pk[i] = q; }
-                    racc |= 1u << i;
-                    const unsigned d = (unsigned)(q - r0);
-                    if (d < 32u) todo &= ~(1u << d);
-                    stale |= __ballot_sync(0xffffffffu, p == q || p == r0 + i);
-                }
-                __syncwarp();
-                continue;
             }
-            const uint2 f = info[i];
-            done |= 1u << i;
-            todo &= ~f.x;
-            stale |= f.y;
+            if (best < 0 && mine) done = true;   // visited without a partner
+            if (!done) atomicMin(cur + u, mark | (unsigned)u);
+            if (done) u = -1;
         }
-        const unsigned acc = (done & has) | racc;
-        const unsigned w = done & has & ~written;
-        if ((w >> lane) & 1u) { ring.set(r0 + lane); ring.set(p); }
-        if (lane == 0) accepted[t & 1] = acc;
-        __syncthreads();   // tile t walked; tile t + 1 staged
+        // rows for the threads without one, ascending
+        const unsigned need = __ballot_sync(0xffffffffu, u < 0);
+        int base = n;
+        const int lead = __ffs(need) - 1;
+        if (more && lane == lead) base = atomicAdd(next, __popc(need));
+        const bool vote = u >= 0 || more;
+        bool any;
+        if (CLUSTER) {
+            namespace cg = cooperative_groups;
+            cg::cluster_group cl = cg::this_cluster();
+            const int v = __syncthreads_or(vote);
+            if (threadIdx.x < gridDim.x)
+                *cl.map_shared_rank(&s_vote[r & 1u][blockIdx.x], threadIdx.x) = v;
+            cl.sync();
+            any = false;
+            for (unsigned q = 0; q < gridDim.x; ++q) any |= s_vote[r & 1u][q] != 0;
+        } else if (!grid_vote(bar, r * gridDim.x, vote, &votes, &any, err)) {
+            return;
+        }
+        if (!any) return;
+        if (need) {
+            base = __shfl_sync(0xffffffffu, base, lead);
+            pending = n;
+            if (u < 0) pending = min(n, base + __popc(need & ((1u << lane) - 1u)));
+            if (base >= n) more = false;
+        }
+        if (r >= max_round) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) *err = 1;
+            return;
+        }
+    }
+}
+
+// pairs numbered by their visiting row (state[k] == k), as the walk counts
+__global__ void k_hem_visitors(int n, const int *__restrict__ state, int *flag) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+        flag[k] = state[k] == k;
+}
+// state (visiting rows) -> aggregate ids, and the members counted for pass 2
+__global__ void k_hem_number(int n, const int *__restrict__ pos, int *state, int *cnt) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int v = state[k];
+        if (v >= 0) {
+            state[k] = pos[v];
+            if (v == k) cnt[pos[v]] = 2;
+        }
     }
 }
 
@@ -615,43 +491,65 @@ __global__ void k_compact(int n, const int *__restrict__ flag, const int *__rest
         if (flag[i]) list[pos[i]] = i;
 }
 
-// pass 2 over the leftover list (ascending), one warp, reference semantics
+// Pass 2 over the leftover list (ascending), one warp: a leftover joins the
+// adjacent aggregate with the fewest members, the first such entry on ties,
+// and the next leftover sees that aggregate one larger.  A lane takes one
+// leftover each and chooses as if no other lane did; the choice stands unless
+// an earlier lane chose an aggregate that this row looks at, or is itself a
+// neighbour of this row.  Those are looked up by hash in two shared tables of
+// the first lane per slot (a false hit only ends the batch early), the lanes
+// before the first doubtful one commit, and the next batch starts there.  One
+// row at a time took 1.06 ms for the leftovers of the 128^3 log-normal level,
+// a chain of four dependent loads each.
 __global__ void __launch_bounds__(32)
 k_hem_pass2_list(int m, const int *__restrict__ list, const int *__restrict__ ia,
                  const int *__restrict__ ja, int *mask_, int *cnt_, int *out) {
+    constexpr int H = 1024;
+    __shared__ int lane_of_agg[H], lane_of_row[H];
     volatile int *mask = mask_;
     volatile int *cnt = cnt_;
     const int lane = threadIdx.x;
+    for (int q = lane; q < H; q += 32) lane_of_agg[q] = lane_of_row[q] = 32;
+    __syncwarp();
     int status = 0;
-    for (int q = 0; q < m; ++q) {
-        const int k = list[q];
-        const int b0 = ia[k], b1 = ia[k + 1];
-        double bwgt = 0.0;
-        int bp = -1, bc = -1;
-        for (int p = b0 + lane; p < b1; p += 32) {
+    for (int q0 = 0; q0 < m;) {
+        const int q = q0 + lane;
+        const bool on = q < m;
+        const int k = on ? list[q] : 0;
+        const int b0 = on ? ia[k] : 0, b1 = on ? ia[k + 1] : 0;
+        int bc = -1, bn = 0;
+        for (int p = b0; p < b1; ++p) {
             const int kc = mask[ja[p]];
-            if (kc >= 0) {
-                double w2 = (double)(-cnt[kc]);
-                int oldp = bp;
-                better_first(bwgt, bp, w2, p);
-                if (bp != oldp) bc = kc;
-            }
+            if (kc < 0) continue;
+            const int c = cnt[kc];
+            if (bc < 0 || c < bn) { bc = kc; bn = c; }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double w2 = __shfl_xor_sync(0xffffffffu, bwgt, o);
-            int p2 = __shfl_xor_sync(0xffffffffu, bp, o);
-            int c2 = __shfl_xor_sync(0xffffffffu, bc, o);
-            int oldp = bp;
-            better_first(bwgt, bp, w2, p2);
-            if (bp != oldp) bc = c2;
-        }
-        if (bp < 0) { status = -1; break; }
-        if (lane == 0) {
-            mask[k] = bc;
-            cnt[bc] = cnt[bc] + 1;
+        if (on) {
+            if (bc >= 0) atomicMin(lane_of_agg + (bc & (H - 1)), lane);
+            atomicMin(lane_of_row + (k & (H - 1)), lane);
         }
         __syncwarp();
+        bool doubt = false;
+        for (int p = b0; p < b1; ++p) {
+            const int j = ja[p], kc = mask[j];
+            doubt |= lane_of_row[j & (H - 1)] < lane;
+            if (kc >= 0) doubt |= lane_of_agg[kc & (H - 1)] < lane;
+        }
+        const unsigned dm = __ballot_sync(0xffffffffu, doubt);
+        const int stop = dm ? __ffs(dm) - 1 : min(32, m - q0);   // lane 0 has no doubt
+        // a row without an aggregated neighbour: the reference stops there
+        const unsigned none = __ballot_sync(0xffffffffu, on && lane < stop && bc < 0);
+        const int last = none ? __ffs(none) - 1 : stop;
+        if (on && bc >= 0) lane_of_agg[bc & (H - 1)] = 32;
+        if (on) lane_of_row[k & (H - 1)] = 32;
+        if (on && lane < last) {
+            mask[k] = bc;
+            cnt[bc] = bn + 1;   // no other lane below last chose bc
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (none) { status = -1; break; }
+        q0 += stop;
     }
     if (lane == 0) out[1] = status;
 }
@@ -664,100 +562,111 @@ __global__ void k_hem_final(int n, int *mask) {
 
 int hem_exact(int n, const int *nia, const int *nja, const double *nval,
               int *agg, int *nagg, int *work_n, cudaStream_t s) {
+    // out: aggregates, status | longest row | next row | barrier (2) | error
+    enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 6, O_N = 8 };
     int *out = nullptr;
-    HZB_TRY(dalloc(&out, 4));
-    HZB_CUDA(cudaMemsetAsync(out, 0, 4 * sizeof(int), s));
-    k_graph_bandwidth<<<grid_for(n), 256, 0, s>>>(n, nia, nja, out + 2);
+    HZB_TRY(dalloc(&out, O_N));
+    int h[O_N] = {0};
+    int gnnz = 0, rc = SUCCESS;
+    const int g = grid_for(n);
+    cudaError_t e = cudaMemsetAsync(out, 0, O_N * sizeof(int), s);
+    k_longest_row<<<g, 256, 0, s>>>(n, nia, out + O_LEN);
     count_launch();
-    int gb[3] = {0, 0, 0};
-    HZB_CUDA(cudaMemcpyAsync(gb, out + 2, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    HZB_CUDA(cudaMemcpyAsync(gb + 2, nia + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    HZB_CUDA(cudaStreamSynchronize(s));
-    const int bw = gb[0], maxlen = gb[1], gnnz = gb[2];
-    // Four implementations with the same decisions, the fastest that the
-    // graph allows: 1 ranked lists + byte ring, 2 ranked lists + bit ring,
-    // 3 bit ring over the raw rows, 4 state in global memory.  HZB_HEM_PATH
-    // names one (if the graph allows it) for tests of the others.
-    int path = 4;
-    if (2 * bw + 64 < (int)HemRing<true>::SIZE && maxlen <= HEM_RANK_MAXLEN) path = 1;
-    else if (2 * bw + 64 < HEM_RING_BITS && maxlen <= HEM_RANK_MAXLEN) path = 2;
-    else if (2 * bw + 2 < HEM_RING_BITS) path = 3;
-    if (const char *f = getenv("HZB_HEM_PATH")) {
-        const int want = atoi(f);
-        if (want >= path && want <= 4) path = want;
-    }
-    int rc = SUCCESS;
-    if (path <= 3) {
-        int *flag = nullptr, *pos = nullptr, *list = nullptr, *tmp = nullptr;
-        const int g = grid_for(n);
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_hem_pass1_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 HEM_RING_WORDS * 4);
-            attr = true;
-        }
-        if ((rc = dalloc(&flag, n)) || (rc = dalloc(&pos, n + 1)) || (rc = dalloc(&list, n)) ||
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h, out, O_N * sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&gnnz, nia + n, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) { dfree(out); set_error(e, __FILE__, __LINE__); return ERROR_SOLVER_MISC; }
+    // 1: rounds over ranked lists; 4: one warp walks the rows, for rows longer
+    // than the ranking takes (its work grows with the square of a row's
+    // length).  HZB_HEM_PATH=4 names the walk for tests.
+    int path = h[O_LEN] <= HEM_RANK_MAXLEN ? 1 : 4;
+    if (const char *f = getenv("HZB_HEM_PATH"))
+        if (atoi(f) == 4) path = 4;
+    if (path == 1) {
+        int *cand = nullptr, *flag = nullptr, *pos = nullptr, *tmp = nullptr;
+        unsigned long long *post = nullptr;
+        if ((rc = dalloc(&cand, gnnz)) || (rc = dalloc(&post, (size_t)2 * n)) ||
+            (rc = dalloc(&flag, n)) || (rc = dalloc(&pos, n + 1)) ||
             (rc = dalloc(&tmp, scan_tmp_size(n + 1)))) {
-            dfree(flag); dfree(pos); dfree(list); dfree(tmp); dfree(out);
+            dfree(cand); dfree(post); dfree(flag); dfree(pos); dfree(tmp); dfree(out);
             return rc;
         }
-        k_hem_init<<<g, 256, 0, s>>>(n, nia, agg, work_n);
-        count_launch();
-        int *cand = nullptr;
-        if (path <= 2 && dalloc(&cand, std::max(1, gnnz)) == SUCCESS) {
-            static bool attr2 = false;
-            if (!attr2) {
-                cudaFuncSetAttribute(k_hem_pass1_staged<true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)HEM_STAGED_SMEM);
-                cudaFuncSetAttribute(k_hem_pass1_staged<false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)HEM_STAGED_SMEM);
-                attr2 = true;
-            }
-            k_hem_rank<<<std::min(div_up(n, 8), 148 * 64), 256, 0, s>>>(n, nia, nja, nval, cand);
-            if (path == 1)
-                k_hem_pass1_staged<true><<<1, 64, HEM_STAGED_SMEM, s>>>(n, bw, nia, cand, agg,
-                                                                        work_n, out);
-            else
-                k_hem_pass1_staged<false><<<1, 64, HEM_STAGED_SMEM, s>>>(n, bw, nia, cand, agg,
-                                                                         work_n, out);
-            count_launch(2);
-            dfree(cand);
-        } else {
-            k_hem_pass1_ring<<<1, 32, HEM_RING_WORDS * 4, s>>>(n, bw, nia, nja, nval, agg,
-                                                              work_n, out);
-            count_launch();
+        int *cnt = work_n;
+        k_hem_init<<<g, 256, 0, s>>>(n, nia, agg);
+        k_hem_rank<<<std::min(div_up(n, 8), 148 * 64), 256, 0, s>>>(n, nia, nja, nval, cand);
+        count_launch(2);
+        // all ones: older than any round's post
+        e = cudaMemsetAsync(post, 0xff, sizeof(unsigned long long) * 2 * n, s);
+        // one CTA per SM; a cluster of 1 to 8 on small levels
+        const bool cluster = n <= HEM_CLUSTER_ROWS;
+        int grid = std::min(sm_count(), div_up(n, HEM_BLOCK));
+        if (cluster) {
+            const int want = std::min(grid, HEM_CLUSTER);
+            for (grid = 1; grid < want;) grid *= 2;
         }
-        k_flag_eq<<<g, 256, 0, s>>>(n, agg, -1, flag);
+        const int first = grid * HEM_BLOCK;
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(out + O_NEXT, &first, sizeof(int), cudaMemcpyHostToDevice, s);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(HEM_BLOCK);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        if (cluster) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = grid;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        }
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia, (const int *)cand, agg, post,
+                                   out + O_NEXT, (unsigned long long *)(out + O_BAR),
+                                   out + O_ERR);
         count_launch();
+        k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
         rc = scan_exclusive(flag, pos, n, tmp, s);
         int m = 0;
         if (!rc) {
+            k_hem_number<<<g, 256, 0, s>>>(n, pos, agg, cnt);
+            cudaMemcpyAsync(out + O_NC, pos + n, sizeof(int), cudaMemcpyDeviceToDevice, s);
+            k_flag_eq<<<g, 256, 0, s>>>(n, agg, -1, flag);
+            rc = scan_exclusive(flag, pos, n, tmp, s);
+        }
+        if (!rc) {
+            int *list = cand;   // the ranked lists are done with (gnnz >= leftovers)
             k_compact<<<g, 256, 0, s>>>(n, flag, pos, list);
-            count_launch();
+            count_launch(4);
             cudaMemcpyAsync(&m, pos + n, sizeof(int), cudaMemcpyDeviceToHost, s);
             cudaStreamSynchronize(s);
             if (m > 0) {
-                k_hem_pass2_list<<<1, 32, 0, s>>>(m, list, nia, nja, agg, work_n, out);
+                k_hem_pass2_list<<<1, 32, 0, s>>>(m, list, nia, nja, agg, cnt, out);
                 count_launch();
             }
             k_hem_final<<<g, 256, 0, s>>>(n, agg);
             count_launch();
         }
-        dfree(flag); dfree(pos); dfree(list); dfree(tmp);
-    } else {   // wide graph: the whole state in global memory
+        dfree(cand); dfree(post); dfree(flag); dfree(pos); dfree(tmp);
+    } else {   // the whole state in global memory
         k_hem_seq<<<1, 32, 0, s>>>(n, nia, nja, nval, agg, work_n, out);
         count_launch();
     }
-    int h[2] = {0, 0};
-    cudaError_t e = cudaMemcpyAsync(h, out, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, out, O_N * sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     dfree(out);
     if (rc) return rc;
     if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); return ERROR_SOLVER_MISC; }
-    *nagg = h[0];
-    return h[1] < 0 ? ERROR_AMG_COARSEING : SUCCESS;
+    if (h[O_ERR]) {
+        set_error_msg("the rounds of the heavy edge matching ran out of time");
+        return ERROR_SOLVER_MISC;
+    }
+    *nagg = h[O_NC];
+    return h[O_STATUS] < 0 ? ERROR_AMG_COARSEING : SUCCESS;
 }
 
 // ---------------------------------------------------------------------------

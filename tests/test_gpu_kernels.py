@@ -112,6 +112,38 @@ def test_hem_implementations_agree(golden, port, monkeypatch, path):
     assert nc == nc_o and np.array_equal(agg, agg_o)
 
 
+def _random_graph(n, deg, seed, symmetric):
+    """Random CSR with negative off-diagonals of few distinct weights (ties),
+    wide rows and any bandwidth."""
+    rng = np.random.default_rng(seed)
+    m = max(1, n * deg // 2)
+    i, j = rng.integers(0, n, m), rng.integers(0, n, m)
+    i, j = i[i != j], j[i != j]
+    w = -rng.integers(1, 6, len(i)).astype(float)
+    if symmetric:
+        i, j, w = np.r_[i, j], np.r_[j, i], np.r_[w, w]
+    key, first = np.unique(i * n + j, return_index=True)
+    k = np.r_[key, np.arange(n) * (n + 1)]
+    v = np.r_[w[first], np.full(n, 50.0)]
+    order = np.argsort(k)
+    k, v = k[order], v[order]
+    ia = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(k // n, minlength=n), out=ia[1:])
+    return ia.astype(np.int32), (k % n).astype(np.int32), v
+
+
+@pytest.mark.parametrize("n,deg,symmetric", [
+    (2, 2, True), (1024, 6, True), (1025, 6, True), (2049, 5, False), (8193, 40, True),
+    (16384, 6, True), (16385, 6, True), (40000, 7, False), (200001, 8, True)])
+def test_hem_rounds_vs_oracle(port, n, deg, symmetric):
+    """One CTA, clusters of 2 to 8, the grid, a window smaller than the graph;
+    rows without a partner and graphs that are not symmetric."""
+    ia, ja, val = _random_graph(n, deg, n, symmetric)
+    nc_o, agg_o = port.hem(ia, ja, val, 0.0)
+    nc, agg = _hem(ia, ja, val, 0.0)
+    assert nc == nc_o and np.array_equal(agg, agg_o)
+
+
 def test_rap_bit_exact(golden):
     g = golden("rap.npz")
     A = DevCSR(g["ia"], g["ja"], g["val"])
