@@ -1,13 +1,20 @@
 // hzb_dense.cu -- coarsest-level dense factorisation (FP64).
 //
 // The coarsest matrix (<= coarse_dof rows, ~1-2k) is expanded to a dense
-// lower triangle, factored A = L L^T with a blocked right-looking Cholesky
-// (32-wide panels: diagonal block in shared memory, panel solve, tiled
-// trailing update), L is inverted block row by block row (tiled product with
-// the rows already inverted, then a 32-row triangular solve per column), and
-// A^{-1} = L^{-T} L^{-1} is formed once, so that every V-cycle applies the
-// coarse solve as one dense matrix-vector product (n^2 FP64 reads from L2)
-// instead of two dependent triangular sweeps.  About 5 n/32 launches.
+// lower triangle and factored A = L L^T, L is inverted, and A^{-1} =
+// L^{-T} L^{-1} is formed once, so that every V-cycle applies the coarse
+// solve as one dense matrix-vector product (n^2 FP64 reads from L2) instead
+// of two dependent triangular sweeps.
+//
+// The arithmetic (n^3 multiply-adds, 0.3 ms at the FP64 rate for n = 2000) is
+// short against the chain of n / 32 panel steps, so the chain is what the
+// layout serves: one launch per 32-column step, in which the CTA of the
+// first trailing tile also factors and inverts the next diagonal block (it
+// alone holds it, updated), and the inverse of L by doubling block sizes
+// (2 log2(n / 32) launches of independent tiles) instead of block row by
+// block row.  n = 1600: 6.5 -> 2.0 ms; n = 1999: 9.5 -> 2.6 ms.  What bounds a
+// step now is shared memory bandwidth while many tiles are left, then the 32
+// dependent columns of the diagonal block.
 // This file may contract a*b+c into FMA: the coarse solve is a direct
 // solve that agrees with the reference's sparse LDL^T only to rounding.
 #include <algorithm>
@@ -15,7 +22,9 @@
 
 namespace hzb {
 
-constexpr int NB = 32;
+constexpr int NB = 32;          // panel width
+constexpr int TB = 64;          // tile of the updates and products
+constexpr int TK = 16;          // depth of a staged slice of the products
 
 __global__ void k_dense_from_csr(int n, const int *__restrict__ ia,
                                  const int *__restrict__ ja,
@@ -25,160 +34,279 @@ __global__ void k_dense_from_csr(int n, const int *__restrict__ ia,
         for (int k = ia[i]; k < ia[i + 1]; ++k) D[(size_t)i * n + ja[k]] += a[k];
 }
 
-// Cholesky of the jb x jb diagonal block at (j0, j0), in shared memory.
-// blockDim = (32, 32).
-__global__ void k_potrf_diag(int n, int j0, int jb, double *D, int *bad) {
-    __shared__ double T[NB][NB + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    T[ty][tx] = (tx < jb && ty < jb) ? D[(size_t)(j0 + ty) * n + j0 + tx] : 0.0;
+// Inverse of the Cholesky factor of a 32 x 32 SPD block, by 256 threads:
+// elimination in place (below the diagonal the factors of the unit lower
+// inverse replace the eliminated entries), then a scaling by the pivots'
+// roots.  W: the block (read) and the result; V: a second buffer, the two
+// alternate so that a column costs one barrier.  Returns false on a pivot
+// that is not positive (every thread sees the same pivots).
+using Block = double[NB][NB + 1];
+__device__ __forceinline__ bool invert_factor(Block *W, Block *V) {
+    const int k = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = (*W)[w + 8 * q][k];
     __syncthreads();
-    for (int j = 0; j < jb; ++j) {
-        const double piv = T[j][j];
-        if (!(piv > 0.0)) {
-            if (tx == 0 && ty == 0) *bad = 1;
-            return;   // uniform: every thread read the same pivot
+    Block *in = W, *out = V;
+    for (int j = 0; j < NB; ++j) {
+        const double piv = (*in)[j][j];
+        if (!(piv > 0.0)) return false;
+        const double rp = 1.0 / piv, jk = (*in)[j][k];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = w + 8 * q;
+            if (i > j) {
+                const double f = (*in)[i][j] * rp;
+                v[q] = k == j ? -f : v[q] - f * jk;
+            }
+            (*out)[i][k] = v[q];
         }
-        const double l = sqrt(piv);
         __syncthreads();
-        if (ty == 0 && tx == j) T[j][j] = l;
-        if (ty == 0 && tx > j && tx < jb) T[tx][j] /= l;
-        __syncthreads();
-        if (ty > j && tx > j && tx <= ty && ty < jb) T[ty][tx] -= T[ty][j] * T[tx][j];
-        __syncthreads();
+        Block *t = in; in = out; out = t;
     }
-    if (tx < jb && ty < jb && tx <= ty) D[(size_t)(j0 + ty) * n + j0 + tx] = T[ty][tx];
+    // *in: pivots on the diagonal, the unit lower inverse below it
+    double r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = w + 8 * q;
+        const double root = sqrt((*in)[i][i]);
+        r[q] = k < i ? (*in)[i][k] / root : k == i ? 1.0 / root : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) (*W)[w + 8 * q][k] = r[q];
+    __syncthreads();
+    return true;
 }
 
-// L[i, j0:j0+jb] = A[i, j0:j0+jb] L_JJ^{-T} for the rows below the block
-__global__ void k_trsm_panel(int n, int j0, int jb, double *D, const int *bad) {
-    __shared__ double Ljj[NB][NB + 1];
-    if (*bad) return;
-    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
-        const int r = t / NB, c = t % NB;
-        Ljj[r][c] = (r < jb && c < jb) ? D[(size_t)(j0 + r) * n + j0 + c] : 0.0;
+// the block at (r0, r0), padded with the identity, inverted into X
+__device__ __forceinline__ void factor_diag(int n, int r0, Block *W, Block *V, double *X,
+                                            int *bad) {
+    if (!invert_factor(W, V)) {
+        if (threadIdx.x == 0) *bad = 1;
+        return;
     }
-    __syncthreads();
-    const int i = j0 + jb + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double x[NB];
-    double *row = D + (size_t)i * n + j0;
-#pragma unroll
-    for (int c = 0; c < NB; ++c) x[c] = c < jb ? row[c] : 0.0;
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-        if (c < jb) {
-            double v = x[c];
-            for (int k = 0; k < c; ++k) v -= x[k] * Ljj[c][k];
-            x[c] = v / Ljj[c][c];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < NB; ++c)
-        if (c < jb) row[c] = x[c];
+    const int k = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < NB; i += 8)
+        if (r0 + i < n && k <= i) X[(size_t)(r0 + i) * n + r0 + k] = (*W)[i][k];
 }
 
-// trailing update D[i][k] -= sum_t L[i][j0+t] L[k][j0+t], r0 <= k <= i < n,
-// r0 = j0 + jb; 32 x 32 output tiles of the lower triangle.
-__global__ void k_syrk_update(int n, int j0, int jb, double *D, const int *bad) {
-    __shared__ double Li[NB][NB + 1], Lk[NB][NB + 1];
-    if (*bad) return;
-    const int r0 = j0 + jb;
-    const int bi = blockIdx.y, bk = blockIdx.x;
-    if (bk > bi) return;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i = r0 + bi * NB + ty, k = r0 + bk * NB + tx;
-    const int ii = r0 + bi * NB + tx;   // loader indices
-    const int kk = r0 + bk * NB + tx;
-    // load panel rows: Li[row][t] = L[r0 + bi*NB + row][j0 + t]
-    for (int row = ty; row < NB; row += blockDim.y) {
-        const int gi = r0 + bi * NB + row, gk = r0 + bk * NB + row;
-        Li[row][tx] = (gi < n && tx < jb) ? D[(size_t)gi * n + j0 + tx] : 0.0;
-        Lk[row][tx] = (gk < n && tx < jb) ? D[(size_t)gk * n + j0 + tx] : 0.0;
+__global__ void __launch_bounds__(256)
+k_chol_first(int n, const double *__restrict__ D, double *X, int *bad) {
+    __shared__ Block W, V;
+    const int k = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < NB; i += 8) {
+        const int a = max(i, k), b = min(i, k);   // the lower triangle is the one kept
+        W[i][k] = a < n ? D[(size_t)a * n + b] : (i == k ? 1.0 : 0.0);
     }
-    (void)ii; (void)kk;
     __syncthreads();
-    if (i >= n || k >= n || k > i) return;
-    double acc = 0.0;
+    factor_diag(n, 0, &W, &V, X, bad);
+}
+
+// Step j0: the panel L[:, j0:j0+32] = D[:, j0:j0+32] X_JJ^T and the trailing
+// update D -= L L^T, one 64 x 64 tile of the lower triangle per CTA.  Every
+// tile forms the two panel slices it needs (a third of its arithmetic), so
+// panel and update need no launch between them; tiles of the first column
+// store theirs.  The first tile goes on to the next diagonal block.
+__global__ void __launch_bounds__(256)
+k_chol_step(int n, int j0, double *D, double *L, double *X, int *bad) {
+    __shared__ double Pi[TB][NB + 1], Pk[TB][NB + 1], Ij[NB][NB + 1];
+    if (*(volatile int *)bad) return;
+    int bi = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
+    while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
+    while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
+    const int bk = (int)blockIdx.x - bi * (bi + 1) / 2;
+    const int r0 = j0 + NB, ri = r0 + bi * TB, rk = r0 + bk * TB;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = w; i < TB; i += 8) {
+        Pi[i][lane] = ri + i < n ? D[(size_t)(ri + i) * n + j0 + lane] : 0.0;
+        if (bi != bk) Pk[i][lane] = rk + i < n ? D[(size_t)(rk + i) * n + j0 + lane] : 0.0;
+        if (i < NB) Ij[i][lane] = lane <= i ? X[(size_t)(j0 + i) * n + j0 + lane] : 0.0;
+    }
+    __syncthreads();
+    double li[8], lk[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) li[q] = lk[q] = 0.0;
 #pragma unroll 8
-    for (int t = 0; t < NB; ++t) acc += Li[ty][t] * Lk[tx][t];
-    D[(size_t)i * n + k] -= acc;
-}
-
-// Inverse of L, block row I (rows i0..i0+ib): first
-//   X[I, c] = -sum_{k=c..i0-1} L[I][k] X[k][c]   for columns c < i0
-// (32 x 32 output tiles), then the diagonal solve below.
-__global__ void k_trinv_gemm(int n, int i0, int ib, const double *__restrict__ L,
-                             double *X) {
-    __shared__ double Ls[NB][NB + 1], Xs[NB][NB + 1];
-    const int c0 = blockIdx.x * NB;
-    if (c0 >= i0) return;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int r = i0 + ty, c = c0 + tx;
-    double acc = 0.0;
-    for (int k0 = c0; k0 < i0; k0 += NB) {
-        const int lk = k0 + tx, xk = k0 + ty;
-        Ls[ty][tx] = (ty < ib && lk < i0) ? L[(size_t)r * n + lk] : 0.0;
-        Xs[ty][tx] = (xk < i0 && c < n) ? X[(size_t)xk * n + c] : 0.0;
-        __syncthreads();
-#pragma unroll 8
-        for (int t = 0; t < NB; ++t) acc += Ls[ty][t] * Xs[t][tx];
-        __syncthreads();
-    }
-    if (ty < ib && c < i0) X[(size_t)r * n + c] = -acc;
-}
-
-// X[I, c] = L_II^{-1} rhs(c) for every column c < i0 + ib, where rhs is the
-// tile product above (c < i0) or the identity (c >= i0).
-__global__ void k_trinv_diag(int n, int i0, int ib, const double *__restrict__ L,
-                             double *X) {
-    __shared__ double Lii[NB][NB + 1];
-    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
-        const int rr = t / NB, cc = t % NB;
-        Lii[rr][cc] = (rr < ib && cc < ib) ? L[(size_t)(i0 + rr) * n + i0 + cc] : 0.0;
-    }
-    __syncthreads();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= i0 + ib) return;
-    double x[NB];
+    for (int t = 0; t < NB; ++t) {
+        const double x = Ij[lane][t];
 #pragma unroll
-    for (int rr = 0; rr < NB; ++rr) {
-        if (rr < ib) {
-            double v = (c < i0) ? X[(size_t)(i0 + rr) * n + c] : (c == i0 + rr ? 1.0 : 0.0);
-            for (int t = 0; t < rr; ++t) v -= Lii[rr][t] * x[t];
-            x[rr] = v / Lii[rr][rr];
-        } else {
-            x[rr] = 0.0;
+        for (int q = 0; q < 8; ++q) {
+            li[q] += Pi[w + 8 * q][t] * x;
+            if (bi != bk) lk[q] += Pk[w + 8 * q][t] * x;
         }
     }
+    __syncthreads();
 #pragma unroll
-    for (int rr = 0; rr < NB; ++rr)
-        if (rr < ib) X[(size_t)(i0 + rr) * n + c] = x[rr];
+    for (int q = 0; q < 8; ++q) {
+        const int i = w + 8 * q;
+        Pi[i][lane] = li[q];
+        Pk[i][lane] = bi != bk ? lk[q] : li[q];
+        if (bk == 0 && ri + i < n) L[(size_t)(ri + i) * n + j0 + lane] = li[q];
+    }
+    __syncthreads();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) acc[q][p] = 0.0;
+#pragma unroll 8
+    for (int t = 0; t < NB; ++t) {
+        double a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { a[q] = Pi[ty + 16 * q][t]; b[q] = Pk[tx + 16 * q][t]; }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) acc[q][p] += a[q] * b[p];
+    }
+    const bool next = blockIdx.x == 0;   // this tile holds the next diagonal block
+    if (next) __syncthreads();           // Pi becomes its buffers
+    Block *W = reinterpret_cast<Block *>(&Pi[0][0]);
+    Block *V = reinterpret_cast<Block *>(&Pi[NB][0]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int i = ty + 16 * q, k = tx + 16 * p;
+            double d = 0.0;
+            if (ri + i < n && rk + k <= ri + i) {
+                const size_t at = (size_t)(ri + i) * n + rk + k;
+                d = D[at] - acc[q][p];
+                D[at] = d;
+            }
+            if (next && i < NB && k <= i) {
+                if (ri + i >= n) d = i == k ? 1.0 : 0.0;
+                (*W)[i][k] = d;
+                (*W)[k][i] = d;
+            }
+        }
+    if (next) {
+        __syncthreads();
+        factor_diag(n, r0, W, V, X, bad);
+    }
 }
 
-// Ainv = X^T X (16 x 16 tiles; X lower triangular)
-__global__ void k_xtx(int n, const double *__restrict__ X, double *Ainv) {
-    __shared__ double ta[16][17], tb[16][17];
-    const int a = blockIdx.y * 16 + threadIdx.y;   // output row
-    const int b = blockIdx.x * 16 + threadIdx.x;   // output column
-    const int i0 = max(blockIdx.y, blockIdx.x) * 16;   // X[i][a] = 0 for i < a
-    double acc = 0.0;
-    for (int it = i0; it < n; it += 16) {
-        const int ir = it + threadIdx.y;
-        const int ca = blockIdx.y * 16 + threadIdx.x;
-        const int cb = blockIdx.x * 16 + threadIdx.x;
-        ta[threadIdx.y][threadIdx.x] = (ir < n && ca < n) ? X[(size_t)ir * n + ca] : 0.0;
-        tb[threadIdx.y][threadIdx.x] = (ir < n && cb < n) ? X[(size_t)ir * n + cb] : 0.0;
-        __syncthreads();
+// One 64 x 64 tile of a product, C(i, c) = sum over k in [k0, k1) of
+// a(i, k) b(k, c): 256 threads, 4 x 4 values each, slices of 16 staged in
+// shared memory with the next slice's loads in flight.
+template <typename FA, typename FB>
+__device__ __forceinline__ void tile_product(int k0, int k1, FA fa, FB fb, bool a_by_k,
+                                             double acc[4][4]) {
+    __shared__ double As[TK][TB + 1], Bs[TK][TB + 1];
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc += ta[q][threadIdx.y] * tb[q][threadIdx.x];
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) acc[q][p] = 0.0;
+    double ra[4], rb[4];
+    // a row-major over k (a_by_k false): 16 threads along k; else 64 along i
+    const int ai = a_by_k ? (threadIdx.x & 63) : (threadIdx.x >> 4);
+    const int ak = a_by_k ? (threadIdx.x >> 6) : (threadIdx.x & 15);
+    const int bc = threadIdx.x & 63, bk = threadIdx.x >> 6;
+    auto fetch = [&](int kb) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = a_by_k ? ai : ai + 16 * q, k = a_by_k ? ak + 4 * q : ak;
+            ra[q] = kb + k < k1 ? fa(i, kb + k) : 0.0;
+            rb[q] = kb + bk + 4 * q < k1 ? fb(kb + bk + 4 * q, bc) : 0.0;
+        }
+    };
+    fetch(k0);
+    for (int kb = k0; kb < k1; kb += TK) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            As[a_by_k ? ak + 4 * q : ak][a_by_k ? ai : ai + 16 * q] = ra[q];
+            Bs[bk + 4 * q][bc] = rb[q];
+        }
+        __syncthreads();
+        if (kb + TK < k1) fetch(kb + TK);
+#pragma unroll
+        for (int t = 0; t < TK; ++t) {
+            double a[4], b[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { a[q] = As[t][ty + 16 * q]; b[q] = Bs[t][tx + 16 * q]; }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) acc[q][p] += a[q] * b[p];
+        }
         __syncthreads();
     }
-    if (a < n && b < n) Ainv[(size_t)a * n + b] = acc;
+}
+
+// Doubling step of X = L^{-1} for blocks of s rows, pair blockIdx.z: with
+// [L11 0; L21 L22] and X11, X22 known, X21 = -X22 (L21 X11).  half 0 forms
+// T = L21 X11, half 1 X21 = -X22 T.
+__global__ void __launch_bounds__(256)
+k_trinv_pair(int n, int s, int half, const double *__restrict__ L, double *X, double *T) {
+    const int r1 = blockIdx.z * 2 * s, r2 = r1 + s;    // block rows 1 and 2
+    const int i0 = blockIdx.y * TB, c0 = blockIdx.x * TB;
+    const int m = min(s, n - r2);                      // rows of block 2
+    if (i0 >= m) return;
+    double acc[4][4];
+    if (half == 0)   // X11 is lower triangular: k >= c
+        tile_product(c0, s,
+                     [&](int i, int k) {
+                         return i0 + i < m ? L[(size_t)(r2 + i0 + i) * n + r1 + k] : 0.0;
+                     },
+                     [&](int k, int c) {
+                         return c0 + c <= k ? X[(size_t)(r1 + k) * n + r1 + c0 + c] : 0.0;
+                     }, false, acc);
+    else             // X22 is lower triangular: k <= i
+        tile_product(0, min(m, i0 + TB),
+                     [&](int i, int k) {
+                         return i0 + i < m && k <= i0 + i
+                                    ? X[(size_t)(r2 + i0 + i) * n + r2 + k] : 0.0;
+                     },
+                     [&](int k, int c) {
+                         return c0 + c < s ? T[(size_t)(r2 + k) * n + r1 + c0 + c] : 0.0;
+                     }, false, acc);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double *out = half == 0 ? T : X;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int i = i0 + ty + 16 * q, c = c0 + tx + 16 * p;
+            if (i < m && c < s)
+                out[(size_t)(r2 + i) * n + r1 + c] = half == 0 ? acc[q][p] : -acc[q][p];
+        }
+}
+
+// Ainv = X^T X, X lower triangular: the tiles of the lower triangle, each
+// written twice
+__global__ void __launch_bounds__(256)
+k_xtx(int n, const double *__restrict__ X, double *Ainv) {
+    if (blockIdx.x > blockIdx.y) return;
+    const int i0 = blockIdx.y * TB, c0 = blockIdx.x * TB;
+    double acc[4][4];
+    tile_product(i0, n,   // X[k][i] = 0 for k < i
+                 [&](int i, int k) {
+                     return i0 + i <= k ? X[(size_t)k * n + i0 + i] : 0.0;
+                 },
+                 [&](int k, int c) {
+                     return c0 + c <= k ? X[(size_t)k * n + c0 + c] : 0.0;
+                 }, true, acc);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int i = i0 + ty + 16 * q, c = c0 + tx + 16 * p;
+            if (i < n && c <= i) {
+                Ainv[(size_t)i * n + c] = acc[q][p];
+                Ainv[(size_t)c * n + i] = acc[q][p];
+            }
+        }
 }
 
 int dense_inverse(const DCsr<double> &A, double **Ainv_out, cudaStream_t s) {
     const int n = A.n;
     *Ainv_out = nullptr;
+    // D: the trailing matrix, then the products of the doubling steps;
+    // Ainv holds L until the inverse of L is complete
     double *D = nullptr, *X = nullptr, *Ainv = nullptr;
     int *bad = nullptr;
     const size_t nn = (size_t)n * n;
@@ -189,42 +317,27 @@ int dense_inverse(const DCsr<double> &A, double **Ainv_out, cudaStream_t s) {
     if ((rc = dalloc(&Ainv, nn))) goto done;
     if ((rc = dalloc(&bad, 1))) goto done;
     cudaMemsetAsync(D, 0, nn * sizeof(double), s);
-    cudaMemsetAsync(X, 0, nn * sizeof(double), s);
     cudaMemsetAsync(bad, 0, sizeof(int), s);
     k_dense_from_csr<<<grid_for(n), 256, 0, s>>>(n, A.ia, A.ja, A.val, D);
-    count_launch();
-    for (int j0 = 0; j0 < n; j0 += NB) {
-        const int jb = std::min(NB, n - j0);
-        const int rest = n - j0 - jb;
-        k_potrf_diag<<<1, dim3(NB, NB), 0, s>>>(n, j0, jb, D, bad);
+    k_chol_first<<<1, 256, 0, s>>>(n, D, X, bad);
+    count_launch(2);
+    for (int j0 = 0; j0 + NB < n; j0 += NB) {
+        const int nt = div_up(n - j0 - NB, TB);
+        k_chol_step<<<nt * (nt + 1) / 2, 256, 0, s>>>(n, j0, D, Ainv, X, bad);
         count_launch();
-        if (rest > 0) {
-            k_trsm_panel<<<div_up(rest, 128), 128, 0, s>>>(n, j0, jb, D, bad);
-            const int nt = div_up(rest, NB);
-            k_syrk_update<<<dim3(nt, nt), dim3(NB, NB), 0, s>>>(n, j0, jb, D, bad);
-            count_launch(2);
-        }
     }
+    for (int b = NB; b < n; b *= 2) {
+        const int pairs = div_up(n - b, 2 * b), t = div_up(b, TB);
+        for (int half = 0; half < 2; ++half)
+            k_trinv_pair<<<dim3(t, t, pairs), 256, 0, s>>>(n, b, half, Ainv, X, D);
+        count_launch(2);
+    }
+    k_xtx<<<dim3(div_up(n, TB), div_up(n, TB)), 256, 0, s>>>(n, X, Ainv);
+    count_launch();
     e = cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto done; }
     if (hbad) { set_error_msg("coarse matrix is not positive definite"); rc = ERROR_DATA_ZERODIAG; goto done; }
-    for (int i0 = 0; i0 < n; i0 += NB) {
-        const int ib = std::min(NB, n - i0);
-        if (i0 > 0) {
-            k_trinv_gemm<<<div_up(i0, NB), dim3(NB, NB), 0, s>>>(n, i0, ib, D, X);
-            count_launch();
-        }
-        k_trinv_diag<<<div_up(i0 + ib, 128), 128, 0, s>>>(n, i0, ib, D, X);
-        count_launch();
-    }
-    {
-        dim3 blk(16, 16), grd(div_up(n, 16), div_up(n, 16));
-        k_xtx<<<grd, blk, 0, s>>>(n, X, Ainv);
-        count_launch();
-    }
-    e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto done; }
     *Ainv_out = Ainv;
     Ainv = nullptr;
 done:
