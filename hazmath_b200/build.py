@@ -26,6 +26,7 @@ SOURCES = [
     ("hzb_kernels.cu", False),
     ("hzb_sell.cu", False),
     ("hzb_setup.cu", False),
+    ("hzb_match.cu", False),
     ("hzb_dense.cu", True),
     ("hzb_solver.cu", False),
     ("hzb_batch.cu", False),

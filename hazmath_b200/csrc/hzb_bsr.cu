@@ -545,14 +545,13 @@ static int bsr_build(hzb_solver *S, int nrow, int nnzb, int nb, const int *d_ia,
         if ((rc = bundle_capacity(m, pia, s, &PP.bundle_cap))) break;
         if ((rc = tmpv.get(&nia, m + 1)) || (rc = tmpv.get(&nja, pnnz > 0 ? pnnz : 1)) ||
             (rc = tmpv.get(&nval, pnnz > 0 ? pnnz : 1)) || (rc = dalloc(&L.agg, m)) ||
-            (rc = tmpv.get(&work, par ? (size_t)6 * m + scan_tmp_size(m + 1) + 8
-                                      : (size_t)(vmb ? 2 : 1) * m)))
+            (rc = tmpv.get(&work, (size_t)(vmb ? 2 : 1) * m)))
             break;
-        rc = strength_graph(PP, S->amg.strong_coupled, nia, nja, nval, &nnnz, tmp, s);
+        if (!par) rc = strength_graph(PP, S->amg.strong_coupled, nia, nja, nval, &nnnz, tmp, s);
         if (!rc) {
             if (vmb)
                 rc = vmb_aggregate(m, nia, nja, S->amg.max_aggregation, L.agg, &nagg, work, s);
-            else if (par) rc = hem_parallel(m, nia, nja, nval, L.agg, &nagg, work, s);
+            else if (par) rc = match_parallel(PP, S->amg.strong_coupled, L.agg, &nagg, s);
             else rc = hem_exact(m, nia, nja, nval, L.agg, &nagg, work, s);
         }
         if (rc) break;

@@ -121,6 +121,42 @@ __device__ __forceinline__ T block_max(T v, T *sh) {
     return v;
 }
 
+// Integer hash of the matching's coins and the colouring's priorities.
+__device__ __forceinline__ unsigned hash_u32(unsigned x) {
+    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
+    return x;
+}
+
+// Exclusive prefix sum of v over the block (multiple of 32 threads, <= 1024),
+// *total its sum; sh: 32 ints.
+__device__ __forceinline__ int block_exscan(int v, int *sh, int *total) {
+    // inclusive warp scan
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sh[wid] = x;
+    __syncthreads();
+    const int nw = blockDim.x >> 5;
+    if (wid == 0) {
+        int w = lane < nw ? sh[lane] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        if (lane < nw) sh[lane] = w;   // inclusive warp totals
+    }
+    __syncthreads();
+    const int before = wid > 0 ? sh[wid - 1] : 0;
+    *total = sh[nw - 1];
+    __syncthreads();
+    return before + x - v;
+}
+
 // Launch counter of the calling thread (kernels issued by this library).
 void count_launch(int k = 1);
 long long launch_count();

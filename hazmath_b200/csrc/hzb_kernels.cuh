@@ -162,22 +162,45 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, in
     return !s_bad;
 }
 
-// The same barrier for kernels that cross it hundreds of times, with a vote:
+// The same barrier for kernels that cross it often: arrivals only ever count up
+// (the k-th crossing waits for k * nblocks, so nothing is reset and no
+// generation word follows the last arrival), and the wait polls without
+// sleeping.  *count starts at zero; *err as above, looked at every 64 polls.
+__device__ __forceinline__ bool grid_step(unsigned *count, unsigned target, int *err) {
+    __shared__ int s_stop;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int bad = 0;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        for (unsigned spin = 0;; ++spin) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((spin & 63u) == 63u && *(volatile int *)err) { bad = 1; break; }
+            if (spin > GRID_SPIN_LIMIT) {
+                atomicExch(err, 1);
+                bad = 1;
+                break;
+            }
+        }
+        s_stop = bad;
+    }
+    __syncthreads();
+    return !s_stop;
+}
+
+// The same with a vote:
 // *word counts arrivals in its lower half and arrivals with a true vote in its
-// upper half, both only ever up (the k-th crossing waits for k * nblocks, so
-// nothing is reset and no generation word follows the last arrival), and the
-// wait polls without sleeping.  *any: somebody voted true in this crossing
+// upper half.  *any: somebody voted true in this crossing
 // (votes: the thread 0's count of true votes so far, 0 at the first).  Only
 // when nobody did may the CTAs leave the loop, so a CTA that reads the word
-// late cannot miss a vote of this crossing.  *word starts at zero; *err as
-// above, looked at every 64 polls.
+// late cannot take a later crossing's votes for this one's.
 __device__ __forceinline__ bool grid_vote(unsigned long long *word, unsigned target, bool vote,
                                           unsigned *votes, bool *any, int *err) {
     __shared__ int s_go;
     const int v = __syncthreads_or(vote);
     if (threadIdx.x == 0) {
         int go = 1;
-        __threadfence();
         const unsigned long long one = v ? 0x100000001ull : 1ull;
         asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(one) : "memory");
         unsigned long long w;

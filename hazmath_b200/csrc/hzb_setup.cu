@@ -15,34 +15,6 @@ namespace hzb {
 // ---------------------------------------------------------------------------
 constexpr int SCAN_BLOCK = 256, SCAN_ITEMS = 8, SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
 
-__device__ __forceinline__ int block_exscan(int v, int *sh, int *total) {
-    // inclusive warp scan
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) sh[wid] = x;
-    __syncthreads();
-    const int nw = blockDim.x >> 5;
-    if (wid == 0) {
-        int w = lane < nw ? sh[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < nw) sh[lane] = w;   // inclusive warp totals
-    }
-    __syncthreads();
-    const int before = wid > 0 ? sh[wid - 1] : 0;
-    *total = sh[nw - 1];
-    __syncthreads();
-    return before + x - v;
-}
-
 __global__ void k_scan_tiles(const int *__restrict__ in, int n, int *tiles) {
     __shared__ int sh[32];
     const int base = blockIdx.x * SCAN_TILE;
@@ -667,263 +639,6 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
     }
     *nagg = h[O_NC];
     return h[O_STATUS] < 0 ? ERROR_AMG_COARSEING : SUCCESS;
-}
-
-// ---------------------------------------------------------------------------
-// deterministic parallel matching (fast mode)
-//   PM_LEAD rounds of mutual choice: every free vertex points at its heaviest
-//   free neighbour and mutual pairs match -- the edges that dominate both
-//   their ends, which the reference's greedy walk takes too; then red/blue
-//   handshake rounds until no pair forms.  Pairs are numbered through a scan.
-//   Leftovers join the adjacent aggregate with the fewest members counted
-//   before the leftover pass (first such neighbour on ties).  Mutual choice
-//   alone stalls on chains of ever heavier edges (smooth coefficient fields);
-//   the handshake alone pairs a vertex only with a neighbour of the other
-//   colour, which on the 128^3 log-normal problem (sigma 1) left coarser
-//   levels and 43 instead of the reference's 38 iterations; a few mutual
-//   rounds first gave 39.
-// ---------------------------------------------------------------------------
-__global__ void k_pm_init(int n, const int *__restrict__ ia, int *state) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x)
-        state[k] = (ia[k + 1] - ia[k] > 1) ? -1 : -2;   // -1 free, -2 isolated
-}
-
-__device__ __forceinline__ unsigned hash_u32(unsigned x) {
-    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-    return x;
-}
-
-__device__ __forceinline__ unsigned edge_hash(int i, int j) {
-    unsigned lo = (unsigned)min(i, j), hi = (unsigned)max(i, j);
-    unsigned x = lo * 0x9e3779b1u ^ (hi + 0x7f4a7c15u + (lo << 6) + (lo >> 2));
-    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-    return x;
-}
-
-// Red/blue handshake (one round): a hashed coin splits the free vertices;
-// every free red vertex proposes to its heaviest free blue neighbour (edge
-// key: |a_ij| in FP32, then a hash of the unordered pair), every blue vertex
-// accepts its heaviest proposer.  Accepted pairs are disjoint, and a constant
-// fraction of the free vertices pairs up per round whatever the weights look
-// like (heaviest-neighbour pointers alone form long chains on smooth
-// coefficient fields).
-__device__ __forceinline__ bool pm_red(int k, int round) {
-    return (hash_u32((unsigned)k * 2654435761u + (unsigned)round * 0x632be5abu) >> 7) & 1u;
-}
-
-__device__ __forceinline__ bool pm_better(float w, unsigned h, int j, float bw,
-                                          unsigned bh, int best) {
-    return best < 0 || w > bw || (w == bw && (h > bh || (h == bh && j > best)));
-}
-
-constexpr int PM_LEAD = 4;
-
-// red k proposes to its heaviest free blue neighbour; in a mutual round
-// (round < PM_LEAD) every free k points at its heaviest free neighbour
-__global__ void k_pm_propose(int n, int round, const int *__restrict__ ia,
-                             const int *__restrict__ ja, const double *__restrict__ a,
-                             const int *__restrict__ state, int *ptr) {
-    const bool mutual = round < PM_LEAD;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x) {
-        int best = -1;
-        if (state[k] == -1 && (mutual || pm_red(k, round))) {
-            float bw = -1.0f;
-            unsigned bh = 0u;
-            for (int p = ia[k]; p < ia[k + 1]; ++p) {
-                const int j = ja[p];
-                if (j == k || state[j] != -1 || (!mutual && pm_red(j, round))) continue;
-                const float w = (float)fabs(a[p]);
-                const unsigned h = edge_hash(k, j);
-                if (pm_better(w, h, j, bw, bh, best)) { best = j; bw = w; bh = h; }
-            }
-        }
-        ptr[k] = best;
-    }
-}
-
-// blue j: acc[j] = heaviest red neighbour proposing to j (or -1); flag marks
-// accepted pairs, numbered by their blue end
-__global__ void k_pm_accept(int n, int round, const int *__restrict__ ia,
-                            const int *__restrict__ ja, const double *__restrict__ a,
-                            const int *__restrict__ state, const int *__restrict__ ptr,
-                            int *acc, int *flag, int *any) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n;
-         j += gridDim.x * blockDim.x) {
-        int best = -1;
-        if (state[j] == -1 && !pm_red(j, round)) {
-            float bw = -1.0f;
-            unsigned bh = 0u;
-            for (int p = ia[j]; p < ia[j + 1]; ++p) {
-                const int i = ja[p];
-                if (i == j || ptr[i] != j) continue;
-                const float w = (float)fabs(a[p]);
-                const unsigned h = edge_hash(i, j);
-                if (pm_better(w, h, i, bw, bh, best)) { best = i; bw = w; bh = h; }
-            }
-        }
-        acc[j] = best;
-        flag[j] = best >= 0;
-        if (best >= 0) *any = 1;
-    }
-}
-
-// mutual round: j pairs with i = ptr[j] when ptr[i] = j, numbered by the
-// higher end
-__global__ void k_pm_mutual(int n, const int *__restrict__ state, const int *__restrict__ ptr,
-                            int *acc, int *flag, int *any) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        int i = -1;
-        if (state[j] == -1) {
-            const int p = ptr[j];
-            if (p >= 0 && p < j && ptr[p] == j) i = p;
-        }
-        acc[j] = i;
-        flag[j] = i >= 0;
-        if (i >= 0) *any = 1;
-    }
-}
-
-__global__ void k_pm_assign(int n, const int *__restrict__ acc,
-                            const int *__restrict__ flag,
-                            const int *__restrict__ pos, const int *__restrict__ base,
-                            int *state) {
-    const int b = *base;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n;
-         j += gridDim.x * blockDim.x)
-        if (flag[j]) {
-            const int c = b + pos[j];
-            state[j] = c;
-            state[acc[j]] = c;
-        }
-}
-// the aggregate count after a round: base += the round's pairs
-__global__ void k_pm_advance(int *base, const int *__restrict__ cnt) { *base += *cnt; }
-
-// Renumbering by leader: aggregate ids follow their smallest member vertex,
-// so coarse rows keep the fine ordering's locality (ids were handed out round
-// by round).
-__global__ void k_pm_lead(int n, const int *__restrict__ agg, int *lead) {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n;
-         v += gridDim.x * blockDim.x)
-        if (agg[v] >= 0) atomicMin(lead + agg[v], v);
-}
-__global__ void k_pm_leadflag(int n, const int *__restrict__ agg, const int *__restrict__ lead,
-                              int *flag) {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n;
-         v += gridDim.x * blockDim.x)
-        flag[v] = agg[v] >= 0 && lead[agg[v]] == v;
-}
-__global__ void k_pm_renumber(int n, const int *__restrict__ lead, const int *__restrict__ pos,
-                              int *agg) {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n;
-         v += gridDim.x * blockDim.x)
-        if (agg[v] >= 0) agg[v] = pos[lead[agg[v]]];
-}
-
-__global__ void k_pm_sizes(int n, const int *__restrict__ state, int *size) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x)
-        if (state[k] >= 0) atomicAdd(size + state[k], 1);
-}
-
-// Leftover free vertices join the adjacent aggregate with the fewest members
-// (sizes counted before this pass; the first such neighbour on ties).  A
-// free vertex without an aggregated neighbour becomes its own aggregate:
-// flag[k] = 1, numbered after the pairs through a scan.
-__global__ void k_pm_leftover(int n, const int *__restrict__ ia,
-                              const int *__restrict__ ja,
-                              const int *__restrict__ state,
-                              const int *__restrict__ size, int *out, int *flag) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x) {
-        int st = state[k], f = 0;
-        if (st == -1) {
-            int bc = -1, bs = 0;
-            for (int p = ia[k]; p < ia[k + 1]; ++p) {
-                const int c = state[ja[p]];
-                if (c >= 0 && (bc < 0 || size[c] < bs)) { bc = c; bs = size[c]; }
-            }
-            st = bc;
-            f = bc < 0;
-        }
-        out[k] = st < 0 ? UNPT : st;
-        flag[k] = f;
-    }
-}
-
-__global__ void k_pm_singletons(int n, const int *__restrict__ flag,
-                                const int *__restrict__ pos, int base, int *out) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += gridDim.x * blockDim.x)
-        if (flag[k]) out[k] = base + pos[k];
-}
-
-int hem_parallel(int n, const int *nia, const int *nja, const double *nval,
-                 int *agg, int *nagg, int *work, cudaStream_t s) {
-    // work layout (ints): state n | ptr n | flag n | pos n+1 | size n | scan tmp
-    int *state = work, *ptr = work + n, *flag = work + 2 * n, *pos = work + 3 * n;
-    int *size = work + 4 * n + 1, *tmp = work + 5 * n + 1;
-    int *dflag = nullptr;
-    HZB_TRY(dalloc(&dflag, 2));
-    const int g = grid_for(n);
-    k_pm_init<<<g, 256, 0, s>>>(n, nia, state);
-    count_launch();
-    cudaMemsetAsync(dflag + 1, 0, sizeof(int), s);   // the aggregate count
-    int nc = 0;
-    int *acc = size;   // free during the rounds
-    for (int round = 0, idle = 0; round < 96 + PM_LEAD && idle < 4; ++round) {
-        cudaMemsetAsync(dflag, 0, sizeof(int), s);
-        k_pm_propose<<<g, 256, 0, s>>>(n, round, nia, nja, nval, state, ptr);
-        if (round < PM_LEAD)
-            k_pm_mutual<<<g, 256, 0, s>>>(n, state, ptr, acc, flag, dflag);
-        else
-            k_pm_accept<<<g, 256, 0, s>>>(n, round, nia, nja, nval, state, ptr, acc, flag,
-                                          dflag);
-        count_launch(2);
-        int rc = scan_exclusive(flag, pos, n, tmp, s);
-        if (rc) { dfree(dflag); return rc; }
-        k_pm_assign<<<g, 256, 0, s>>>(n, acc, flag, pos, dflag + 1, state);
-        k_pm_advance<<<1, 1, 0, s>>>(dflag + 1, pos + n);
-        count_launch(2);
-        int h[2];
-        cudaMemcpyAsync(h, dflag, sizeof(h), cudaMemcpyDeviceToHost, s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) { dfree(dflag); set_error(e, __FILE__, __LINE__); return ERROR_SOLVER_MISC; }
-        nc = h[1];
-        // stop after a few handshake rounds in a row without a new pair
-        idle = h[0] || round < PM_LEAD ? 0 : idle + 1;
-    }
-    cudaMemsetAsync(size, 0, sizeof(int) * (nc > 0 ? nc : 1), s);
-    k_pm_sizes<<<g, 256, 0, s>>>(n, state, size);
-    k_pm_leftover<<<g, 256, 0, s>>>(n, nia, nja, state, size, agg, flag);
-    count_launch(2);
-    int rc = scan_exclusive(flag, pos, n, tmp, s);
-    int extra = 0;
-    if (!rc) {
-        k_pm_singletons<<<g, 256, 0, s>>>(n, flag, pos, nc, agg);
-        count_launch();
-        cudaMemcpyAsync(&extra, pos + n, sizeof(int), cudaMemcpyDeviceToHost, s);
-    }
-    if (!rc) {   // ids in the order of each aggregate's smallest vertex
-        int *lead = size;
-        cudaMemsetAsync(lead, 0x7f, sizeof(int) * (size_t)n, s);
-        k_pm_lead<<<g, 256, 0, s>>>(n, agg, lead);
-        k_pm_leadflag<<<g, 256, 0, s>>>(n, agg, lead, flag);
-        count_launch(2);
-        rc = scan_exclusive(flag, pos, n, tmp, s);
-        if (!rc) {
-            k_pm_renumber<<<g, 256, 0, s>>>(n, lead, pos, agg);
-            count_launch();
-        }
-    }
-    cudaError_t e = cudaStreamSynchronize(s);
-    dfree(dflag);
-    if (rc) return rc;
-    if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); return ERROR_SOLVER_MISC; }
-    *nagg = nc + extra;
-    return SUCCESS;
 }
 
 // ---------------------------------------------------------------------------

@@ -22,10 +22,11 @@ int strength_graph(const DCsr<double> &A, double theta, int *nia, int *nja,
 // isolated point on the second pass).
 int hem_exact(int n, const int *nia, const int *nja, const double *nval,
               int *agg, int *nagg, int *work_n, cudaStream_t s);
-// deterministic parallel matching (mutual heaviest neighbour rounds + the
-// same leftover rule against pre-pass-2 sizes); not bit-exact.
-int hem_parallel(int n, const int *nia, const int *nja, const double *nval,
-                 int *agg, int *nagg, int *work, cudaStream_t s);
+// deterministic parallel matching (mutual heaviest neighbour and handshake
+// rounds, leftovers to their first aggregated neighbour) on A's strength graph
+// for the threshold theta, aggregates numbered by their smallest vertex; not
+// bit-exact (hzb_match.cu).  agg: n outputs.
+int match_parallel(const DCsr<double> &A, double theta, int *agg, int *nagg, cudaStream_t s);
 
 // VMB aggregation (aggregation_vmb, amg_setup_ua.c:596-736) on the strength
 // graph in the reference's three sequential steps and visiting orders;

@@ -778,11 +778,13 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
         const bool vmb = S->amg.aggregation_type == VMB;
         const bool par = !vmb && S->bp.matching == HZB_MATCH_PARALLEL;
         const bool hec = !vmb && !par && S->amg.aggregation_type == HEC;
-        if ((rc = dalloc(&nia, m + 1)) || (rc = dalloc(&nja, L.nnz)) ||
-            (rc = dalloc(&nval, L.nnz)) || (rc = dalloc(&agg, m)) ||
-            (rc = dalloc(&work, par ? (size_t)6 * m + scan_tmp_size(m + 1) + 8
-                                : hec ? hec_work_ints(m)
-                                      : (size_t)(vmb ? 2 : 1) * m))) {
+        // the parallel matching reads A itself; smoothed aggregation needs the
+        // strength graph whichever matching runs
+        const bool graph = !par || sa;
+        if ((rc = dalloc(&agg, m)) ||
+            (graph && ((rc = dalloc(&nia, m + 1)) || (rc = dalloc(&nja, L.nnz)) ||
+                       (rc = dalloc(&nval, L.nnz)))) ||
+            (!par && (rc = dalloc(&work, hec ? hec_work_ints(m) : (size_t)(vmb ? 2 : 1) * m)))) {
             dfree(nia); dfree(nja); dfree(nval); dfree(agg); dfree(work);
             break;
         }
@@ -791,11 +793,11 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
             if (!S->hec_state) rc = dalloc(&S->hec_state, 35);
             if (!rc) rc = hec_seed(S->hec_state, 1u, s);
         }
-        if (!rc) rc = strength_graph(L.A64(), S->amg.strong_coupled, nia, nja, nval, &nnnz,
-                                     tmp, s);
+        if (!rc && graph)
+            rc = strength_graph(L.A64(), S->amg.strong_coupled, nia, nja, nval, &nnnz, tmp, s);
         if (!rc) {
             if (vmb) rc = vmb_aggregate(m, nia, nja, S->amg.max_aggregation, agg, &nagg, work, s);
-            else if (par) rc = hem_parallel(m, nia, nja, nval, agg, &nagg, work, s);
+            else if (par) rc = match_parallel(L.A64(), S->amg.strong_coupled, agg, &nagg, s);
             else if (hec) rc = hec_aggregate(m, nia, nja, nval, agg, &nagg, S->hec_state, work, s);
             else rc = hem_exact(m, nia, nja, nval, agg, &nagg, work, s);
         }
