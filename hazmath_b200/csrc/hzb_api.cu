@@ -1476,6 +1476,10 @@ extern "C" INT hzb_rap_agg_device(INT n, INT nnz, const INT *ia, const INT *ja,
     rc = check_rap_inputs(n, nnz, ia, ja, nc, agg, ria, s);
     if (!rc) rc = restriction_pattern(n, nc, agg, ria, rja, tmp, s);
     if (!rc) rc = rap_agg(A, nc, agg, ria, rja, rap_ia, rap_ja, rap_val, rap_nnz, s);
+    if (!rc) {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; }
+    }
 done:
     dfree(ria); dfree(rja); dfree(tmp);
     return rc;

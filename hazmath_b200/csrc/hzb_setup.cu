@@ -793,107 +793,7 @@ __global__ void k_rap_build(int nc, const int *__restrict__ ria,
     }
 }
 
-// The same slot lists with a warp per coarse row, for rows whose bound ub
-// (1 + the fine rows' lengths) is at most 64: slot t lives in lane t % 32,
-// register t / 32.  The warp loads 32 entries of a fine row at a time (their
-// coarse columns in parallel), then takes the products one by one in CSR
-// order: a ballot finds the slot holding the column, whose lane adds the
-// value, or the next free slot takes it.  Every slot receives its values in
-// the same order as above, so the sums are the same bit for bit.  Rows with
-// a larger bound are left to k_rap_build (rowcnt untouched here).
-__global__ void __launch_bounds__(256)
-k_rap_build_warp(int nc, const int *__restrict__ ria, const int *__restrict__ rja,
-                 const int *__restrict__ ia, const int *__restrict__ ja,
-                 const double *__restrict__ a, const int *__restrict__ agg,
-                 const int *__restrict__ off, const int *__restrict__ ub, int *scol,
-                 double *sval, int *rowcnt, int *nbig) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nc; c += warps) {
-        if (ub[c] > 64) {
-            if (lane == 0) atomicAdd(nbig, 1);
-            continue;
-        }
-        int col0 = lane == 0 ? c : -1, col1 = -1;
-        double val0 = 0.0, val1 = 0.0;
-        int cnt = 1;
-        for (int q = ria[c]; q < ria[c + 1]; ++q) {
-            const int i = rja[q];
-            const int k0 = ia[i], k1 = ia[i + 1];
-            for (int kb = k0; kb < k1; kb += 32) {
-                const int k = kb + lane;
-                int cc_l = -1;
-                double v_l = 0.0;
-                if (k < k1) {
-                    cc_l = agg[ja[k]];
-                    v_l = a[k];
-                }
-                const int m = min(32, k1 - kb);
-                for (int j = 0; j < m; ++j) {
-                    const int cc = __shfl_sync(FULL, cc_l, j);
-                    const double v = __shfl_sync(FULL, v_l, j);
-                    if (cc < 0) continue;
-                    const unsigned h0 = __ballot_sync(FULL, col0 == cc);
-                    const unsigned h1 = __ballot_sync(FULL, col1 == cc);
-                    if (h0) {
-                        if (lane == __ffs(h0) - 1) val0 += v;
-                    } else if (h1) {
-                        if (lane == __ffs(h1) - 1) val1 += v;
-                    } else {
-                        if (lane == (cnt & 31)) {
-                            if (cnt < 32) { col0 = cc; val0 = v; }
-                            else { col1 = cc; val1 = v; }
-                        }
-                        ++cnt;
-                    }
-                }
-            }
-        }
-        int *cols = scol + off[c];
-        double *vals = sval + off[c];
-        if (lane < cnt) { cols[lane] = col0; vals[lane] = val0; }
-        if (lane + 32 < cnt) { cols[lane + 32] = col1; vals[lane + 32] = val1; }
-        if (lane == 0) rowcnt[c] = cnt;
-    }
-}
-
-// k_rap_build for the rows k_rap_build_warp left (bound above 64)
-__global__ void k_rap_build_big(int nc, const int *__restrict__ ria,
-                                const int *__restrict__ rja, const int *__restrict__ ia,
-                                const int *__restrict__ ja, const double *__restrict__ a,
-                                const int *__restrict__ agg, const int *__restrict__ off,
-                                const int *__restrict__ ub, int *scol, double *sval,
-                                int *rowcnt) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc;
-         c += gridDim.x * blockDim.x) {
-        if (ub[c] <= 64) continue;
-        int *cols = scol + off[c];
-        double *vals = sval + off[c];
-        int cnt = 1;
-        cols[0] = c;
-        vals[0] = 0.0;
-        for (int q = ria[c]; q < ria[c + 1]; ++q) {
-            const int i = rja[q];
-            for (int k = ia[i]; k < ia[i + 1]; ++k) {
-                const int cc = agg[ja[k]];
-                if (cc < 0) continue;
-                int pos = -1;
-                for (int t = 0; t < cnt; ++t)
-                    if (cols[t] == cc) { pos = t; break; }
-                if (pos >= 0) {
-                    vals[pos] += a[k];
-                } else {
-                    cols[cnt] = cc;
-                    vals[cnt] = a[k];
-                    ++cnt;
-                }
-            }
-        }
-        rowcnt[c] = cnt;
-    }
-}
-
+// slot lists in scratch to CSR
 __global__ void k_rap_compact(int nc, const int *__restrict__ off,
                               const int *__restrict__ cia,
                               const int *__restrict__ scol,
@@ -909,63 +809,392 @@ __global__ void k_rap_compact(int nc, const int *__restrict__ off,
     }
 }
 
+// The same slot lists by a warp per coarse row, without scratch: one pass
+// counts a row's slots, and after the scan of the counts a second one forms
+// the row and writes it in place (5.4 GB at the 256^3 fine level against 7.2
+// for one pass through scratch and a compaction).  The row's entries are taken
+// 32 at a time, whatever fine rows they come from.  Lanes with the same coarse
+// column find each other with a match; the first of them finds the column's
+// slot (a small hash table in shared memory, which a row of at most 32 entries
+// does not need), columns seen for the first time take slots in lane order,
+// and the first lane adds the values of its group in lane order to the slot.
+// Slot numbers and every sum are those of the loop above, bit for bit.  Taking
+// the entries one by one (two ballots each) had cost 12.3 ms at that level,
+// the compaction by a thread per row 2.4.
+// A row whose bound (1 + its entries) exceeds CAP goes to a list for the next
+// instantiation; list 2 (above RAP_CAP2) is left to k_rap_build_big.
+constexpr int RAP_CAP0 = 64, RAP_CAP1 = 256, RAP_CAP2 = 2048;
+
+template <int CAP>
+struct RapTable {
+    int key[2 * CAP];               // coarse column, -1 free
+    unsigned short slot[2 * CAP];
+    int col[CAP];
+    double val[CAP];
+};
+
+// Sum, in lane order, of the values of the group that this lane leads (mask:
+// its lanes; 0 for the others), added to acc.
+__device__ __forceinline__ double rap_group_sum(unsigned mask, double acc, double v) {
+    const int most = __reduce_max_sync(0xffffffffu, __popc(mask));
+    for (int r = 0; r < most; ++r) {
+        const double x = __shfl_sync(0xffffffffu, v, __ffs(mask) - 1);
+        if (mask) acc += x;
+        mask &= mask - 1u;
+    }
+    return acc;
+}
+
+// entry t of a batch of nf <= 32 fine rows (lane q: row q from entry b on,
+// `start` entries before it)
+__device__ __forceinline__ int rap_entry(int t, int nf, int b, int start) {
+    int base = 0;
+    for (int r = 0; r < nf; ++r) {
+        const int sr = __shfl_sync(0xffffffffu, start, r), br = __shfl_sync(0xffffffffu, b, r);
+        if (t >= sr) base = br - sr;
+    }
+    return base + t;
+}
+
+// inclusive sums of len over the lanes
+__device__ __forceinline__ int rap_lane_sums(int len) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, len, o);
+        if (lane >= o) len += y;
+    }
+    return len;
+}
+
+// Coarse row c of at most 32 entries (m) from nf <= 32 fine rows: the slot
+// count, after writing the row (FILL).
+template <bool FILL>
+__device__ __forceinline__ int rap_short_row(int c, int m, int nf, int b, int start,
+                                             const int *__restrict__ ja,
+                                             const double *__restrict__ a,
+                                             const int *__restrict__ agg, int *cols,
+                                             double *vals) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int k = rap_entry(lane, nf, b, start);
+    int cc = -1;
+    double v = 0.0;
+    if (lane < m) {
+        cc = agg[ja[k]];
+        if (FILL) v = a[k];
+    }
+    const unsigned grp = __match_any_sync(FULL, cc);
+    const bool lead = cc >= 0 && lane == __ffs(grp) - 1;
+    const unsigned fresh = __ballot_sync(FULL, lead && cc != c);
+    if (FILL) {
+        const bool self = lead && cc == c;
+        const double acc = rap_group_sum(lead ? grp & (grp - 1u) : 0u, self ? 0.0 + v : v, v);
+        const int slot = self ? 0 : 1 + __popc(fresh & ((1u << lane) - 1u));
+        if (lead) {
+            cols[slot] = cc;
+            vals[slot] = acc;
+        }
+        // the diagonal slot is there even when no entry maps to it
+        if (!__any_sync(FULL, self) && lane == 0) {
+            cols[0] = c;
+            vals[0] = 0.0;
+        }
+    }
+    return 1 + __popc(fresh);
+}
+
+// Any other coarse row c, from the fine rows rja[q0, q1) (the first batch's
+// b and len at hand), through the table.
+template <int CAP, bool FILL>
+__device__ __forceinline__ int rap_row(int c, int q0, int q1, int b, int len, RapTable<CAP> *T,
+                                       const int *__restrict__ rja, const int *__restrict__ ia,
+                                       const int *__restrict__ ja, const double *__restrict__ a,
+                                       const int *__restrict__ agg, int *cols, double *vals) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned HM = 2 * CAP - 1;
+    auto hash = [](int col) { return ((unsigned)col * 2654435761u >> 7) & HM; };
+    int cnt = 1;
+    for (int t = lane; t < 2 * CAP; t += 32) T->key[t] = -1;
+    __syncwarp();
+    if (lane == 0) {
+        T->key[hash(c)] = c;
+        T->slot[hash(c)] = 0;
+        T->col[0] = c;
+        T->val[0] = 0.0;
+    }
+    __syncwarp();
+    for (int qb = q0; qb < q1; qb += 32) {
+        const int nf = min(32, q1 - qb);
+        if (qb > q0) {
+            b = len = 0;
+            if (lane < nf) {
+                const int i = rja[qb + lane];
+                b = ia[i];
+                len = ia[i + 1] - b;
+            }
+        }
+        const int end = rap_lane_sums(len);
+        const int m = __shfl_sync(FULL, end, 31);
+        for (int tb = 0; tb < m; tb += 32) {
+            const int k = rap_entry(tb + lane, nf, b, end - len);
+            int cc = -1;
+            double v = 0.0;
+            if (tb + lane < m) {
+                cc = agg[ja[k]];
+                if (FILL) v = a[k];
+            }
+            const unsigned grp = __match_any_sync(FULL, cc);
+            const bool lead = cc >= 0 && lane == __ffs(grp) - 1;
+            int slot = -1;
+            unsigned h = 0;
+            if (lead) {
+                h = hash(cc);
+                for (int key; (key = T->key[h]) != -1; h = (h + 1) & HM)
+                    if (key == cc) { slot = T->slot[h]; break; }
+            }
+            const bool fresh = lead && slot < 0;
+            const unsigned nb = __ballot_sync(FULL, fresh);
+            if (fresh) {            // distinct columns: only a place can be contended
+                slot = cnt + __popc(nb & ((1u << lane) - 1u));
+                while (atomicCAS(&T->key[h], -1, cc) != -1) h = (h + 1) & HM;
+                T->slot[h] = (unsigned short)slot;
+            }
+            cnt += __popc(nb);
+            if (FILL) {
+                const double acc = rap_group_sum(lead ? grp & (grp - 1u) : 0u,
+                                                 lead && !fresh ? T->val[slot] + v : v, v);
+                if (lead) {
+                    T->col[slot] = cc;
+                    T->val[slot] = acc;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    if (FILL) {
+        for (int t = lane; t < cnt; t += 32) {
+            cols[t] = T->col[t];
+            vals[t] = T->val[t];
+        }
+        __syncwarp();
+    }
+    return cnt;
+}
+
+// All rows (CAP = RAP_CAP0), or the rows of list `tier` - 1 (nrow of them,
+// read on the device).  list: the rows for the next instantiations, nc each;
+// ctl[t]: their number.
+template <int CAP, int WARPS, bool FILL, bool LISTED>
+__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS)
+k_rap_rows(int nc, const int *__restrict__ ria, const int *__restrict__ rja,
+           const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
+           const int *__restrict__ agg, const int *__restrict__ cia, int *rowcnt, int *cja,
+           double *cval, int *list, int *ctl, int tier) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RapTable<CAP> *T = reinterpret_cast<RapTable<CAP> *>(smem_raw) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * WARPS;
+    const int *mine = list + (size_t)(tier - 1) * nc;
+    const int nrow = LISTED ? ctl[tier - 1] : nc;
+    // A row's metadata is a chain of three loads (ria, rja, ia), each issued one
+    // row ahead of the load that needs it, so that none of them is waited for.
+    int c1 = 0, c2 = 0, c3 = 0, p1 = 0, p2 = 0, p3 = 0, n1 = 0, n2 = 0, n3 = 0;
+    int i2 = 0, b1 = 0, e1 = 0;
+    auto advance = [&](int at) {    // at: the row whose pointers are loaded now
+        c1 = c2; p1 = p2; n1 = n2;
+        b1 = e1 = 0;
+        if (p1 + lane < n1) { b1 = ia[i2]; e1 = ia[i2 + 1]; }
+        c2 = c3; p2 = p3; n2 = n3;
+        i2 = p2 + lane < n2 ? rja[p2 + lane] : 0;
+        p3 = n3 = 0;
+        if (at < nrow) {
+            c3 = LISTED ? mine[at] : at;
+            p3 = ria[c3];
+            n3 = ria[c3 + 1];
+        }
+    };
+    int at = blockIdx.x * WARPS + (threadIdx.x >> 5);
+    advance(at);
+    advance(at + warps);
+    advance(at + 2 * warps);
+    for (; at < nrow; at += warps) {
+        const int cc = c1, r0 = p1, r1 = n1, rb = b1, rl = e1 - b1;
+        advance(at + 3 * warps);
+        const int end = rap_lane_sums(rl);
+        const int m = __shfl_sync(0xffffffffu, end, 31);
+        int ub = 1 + m;
+        for (int qb = r0 + 32; qb < r1; qb += 32) {
+            int l = 0;
+            if (qb + lane < r1) {
+                const int i = rja[qb + lane];
+                l = ia[i + 1] - ia[i];
+            }
+            ub += __reduce_add_sync(0xffffffffu, l);
+        }
+        if (ub > CAP) {
+            // counted and listed by the count pass; the fill pass leaves it too
+            if (!FILL && lane == 0) {
+                const int k = ub <= RAP_CAP1 ? 0 : ub <= RAP_CAP2 ? 1 : 2;
+                if (!LISTED) list[(size_t)k * nc + atomicAdd(ctl + k, 1)] = cc;
+                if (k == 2) rowcnt[cc] = 0;
+            }
+            continue;
+        }
+        int *cols = FILL ? cja + cia[cc] : nullptr;
+        double *vals = FILL ? cval + cia[cc] : nullptr;
+        int cnt;
+        if (!LISTED && m <= 32 && r1 - r0 <= 32)
+            cnt = rap_short_row<FILL>(cc, m, r1 - r0, rb, end - rl, ja, a, agg, cols, vals);
+        else
+            cnt = rap_row<CAP, FILL>(cc, r0, r1, rb, rl, T, rja, ia, ja, a, agg, cols, vals);
+        if (!FILL && lane == 0) rowcnt[cc] = cnt;
+    }
+}
+
+// Rows with a bound above RAP_CAP2, a thread each, slots in scratch at off[c]
+__global__ void k_rap_build_big(int nc, const int *__restrict__ ria,
+                                const int *__restrict__ rja, const int *__restrict__ ia,
+                                const int *__restrict__ ja, const double *__restrict__ a,
+                                const int *__restrict__ agg, const int *__restrict__ off,
+                                const int *__restrict__ list, int nlist, int *scol, double *sval,
+                                int *rowcnt) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nlist;
+         t += gridDim.x * blockDim.x) {
+        const int c = list[t];
+        int *cols = scol + off[c];
+        double *vals = sval + off[c];
+        int cnt = 1;
+        cols[0] = c;
+        vals[0] = 0.0;
+        for (int q = ria[c]; q < ria[c + 1]; ++q) {
+            const int i = rja[q];
+            for (int k = ia[i]; k < ia[i + 1]; ++k) {
+                const int cc = agg[ja[k]];
+                if (cc < 0) continue;
+                int pos = -1;
+                for (int u = 0; u < cnt; ++u)
+                    if (cols[u] == cc) { pos = u; break; }
+                if (pos >= 0) {
+                    vals[pos] += a[k];
+                } else {
+                    cols[cnt] = cc;
+                    vals[cnt] = a[k];
+                    ++cnt;
+                }
+            }
+        }
+        rowcnt[c] = cnt;
+    }
+}
+// and their rows copied to the product, a warp each
+__global__ void k_rap_copy_big(const int *__restrict__ list, int nlist,
+                               const int *__restrict__ off, const int *__restrict__ cia,
+                               const int *__restrict__ scol, const double *__restrict__ sval,
+                               int *cja, double *cval) {
+    for (int t = blockIdx.x; t < nlist; t += gridDim.x) {
+        const int c = list[t], src = off[c], dst = cia[c], m = cia[c + 1] - dst;
+        for (int u = threadIdx.x; u < m; u += blockDim.x) {
+            cja[dst + u] = scol[src + u];
+            cval[dst + u] = sval[src + u];
+        }
+    }
+}
+
 int rap_agg(const DCsr<double> &A, int nc, const int *agg, const int *ria,
             const int *rja, int **cia_out, int **cja_out, double **cval_out,
             int *cnnz, cudaStream_t s) {
     *cia_out = nullptr; *cja_out = nullptr; *cval_out = nullptr;
-    int *ub = nullptr, *off = nullptr, *tmp = nullptr, *rowcnt = nullptr;
-    int *scol = nullptr, *cia = nullptr, *cja = nullptr;
+    int *tmp = nullptr, *rowcnt = nullptr, *list = nullptr, *ctl = nullptr;
+    int *ub = nullptr, *off = nullptr, *scol = nullptr, *cia = nullptr, *cja = nullptr;
     double *sval = nullptr, *cval = nullptr;
-    int rc = SUCCESS, total = 0;
-    const int g = grid_for(nc);
+    int rc = SUCCESS, h[4] = {0, 0, 0, 0};
     cudaError_t e;
-    if ((rc = dalloc(&ub, nc))) goto fail;
-    if ((rc = dalloc(&off, nc + 1))) goto fail;
+    constexpr int W0 = 8, W1 = 4, W2 = 1;   // warps per CTA of the instantiations
+    constexpr size_t S0 = W0 * sizeof(RapTable<RAP_CAP0>), S1 = W1 * sizeof(RapTable<RAP_CAP1>),
+                     S2 = W2 * sizeof(RapTable<RAP_CAP2>);
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(k_rap_rows<RAP_CAP2, W2, false, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S2);
+        cudaFuncSetAttribute(k_rap_rows<RAP_CAP2, W2, true, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S2);
+        attr = true;
+    }
+    const int g0 = grid_for(32LL * nc), g1 = std::min(div_up(nc, W1), 4 * sm_count()),
+              g2 = std::min(nc, 4 * sm_count());
     if ((rc = dalloc(&tmp, scan_tmp_size(nc + 1)))) goto fail;
     if ((rc = dalloc(&rowcnt, nc))) goto fail;
+    if ((rc = dalloc(&list, (size_t)3 * nc))) goto fail;
+    if ((rc = dalloc(&ctl, 4))) goto fail;
     if ((rc = dalloc(&cia, nc + 1))) goto fail;
-    k_rap_bound<<<g, 256, 0, s>>>(nc, ria, rja, A.ia, ub);
-    count_launch();
-    if ((rc = scan_exclusive(ub, off, nc, tmp, s))) goto fail;
-    e = cudaMemcpyAsync(&total, off + nc, sizeof(int), cudaMemcpyDeviceToHost, s);
+    e = cudaMemsetAsync(ctl, 0, 4 * sizeof(int), s);
+    if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
+    k_rap_rows<RAP_CAP0, W0, false, false><<<g0, 32 * W0, S0, s>>>(
+        nc, ria, rja, A.ia, A.ja, A.val, agg, nullptr, rowcnt, nullptr, nullptr, list, ctl, 0);
+    k_rap_rows<RAP_CAP1, W1, false, true><<<g1, 32 * W1, S1, s>>>(
+        nc, ria, rja, A.ia, A.ja, A.val, agg, nullptr, rowcnt, nullptr, nullptr, list, ctl, 1);
+    k_rap_rows<RAP_CAP2, W2, false, true><<<g2, 32 * W2, S2, s>>>(
+        nc, ria, rja, A.ia, A.ja, A.val, agg, nullptr, rowcnt, nullptr, nullptr, list, ctl, 2);
+    count_launch(3);
+    if ((rc = scan_exclusive(rowcnt, cia, nc, tmp, s))) goto fail;
+    e = cudaMemcpyAsync(ctl + 3, cia + nc, sizeof(int), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
-    if ((rc = dalloc(&scol, total))) goto fail;
-    if ((rc = dalloc(&sval, total))) goto fail;
-    {
-        // a warp per coarse row; rows with a bound above 64 slots by a thread
-        int *nbig = tmp;   // the scan scratch is free until the next scan
-        e = cudaMemsetAsync(nbig, 0, sizeof(int), s);
-        if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
-        k_rap_build_warp<<<grid_for(32LL * nc), 256, 0, s>>>(nc, ria, rja, A.ia, A.ja, A.val,
-                                                            agg, off, ub, scol, sval, rowcnt,
-                                                            nbig);
-        int hbig = 0;
-        e = cudaMemcpyAsync(&hbig, nbig, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (h[2]) {
+        // rows of thousands of entries: bounds, scratch and a thread per row
+        int total = 0;
+        if ((rc = dalloc(&ub, nc))) goto fail;
+        if ((rc = dalloc(&off, nc + 1))) goto fail;
+        k_rap_bound<<<grid_for(nc), 256, 0, s>>>(nc, ria, rja, A.ia, ub);
+        count_launch();
+        if ((rc = scan_exclusive(ub, off, nc, tmp, s))) goto fail;
+        e = cudaMemcpyAsync(&total, off + nc, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
+        if ((rc = dalloc(&scol, total))) goto fail;
+        if ((rc = dalloc(&sval, total))) goto fail;
+        k_rap_build_big<<<grid_for(h[2], 128), 128, 0, s>>>(
+            nc, ria, rja, A.ia, A.ja, A.val, agg, off, list + (size_t)2 * nc, h[2], scol, sval,
+            rowcnt);
         count_launch();
-        if (hbig) {
-            k_rap_build_big<<<g, 128, 0, s>>>(nc, ria, rja, A.ia, A.ja, A.val, agg, off, ub,
-                                              scol, sval, rowcnt);
-            count_launch();
-        }
+        if ((rc = scan_exclusive(rowcnt, cia, nc, tmp, s))) goto fail;
+        e = cudaMemcpyAsync(&h[3], cia + nc, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
     }
-    if ((rc = scan_exclusive(rowcnt, cia, nc, tmp, s))) goto fail;
-    e = cudaMemcpyAsync(cnnz, cia + nc, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
+    *cnnz = h[3];
     if ((rc = dalloc(&cja, *cnnz))) goto fail;
     if ((rc = dalloc(&cval, *cnnz))) goto fail;
-    k_rap_compact<<<g, 256, 0, s>>>(nc, off, cia, scol, sval, cja, cval);
+    k_rap_rows<RAP_CAP0, W0, true, false><<<g0, 32 * W0, S0, s>>>(
+        nc, ria, rja, A.ia, A.ja, A.val, agg, cia, rowcnt, cja, cval, list, ctl, 0);
     count_launch();
-    e = cudaStreamSynchronize(s);
+    if (h[0]) {
+        k_rap_rows<RAP_CAP1, W1, true, true><<<std::min(div_up(h[0], W1), g1), 32 * W1, S1, s>>>(
+            nc, ria, rja, A.ia, A.ja, A.val, agg, cia, rowcnt, cja, cval, list, ctl, 1);
+        count_launch();
+    }
+    if (h[1]) {
+        k_rap_rows<RAP_CAP2, W2, true, true><<<std::min(h[1], g2), 32 * W2, S2, s>>>(
+            nc, ria, rja, A.ia, A.ja, A.val, agg, cia, rowcnt, cja, cval, list, ctl, 2);
+        count_launch();
+    }
+    if (h[2]) {
+        k_rap_copy_big<<<std::min(h[2], 4 * sm_count()), 128, 0, s>>>(
+            list + (size_t)2 * nc, h[2], off, cia, scol, sval, cja, cval);
+        count_launch();
+    }
+    e = cudaGetLastError();
     if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
-    dfree(ub); dfree(off); dfree(tmp); dfree(rowcnt); dfree(scol); dfree(sval);
+    dfree(tmp); dfree(rowcnt); dfree(list); dfree(ctl);
+    dfree(ub); dfree(off); dfree(scol); dfree(sval);
     *cia_out = cia; *cja_out = cja; *cval_out = cval;
     return SUCCESS;
 fail:
-    dfree(ub); dfree(off); dfree(tmp); dfree(rowcnt); dfree(scol); dfree(sval);
+    dfree(tmp); dfree(rowcnt); dfree(list); dfree(ctl);
+    dfree(ub); dfree(off); dfree(scol); dfree(sval);
     dfree(cia); dfree(cja); dfree(cval);
     return rc;
 }

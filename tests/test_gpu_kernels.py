@@ -165,3 +165,65 @@ def test_rap_bit_exact(golden):
     assert np.array_equal(out[1], g["cja"])
     assert np.array_equal(out[2], g["cval"])
 
+
+def _rap_plain(ia, ja, val, nc, agg):
+    """A_c = R A P in the reference's slot order: the diagonal first (from
+    0.0), other columns where they are first met, sums in traversal order."""
+    members = [[] for _ in range(nc)]
+    for i, c in enumerate(agg):
+        if c >= 0:
+            members[c].append(i)
+    cia, cja, cval = [0], [], []
+    for c in range(nc):
+        slot, vals = {c: 0}, [0.0]
+        for i in members[c]:
+            for k in range(ia[i], ia[i + 1]):
+                cc = int(agg[ja[k]])
+                if cc < 0:
+                    continue
+                if cc in slot:
+                    vals[slot[cc]] += val[k]
+                else:
+                    slot[cc] = len(vals)
+                    vals.append(float(val[k]))
+        cja += list(slot)
+        cval += vals
+        cia.append(len(cja))
+    return np.array(cia, np.int32), np.array(cja, np.int32), np.array(cval)
+
+
+@pytest.mark.parametrize("n,lens,members", [
+    (40, (0, 3), 2),           # rows of at most 32 entries together, empty rows
+    (300, (14, 18), 2),        # around 32 entries: with and without the table
+    (300, (30, 33), 2),        # around 64: the first list's bound
+    (200, (60, 130), 2),       # around 256: the second list
+    (400, (1, 3), 40),         # more than 32 fine rows in an aggregate
+    (1500, (900, 1100), 2),    # around 2048: the scratch rows
+])
+def test_rap_row_sizes_bit_exact(n, lens, members):
+    rng = np.random.default_rng(n + lens[1])
+    m = rng.integers(lens[0], lens[1] + 1, n)
+    ia = np.zeros(n + 1, np.int32)
+    np.cumsum(m, out=ia[1:])
+    ja = np.concatenate([rng.permutation(n)[:k] for k in m]).astype(np.int32)
+    val = rng.uniform(-1.0, 1.0, len(ja))
+    val[rng.random(len(val)) < 0.05] = -0.0
+    nc = n // members
+    agg = np.r_[np.arange(nc), rng.integers(0, nc, n - nc)].astype(np.int32)
+    agg[nc:][rng.random(n - nc) < 0.05] = -1
+    A = DevCSR(ia, ja, val)
+    nnz = C.c_int()
+    pia, pja, pval = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    rc = hz.lib().hzb_rap_agg_device(*A.args(), nc, ptr(dev(agg)), C.byref(nnz), C.byref(pia),
+                                     C.byref(pja), C.byref(pval))
+    assert rc == 0, hz.last_error()
+    cia, cja, cval = _rap_plain(ia, ja, val, nc, agg)
+    got = []
+    for q, like in ((pia, cia), (pja, cja), (pval, cval)):
+        a = np.empty_like(like)
+        assert nnz.value == len(cja)
+        assert hz.lib().hzb_copy_to_host(a.ctypes.data, q, a.nbytes) == 0
+        hz.lib().hzb_free_device(q)
+        got.append(a)
+    assert np.array_equal(got[0], cia) and np.array_equal(got[1], cja)
+    assert np.array_equal(got[2].view(np.int64), cval.view(np.int64))
