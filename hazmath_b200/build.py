@@ -29,6 +29,7 @@ SOURCES = [
     ("hzb_match.cu", False),
     ("hzb_dense.cu", True),
     ("hzb_solver.cu", False),
+    ("hzb_small.cu", False),
     ("hzb_batch.cu", False),
     ("hzb_gmres.cu", False),
     ("hzb_cycles.cu", False),

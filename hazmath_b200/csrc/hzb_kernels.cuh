@@ -166,12 +166,17 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, in
 // (the k-th crossing waits for k * nblocks, so nothing is reset and no
 // generation word follows the last arrival), and the wait polls without
 // sleeping.  *count starts at zero; *err as above, looked at every 64 polls.
-__device__ __forceinline__ bool grid_step(unsigned *count, unsigned target, int *err) {
-    __shared__ int s_stop;
+// Work that depends on nobody (loads of constant data) goes between the arrival
+// and the wait.
+__device__ __forceinline__ void grid_arrive(unsigned *count) {
     __syncthreads();
+    if (threadIdx.x == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(unsigned *count, unsigned target, int *err) {
+    __shared__ int s_stop;
     if (threadIdx.x == 0) {
         int bad = 0;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         for (unsigned spin = 0;; ++spin) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
@@ -187,6 +192,10 @@ __device__ __forceinline__ bool grid_step(unsigned *count, unsigned target, int 
     }
     __syncthreads();
     return !s_stop;
+}
+__device__ __forceinline__ bool grid_step(unsigned *count, unsigned target, int *err) {
+    grid_arrive(count);
+    return grid_wait(count, target, err);
 }
 
 // The same with a vote:

@@ -118,7 +118,7 @@ static int coarse_apply(hzb_solver *S) {
     Level &L1 = S->lv[1];
     HZB_TRY(vzero<double>(L1.n, L1.x, S->s));
     if (S->nl == 2) return dense_gemv<double>(L1.n, S->Ainv, L1.b, L1.x, S->s);
-    return cycle64(S, plain_cycle(S), 1);
+    return cycle64(S, plain_cycle(S), 1, true);
 }
 
 // e <- e - P B_c R (A e)       (forward coarse correction)

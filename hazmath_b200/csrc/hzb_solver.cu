@@ -125,6 +125,7 @@ void Level::release() {
     dfree(d_jac); dfree(d_gs_f); dfree(d_gs_b); dfree(d_sor_f); dfree(d_sor_b);
     dfree(d_gs32);
     dfree(l1_32);
+    dfree(l1_64);
     dfree(tia); dfree(tja); dfree(tval);
     fwd.release(); bwd.release(); col.release();
 }
@@ -173,7 +174,7 @@ static int fetch(hzb_solver *S, KrylovWork &w) {
     memcpy(&e, w.h_sc + SC_ERR, sizeof(int));
     if (e) {
         cudaMemsetAsync(w.sc + SC_ERR, 0, sizeof(double), S->s);
-        set_error_msg("a grid barrier of a Gauss-Seidel sweep ran out of time");
+        set_error_msg("a grid barrier of the cycle ran out of time");
         return ERROR_SOLVER_MISC;
     }
     return SUCCESS;
@@ -188,7 +189,7 @@ int check_waits(hzb_solver *S) {
     HZB_CUDA(cudaStreamSynchronize(S->s));
     if (e) {
         cudaMemsetAsync(S->kw.sc + SC_ERR, 0, sizeof(double), S->s);
-        set_error_msg("a grid barrier of a Gauss-Seidel sweep ran out of time");
+        set_error_msg("a grid barrier of the cycle ran out of time");
         return ERROR_SOLVER_MISC;
     }
     return SUCCESS;
@@ -382,8 +383,25 @@ int coarse_alpha(hzb_solver *S, int c, const double *rc, double *alpha) {
 
 // l0 > 0 runs the same cycle on the sub-hierarchy below level l0 (the
 // coarse-grid operator B_c used by the learned-weight training).
-int cycle64(hzb_solver *S, const AMG_param &cyc, int l0) {
+int cycle64(hzb_solver *S, const AMG_param &cyc, int l0, bool zero) {
     const int nl = S->nl;
+    const int small = small_first_level<double>(S, cyc, l0, zero);
+    if (small < nl) {
+        for (int l = l0; l < small; ++l) {
+            Level &L = S->lv[l];
+            HZB_TRY(smooth64(S, l, true, cyc));
+            HZB_TRY(spmv<double>(L.A64(), SPMV_RES, L.x, L.b, L.w, 1.0, nullptr, S->s));
+            if (l + 1 == small) break;
+            HZB_TRY(restrict_level(S, l, L.w, S->lv[l + 1].b));
+            HZB_TRY(vzero<double>(S->lv[l + 1].n, S->lv[l + 1].x, S->s));
+        }
+        HZB_TRY(small_levels<double>(S, small, l0, cyc));
+        for (int l = small - 1; l >= l0; --l) {
+            if (l + 1 < small) HZB_TRY(prolong_level(S, l, S->lv[l + 1].x, S->lv[l].x, 1.0));
+            HZB_TRY(smooth64(S, l, false, cyc));
+        }
+        return SUCCESS;
+    }
     int num_lvl[MAX_AMG_LVL] = {0};
     int l = l0;
     double alpha = 1.0;
@@ -422,7 +440,7 @@ static int precond64_body(hzb_solver *S, const double *r, double *z,
     L0.b = const_cast<double *>(r);
     L0.x = z;
     int rc = vzero<double>(L0.n, z, S->s);
-    for (int i = 0; rc == SUCCESS && i < cyc.maxit; ++i) rc = cycle64(S, cyc);
+    for (int i = 0; rc == SUCCESS && i < cyc.maxit; ++i) rc = cycle64(S, cyc, 0, i == 0);
     L0.b = sb;
     L0.x = sx;
     return rc;
@@ -486,6 +504,24 @@ static int smooth32(hzb_solver *S, int l, bool pre, const AMG_param &cyc, bool x
 // level0_zero: the caller left x32 of level 0 at zero
 int cycle32(hzb_solver *S, const AMG_param &cyc, bool level0_zero) {
     const int nl = S->nl;
+    const int small = small_first_level<float>(S, cyc, 0, level0_zero);
+    if (small < nl) {
+        for (int l = 0; l < small; ++l) {
+            Level &L = S->lv[l];
+            HZB_TRY(smooth32(S, l, true, cyc, l > 0 || level0_zero));
+            HZB_TRY(spmv<float>(L.A32(), SPMV_RES, L.x32, L.b32, L.w32, 1.0f, nullptr, S->s));
+            if (l + 1 < small)
+                HZB_TRY(restrict_agg<float>(L.nc, L.ria, L.rja, L.w32, S->lv[l + 1].b32, S->s));
+        }
+        HZB_TRY(small_levels<float>(S, small, 0, cyc));
+        for (int l = small - 1; l >= 0; --l) {
+            Level &L = S->lv[l];
+            if (l + 1 < small)
+                HZB_TRY(prolong_agg<float>(L.n, L.agg, S->lv[l + 1].x32, L.x32, 1.0f, S->s));
+            HZB_TRY(smooth32(S, l, false, cyc, false));
+        }
+        return SUCCESS;
+    }
     int num_lvl[MAX_AMG_LVL] = {0};
     bool zero[MAX_AMG_LVL] = {false};
     zero[0] = level0_zero;
@@ -894,6 +930,14 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
             L.bundle_cap = A.bundle_cap;
         }
     }
+    // the merged kernels of the l1-Jacobi cycle's small levels read the norms
+    if (S->amg.smoother == SMOOTHER_L1DIAG && S->bp.precision == HZB_PREC_FP64 && !batch)
+        for (int l = 0; l < S->nl - 1; ++l) {
+            Level &L = S->lv[l];
+            if (L.nnz > SMALL_NNZ_64) continue;
+            HZB_TRY(dalloc(&L.l1_64, L.n));
+            HZB_TRY(l1_norms<double>(L.A64(), L.l1_64, s));
+        }
     trace.mark("smoothers");
     HZB_TRY(S->kw.alloc(n, s));
     if (S->amg.coarse_solver != SOLVER_UMFPACK)

@@ -56,6 +56,7 @@ struct Level {
     double *d_sor_f = nullptr, *d_sor_b = nullptr;
     float *d_gs32 = nullptr;
     float *l1_32 = nullptr;           // l1 row norms for the FP32 first sweep
+    double *l1_64 = nullptr;          // the FP64 cycle's, on small levels
     Schedule fwd, bwd, col;
     // coarsest level with the direct solver: the transposed matrix the
     // reference factors (and leaves in mgl[nl-1].A)
@@ -176,8 +177,27 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
 // z = B r with B = maxit V/W cycles of the FP64 hierarchy (precond_amg)
 int precond64(hzb_solver *S, const double *r, double *z, const AMG_param &cyc);
 // one cycle on level-0 b/x already in place (mgcycle)
-int cycle64(hzb_solver *S, const AMG_param &cyc, int l0 = 0);
+// (zero: level l0's x holds zeros)
+int cycle64(hzb_solver *S, const AMG_param &cyc, int l0 = 0, bool zero = false);
 int cycle32(hzb_solver *S, const AMG_param &cyc, bool level0_zero);
+// The small levels of the l1-Jacobi V-cycle through merged kernels
+// (hzb_small.cu).  small_first_level: the first level small_levels may start
+// from in a cycle on levels l0.. (zero: level l0's x is zero), S->nl when it
+// does not apply.  small_levels(lb): with lb > l0 from level lb - 1's w to its
+// x (b_lb = R w, x += P x_lb); with lb = l0 from that level's b to its x.
+// A level is small while its launch and chain of loads outlast its memory
+// traffic, that is up to SMALL_ROWS_32 rows in FP32 (4 lanes a row; measured
+// with limits of 65,536, 262,144 and 524,288 rows: 100^3-cube setup and solve
+// 23.9, 23.3 and 24.3 ms, 1022^2 vertices 38.3, 37.5 and 39.7) and
+// SMALL_NNZ_64 entries in FP64 (a thread a row: with 0.9 and 1.8 million
+// entries in, the 64^3 solve takes 8.45 and 9.05 ms; with 0.5 and 1.1 million
+// the 400^2 one 6.4 and 5.9).  Above, the bundles and the sliced ELL copy
+// stream their rows better.
+constexpr int SMALL_ROWS_32 = 262144, SMALL_NNZ_64 = 1250000;
+template <typename T>
+int small_first_level(const hzb_solver *S, const AMG_param &cyc, int l0, bool zero);
+template <typename T>
+int small_levels(hzb_solver *S, int lb, int l0, const AMG_param &cyc);
 // reference PCG on level-0 operator
 int pcg(hzb_solver *S, const DCsr<double> &A, const double *b, double *u,
         int pc_kind, HostPrecond *hp, double tol, int maxit, int stop_type,
