@@ -324,18 +324,150 @@ k_bsr_gs_set(const int *__restrict__ rows, int cnt, const int *__restrict__ ia,
         bsr_relax_row<NB>(rows[q], ia, ja, val, dinv, b, x, x);
 }
 
-// a run of small level sets [first, last) by one CTA, sets in order
+// A run of small level sets [first, last) by one cluster of up to 8 CTAs, the
+// sets separated by its barrier (0.3 us).  One CTA with a thread per block row
+// took 16 us a set on the 24^3-cube system with 3 x 3 blocks (1.08 ms a sweep
+// of level 0, 14 MB of blocks through one SM, and each row a chain of loads):
+// here a lane per row of the block keeps the row's part of the first U blocks
+// in registers, loaded while the barrier is under way, from row indices and
+// pointers loaded one and two sets earlier, so that only the gathers of x and
+// the chain of subtractions stay between barriers: 0.13 ms.  The subtractions
+// run in row order (blocks in order, a block's columns in order), as above.
+// x is read and written at L2, which the CTAs share.
 template <int NB>
-__global__ void __launch_bounds__(256)
-k_bsr_gs_run(const int *__restrict__ rows, const int *__restrict__ set_ptr, int first,
-             int last, const int *__restrict__ ia, const int *__restrict__ ja,
-             const double *__restrict__ val, const double *__restrict__ dinv,
-             const double *__restrict__ b, double *x) {
+struct GsLane {
+    // lanes per block row, and blocks of a row held in registers
+    static constexpr int G = NB == 1 ? 1 : NB == 2 ? 2 : NB <= 4 ? 4 : 8;
+    static constexpr int U = NB <= 3 ? 16 : NB == 4 ? 8 : 4;
+    static constexpr int NT = 256, CLUSTER = 8;
+    static constexpr int ROWS = NT / G;     // block rows of a CTA at a time
+};
+
+template <int NB>
+__global__ void __launch_bounds__(GsLane<NB>::NT, 1)
+k_bsr_gs_cluster(const int *__restrict__ rows, const int *__restrict__ set_ptr, int first,
+                 int last, const int *__restrict__ ia, const int *__restrict__ ja,
+                 const double *__restrict__ val, const double *__restrict__ dinv,
+                 const double *__restrict__ b, double *x) {
+    using P = GsLane<NB>;
+    constexpr int G = P::G, U = P::U;
+    const int sub = threadIdx.x % G, r = min(sub, NB - 1);   // idle lanes repeat the last row
+    const int base = (threadIdx.x & 31) - sub;
+    const int at = blockIdx.x * P::ROWS + threadIdx.x / G;    // place in a set
+    const int cap = gridDim.x * P::ROWS;
+    auto row_at = [&](int k) {
+        if (k >= last) return -1;
+        const int q = __ldg(set_ptr + k) + at;
+        return q < __ldg(set_ptr + k + 1) ? __ldg(rows + q) : -1;
+    };
+    int i, k0, k1, c[U];             // the row at hand
+    double v[U][NB], d[NB], bi;
+    int i1, p0 = 0, p1 = 0;          // the next set's row and its pointers
+    int i2;                          // the row after that
+    auto load = [&]() {              // the next set's row becomes the one at hand
+        i = i1;
+        k0 = p0;
+        k1 = p1;
+        bi = 0.0;
+        if (i >= 0) {
+            bi = __ldg(b + (size_t)i * NB + r);
+#pragma unroll
+            for (int q = 0; q < NB; ++q) d[q] = __ldg(dinv + (size_t)i * (NB * NB) + r * NB + q);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            c[u] = k0 + u < k1 ? __ldg(ja + k0 + u) : -1;
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                v[u][q] = k0 + u < k1 ? __ldg(val + (size_t)(k0 + u) * (NB * NB) + r * NB + q)
+                                      : 0.0;
+        }
+    };
+    auto bounds = [&]() {
+        i1 = i2;
+        p0 = p1 = 0;
+        if (i1 >= 0) { p0 = __ldg(ia + i1); p1 = __ldg(ia + i1 + 1); }
+    };
+    i2 = row_at(first);
+    bounds();
+    load();
+    i2 = row_at(first + 1);
+    bounds();
+    i2 = row_at(first + 2);
     for (int k = first; k < last; ++k) {
-        for (int q = set_ptr[k] + threadIdx.x; q < set_ptr[k + 1]; q += blockDim.x)
-            bsr_relax_row<NB>(rows[q], ia, ja, val, dinv, b, x, x);
-        __syncthreads();
+        double t = bi;
+        {
+            double xv[U][NB];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < NB; ++q)
+                    xv[u][q] = c[u] >= 0 && c[u] != i ? __ldcg(x + (size_t)c[u] * NB + q) : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c[u] >= 0 && c[u] != i) {
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) t -= v[u][q] * xv[u][q];
+                }
+        }
+        constexpr int W = 4;         // the rest of a longer row
+        for (int kb = k0 + U; kb < k1; kb += W) {
+            int J[W];
+            double xr[W][NB];
+#pragma unroll
+            for (int u = 0; u < W; ++u) J[u] = kb + u < k1 ? __ldg(ja + kb + u) : i;
+#pragma unroll
+            for (int u = 0; u < W; ++u)
+#pragma unroll
+                for (int q = 0; q < NB; ++q)
+                    xr[u][q] = J[u] != i ? __ldcg(x + (size_t)J[u] * NB + q) : 0.0;
+#pragma unroll
+            for (int u = 0; u < W; ++u)
+                if (J[u] != i) {
+                    const double *a = val + (size_t)(kb + u) * (NB * NB) + r * NB;
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) t -= __ldg(a + q) * xr[u][q];
+                }
+        }
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) s += d[q] * __shfl_sync(0xffffffffu, t, base + q);
+        if (i >= 0 && sub < NB) __stcg(x + (size_t)i * NB + sub, s);
+        // a set of more rows than the cluster takes at a time
+        const int q1 = __ldg(set_ptr + k + 1);
+        for (int q = __ldg(set_ptr + k) + cap + blockIdx.x * P::NT + threadIdx.x; q < q1;
+             q += gridDim.x * P::NT)
+            bsr_relax_row<NB, true>(rows[q], ia, ja, val, dinv, b, x, x);
+        if (k + 1 == last) break;
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        load();
+        bounds();
+        i2 = row_at(k + 3);
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
+}
+
+template <int NB>
+int bsr_gs_cluster(const Schedule &sc, int run, const int *ia, const int *ja, const double *val,
+                   const double *dinv, const double *b, double *x, cudaStream_t s) {
+    using P = GsLane<NB>;
+    int grid = 1;
+    while (grid < P::CLUSTER && grid * P::ROWS < sc.run_max[run]) grid *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(P::NT);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = grid;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HZB_CUDA(cudaLaunchKernelEx(&cfg, k_bsr_gs_cluster<NB>, (const int *)sc.rows,
+                                (const int *)sc.set_ptr, sc.run_first[run], sc.run_last[run], ia,
+                                ja, val, dinv, b, x));
+    return SUCCESS;
 }
 
 // consecutive large level sets [first, last) in one cooperative launch,
@@ -440,6 +572,7 @@ struct Scratch {
 };
 
 void bsr_release(hzb_solver *S) {
+    S->gbsr.release();
     if (!S->bsr) return;
     S->bsr->release();
     delete S->bsr;
@@ -692,8 +825,7 @@ static int bsr_smooth(hzb_solver *S, BsrLevel &L, int kind, int sweeps) {
                     k_bsr_gs_set<NB><<<grid_for(cnt, 128), 128, 0, s>>>(
                         sc.rows + sc.h_ptr[f], cnt, L.ia, L.ja, L.val, L.dinv, E.b, E.x);
                 } else {
-                    k_bsr_gs_run<NB><<<1, 256, 0, s>>>(sc.rows, sc.set_ptr, f, l, L.ia, L.ja,
-                                                        L.val, L.dinv, E.b, E.x);
+                    rc = bsr_gs_cluster<NB>(sc, (int)q, L.ia, L.ja, L.val, L.dinv, E.b, E.x, s);
                 }
             });
             HZB_TRY(rc);
@@ -757,10 +889,14 @@ forward:
         Level &Cn = H.lv[nl - 1].s;
         const int csize = Cn.n;
         const int cmaxit = (int)std::min<long long>((long long)csize * csize, 200);
-        double rel = 0.0;
-        const int it = gmres(S, Cn.A64(), Cn.b, Cn.x, PC_NONE, nullptr, cyc.tol, cmaxit, 25,
-                             STOP_REL_RES, 0, false, &rel, MAX_AMG_LVL + 1);
-        if (it == ERROR_SOLVER_MISC || it == ERROR_ALLOC_MEM) return it;
+        if (gmres_cta_ok(csize, 25)) {
+            HZB_TRY(gmres_cta(Cn.A64(), Cn.b, Cn.x, cyc.tol, cmaxit, 25, s));
+        } else {
+            double rel = 0.0;
+            const int it = gmres(S, Cn.A64(), Cn.b, Cn.x, PC_NONE, nullptr, cyc.tol, cmaxit, 25,
+                                 STOP_REL_RES, 0, false, &rel, MAX_AMG_LVL + 1);
+            if (it == ERROR_SOLVER_MISC || it == ERROR_ALLOC_MEM) return it;
+        }
     }
     while (l > 0) {
         --l;
@@ -841,16 +977,27 @@ int bsr_time_kernel(hzb_solver *S, int which, int l, int reps, double *ms_per_la
 }
 
 // precond_dbsr_amg (precond.c:1311-1335): maxit cycles from zero
+// Nothing of the cycle reads a device value on the host: no coarse scaling,
+// the coarsest solve in one launch.
+bool bsr_capturable(const hzb_solver *S) {
+    return S->bsr && S->bsr_cyc.coarse_scaling != ON &&
+           gmres_cta_ok(S->bsr->lv[S->bsr->nl - 1].s.n, 25);
+}
+
 int bsr_precond(hzb_solver *S, const double *r, double *z) {
     BsrHier &H = *S->bsr;
     Level &E = H.lv[0].s;
-    double *sx = E.x;
-    HZB_TRY(vcopy<double>(E.n, r, E.b, S->s));   // the residual is an input
-    E.x = z;
-    int rc = vzero<double>(E.n, z, S->s);
-    for (int i = 0; rc == SUCCESS && i < S->bsr_cyc.maxit; ++i) rc = bsr_cycle(S, S->bsr_cyc);
-    E.x = sx;
-    return rc;
+    auto body = [&]() {
+        double *sx = E.x;
+        HZB_TRY(vcopy<double>(E.n, r, E.b, S->s));   // the residual is an input
+        E.x = z;
+        int rc = vzero<double>(E.n, z, S->s);
+        for (int i = 0; rc == SUCCESS && i < S->bsr_cyc.maxit; ++i) rc = bsr_cycle(S, S->bsr_cyc);
+        E.x = sx;
+        return rc;
+    };
+    if (!bsr_capturable(S)) return body();
+    return with_graph(S, S->gbsr, r, z, cycle_tag(S, S->bsr_cyc), body);
 }
 
 }  // namespace hzb

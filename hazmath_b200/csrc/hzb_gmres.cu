@@ -89,6 +89,207 @@ __global__ void k_gm_add(int n, const double *__restrict__ x, double *y) {
         y[k] += x[k];
 }
 
+// The unpreconditioned variable-restart GMRES (STOP_REL_RES) of a small system
+// in one CTA: the loop of gmres() below, basis in shared memory, scalars by
+// thread 0, no host.  A coarsest level of some hundred rows took 14 launches
+// and a host read per step there (2.3 ms for 24 steps); every operation rounds
+// as there (n <= 1024 rows, which dot() reduces with one block of 256 threads
+// too), so the iterates are the same bit for bit.
+constexpr int GM_CTA = 256, GM_CTA_ROWS = 1024, GM_CTA_SMEM = 200 * 1024;
+
+__global__ void __launch_bounds__(GM_CTA)
+k_gmres_cta(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+            const double *__restrict__ a, const double *__restrict__ b, double *x, double tol,
+            int MaxIt, int restart) {
+    extern __shared__ __align__(16) double gm_smem[];
+    double *P = gm_smem;                               // restart + 1 vectors
+    double *r = P + (size_t)(restart + 1) * n;
+    double *hh = r + n;                                // (restart + 1)^2, by rows
+    double *c = hh + (restart + 1) * (restart + 1), *sn = c + restart + 1, *rs = sn + restart + 1;
+    double *h = rs + restart + 2;                      // Hessenberg column, restart + 2
+    __shared__ double sh[32], s_val;
+    const int tid = threadIdx.x, ld = restart + 1;
+    auto total = [&](double v) {                       // block sum, to every thread
+        v = block_sum(v, sh);
+        if (tid == 0) s_val = v;
+        __syncthreads();
+        v = s_val;
+        __syncthreads();
+        return v;
+    };
+    auto norm2 = [&](const double *u) {
+        double v = 0.0;
+        for (int k = tid; k < n; k += GM_CTA) v += u[k] * u[k];
+        return total(v);
+    };
+    auto row_times = [&](int i, const double *v) {     // (A v)_i in CSR order
+        constexpr int G = 8;
+        double t = 0.0;
+        const int k1 = ia[i + 1];
+        for (int kb = ia[i]; kb < k1; kb += G) {
+            double av[G], xv[G];
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                av[q] = kb + q < k1 ? a[kb + q] : 0.0;
+                xv[q] = kb + q < k1 ? v[ja[kb + q]] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                if (kb + q < k1) t += av[q] * xv[q];
+        }
+        return t;
+    };
+    const double cr_max = 0.99, cr_min = 0.174, epsmac = SMALLREAL;
+    const int d = 3, restart_min = 3, restart_max = restart;
+    int Restart = restart, iter = 0;
+    double cr = 1.0;
+    for (int k = tid; k < n; k += GM_CTA) P[k] = b[k] - row_times(k, x);
+    __syncthreads();
+    double r_norm = sqrt(norm2(P));
+    const double absres0 = fmax(SMALLREAL, r_norm);
+    double relres = r_norm / absres0;
+    if (relres < tol || absres0 < 1e-3 * tol) return;
+    while (iter < MaxIt) {
+        const double r_norm_old = r_norm;
+        if (tid == 0) rs[0] = r_norm;
+        if (cr > cr_max || iter == 0) {
+            Restart = restart_max;
+        } else if (cr < cr_min) {
+            // keep it
+        } else if (Restart - d > restart_min) {
+            Restart -= d;
+        } else {
+            Restart = restart_max;
+        }
+        const double scale = 1.0 / r_norm;
+        for (int k = tid; k < n; k += GM_CTA) P[k] *= scale;
+        __syncthreads();
+        int i = 0;
+        while (i < Restart && iter < MaxIt) {
+            ++i;
+            ++iter;
+            const double *pv = P + (size_t)(i - 1) * n;
+            double *pi = P + (size_t)i * n;
+            double acc = 0.0;
+            for (int k = tid; k < n; k += GM_CTA) {
+                const double v = row_times(k, pv);
+                pi[k] = v;
+                acc += P[k] * v;
+            }
+            double hj = total(acc);
+            if (tid == 0) h[0] = hj;
+            for (int j = 0; j < i; ++j) {
+                const double m = -hj, *pj = P + (size_t)j * n;
+                const double *q = j + 1 < i ? P + (size_t)(j + 1) * n : nullptr;
+                acc = 0.0;
+                for (int k = tid; k < n; k += GM_CTA) {
+                    const double v = pi[k] + m * pj[k];
+                    pi[k] = v;
+                    acc += (q ? q[k] : v) * v;
+                }
+                hj = total(acc);
+                if (tid == 0) h[j + 1] = hj;
+            }
+            const double t = sqrt(hj);
+            if (t != 0.0) {
+                const double ri = 1.0 / t;
+                for (int k = tid; k < n; k += GM_CTA) pi[k] *= ri;
+            }
+            if (tid == 0) {
+                h[i] = t;
+                for (int j = 0; j <= i; ++j) hh[j * ld + i - 1] = h[j];
+                for (int j = 1; j < i; ++j) {
+                    const double u = hh[(j - 1) * ld + i - 1];
+                    hh[(j - 1) * ld + i - 1] = sn[j - 1] * hh[j * ld + i - 1] + c[j - 1] * u;
+                    hh[j * ld + i - 1] = -sn[j - 1] * u + c[j - 1] * hh[j * ld + i - 1];
+                }
+                double g2 = hh[i * ld + i - 1] * hh[i * ld + i - 1];
+                g2 += hh[(i - 1) * ld + i - 1] * hh[(i - 1) * ld + i - 1];
+                double gamma = sqrt(g2);
+                if (gamma == 0.0) gamma = epsmac;
+                c[i - 1] = hh[(i - 1) * ld + i - 1] / gamma;
+                sn[i - 1] = hh[i * ld + i - 1] / gamma;
+                rs[i] = -sn[i - 1] * rs[i - 1];
+                rs[i - 1] = c[i - 1] * rs[i - 1];
+                hh[(i - 1) * ld + i - 1] =
+                    sn[i - 1] * hh[i * ld + i - 1] + c[i - 1] * hh[(i - 1) * ld + i - 1];
+                s_val = fabs(rs[i]);
+            }
+            __syncthreads();
+            r_norm = s_val;
+            relres = r_norm / absres0;
+            __syncthreads();
+            if (relres < tol) break;
+        }
+        if (tid == 0) {   // the upper triangular system
+            rs[i - 1] = rs[i - 1] / hh[(i - 1) * ld + i - 1];
+            for (int k = i - 2; k >= 0; --k) {
+                double t = 0.0;
+                for (int j = k + 1; j < i; ++j) t -= hh[k * ld + j] * rs[j];
+                t += rs[k];
+                rs[k] = t / hh[k * ld + k];
+            }
+        }
+        __syncthreads();
+        for (int k = tid; k < n; k += GM_CTA) {
+            double v = P[(size_t)(i - 1) * n + k];
+            if (rs[i - 1] != 1.0) v *= rs[i - 1];
+            for (int j = i - 2; j >= 0; --j) v = v + rs[j] * P[(size_t)j * n + k];
+            x[k] += v;
+        }
+        __syncthreads();
+        if (relres < tol) {   // the true residual decides
+            for (int k = tid; k < n; k += GM_CTA) r[k] = b[k] - row_times(k, x);
+            r_norm = sqrt(norm2(r));
+            relres = r_norm / absres0;
+            if (relres < tol) return;
+            for (int k = tid; k < n; k += GM_CTA) P[k] = r[k];
+            i = 0;
+            __syncthreads();
+        }
+        if (i) {   // the residual direction for the next cycle
+            if (tid == 0)
+                for (int j = i; j > 0; --j) {
+                    rs[j - 1] = -sn[j - 1] * rs[j];
+                    rs[j] = c[j - 1] * rs[j];
+                }
+            __syncthreads();
+            for (int k = tid; k < n; k += GM_CTA) {
+                double v = P[(size_t)i * n + k];
+                v = v + (rs[i] - 1.0) * v;
+                for (int j = i - 1; j > 0; --j) v = v + rs[j] * P[(size_t)j * n + k];
+                P[(size_t)i * n + k] = v;
+                double u = P[k];
+                u = u + (rs[0] - 1.0) * u;
+                P[k] = u + v;
+            }
+            __syncthreads();
+        }
+        cr = r_norm / r_norm_old;
+    }
+}
+
+static size_t gmres_cta_smem(int n, int restart) {
+    const size_t ld = restart + 1;
+    return ((ld + 1) * n + ld * ld + 2 * ld + 2 * (ld + 1)) * sizeof(double);
+}
+
+bool gmres_cta_ok(int n, int restart) {
+    return n >= 1 && n <= GM_CTA_ROWS && restart >= 1 &&
+           gmres_cta_smem(n, restart) <= (size_t)GM_CTA_SMEM;
+}
+
+int gmres_cta(const DCsr<double> &A, const double *b, double *x, double tol, int MaxIt,
+              int restart, cudaStream_t s) {
+    HZB_CUDA(cudaFuncSetAttribute(k_gmres_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  GM_CTA_SMEM));
+    k_gmres_cta<<<1, GM_CTA, gmres_cta_smem(A.n, restart), s>>>(A.n, A.ia, A.ja, A.val, b, x, tol,
+                                                               MaxIt, restart);
+    count_launch();
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
+
 struct GmresWork {
     int n = 0, restart = 0, req = 0;   // allocated / requested restart
     bool flexible = false;
@@ -185,7 +386,7 @@ static int arnoldi(hzb_solver *S, GmresWork &g, const DCsr<double> &A, int kind,
                    HostPrecond *hp, int i, double *zout, std::vector<double> &h) {
     const int n = g.n;
     cudaStream_t s = S->s;
-    HZB_TRY(apply_precond(S, kind, hp, n, g.p[i - 1], zout));   // z = M p_{i-1}
+    HZB_TRY(apply_precond_staged(S, kind, hp, n, g.p[i - 1], zout));   // z = M p_{i-1}
     HZB_TRY(spmv<double>(A, SPMV_Y, zout, nullptr, g.p[i], 1.0, nullptr, s));
     const int G = reduce_blocks(n);
     HZB_TRY(dot(n, g.p[0], g.p[i], g.part, g.col + 0, s));
@@ -281,7 +482,7 @@ int gmres(hzb_solver *S, const DCsr<double> &A, const double *b, double *x, int 
             relres = r_norm / absres0;
             break;
         case STOP_REL_PRECRES: {
-            HZB_TRY(apply_precond(S, kind, hp, n, g.p[0], g.r));
+            HZB_TRY(apply_precond_staged(S, kind, hp, n, g.p[0], g.r));
             double t = 0.0;
             HZB_TRY(dot_host(S, g, g.p[0], g.r, &t));
             const double r_normb = sqrt(t);
@@ -378,7 +579,7 @@ int gmres(hzb_solver *S, const DCsr<double> &A, const double *b, double *x, int 
             std::vector<double> cf(rs.begin(), rs.begin() + i);
             if (!flexible) {
                 HZB_TRY(combine(S, g, g.d_p, i, cf, g.w));
-                HZB_TRY(apply_precond(S, kind, hp, n, g.w, g.r));
+                HZB_TRY(apply_precond_staged(S, kind, hp, n, g.w, g.r));
             } else {
                 HZB_TRY(combine(S, g, g.d_z, i, cf, g.r));
             }
@@ -394,7 +595,7 @@ int gmres(hzb_solver *S, const DCsr<double> &A, const double *b, double *x, int 
             double measure = r_norm;
             if (stop_type == STOP_REL_PRECRES) {
                 double *dst = flexible ? g.p[0] : g.w;
-                HZB_TRY(apply_precond(S, kind, hp, n, g.r, dst));
+                HZB_TRY(apply_precond_staged(S, kind, hp, n, g.r, dst));
                 double t = 0.0;
                 HZB_TRY(dot_host(S, g, dst, g.r, &t));
                 measure = sqrt(t);

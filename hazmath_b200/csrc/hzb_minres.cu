@@ -150,7 +150,7 @@ int minres(hzb_solver *S, const DCsr<double> &A, const double *b, double *u, int
         *out = w.h[slot];
         return SUCCESS;
     };
-    auto pc = [&](const double *r, double *z) { return apply_precond(S, kind, hp, m, r, z); };
+    auto pc = [&](const double *r, double *z) { return apply_precond_staged(S, kind, hp, m, r, z); };
     // the residual measure of the stopping type from the current r (uses t)
     auto measure = [&](double nu2, double *absr, double *relr) -> int {
         double v = 0.0;

@@ -750,6 +750,7 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
     S->g32.release();
     S->g32c.release();
     S->gcyc.release();
+    S->gbsr.release();
     gmres_release(S);
     gcg_release(S);
     for (auto &L : S->lv) L.release();
@@ -1057,9 +1058,31 @@ static int apply_pc(hzb_solver *S, int kind, HostPrecond *hp, int n,
     return vcopy<double>(n, r, z, S->s);
 }
 
+// whether a kind's application is replayed from a captured graph
+static bool precond_captured(const hzb_solver *S, int kind) {
+    if (!S->bp.use_graph) return false;
+    if (kind == PC_BSR) return bsr_capturable(S);
+    return (kind == PC_AMG || kind == PC_AMLI || kind == PC_ADD) &&
+           S->pc_cyc.coarse_solver == SOLVER_UMFPACK && S->Ainv && S->pc_cyc.coarse_scaling != ON;
+}
+
 int apply_precond(hzb_solver *S, int kind, HostPrecond *hp, int n, const double *r,
                   double *z) {
     return apply_pc(S, kind, hp, n, r, z);
+}
+
+// For loops whose vectors change from step to step (a Krylov basis): through
+// kw's r and z, which a captured application keeps its addresses of.  Two
+// copies instead of a capture and an instantiation per step, which took 0.5
+// ms (2D 255^2: 24 steps).
+int apply_precond_staged(hzb_solver *S, int kind, HostPrecond *hp, int n, const double *r,
+                         double *z) {
+    KrylovWork &w = S->kw;
+    if (w.n != n || r == w.r || r == w.z || z == w.r || z == w.z || !precond_captured(S, kind))
+        return apply_pc(S, kind, hp, n, r, z);
+    HZB_TRY(vcopy<double>(n, r, w.r, S->s));
+    HZB_TRY(apply_pc(S, kind, hp, n, w.r, w.z));
+    return vcopy<double>(n, w.z, z, S->s);
 }
 
 // residual measure for the stopping type (krylov.c:157-170, 211-227)
@@ -1262,44 +1285,7 @@ static int apply_pc32_body(hzb_solver *S, const double *r, double *z) {
     return f2d(L0.n, L0.x32, z, S->s);
 }
 
-// Replays `body` from a CUDA graph captured on the solver's stream; the
-// capture is redone whenever the key (vector pointers, tag) changes.
-template <typename F>
-static int with_graph(hzb_solver *S, GraphCache &G, const void *k0, const void *k1,
-                      long long tag, F body, long long tag2 = 0) {
-    if (!S->bp.use_graph) return body();
-    if (!G.exec || G.k0 != k0 || G.k1 != k1 || G.tag != tag || G.tag2 != tag2) {
-        G.release();
-        const long long before = launch_count();
-        HZB_CUDA(cudaStreamBeginCapture(S->s, cudaStreamCaptureModeThreadLocal));
-        int rc = body();
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(S->s, &g);
-        if (rc || e != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            if (e != cudaSuccess) set_error(e, __FILE__, __LINE__);
-            return rc ? rc : ERROR_SOLVER_MISC;
-        }
-        e = cudaGraphInstantiate(&G.exec, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            G.exec = nullptr;
-            set_error(e, __FILE__, __LINE__);
-            return ERROR_SOLVER_MISC;
-        }
-        G.k0 = k0;
-        G.k1 = k1;
-        G.tag = tag;
-        G.tag2 = tag2;
-        G.kernels = launch_count() - before;   // counted once by the capture
-    } else {
-        count_launch((int)G.kernels);
-    }
-    HZB_CUDA(cudaGraphLaunch(G.exec, S->s));
-    return SUCCESS;
-}
-
-static long long cycle_tag(const hzb_solver *S, const AMG_param &c) {
+long long cycle_tag(const hzb_solver *S, const AMG_param &c) {
     return (long long)c.maxit | ((long long)c.cycle_type << 8) |
            ((long long)c.smoother << 12) | ((long long)c.presmooth_iter << 20) |
            ((long long)c.postsmooth_iter << 26) | ((long long)S->omega_active << 32) |
@@ -1431,6 +1417,7 @@ void destroy(hzb_solver *S) {
     S->g32.release();
     S->g32c.release();
     S->gcyc.release();
+    S->gbsr.release();
     gmres_release(S);
     gcg_release(S);
     for (auto &L : S->lv) L.release();

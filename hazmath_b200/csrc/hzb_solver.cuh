@@ -153,6 +153,7 @@ struct hzb_solver {
     hzb::GraphCache g64, g32;         // captured FP64 / FP32 preconditioners
     hzb::GraphCache g32c;             // the FP32 cycles alone (level-0 b32 given)
     hzb::GraphCache gcyc;             // captured AMLI / additive preconditioner
+    hzb::GraphCache gbsr;             // captured block (BSR) preconditioner
     std::vector<double> amli_coef;    // polynomial of the AMLI cycle (degree + 1)
     // Krylov work kept per level for the coarse-level solves of the
     // nonlinear AMLI cycle and the coarse GMRES fallback
@@ -213,6 +214,9 @@ int pc_kind_of_cycle(int cycle_type);
 // z = M r for a preconditioner kind of pcg / gmres
 int apply_precond(hzb_solver *S, int kind, HostPrecond *hp, int n, const double *r,
                   double *z);
+// the same for vectors that change from call to call
+int apply_precond_staged(hzb_solver *S, int kind, HostPrecond *hp, int n, const double *r,
+                         double *z);
 // variable-restart GMRES (flexible = false, dcsr_pvgmres) or flexible GMRES
 // (dcsr_pvfgmres), right-preconditioned (hzb_gmres.cu)
 // (hzb_gmres.cu); ws_slot >= 0 keeps the basis in S->gm_ws[ws_slot] for the
@@ -221,6 +225,11 @@ int gmres(hzb_solver *S, const DCsr<double> &A, const double *b, double *x, int 
           HostPrecond *hp, double tol, int MaxIt, int restart, int stop_type, int prtlvl,
           bool flexible, double *relres_out, int ws_slot = -1);
 void gmres_release(hzb_solver *S);
+// the unpreconditioned GMRES (not flexible, STOP_REL_RES) of a small system in
+// one launch, the same iterates; gmres_cta_ok: whether the system fits
+bool gmres_cta_ok(int n, int restart);
+int gmres_cta(const DCsr<double> &A, const double *b, double *x, double tol, int MaxIt,
+              int restart, cudaStream_t s);
 // preconditioned MINRES, dcsr_pminres (hzb_minres.cu)
 int minres(hzb_solver *S, const DCsr<double> &A, const double *b, double *u, int kind,
            HostPrecond *hp, double tol, int MaxIt, int stop_type, int prtlvl,
@@ -306,6 +315,7 @@ bool batch_has_terminal(const hzb_solver *S, int lvl);
 int bsr_setup(hzb_solver *S, int nrow, int nnzb, int nb, const int *d_ia, const int *d_ja,
               const double *d_val);
 int bsr_precond(hzb_solver *S, const double *r, double *z);
+bool bsr_capturable(const hzb_solver *S);
 int bsr_cycle(hzb_solver *S, const AMG_param &cyc);
 DCsr<double> bsr_scalar_A(hzb_solver *S);
 int bsr_block_size(const hzb_solver *S);
@@ -315,4 +325,42 @@ void bsr_release(hzb_solver *S);
 // hzb_time_kernel's block kernels (HZB_K_BSR_*)
 int bsr_time_kernel(hzb_solver *S, int which, int l, int reps, double *ms_per_launch,
                     double *bytes_per_launch);
+// the cycle parameters a captured cycle depends on
+long long cycle_tag(const hzb_solver *S, const AMG_param &c);
+// Replays `body` from a CUDA graph captured on the solver's stream; the
+// capture is redone whenever the key (vector pointers, tag) changes.
+template <typename F>
+int with_graph(hzb_solver *S, GraphCache &G, const void *k0, const void *k1,
+                      long long tag, F body, long long tag2 = 0) {
+    if (!S->bp.use_graph) return body();
+    if (!G.exec || G.k0 != k0 || G.k1 != k1 || G.tag != tag || G.tag2 != tag2) {
+        G.release();
+        const long long before = launch_count();
+        HZB_CUDA(cudaStreamBeginCapture(S->s, cudaStreamCaptureModeThreadLocal));
+        int rc = body();
+        cudaGraph_t g = nullptr;
+        cudaError_t e = cudaStreamEndCapture(S->s, &g);
+        if (rc || e != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            if (e != cudaSuccess) set_error(e, __FILE__, __LINE__);
+            return rc ? rc : ERROR_SOLVER_MISC;
+        }
+        e = cudaGraphInstantiate(&G.exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            G.exec = nullptr;
+            set_error(e, __FILE__, __LINE__);
+            return ERROR_SOLVER_MISC;
+        }
+        G.k0 = k0;
+        G.k1 = k1;
+        G.tag = tag;
+        G.tag2 = tag2;
+        G.kernels = launch_count() - before;   // counted once by the capture
+    } else {
+        count_launch((int)G.kernels);
+    }
+    HZB_CUDA(cudaGraphLaunch(G.exec, S->s));
+    return SUCCESS;
+}
 }  // namespace hzb

@@ -155,3 +155,26 @@ def test_bsr_rejects_what_the_reference_rejects(golden):
     zval[d0] = 0.0
     assert S.setup_bsr_host(3, big[0], big[1], zval.reshape(-1)) == hz.ERROR_DATA_ZERODIAG
     S.close()
+
+
+@pytest.mark.parametrize("nb,N,smoother", [
+    (1, 20, hz.SMOOTHER_GS), (2, 26, hz.SMOOTHER_GS), (3, 34, hz.SMOOTHER_GS),
+    (3, 12, hz.SMOOTHER_SGS), (4, 18, hz.SMOOTHER_GS), (5, 14, hz.SMOOTHER_GS),
+    (6, 12, hz.SMOOTHER_SGS), (7, 12, hz.SMOOTHER_GS), (8, 14, hz.SMOOTHER_GS)])
+def test_bsr_precond_block_sizes_vs_oracle(port, nb, N, smoother):
+    """Every block size, level sets of one CTA to more rows than a cluster
+    takes at a time (N = 34, nb = 3 and N = 14, nb = 8), rows longer than the
+    blocks held in registers (the coarse levels; nb >= 4 everywhere)."""
+    kia, kja, kval = P.kuhn3d_p1(N, P.lognormal_field(N, 1.0, 4.0, nb))
+    B = 2.0 * np.eye(nb) + 0.3 / nb * np.add.outer(np.arange(nb), np.arange(nb)) / nb
+    P.BLOCK_COUPLING.setdefault(nb, B)
+    ia, ja, val = P.block_system(kia, kja, kval, nb, 40 + nb)
+    r = P.rhs_uniform((len(ia) - 1) * nb, 7)
+    port.bsr_hierarchy(nb, ia, ja, val, coarse_dof=100)
+    z_o = port.bsr_precond(r, cycle_type=1, smoother=smoother, presmooth_iter=1)
+    S = hz.Solver(hz.bench_amg(coarse_dof=100, coarse_solver=0, smoother=smoother), itparam("pcg"))
+    assert S.setup_bsr_host(nb, ia, ja, val) == 0, hz.last_error()
+    z = S.bsr_precond_host(r)
+    assert np.array_equal(z, S.bsr_precond_host(r))
+    S.close()
+    np.testing.assert_allclose(z, z_o, rtol=0, atol=ZTOL * np.abs(z_o).max())
