@@ -27,6 +27,7 @@ SOURCES = [
     ("hzb_sell.cu", False),
     ("hzb_setup.cu", False),
     ("hzb_match.cu", False),
+    ("hzb_gs.cu", False),
     ("hzb_dense.cu", True),
     ("hzb_solver.cu", False),
     ("hzb_small.cu", False),

@@ -1429,8 +1429,9 @@ extern "C" INT hzb_smoother_device(SHORT smoother, SHORT forward, INT sweeps,
     rc = bundle_capacity(n, ia, S->s, &L.bundle_cap);
     if (!rc) rc = dalloc(&L.t, n);
     if (!rc) rc = level_smoother_data(S, L);
+    if (!rc) rc = S->kw.alloc(n, S->s);   // its error word
     if (!rc) rc = smooth64(S, 0, forward != 0, amg);
-    if (!rc && cudaStreamSynchronize(S->s) != cudaSuccess) rc = ERROR_SOLVER_MISC;
+    if (!rc) rc = check_waits(S);
     L.b = nullptr;   // not owned
     L.x = nullptr;
     }

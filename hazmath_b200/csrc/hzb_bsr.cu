@@ -741,8 +741,8 @@ static int bsr_build(hzb_solver *S, int nrow, int nnzb, int nb, const int *d_ia,
     if (S->amg.smoother == SMOOTHER_GS || S->amg.smoother == SMOOTHER_SGS)
         for (int l = 0; l < H.nl - 1; ++l) {
             BsrLevel &L = H.lv[l];
-            HZB_TRY(gs_schedule(L.nrow, L.ia, L.ja, L.nnzb, 0, &L.asc, s));
-            HZB_TRY(gs_schedule(L.nrow, L.ia, L.ja, L.nnzb, 1, &L.desc, s));
+            HZB_TRY(gs_schedule(L.nrow, L.ia, L.ja, L.nnzb, &L.asc, s));
+            HZB_TRY(gs_schedule_reverse(L.asc, L.nrow, &L.desc, s));
         }
     HZB_TRY(H.kwc.alloc(H.lv[0].s.n));
     HZB_TRY(S->kw.alloc(H.lv[0].s.n));

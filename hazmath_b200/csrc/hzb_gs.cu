@@ -1,0 +1,474 @@
+// hzb_gs.cu -- exact Gauss-Seidel over small level sets, streamed.
+//
+// A level set of the lexicographic order depends on the one before it, so what
+// bounds a sweep is the time from one set to the next.  One CTA runs the sets
+// in order and keeps everything a set needs in shared memory: the matrix rows
+// are stored a second time in the schedule's order (a set's rows of one length,
+// filled up with zeros against a place that holds zero, the diagonal left out), x, b and the diagonals are put
+// into that order before the sweep and x back after it, so that a warp of its
+// own copies whole groups of sets ahead by a few contiguous bulk copies.  x
+// lies in a ring indexed by place in the schedule, wide enough that every
+// entry's value is in it: new values of earlier sets, the old iterate for
+// later ones.  A set is then one barrier, the shared loads of x (a thread has
+// its row's first entries in registers by then) and the chain of subtractions.
+//   Measured on the sets of 2D 5-point levels: 0.47 us a set with loads
+// rotated through registers and x in shared memory, 1.3 with x in global
+// memory (gathers of just written values miss L1), 0.7 to 1.3 with
+// asynchronous 8-byte gathers in place of the permuted vectors (along an
+// anti-diagonal each touches a line of its own, and they fill the queue that
+// the shared loads of the computing warps go through), 0.6 with a set's copies
+// issued inside its barrier, 0.6 with a test per entry (200 instructions a set,
+// each waiting for the one before), 0.27 to 0.35 now.
+//   The row sum runs in CSR order from b_i with the diagonal skipped, each
+// value rounded as in gs_rows: the same bits.
+#include "hzb_solver.cuh"
+#include <algorithm>
+
+namespace hzb {
+
+namespace {
+
+constexpr int GS_ROWS = 256;           // a set's rows: one per computing thread
+constexpr int GS_SETS = 2048;          // sets of a schedule (their sizes lie in shared memory)
+constexpr int GS_BLOCK = 256;          // places per copy of x
+constexpr int GS_PAD = 8;              // set starts and slot pitches, in places
+constexpr size_t GS_SMEM = 220 * 1024;
+
+// set s: first place (x), rows and entries per row (y; the latter even and in
+// the upper half), the first place's place in the ring (z), first entry (w); its
+// rows are rounded up to GS_PAD
+__host__ __device__ inline int gs_pitch(int rows) { return (rows + GS_PAD - 1) / GS_PAD * GS_PAD; }
+__host__ __device__ inline int gs_rows(int4 I) { return I.y & 0xffff; }
+__host__ __device__ inline int gs_width(int4 I) { return I.y >> 16; }
+// the places and entries behind a set
+__host__ __device__ inline int gs_end_place(int4 I) { return I.x + gs_pitch(gs_rows(I)); }
+__host__ __device__ inline int gs_end_entry(int4 I) {
+    return I.w + gs_width(I) * gs_pitch(gs_rows(I));
+}
+
+// one stage, a group of sets of E entries and R places: values, (b, d), columns
+__host__ __device__ inline size_t gs_stage(int E, int R) {
+    return (size_t)E * 8 + (size_t)R * 16 + (size_t)E * 2;
+}
+inline size_t gs_smem(int ns, int E, int R, int ring, int stages) {
+    return (size_t)ns * 16 + (size_t)(ring + 2) * 8 + (size_t)stages * gs_stage(E, R) +
+           (size_t)stages * 16;
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes,
+                                          unsigned long long *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
+                 "[%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
+                 "r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void bar_init(unsigned long long *bar, unsigned count) {
+    asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+// wait for the phase of the given parity; bounded: a copy that never arrives
+// is reported, and nobody waits any more
+__device__ __forceinline__ void bar_wait(unsigned long long *bar, unsigned parity, int *dead,
+                                         int *err) {
+    unsigned done = 0;
+    for (unsigned spin = 0; !done; ++spin) {
+        asm volatile("{\n.reg .pred p;\n"
+                     "mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n"
+                     "selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (done || *(volatile int *)dead) return;
+        if (spin > (1u << 20)) {
+            *(volatile int *)dead = 1;
+            atomicExch(err, 1);
+            return;
+        }
+    }
+}
+
+// What a sweep runs on; group: sets per stage, E and R a stage's capacity.
+struct GsSweep {
+    const int4 *info;
+    const unsigned short *col;
+    const double *val;
+    const double2 *bd;
+    double *x;
+    int ns, group, E, R, stages, ring, dist, places, skip_place;
+};
+
+// A thread's row of a set with Z entries: loaded before the barrier that
+// completes the previous set, finished behind it.
+template <int Z>
+struct GsRow {
+    unsigned c[Z / 2];              // two ring places each
+    double v[Z];
+    __device__ __forceinline__ void load(const unsigned short *col, const double *val) {
+        if (Z % 4 == 0) {
+#pragma unroll
+            for (int q = 0; q < Z / 4; ++q) {
+                const uint2 u = reinterpret_cast<const uint2 *>(col)[q];
+                c[2 * q] = u.x;
+                c[2 * q + 1] = u.y;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < Z / 2; ++q) c[q] = reinterpret_cast<const unsigned *>(col)[q];
+        }
+#pragma unroll
+        for (int q = 0; q < Z / 2; ++q) {
+            const double2 u = reinterpret_cast<const double2 *>(val)[q];
+            v[2 * q] = u.x;
+            v[2 * q + 1] = u.y;
+        }
+    }
+    __device__ __forceinline__ double sum(const double *ring, double acc) const {
+        double x[Z];
+#pragma unroll
+        for (int q = 0; q < Z / 2; ++q) {
+            x[2 * q] = ring[c[q] & 0xffffu];
+            x[2 * q + 1] = ring[c[q] >> 16];
+        }
+#pragma unroll
+        for (int q = 0; q < Z; ++q) acc -= v[q] * x[q];
+        return acc;
+    }
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(GS_ROWS + 32, 1)
+k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    int4 *info = reinterpret_cast<int4 *>(smem);
+    double *ring = reinterpret_cast<double *>(info + A.ns);   // and a place that holds zero
+    unsigned char *stage0 = reinterpret_cast<unsigned char *>(ring + A.ring + 2);
+    const int stage_bytes = (int)gs_stage(A.E, A.R);
+    unsigned long long *full =
+        reinterpret_cast<unsigned long long *>(stage0 + A.stages * stage_bytes);
+    unsigned long long *empty = full + A.stages;
+    __shared__ int s_dead;
+    const int t = threadIdx.x, ns = A.ns;
+    for (int k = t; k < ns; k += blockDim.x) info[k] = A.info[k];
+    if (t == 0) {
+        s_dead = 0;
+        ring[A.ring] = 0.0;
+        for (int k = 0; k < A.stages; ++k) {
+            bar_init(full + k, 1);
+            bar_init(empty + k, 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (t >= GS_ROWS) {
+        // groups of sets into their stages, and x as far as their rows reach
+        if (t > GS_ROWS) return;
+        int loaded = 0, to = 0, k = 0;  // places of x copied or on their way; the stage
+        unsigned parity = 1;            // the first round finds every stage empty
+        for (int s0 = 0; s0 < ns; s0 += A.group) {
+            const int4 I0 = info[s0], I1 = info[min(s0 + A.group, ns) - 1];
+            const int rows = gs_end_place(I1) - I0.x, e = gs_end_entry(I1) - I0.w;
+            int upto = (gs_end_place(I1) + A.dist + GS_BLOCK - 1) / GS_BLOCK * GS_BLOCK;
+            upto = max(min(upto, A.places), loaded);
+            bar_wait(empty + k, parity, &s_dead, err);
+            double *val = reinterpret_cast<double *>(stage0 + k * stage_bytes);
+            double2 *bd = reinterpret_cast<double2 *>(val + A.E);
+            unsigned short *col = reinterpret_cast<unsigned short *>(bd + A.R);
+            const unsigned bytes = (unsigned)(e * 10 + rows * 16 + (upto - loaded) * 8);
+            asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;"
+                         ::"r"(smem_u32(full + k)), "r"(bytes) : "memory");
+            if (e) {
+                bulk_copy(val, A.val + I0.w, e * 8, full + k);
+                bulk_copy(col, A.col + I0.w, e * 2, full + k);
+            }
+            bulk_copy(bd, A.bd + I0.x, rows * 16, full + k);
+            for (; loaded < upto; loaded += GS_BLOCK) {   // the ring is a multiple of GS_BLOCK
+                bulk_copy(ring + to, A.x + loaded, GS_BLOCK * 8, full + k);
+                to = to + GS_BLOCK == A.ring ? 0 : to + GS_BLOCK;
+            }
+            if (++k == A.stages) {
+                k = 0;
+                parity ^= 1u;
+            }
+        }
+        return;
+    }
+    int k = 0, in_group = 0;            // the stage at hand, sets of it begun
+    unsigned parity = 0;
+    int e0 = 0, x0 = 0;                 // the group's first entry and place
+    const unsigned char *stage = stage0;
+    const int val_bytes = A.E * 8, col_at = val_bytes + A.R * 16;
+    unsigned long long *release = nullptr;   // the stage that the next barrier frees
+    for (int s = 0; s < ns; ++s) {
+        const int4 I = info[s];
+        if (in_group == 0) {
+            bar_wait(full + k, parity, &s_dead, err);
+            x0 = I.x;
+            e0 = I.w;
+            stage = stage0 + k * stage_bytes;
+        }
+        const int Z = gs_width(I);
+        const bool on = t < gs_rows(I);
+        const int at = on ? I.w - e0 + t * Z : 0;   // idle threads load the first row
+        const double *val = reinterpret_cast<const double *>(stage) + at;
+        const unsigned short *col = reinterpret_cast<const unsigned short *>(stage + col_at) + at;
+        const double2 bd = reinterpret_cast<const double2 *>(stage + val_bytes)[on ? I.x - x0 + t : 0];
+        // the previous set is complete, and its group when this set begins one
+        auto barrier = [&]() {
+            asm volatile("bar.sync 1, %0;" ::"n"(GS_ROWS) : "memory");
+            if (release && t == 0)
+                asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(smem_u32(release))
+                             : "memory");
+        };
+        double acc;
+        switch (Z) {   // the same for every thread
+        case 0: barrier(); acc = bd.x; break;
+        case 2: { GsRow<2> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+        case 4: { GsRow<4> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+        case 6: { GsRow<6> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+        case 8: { GsRow<8> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+        default: {
+            barrier();
+            acc = bd.x;
+            for (int u = 0; u < Z; u += 2) {
+                GsRow<2> r;
+                r.load(col + u, val + u);
+                acc = r.sum(ring, acc);
+            }
+        }
+        }
+        release = nullptr;
+        if (on) {
+            const int place = I.x + t;
+            double *px = ring + (I.z + t < A.ring ? I.z + t : I.z + t - A.ring);
+            if (KIND == 0) {
+                const double xn = acc * bd.y;
+                *px = xn;
+                A.x[place] = xn;
+            } else if (place != A.skip_place && fabs(bd.y) > double(SMALLREAL)) {
+                const double xn = KIND == 1 ? w * (acc / bd.y) + (1 - w) * *px : acc / bd.y;
+                *px = xn;
+                A.x[place] = xn;
+            }
+        }
+        if (++in_group == A.group) {
+            // what this group wrote to the ring comes before the copies that
+            // replace it
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            in_group = 0;
+            release = empty + k;
+            if (++k == A.stages) {
+                k = 0;
+                parity ^= 1u;
+            }
+        }
+    }
+}
+
+// vectors into the schedule's order (src: row of a place, -1 for padding)
+__global__ void k_gs_in(int places, const int *__restrict__ src, const double *__restrict__ b,
+                        const double *__restrict__ d, const double *__restrict__ x, double2 *bd,
+                        double *xp) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < places; q += gridDim.x * blockDim.x) {
+        const int i = src[q];
+        bd[q] = i >= 0 ? make_double2(b[i], d[i]) : make_double2(0.0, 0.0);
+        xp[q] = i >= 0 ? x[i] : 0.0;
+    }
+}
+__global__ void k_gs_out(int places, const int *__restrict__ src, const double *__restrict__ xp,
+                         double *x) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < places; q += gridDim.x * blockDim.x) {
+        const int i = src[q];
+        if (i >= 0) x[i] = xp[q];
+    }
+}
+
+// one CTA per set: its rows in ascending order to their places (neighbouring
+// rows lie side by side in the ring then), and the longest row without the
+// diagonal, made even
+__global__ void __launch_bounds__(GS_ROWS)
+k_gs_place(const int *__restrict__ rows, const int *__restrict__ set_ptr,
+           const int *__restrict__ start, const int *__restrict__ ia, const int *__restrict__ ja,
+           int *src, int *place, int *width) {
+    __shared__ int r[GS_ROWS], sh[32];
+    const int s = blockIdx.x, t = threadIdx.x;
+    const int q0 = set_ptr[s], m = set_ptr[s + 1] - q0;
+    const int i = t < m ? rows[q0 + t] : 0x7fffffff;
+    r[t] = i;
+    __syncthreads();
+    int len = 0;
+    if (t < m) {
+        int rank = 0;
+        for (int q = 0; q < m; ++q) rank += r[q] < i;
+        src[start[s] + rank] = i;
+        place[i] = start[s] + rank;
+        for (int k = ia[i]; k < ia[i + 1]; ++k) len += ja[k] != i;
+    }
+    len = block_max(len, sh);
+    if (t == 0) width[s] = (len + 1) / 2 * 2;
+}
+
+// the largest distance in places between a row and one of its columns
+__global__ void k_gs_dist(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+                          const int *__restrict__ place, int *dist) {
+    __shared__ int sh[32];
+    int m = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int p = place[i];
+        for (int k = ia[i]; k < ia[i + 1]; ++k) m = max(m, abs(place[ja[k]] - p));
+    }
+    m = block_max(m, sh);
+    if (threadIdx.x == 0) atomicMax(dist, m);
+}
+
+// one CTA per set: the entries row by row, zeros against the ring's zero place
+// behind a shorter row (subtracting +0.0 * 0.0 changes nothing)
+__global__ void __launch_bounds__(GS_ROWS)
+k_gs_fill(const int4 *__restrict__ info, int ring, const int *__restrict__ src,
+          const int *__restrict__ place, const int *__restrict__ ia, const int *__restrict__ ja,
+          const double *__restrict__ a, unsigned short *col, double *val) {
+    const int4 I = info[blockIdx.x];
+    const int t = threadIdx.x, Z = gs_width(I);
+    if (t >= gs_pitch(gs_rows(I))) return;
+    const int i = t < gs_rows(I) ? src[I.x + t] : -1;
+    col += I.w + t * Z;
+    val += I.w + t * Z;
+    int u = 0;
+    if (i >= 0)
+        for (int k = ia[i]; k < ia[i + 1]; ++k) {
+            const int j = ja[k];
+            if (j == i) continue;
+            col[u] = (unsigned short)(place[j] % ring);
+            val[u] = a[k];
+            ++u;
+        }
+    for (; u < Z; ++u) {
+        col[u] = (unsigned short)ring;
+        val[u] = 0.0;
+    }
+}
+
+}  // namespace
+
+void GsStream::release() {
+    dfree(info);
+    dfree(src);
+    dfree(place);
+    dfree(col);
+    dfree(val);
+    dfree(bd);
+    dfree(xp);
+    stages = 0;
+}
+
+int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
+    GsStream &G = sc->stream;
+    G.release();
+    const int n = A.n, ns = (int)sc->h_ptr.size() - 1;
+    // sets of at most a row per thread throughout, and few enough of them
+    if (ns < 1 || ns > GS_SETS) return SUCCESS;
+    std::vector<int> start(ns), width(ns);
+    int places = 0;
+    for (int k = 0; k < ns; ++k) {
+        const int m = sc->h_ptr[k + 1] - sc->h_ptr[k];
+        if (m > GS_ROWS) return SUCCESS;
+        start[k] = places;
+        places += gs_pitch(m);
+    }
+    places = (places + GS_BLOCK - 1) / GS_BLOCK * GS_BLOCK;
+    int *d_start = nullptr, *d_width = nullptr, dist = 0;
+    int rc = SUCCESS;
+    cudaError_t e = cudaSuccess;
+    auto done = [&](bool keep) {
+        dfree(d_start);
+        dfree(d_width);
+        if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; }
+        if (rc || !keep) G.release();
+        return rc;
+    };
+    if ((rc = dalloc(&d_start, ns)) || (rc = dalloc(&d_width, ns + 1)) ||
+        (rc = dalloc(&G.src, places)) || (rc = dalloc(&G.place, n)))
+        return done(false);
+    e = cudaMemcpyAsync(d_start, start.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(G.src, 0xff, sizeof(int) * places, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_width + ns, 0, sizeof(int), s);
+    if (e != cudaSuccess) return done(false);
+    k_gs_place<<<ns, GS_ROWS, 0, s>>>(sc->rows, sc->set_ptr, d_start, A.ia, A.ja, G.src, G.place,
+                                      d_width);
+    k_gs_dist<<<grid_for(n), 256, 0, s>>>(n, A.ia, A.ja, G.place, d_width + ns);
+    count_launch(2);
+    e = cudaMemcpyAsync(width.data(), d_width, sizeof(int) * ns, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&dist, d_width + ns, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return done(false);
+    std::vector<int4> info(ns);
+    long long ents = 0;
+    for (int k = 0; k < ns; ++k) {
+        const int m = sc->h_ptr[k + 1] - sc->h_ptr[k];
+        if (ents > (1LL << 30)) return done(false);
+        if (width[k] > 0x7fff) return done(false);
+        info[k] = int4{start[k], m | width[k] << 16, 0, (int)ents};
+        ents += (long long)width[k] * gs_pitch(m);
+    }
+    // Sets per stage and stages: large groups keep the copying warp ahead (it
+    // takes about 1 us a group), and the sets in flight have to cover the
+    // copies' latency (2 us, ten sets); the first choice that fits.  The ring
+    // spans the columns on both sides of the sets in flight.
+    static const int choice[][2] = {{8, 3}, {4, 4}, {4, 3}, {2, 6}, {2, 4}, {1, 8}, {1, 4}, {1, 3}, {1, 2}};
+    int ring = 0, stages = 0, group = 0, E = 0, R = 0;
+    for (const auto &c : choice) {
+        E = R = 0;
+        for (int k = 0; k < ns; k += c[0]) {
+            const int l = std::min(k + c[0], ns) - 1;
+            E = std::max(E, gs_end_entry(info[l]) - info[k].w);
+            R = std::max(R, gs_end_place(info[l]) - info[k].x);
+        }
+        const long long span = 2LL * dist + (long long)(c[1] + 1) * R + 2 * GS_BLOCK;
+        ring = (int)((std::min<long long>(span, places) + GS_BLOCK - 1) / GS_BLOCK * GS_BLOCK);
+        if (ring > 0xff00 || gs_smem(ns, E, R, ring, c[1]) > GS_SMEM) continue;
+        group = c[0];
+        stages = c[1];
+        break;
+    }
+    if (!stages) return done(false);
+    for (auto &I : info) I.z = I.x % ring;
+    if ((rc = dalloc(&G.info, ns)) || (rc = dalloc(&G.col, ents)) || (rc = dalloc(&G.val, ents)) ||
+        (rc = dalloc(&G.bd, places)) || (rc = dalloc(&G.xp, places)))
+        return done(false);
+    e = cudaMemcpyAsync(G.info, info.data(), sizeof(int4) * ns, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) {
+        k_gs_fill<<<ns, GS_ROWS, 0, s>>>(G.info, ring, G.src, G.place, A.ia, A.ja, A.val,
+                                         G.col, G.val);
+        count_launch();
+        e = cudaMemcpyAsync(&G.last_place, G.place + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // and the host arrays above
+    }
+    G.ns = ns;
+    G.group = group;
+    G.E = E;
+    G.R = R;
+    G.ring = ring;
+    G.stages = stages;
+    G.dist = dist;
+    G.places = places;
+    return done(true);
+}
+
+int gs_stream_sweep(const Schedule &sc, const double *d, const double *b, double *x,
+                    int kind, double w, int *err, cudaStream_t s) {
+    const GsStream &G = sc.stream;
+    const int skip_place = (kind & GS_SKIP_LAST) ? G.last_place : -1;   // SGS leaves row n - 1
+    auto kernel = (kind & 15) == 0 ? k_gs_stream<0> : (kind & 15) == 1 ? k_gs_stream<1> : k_gs_stream<2>;
+    HZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)GS_SMEM));
+    k_gs_in<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, b, d, x, G.bd, G.xp);
+    const GsSweep A = {G.info, G.col, G.val, G.bd, G.xp, G.ns, G.group, G.E, G.R, G.stages,
+                       G.ring, G.dist, G.places, skip_place};
+    kernel<<<1, GS_ROWS + 32, gs_smem(G.ns, G.E, G.R, G.ring, G.stages), s>>>(A, w, err);
+    k_gs_out<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, G.xp, x);
+    count_launch(3);
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
+
+}  // namespace hzb

@@ -1361,6 +1361,7 @@ void Schedule::release() {
     dfree(rows);
     dfree(set_ptr);
     dfree(bar);
+    stream.release();
     h_ptr.clear();
     run_first.clear();
     run_last.clear();
@@ -1387,17 +1388,17 @@ __global__ void k_transpose_fill(int n, const int *__restrict__ ia,
 // dependency count: neighbours that come earlier in the sweep
 __global__ void k_indeg(int n, const int *__restrict__ ia, const int *__restrict__ ja,
                         const int *__restrict__ tia, const int *__restrict__ tja,
-                        int backward, int *indeg, int *rows, int *tail) {
+                        int *indeg, int *rows, int *tail) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         int c = 0;
         for (int k = ia[i]; k < ia[i + 1]; ++k) {
             const int j = ja[k];
-            c += backward ? (j > i) : (j < i);
+            c += j < i;
         }
         for (int k = tia[i]; k < tia[i + 1]; ++k) {
             const int j = tja[k];
-            c += backward ? (j > i) : (j < i);
+            c += j < i;
         }
         indeg[i] = c;
         atomicMax(tail + 1, c);
@@ -1407,19 +1408,19 @@ __global__ void k_indeg(int n, const int *__restrict__ ia, const int *__restrict
 
 __global__ void k_kahn_round(int head, int cnt, const int *__restrict__ ia,
                              const int *__restrict__ ja, const int *__restrict__ tia,
-                             const int *__restrict__ tja, int backward, int *indeg,
+                             const int *__restrict__ tja, int *indeg,
                              int *rows, int *tail) {
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt;
          q += gridDim.x * blockDim.x) {
         const int i = rows[head + q];
         for (int k = ia[i]; k < ia[i + 1]; ++k) {
             const int j = ja[k];
-            if (backward ? (j < i) : (j > i))
+            if (j > i)
                 if (atomicSub(indeg + j, 1) == 1) rows[atomicAdd(tail, 1)] = j;
         }
         for (int k = tia[i]; k < tia[i + 1]; ++k) {
             const int j = tja[k];
-            if (backward ? (j < i) : (j > i))
+            if (j > i)
                 if (atomicSub(indeg + j, 1) == 1) rows[atomicAdd(tail, 1)] = j;
         }
     }
@@ -1434,7 +1435,7 @@ __global__ void k_kahn_round(int head, int cnt, const int *__restrict__ ia,
 constexpr int KAHN_CTA_MAX_ROWS = 1 << 20;
 __global__ void __launch_bounds__(1024)
 k_kahn_all(int n, const int *__restrict__ ia, const int *__restrict__ ja,
-           const int *__restrict__ tia, const int *__restrict__ tja, int backward,
+           const int *__restrict__ tia, const int *__restrict__ tja,
            int *indeg, int *rows, const int *__restrict__ tail0, int *ptr, int *nsets) {
     __shared__ int s_tail, s_head, s_cur, s_ns;
     if (threadIdx.x == 0) {
@@ -1453,12 +1454,12 @@ k_kahn_all(int n, const int *__restrict__ ia, const int *__restrict__ ja,
             const int i = rows[q];
             for (int k = ia[i]; k < ia[i + 1]; ++k) {
                 const int j = ja[k];
-                if (backward ? (j < i) : (j > i))
+                if (j > i)
                     if (atomicSub(indeg + j, 1) == 1) rows[atomicAdd(&s_tail, 1)] = j;
             }
             for (int k = tia[i]; k < tia[i + 1]; ++k) {
                 const int j = tja[k];
-                if (backward ? (j < i) : (j > i))
+                if (j > i)
                     if (atomicSub(indeg + j, 1) == 1) rows[atomicAdd(&s_tail, 1)] = j;
             }
         }
@@ -1493,7 +1494,7 @@ constexpr size_t kahn_smem_bytes(int n) {
 }
 __global__ void __launch_bounds__(1024)
 k_kahn_smem(int n, const int *__restrict__ ia, const int *__restrict__ ja,
-            const int *__restrict__ tia, const int *__restrict__ tja, int backward,
+            const int *__restrict__ tia, const int *__restrict__ tja,
             const int *__restrict__ indeg, int *rows, const int *__restrict__ tail0, int *ptr,
             int *nsets) {
     extern __shared__ unsigned kahn_sm[];
@@ -1538,7 +1539,7 @@ k_kahn_smem(int n, const int *__restrict__ ia, const int *__restrict__ ja,
                 for (int u = 0; u < 8; ++u) c[u] = k0 + u < k1 ? xj[k0 + u] : -1;
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
-                    if (c[u] >= 0 && (backward ? (c[u] < i) : (c[u] > i))) release(c[u]);
+                    if (c[u] >= 0 && c[u] > i) release(c[u]);
             }
         };
         for (int q = head + threadIdx.x; q < cur; q += blockDim.x) {
@@ -1584,7 +1585,7 @@ static void make_runs(Schedule *sch) {
     }
 }
 
-int gs_schedule(int n, const int *ia, const int *ja, int nnz, int backward,
+int gs_schedule(int n, const int *ia, const int *ja, int nnz,
                 Schedule *sch, cudaStream_t s) {
     sch->release();
     int *tia = nullptr, *tja = nullptr, *fillc = nullptr, *indeg = nullptr;
@@ -1607,7 +1608,7 @@ int gs_schedule(int n, const int *ia, const int *ja, int nnz, int backward,
     if ((rc = scan_exclusive(fillc, tia, n, tmp, s))) goto done;
     cudaMemsetAsync(fillc, 0, sizeof(int) * n, s);
     k_transpose_fill<<<g, 256, 0, s>>>(n, ia, ja, tia, fillc, tja);
-    k_indeg<<<g, 256, 0, s>>>(n, ia, ja, tia, tja, backward, indeg, sch->rows, tail);
+    k_indeg<<<g, 256, 0, s>>>(n, ia, ja, tia, tja, indeg, sch->rows, tail);
     count_launch(2);
     if (n <= KAHN_CTA_MAX_ROWS) {
         // one CTA runs every round; set boundaries and counts come back once
@@ -1633,10 +1634,10 @@ int gs_schedule(int n, const int *ia, const int *ja, int nnz, int backward,
                                      (int)kahn_smem_bytes(KAHN_SMEM_ROWS));
                 attr = true;
             }
-            k_kahn_smem<<<1, 1024, kahn_smem_bytes(n), s>>>(n, ia, ja, tia, tja, backward,
+            k_kahn_smem<<<1, 1024, kahn_smem_bytes(n), s>>>(n, ia, ja, tia, tja,
                                                             indeg, sch->rows, tail, dptr, dns);
         } else {
-            k_kahn_all<<<1, 1024, 0, s>>>(n, ia, ja, tia, tja, backward, indeg, sch->rows,
+            k_kahn_all<<<1, 1024, 0, s>>>(n, ia, ja, tia, tja, indeg, sch->rows,
                                           tail, dptr, dns);
         }
         count_launch();
@@ -1667,7 +1668,7 @@ int gs_schedule(int n, const int *ia, const int *ja, int nnz, int backward,
             ptr.push_back(cur);
             const int cnt = cur - head;
             k_kahn_round<<<grid_for(cnt), 256, 0, s>>>(head, cnt, ia, ja, tia, tja,
-                                                       backward, indeg, sch->rows, tail);
+                                                       indeg, sch->rows, tail);
             count_launch();
             head = cur;
             e = cudaMemcpyAsync(&cur, tail, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -1696,6 +1697,37 @@ done:
     dfree(tia); dfree(tja); dfree(fillc); dfree(indeg); dfree(tail); dfree(tmp);
     if (rc) sch->release();
     return rc;
+}
+
+__global__ void k_reverse(int n, const int *__restrict__ in, int *out) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+        out[q] = in[n - 1 - q];
+}
+
+int gs_schedule_reverse(const Schedule &f, int n, Schedule *sch, cudaStream_t s) {
+    sch->release();
+    const int ns = (int)f.h_ptr.size() - 1;
+    std::vector<int> ptr(ns + 1);
+    for (int k = 0; k <= ns; ++k) ptr[k] = n - f.h_ptr[ns - k];
+    int rc = SUCCESS;
+    if (!(rc = dalloc(&sch->rows, n)) && !(rc = dalloc(&sch->bar, 2)) &&
+        !(rc = dalloc(&sch->set_ptr, ptr.size()))) {
+        k_reverse<<<grid_for(n), 256, 0, s>>>(n, f.rows, sch->rows);
+        count_launch();
+        cudaError_t e = cudaMemsetAsync(sch->bar, 0, 2 * sizeof(unsigned), s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(sch->set_ptr, ptr.data(), sizeof(int) * ptr.size(),
+                                cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; }
+    }
+    if (rc) {
+        sch->release();
+        return rc;
+    }
+    sch->h_ptr = ptr;
+    make_runs(sch);
+    return SUCCESS;
 }
 
 // ---------------------------------------------------------------------------

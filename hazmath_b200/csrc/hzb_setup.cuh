@@ -78,8 +78,20 @@ int smoother_diagonals(const DCsr<double> &A, double *d_jac, double *d_gs_f,
                        cudaStream_t s);
 
 // Level schedule of lexicographic Gauss-Seidel: rows grouped into sets that
-// depend only on earlier sets (forward: on lower-numbered neighbours in A or
-// A^T; backward: higher).  perm (n) and host set pointers.
+// depend only on earlier sets (on lower-numbered neighbours in A or A^T; the
+// backward sweep takes the sets in reverse).  perm (n) and host set pointers.
+// (stream: its rows again in the schedule's order, when every set is small,
+// hzb_gs.cu)
+struct GsStream {
+    int ns = 0, group = 0, E = 0, R = 0, ring = 0, stages = 0;   // stages 0: no stream
+    int dist = 0, places = 0, last_place = 0;
+    int4 *info = nullptr;
+    int *src = nullptr, *place = nullptr;             // row of a place, place of a row
+    unsigned short *col = nullptr;
+    double *val = nullptr, *xp = nullptr;
+    double2 *bd = nullptr;                            // b and the diagonal of a place
+    void release();
+};
 struct Schedule {
     int *rows = nullptr;           // device, n
     int *set_ptr = nullptr;        // device, nsets+1
@@ -88,10 +100,22 @@ struct Schedule {
     std::vector<int> run_last;     // (-1: one large set)
     std::vector<int> run_max;      // the run's largest set
     unsigned *bar = nullptr;       // device, 2 words: grid barrier of gs_sets_grid
+    GsStream stream;
     void release();
 };
-int gs_schedule(int n, const int *ia, const int *ja, int nnz, int backward,
+// The stream of a schedule, for A's values (none when a set is too large), and
+// a sweep of it (kinds as gs_rows', x in place; err: raised if a copy never
+// arrives).
+int gs_stream_build(const DCsr<double> &A, Schedule *sch, cudaStream_t s);
+int gs_stream_sweep(const Schedule &sch, const double *d, const double *b, double *x, int kind,
+                    double w, int *err, cudaStream_t s);
+int gs_schedule(int n, const int *ia, const int *ja, int nnz,
                 Schedule *sch, cudaStream_t s);
+// The schedule of the opposite sweep: the sets in reverse order.  A row comes
+// after its lower neighbours (in A or A^T) in one, so it comes after the higher
+// ones in the other; building it anew took as long as the first (1.3 ms for the
+// 509 sets of a 2D 255^2 level).
+int gs_schedule_reverse(const Schedule &f, int n, Schedule *sch, cudaStream_t s);
 // Colour classes (Jones-Plassmann with hashed priorities, smallest free
 // colour): rows sorted by colour, host colour pointers.
 int multicolor(int n, const int *ia, const int *ja, Schedule *sch,

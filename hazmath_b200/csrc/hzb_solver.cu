@@ -219,6 +219,8 @@ static int run_sets(hzb_solver *S, const DCsr<double> &A, const Schedule &sc,
         return !(e && e[0] == '0');
     }();
     int *err = grid_ok ? wait_err(S) : nullptr;
+    if (!reverse && sc.stream.stages && wait_err(S))
+        return gs_stream_sweep(sc, d, b, x, kind, w, wait_err(S), S->s);
     if (!reverse) {
         const size_t nr = sc.run_first.size();
         for (size_t q = 0; q < nr; ++q) {
@@ -687,8 +689,10 @@ int level_smoother_data(hzb_solver *S, Level &L) {
         if (S->bp.gs_schedule == HZB_GS_MULTICOLOR) {
             HZB_TRY(multicolor(L.n, L.ia, L.ja, &L.col, S->s));
         } else {
-            HZB_TRY(gs_schedule(L.n, L.ia, L.ja, L.nnz, 0, &L.fwd, S->s));
-            HZB_TRY(gs_schedule(L.n, L.ia, L.ja, L.nnz, 1, &L.bwd, S->s));
+            HZB_TRY(gs_schedule(L.n, L.ia, L.ja, L.nnz, &L.fwd, S->s));
+            HZB_TRY(gs_schedule_reverse(L.fwd, L.n, &L.bwd, S->s));
+            HZB_TRY(gs_stream_build(L.A64(), &L.fwd, S->s));
+            HZB_TRY(gs_stream_build(L.A64(), &L.bwd, S->s));
         }
     }
     return SUCCESS;

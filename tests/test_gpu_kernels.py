@@ -227,3 +227,43 @@ def test_rap_row_sizes_bit_exact(n, lens, members):
         got.append(a)
     assert np.array_equal(got[0], cia) and np.array_equal(got[1], cja)
     assert np.array_equal(got[2].view(np.int64), cval.view(np.int64))
+
+
+def _wide(n, seed):
+    """Rows of 0 to 40 off-diagonal entries to both sides, unsorted, the
+    diagonal anywhere."""
+    rng = np.random.default_rng(seed)
+    ia, ja, val = [0], [], []
+    for i in range(n):
+        c = rng.choice(n, size=min(n, int(rng.integers(0, 41))), replace=False)
+        c = rng.permutation(np.r_[c[c != i], i])
+        ja.extend(c)
+        val.extend(np.where(c == i, 60.0, rng.uniform(-1.0, 1.0, len(c))))
+        ia.append(len(ja))
+    return np.array(ia, np.int32), np.array(ja, np.int32), np.array(val)
+
+
+GS_PROBLEMS = {
+    "one_row": lambda: P.poisson2d_5pt(1),
+    "2d_16": lambda: P.poisson2d_5pt(16),
+    "2d_256": lambda: P.poisson2d_5pt(256),      # sets of up to 256 rows: the last that stream
+    "2d_257": lambda: P.poisson2d_5pt(257),      # runs of sets in the row kernels
+    "aniso_61": lambda: P.aniso2d_p1(61, 0.1, 0.5),
+    "kuhn_17": lambda: P.kuhn3d_p1(17, P.lognormal_field(17, 1.0, 4.0, 7)),
+    "wide_300": lambda: _wide(300, 5),
+}
+
+
+@pytest.mark.parametrize("name", sorted(GS_PROBLEMS))
+@pytest.mark.parametrize("sm,pre", [(2, 1), (2, 0), (3, 1), (5, 1), (5, 0), (6, 1)])
+def test_streamed_gauss_seidel_vs_oracle(port, name, sm, pre):
+    """GS, SGS (which leaves the last row out of its way back), SOR and SSOR on
+    schedules with small sets, both directions, several sweeps."""
+    ia, ja, val = GS_PROBLEMS[name]()
+    n = len(ia) - 1
+    rng = np.random.default_rng(n + sm)
+    b, x0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    A = DevCSR(ia, ja, val)
+    x = dev(x0)
+    assert hz.lib().hzb_smoother_device(sm, pre, 2, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
+    assert np.array_equal(host(x), port.smooth(sm, pre, 2, ia, ja, val, b, x0, relax=1.15))
