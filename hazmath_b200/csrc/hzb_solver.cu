@@ -754,6 +754,7 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
     S->g32.release();
     S->g32c.release();
     S->gcyc.release();
+    S->gcoarse.release();
     S->gbsr.release();
     gmres_release(S);
     gcg_release(S);
@@ -1421,6 +1422,7 @@ void destroy(hzb_solver *S) {
     S->g32.release();
     S->g32c.release();
     S->gcyc.release();
+    S->gcoarse.release();
     S->gbsr.release();
     gmres_release(S);
     gcg_release(S);

@@ -153,6 +153,7 @@ struct hzb_solver {
     hzb::GraphCache g64, g32;         // captured FP64 / FP32 preconditioners
     hzb::GraphCache g32c;             // the FP32 cycles alone (level-0 b32 given)
     hzb::GraphCache gcyc;             // captured AMLI / additive preconditioner
+    hzb::GraphCache gcoarse;          // captured cycle on the levels below 0 (training)
     hzb::GraphCache gbsr;             // captured block (BSR) preconditioner
     std::vector<double> amli_coef;    // polynomial of the AMLI cycle (degree + 1)
     // Krylov work kept per level for the coarse-level solves of the
