@@ -294,64 +294,117 @@ __global__ void k_bat_activity(int nlev, int nblk_all, const int *__restrict__ b
 
 static int bat_grid(int nitems) { return std::max(1, std::min(nitems, sm_count() * 8)); }
 
-// rows of every system on a level
+// Rows of every system on a level.  A system's rows are consecutive, so only
+// its first and last row count (one atomic a row, all of a warp's on one word,
+// took 0.7 ms of the setup of 48 systems).
 __global__ void k_bat_count(int n, const int *__restrict__ sys, int *cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        atomicAdd(cnt + sys[i], 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int k = sys[i];
+        if (i == 0 || sys[i - 1] != k) atomicSub(cnt + k, i);
+        if (i == n - 1 || sys[i + 1] != k) atomicAdd(cnt + k, i + 1);
+    }
 }
 
-// Dense inverse of each terminal block (one CTA per block, the block in
-// shared memory): the block's CSR rows [row0, row0 + m) scattered into an
-// m x m matrix (its columns lie in the same range: systems do not couple),
-// then Gauss-Jordan elimination in place without pivoting (the block is
-// SPD): for each k the pivot row is scaled by 1 / a_kk with a_kk replaced by
-// 1, and every other row subtracts its column-k multiple of it with its
-// column-k entry replaced by 0; after m steps the array holds the inverse.
+// Dense inverse of each terminal block: the block's CSR rows [row0, row0 + m)
+// scattered into an m x m matrix (its columns lie in the same range: systems do
+// not couple), then Gauss-Jordan elimination in place without pivoting (the
+// block is SPD): for each k the pivot row is scaled by 1 / a_kk with a_kk
+// replaced by 1, and every other row subtracts its column-k multiple of it with
+// its column-k entry replaced by 0; after m steps the array holds the inverse.
 // A pivot that is not positive and finite sets *bad.
-__global__ void __launch_bounds__(256)
+//   One CTA per block, a warp per 4 rows (i, i + 32, ..) and a lane per 4
+// columns, the matrix in registers: a step exchanges the pivot row, which one
+// warp holds and divides, and column k through two buffers in shared memory,
+// with one barrier.  With the matrix in shared memory a step moved all of it
+// through the 128 bytes a clock (6 us a step, 0.77 ms for 128 rows; 0.28 now,
+// half of it the row's division, which the other warps wait for).
+constexpr int TERM_SPLIT = 8;
+constexpr int TERM_Q = (BAT_TERM_ROWS + 31) / 32;
+__global__ void __launch_bounds__(1024)
 k_bat_term_inverse(int nblk, const int *__restrict__ row0, const int *__restrict__ msz,
                    const long long *__restrict__ off, const int *__restrict__ ia,
                    const int *__restrict__ ja, const double *__restrict__ val,
                    double *inv, float *inv32, int *bad) {
-    extern __shared__ double sa[];
+    extern __shared__ double sa[];           // m x m, row-major, to scatter into
+    __shared__ double pivot_row[2][BAT_TERM_ROWS], col[2][BAT_TERM_ROWS];
+    __shared__ int s_ok[2];
     const int blk = blockIdx.x;
     if (blk >= nblk) return;
     const int m = msz[blk], r0 = row0[blk];
-    double *A = sa;               // m x m, row-major
-    double *colk = sa + m * m;    // column k before the step
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) A[q] = 0.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int q = threadIdx.x; q < m * m; q += blockDim.x) sa[q] = 0.0;
     __syncthreads();
     for (int i = threadIdx.x; i < m; i += blockDim.x)
         for (int p = ia[r0 + i]; p < ia[r0 + i + 1]; ++p) {
             const int j = ja[p] - r0;
-            if (j >= 0 && j < m) A[i * m + j] += val[p];
+            if (j >= 0 && j < m) sa[i * m + j] += val[p];
         }
-    bool ok = true;
-    for (int k = 0; k < m; ++k) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < m; i += blockDim.x) colk[i] = A[i * m + k];
-        __syncthreads();
-        const double piv = colk[k];
-        if (!(piv > 0.0) || !isfinite(piv)) { ok = false; break; }
-        for (int j = threadIdx.x; j < m; j += blockDim.x)
-            A[k * m + j] = (j == k ? 1.0 : A[k * m + j]) / piv;
-        __syncthreads();
-        for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-            const int i = q / m, j = q - i * m;
-            if (i != k) A[q] = (j == k ? 0.0 : A[q]) - colk[i] * A[k * m + j];
-        }
-    }
-    if (!ok) {
-        if (threadIdx.x == 0) atomicOr(bad, 1);
-        return;
-    }
     __syncthreads();
+    double A[TERM_Q][TERM_Q];
+#pragma unroll
+    for (int a = 0; a < TERM_Q; ++a)
+#pragma unroll
+        for (int b = 0; b < TERM_Q; ++b) {
+            const int i = warp + 32 * a, j = lane + 32 * b;
+            A[a][b] = i < m && j < m ? sa[i * m + j] : 0.0;
+        }
+    for (int k = 0; k < m; ++k) {
+        double *pr = pivot_row[k & 1], *ck = col[k & 1];
+        const int kw = k & 31, kq = k >> 5;
+        if (lane == kw) {
+#pragma unroll
+            for (int a = 0; a < TERM_Q; ++a)
+#pragma unroll
+                for (int b = 0; b < TERM_Q; ++b)
+                    if (b == kq) ck[warp + 32 * a] = A[a][b];
+        }
+        if (warp == kw) {
+            double row[TERM_Q], piv = 0.0;
+#pragma unroll
+            for (int a = 0; a < TERM_Q; ++a)
+#pragma unroll
+                for (int b = 0; b < TERM_Q; ++b)
+                    if (a == kq) {
+                        row[b] = A[a][b];
+                        if (b == kq) piv = A[a][b];
+                    }
+            piv = __shfl_sync(0xffffffffu, piv, kw);
+            if (lane == 0) s_ok[k & 1] = (piv > 0.0) && isfinite(piv);
+#pragma unroll
+            for (int b = 0; b < TERM_Q; ++b)
+                pr[lane + 32 * b] = (lane + 32 * b == k ? 1.0 : row[b]) / piv;
+        }
+        __syncthreads();
+        if (!s_ok[k & 1]) {
+            if (threadIdx.x == 0) atomicOr(bad, 1);
+            return;
+        }
+        double rj[TERM_Q];
+#pragma unroll
+        for (int b = 0; b < TERM_Q; ++b) rj[b] = pr[lane + 32 * b];
+#pragma unroll
+        for (int a = 0; a < TERM_Q; ++a) {
+            const int i = warp + 32 * a;
+            const double c = ck[i];
+#pragma unroll
+            for (int b = 0; b < TERM_Q; ++b) {
+                if (i == k) A[a][b] = rj[b];
+                else A[a][b] = (lane + 32 * b == k ? 0.0 : A[a][b]) - c * rj[b];
+            }
+        }
+    }
     double *out = inv + off[blk];
     float *out32 = inv32 + off[blk];
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-        out[q] = A[q];
-        out32[q] = (float)A[q];
-    }
+#pragma unroll
+    for (int a = 0; a < TERM_Q; ++a)
+#pragma unroll
+        for (int b = 0; b < TERM_Q; ++b) {
+            const int i = warp + 32 * a, j = lane + 32 * b;
+            if (i < m && j < m) {
+                out[i * m + j] = A[a][b];
+                out32[i * m + j] = (float)A[a][b];
+            }
+        }
 }
 
 // x = inverse * b on every terminal block of a level (one CTA per block, a
@@ -367,9 +420,12 @@ k_bat_term_solve(int nblk, const int *__restrict__ row0, const int *__restrict__
     for (int j = threadIdx.x; j < m; j += blockDim.x) sb[j] = b[r0 + j];
     __syncthreads();
     const V *M = inv + off[blk];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int i = warp; i < m; i += nw) {
+    // TERM_SPLIT CTAs share a block's rows: one CTA's warps took 16 rows each,
+    // one after the other (14.5 us a launch; 4 now)
+    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * gridDim.y;
+    for (int i = (threadIdx.x >> 5) + (blockDim.x >> 5) * blockIdx.y; i < m; i += nw) {
         T acc = T(0);
+#pragma unroll 4
         for (int j = lane; j < m; j += 32) acc += T(M[(size_t)i * m + j]) * sb[j];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -474,15 +530,14 @@ int batch_level_begin(hzb_solver *S, int lvl, bool force, int *live) {
     HZB_CUDA(cudaMemcpyAsync(B.tl_off[lvl], off.data(), sizeof(long long) * nb,
                              cudaMemcpyHostToDevice, s));
     HZB_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
-    const size_t smem = sizeof(double) * ((size_t)mmax * mmax + mmax);
+    const size_t smem = sizeof(double) * (size_t)mmax * mmax;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_bat_term_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(double) * (BAT_TERM_ROWS * BAT_TERM_ROWS +
-                                                     BAT_TERM_ROWS)));
+                             (int)(sizeof(double) * BAT_TERM_ROWS * BAT_TERM_ROWS));
         attr = true;
     }
-    k_bat_term_inverse<<<nb, 256, smem, s>>>(nb, B.tl_row0[lvl], B.tl_m[lvl], B.tl_off[lvl],
+    k_bat_term_inverse<<<nb, 1024, smem, s>>>(nb, B.tl_row0[lvl], B.tl_m[lvl], B.tl_off[lvl],
                                              L.ia, L.ja, L.val, B.tl_inv[lvl],
                                              B.tl_inv32[lvl], bad);
     count_launch();
@@ -543,11 +598,11 @@ int batch_terminal_solve(hzb_solver *S, int lvl, bool fp32) {
     if (lvl >= (int)B.tl_n.size() || B.tl_n[lvl] == 0) return SUCCESS;
     const Level &L = S->lv[lvl];
     if (fp32)
-        k_bat_term_solve<float, float><<<B.tl_n[lvl], 256, 0, S->s>>>(
+        k_bat_term_solve<float, float><<<dim3(B.tl_n[lvl], TERM_SPLIT), 256, 0, S->s>>>(
             B.tl_n[lvl], B.tl_row0[lvl], B.tl_m[lvl], B.tl_off[lvl], B.tl_inv32[lvl], L.b32,
             L.x32);
     else
-        k_bat_term_solve<double, double><<<B.tl_n[lvl], 256, 0, S->s>>>(
+        k_bat_term_solve<double, double><<<dim3(B.tl_n[lvl], TERM_SPLIT), 256, 0, S->s>>>(
             B.tl_n[lvl], B.tl_row0[lvl], B.tl_m[lvl], B.tl_off[lvl], B.tl_inv[lvl], L.b, L.x);
     count_launch();
     HZB_LAUNCH_CHECK();

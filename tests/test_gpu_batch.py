@@ -122,6 +122,37 @@ def test_batch_rejects_coupled_systems():
     assert rc == hz.ERROR_INPUT_PAR
 
 
+@pytest.mark.parametrize("prec,max_it", [("mixed", 3), ("fp64", 1)])
+def test_batch_terminal_block_sizes(prec, max_it):
+    """Systems small enough to be dense blocks from the start (each size at an
+    edge of the 32-wide register tiles, up to the largest block): 4.5 on the
+    diagonal and -1 at the distances 1 and 7, so the condition number is at
+    most 8.5 / 0.5 and the block's inverse solves the system at once in FP64;
+    in FP32 its relative error is about 1e-6 a cycle, so two or three reach
+    1e-8."""
+    rng = np.random.default_rng(3)
+    mats, rhs = [], []
+    for m in (1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128):
+        A = sp.diags([np.full(m, 4.5)], [0]).tolil()
+        for d in (1, 7):
+            if d < m:
+                A += sp.diags([-np.ones(m - d), -np.ones(m - d)], [d, -d])
+        mats.append(sp.csr_matrix(A))
+        rhs.append(rng.uniform(-1.0, 1.0, m))
+    U = sp.block_diag(mats, format="csr")
+    U.sort_indices()
+    off = np.cumsum([0] + [len(b) for b in rhs]).astype(np.int32)
+    p = hz.HZB_PREC_MIXED if prec == "mixed" else hz.HZB_PREC_FP64
+    rc, its, rel, sec, x, _ = _batch_solve(
+        (off, U.indptr.astype(np.int32), U.indices.astype(np.int32), U.data,
+         np.concatenate(rhs)), p)
+    assert rc > 0, hz.last_error()
+    assert its.max() <= max_it
+    for k, (A, b) in enumerate(zip(mats, rhs)):
+        want = np.linalg.solve(A.toarray(), b)
+        assert np.linalg.norm(x[off[k]:off[k + 1]] - want) <= 1e-6 * np.linalg.norm(want), k
+
+
 def test_batch_against_reference_per_system(golden):
     """Each of the 24 systems solved by the batch (FP32 cycle, parallel
     matching, per-system flexible CG to 1e-8) against the same system solved
