@@ -9,21 +9,30 @@
 
 namespace hzb {
 
-// FP32 sliced-ELL copy of a level's matrix (hzb_sell.cu): slot r of a
-// 256-row window holds row row[r] (-1: none) of len[r] entries, stored at
-// col/val[ptr[r / 32] + 32 u + r % 32]; npad = 0: none.
+// Sliced-ELL copy of a matrix (hzb_sell.cu): slot r of a 256-row window holds
+// one row, slot[r] its index in the window and, above 8 bits, its length;
+// head[r / 32] where its slice's entries, columns and bases begin and its width,
+// base the smallest columns of a pair's two entries; npad = 0: none.
+template <typename T>
 struct SellView {
     int npad = 0;
-    const int *ptr = nullptr, *row = nullptr, *len = nullptr, *col = nullptr;
-    const float *val = nullptr;
+    const unsigned *slot = nullptr;
+    const unsigned short *col = nullptr;
+    const int4 *head = nullptr;
+    const int2 *base = nullptr;
+    const T *val = nullptr;
 };
+template <typename T>
 struct SellArrays {
     int npad = 0;
-    int *ptr = nullptr, *row = nullptr, *len = nullptr, *col = nullptr;
-    float *val = nullptr;
-    SellView view() const {
-        SellView v;
-        v.npad = npad; v.ptr = ptr; v.row = row; v.len = len; v.col = col; v.val = val;
+    unsigned *slot = nullptr;
+    unsigned short *col = nullptr;
+    int4 *head = nullptr;
+    int2 *base = nullptr;
+    T *val = nullptr;
+    SellView<T> view() const {
+        SellView<T> v;
+        v.npad = npad; v.slot = slot; v.col = col; v.head = head; v.base = base; v.val = val;
         return v;
     }
     void release();
@@ -42,7 +51,7 @@ struct DCsr {
     // partial sums are combined across its lanes, so the lanes kernels do
     // not give the sequential CSR-order sum of the FP64 kernels.
     int vec_lanes = 0;
-    SellView sell;
+    SellView<T> sell;
     // Optional activity of 256-row blocks (ACT_ROWS): kernels skip the rows
     // of a block whose byte is 0 (batched solves skip converged systems).
     const unsigned char *act = nullptr;
@@ -67,10 +76,11 @@ int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cud
 // shape, if any
 bool fp32_schedule_known(int n, int nnz, int *lanes);
 
-// Sliced-ELL copy of an FP32 CSR matrix (hzb_sell.cu); *out stays empty
+// Sliced-ELL copy of a CSR matrix (hzb_sell.cu); *out stays empty
 // (npad 0) when its slice offsets would overflow int.  Sweep and SpMV on it
 // (no activity array, no SPMV_Y_DOT).
-int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
+template <typename T>
+int sell_build(int n, const int *ia, const int *ja, const T *a, SellArrays<T> *out,
                cudaStream_t s);
 int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
                   const float *omega, cudaStream_t s);

@@ -1,138 +1,225 @@
-// hzb_sell.cu -- the FP32 cycle's sliced-ELL schedule.
+// hzb_sell.cu -- the sliced-ELL schedule.
 //
-// A level's FP32 matrix is also kept as 32-row slices stored column-major:
-// entry u of the row in slot r of slice s sits at col/val[ptr[s] + 32 u +
-// (r mod 32)], so the 32 threads of a warp, one row each, read entry u of
-// their 32 rows as one coalesced 128-byte line -- no shared-memory staging
-// (full occupancy) and no lanes to combine.  A slice is as wide as its
-// longest row; rows are ordered by length (descending, ties by index)
-// inside each 256-row window, so the rows of a slice have nearly equal
-// lengths, and a thread stops at its own row's length, so the padding is
-// never read.  Each row's entries keep their CSR order and one thread sums
-// them in that order.  For the FP32 cycle, where it competes with the staged
-// bundles and the lanes-per-row kernels in the per-level autotuner.
+// A matrix is also kept as 32-row slices, each as wide as its longest row; rows
+// are ordered by length (descending, ties by index) inside each 256-row window,
+// so the rows of a slice have nearly equal lengths.  Entries 2p and 2p + 1 of a
+// row lie side by side, at val[32 (first + 2p) + 2 (slot mod 32)], the last of
+// an odd width alone in its line of 32, so the threads of a warp, one row each,
+// read their entries with coalesced loads -- no shared-memory staging (full
+// occupancy) and no lanes to combine.  Each row's entries keep their CSR order
+// and one thread sums them in that order; a row shorter than its slice adds
+// zeros times its own last column's x.
+//   The sweeps are bound by the memory, so what counts is the bytes of an
+// entry: its column is held in 16 bits above the smallest column of its slice
+// at its position (base, the same words for the whole warp), which covers any
+// matrix whose neighbouring rows reach to similar places; a slice where some
+// range is wider keeps 32-bit columns.  A row's index and length share a word.
+// 6 bytes an FP32 entry instead of 8, and no test per entry: 222 -> 185 us a
+// sweep of 16.6 million rows of up to 7 entries, 150 -> 131 on the next level.
+// All 64 warps of an SM have to run for it (32 registers; 221 us with 48 of them);
+// fetching entries into L2 some waves ahead gave nothing, several windows a CTA 4 %
+// here and a loss on smaller levels.
 #include "hzb_setup.cuh"
 #include <climits>
+#include <type_traits>
 
 namespace hzb {
 
 namespace {
 constexpr int SELL_WIN = 256;   // rows sorted together (one CTA)
 constexpr int SELL_C = 32;      // rows per slice
+constexpr unsigned SELL_ROW = SELL_WIN - 1;   // a slot's row within its window; the length above
+
+template <typename T> struct SellPair;
+template <> struct SellPair<float> { using type = float2; };
+template <> struct SellPair<double> { using type = double2; };
 
 // One CTA per window: slot of each row by its rank (longer first, then by
-// index), the slice widths (the first slot of a slice holds its longest
-// row), and the slot -> row map (-1 past n).
+// index; rows past n last) and, a warp per slice, its width (the first slot
+// holds the longest row), half of it rounded up, and the lines of 64 bytes of
+// its columns: the width, or twice that where a position's columns span more
+// than 16 bits.
 __global__ void __launch_bounds__(SELL_WIN)
-k_sell_order(int n, const int *__restrict__ ia, int *srow, int *slen, int *width32,
-             unsigned long long *total) {
-    __shared__ int len[SELL_WIN];
-    const int t = threadIdx.x;
-    const int i = blockIdx.x * SELL_WIN + t;
+k_sell_order(int n, const int *__restrict__ ia, const int *__restrict__ ja, unsigned *slot,
+             int *width, int *pairs, int *lines, unsigned long long *total) {
+    __shared__ int len[SELL_WIN], row[SELL_WIN], sum[3];
+    const int t = threadIdx.x, w0 = blockIdx.x * SELL_WIN;
+    const int i = w0 + t;
     const int li = i < n ? ia[i + 1] - ia[i] : -1;
     len[t] = li;
+    if (t < 3) sum[t] = 0;
     __syncthreads();
     int rank = 0;
     for (int q = 0; q < SELL_WIN; ++q) {
         const int lq = len[q];
         rank += lq > li || (lq == li && q < t);
     }
-    const int slot = blockIdx.x * SELL_WIN + rank;
-    srow[slot] = i < n ? i : -1;
-    slen[slot] = li > 0 ? li : 0;
-    if (rank % SELL_C == 0) {
-        width32[slot / SELL_C] = (li > 0 ? li : 0) * SELL_C;
-        atomicAdd(total, (unsigned long long)(li > 0 ? li : 0) * SELL_C);
+    row[rank] = t;
+    if (li >= INT_MAX / SELL_WIN) atomicAdd(total, 1ull << 40);   // no room for the length
+    slot[w0 + rank] = (unsigned)t | (unsigned)max(li, 0) * SELL_WIN;
+    __syncthreads();
+    const int r = row[t], l = max(len[r], 0);
+    const int k0 = l > 0 ? ia[w0 + r] : 0;
+    const int w = __shfl_sync(0xffffffffu, l, 0);
+    bool wide = false;
+    for (int u = 0; u < w; ++u) {
+        const int c = l > 0 ? ja[k0 + min(u, l - 1)] : -1;
+        const int lo = __reduce_min_sync(0xffffffffu, c < 0 ? INT_MAX : c);
+        const int hi = __reduce_max_sync(0xffffffffu, c);
+        wide |= hi - lo > 0xffff;
     }
+    if (t % SELL_C == 0) {
+        const int k = (w0 + t) / SELL_C, np = (w + 1) / 2, nl = wide ? 2 * w : w;
+        width[k] = w;
+        pairs[k] = np;
+        lines[k] = nl;
+        atomicAdd(sum, w);
+        atomicAdd(sum + 1, np);
+        atomicAdd(sum + 2, nl);
+    }
+    __syncthreads();
+    if (t < 3) atomicAdd(total + t, (unsigned long long)sum[t]);
 }
 
-__global__ void k_sell_fill(int npad, const int *__restrict__ ptr, const int *__restrict__ srow,
-                            const int *__restrict__ slen, const int *__restrict__ ia,
-                            const int *__restrict__ ja, const float *__restrict__ a, int *col,
-                            float *val) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < npad; r += gridDim.x * blockDim.x) {
-        const int s = r / SELL_C, lane = r % SELL_C;
-        const int w = (ptr[s + 1] - ptr[s]) / SELL_C;
-        const int i = srow[r], len = slen[r];
-        const int k0 = i >= 0 ? ia[i] : 0;
-        for (int u = 0; u < w; ++u) {
-            const size_t q = (size_t)ptr[s] + (size_t)u * SELL_C + lane;
-            col[q] = u < len ? ja[k0 + u] : 0;
-            val[q] = u < len ? a[k0 + u] : 0.f;
-        }
-    }
-}
-
-// Row sum of slot r's row in CSR order, eight entries' loads and gathers in
-// flight at a time.  L1: t -= v x and d += |v| (t starts at b_i); else
-// t += v x.
-template <bool L1>
-__device__ __forceinline__ void sell_row(int base, int len, const int *__restrict__ col,
-                                         const float *__restrict__ val,
-                                         const float *__restrict__ x, float &t, float &d) {
-    constexpr int G = 8;
-    for (int u0 = 0; u0 < len; u0 += G) {
-        int c[G];
-        float v[G], xv[G];
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            c[q] = 0;
-            v[q] = 0.f;
-            if (u0 + q < len) {
-                const int k = base + (u0 + q) * SELL_C;
-                c[q] = __ldcs(col + k);
-                v[q] = __ldcs(val + k);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < G; ++q) xv[q] = u0 + q < len ? __ldg(x + c[q]) : 0.f;
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            if (u0 + q < len) {
-                if (L1) {
-                    t -= v[q] * xv[q];
-                    d += fabsf(v[q]);
-                } else {
-                    t += v[q] * xv[q];
-                }
-            }
-        }
-    }
-}
-
+// A warp per slice: its entries, columns and bases, and its head: first line of
+// entries, first line of columns (negated and less one where they are 32 bits
+// wide), first pair of bases, width.
+template <typename T>
 __global__ void __launch_bounds__(SELL_WIN)
-k_l1_sell(int npad, const int *__restrict__ ptr, const int *__restrict__ srow,
-          const int *__restrict__ slen, const int *__restrict__ col,
-          const float *__restrict__ val, const float *__restrict__ b,
+k_sell_fill(const int *__restrict__ first, const int *__restrict__ pairs,
+            const int *__restrict__ lines, const unsigned *__restrict__ slot,
+            const int *__restrict__ ia, const int *__restrict__ ja, const T *__restrict__ a,
+            int4 *head, unsigned short *col, int2 *base, T *val) {
+    const int t = blockIdx.x * SELL_WIN + threadIdx.x, s = t / SELL_C, lane = t % SELL_C;
+    const unsigned sl = slot[t];
+    const int len = (int)(sl / SELL_WIN);
+    const int f0 = first[s], w = first[s + 1] - f0, l0 = lines[s], p0 = pairs[s];
+    const bool wide = lines[s + 1] - l0 != w;
+    const int k0 = len > 0 ? ia[blockIdx.x * SELL_WIN + (sl & SELL_ROW)] : 0;
+    if (lane == 0) head[s] = make_int4(f0, wide ? -l0 - 1 : l0, p0, w);
+    for (int u = 0; u < w; ++u) {
+        int c = len > 0 ? ja[k0 + min(u, len - 1)] : INT_MAX;
+        const int lo = __reduce_min_sync(0xffffffffu, c);
+        if (len == 0) c = lo;
+        // two entries side by side, the last of an odd width alone
+        const int at = u + 1 == w && u % 2 == 0 ? u * SELL_C + lane
+                                                : u / 2 * 2 * SELL_C + 2 * lane + u % 2;
+        val[(size_t)f0 * SELL_C + at] = u < len ? a[k0 + u] : T(0);
+        if (lane == 0) reinterpret_cast<int *>(base + p0 + u / 2)[u % 2] = lo;
+        unsigned short *q = col + (size_t)l0 * SELL_C;
+        if (wide) reinterpret_cast<int *>(q)[at] = c;
+        else q[at] = (unsigned short)(c - lo);
+    }
+}
+
+// W entries of a row, all their loads and gathers in flight at once.  L1: t -= v x
+// and d += |v| (t starts at b_i); else t += v x.  val, col and base point at the
+// slice's next entries, lane is the thread's.
+template <typename T, bool L1, bool WIDE, int W>
+__device__ __forceinline__ void sell_entries(const T *__restrict__ val,
+                                             const unsigned short *__restrict__ col,
+                                             const int2 *__restrict__ base, int lane,
+                                             const T *__restrict__ x, T &t, T &d) {
+    using V2 = typename SellPair<T>::type;
+    T v[W], xv[W];
+    int c[W];
+#pragma unroll
+    for (int q = 0; q < W / 2; ++q) {
+        const V2 u = __ldcs(reinterpret_cast<const V2 *>(val) + q * SELL_C + lane);
+        v[2 * q] = u.x;
+        v[2 * q + 1] = u.y;
+        if (WIDE) {
+            const int2 k = __ldcs(reinterpret_cast<const int2 *>(col) + q * SELL_C + lane);
+            c[2 * q] = k.x;
+            c[2 * q + 1] = k.y;
+        } else {
+            const unsigned k = __ldcs(reinterpret_cast<const unsigned *>(col) + q * SELL_C + lane);
+            const int2 b = __ldg(base + q);
+            c[2 * q] = b.x + (int)(k & 0xffffu);
+            c[2 * q + 1] = b.y + (int)(k >> 16);
+        }
+    }
+    if (W % 2) {
+        v[W - 1] = __ldcs(val + (W - 1) * SELL_C + lane);
+        c[W - 1] = WIDE ? __ldcs(reinterpret_cast<const int *>(col) + (W - 1) * SELL_C + lane)
+                        : __ldg(&base[W / 2].x) + (int)__ldcs(col + (W - 1) * SELL_C + lane);
+    }
+#pragma unroll
+    for (int q = 0; q < W; ++q) xv[q] = __ldg(x + c[q]);
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        if (L1) {
+            t -= v[q] * xv[q];
+            d += fabs(v[q]);
+        } else {
+            t += v[q] * xv[q];
+        }
+    }
+}
+
+template <typename T, bool L1, bool WIDE>
+__device__ __forceinline__ void sell_slice(const SellView<T> &V, int4 h, int lane,
+                                           const T *__restrict__ x, T &t, T &d) {
+    const T *val = V.val + (size_t)h.x * SELL_C;
+    const unsigned short *col = V.col + (size_t)(WIDE ? -h.y - 1 : h.y) * SELL_C;
+    const int2 *base = V.base + h.z;
+    int w = h.w;
+    for (; w >= 8; w -= 8) {
+        sell_entries<T, L1, WIDE, 8>(val, col, base, lane, x, t, d);
+        val += 8 * SELL_C;
+        col += 8 * SELL_C * (WIDE ? 2 : 1);
+        base += 4;
+    }
+    switch (w) {                   // the same for the whole warp
+    case 1: sell_entries<T, L1, WIDE, 1>(val, col, base, lane, x, t, d); break;
+    case 2: sell_entries<T, L1, WIDE, 2>(val, col, base, lane, x, t, d); break;
+    case 3: sell_entries<T, L1, WIDE, 3>(val, col, base, lane, x, t, d); break;
+    case 4: sell_entries<T, L1, WIDE, 4>(val, col, base, lane, x, t, d); break;
+    case 5: sell_entries<T, L1, WIDE, 5>(val, col, base, lane, x, t, d); break;
+    case 6: sell_entries<T, L1, WIDE, 6>(val, col, base, lane, x, t, d); break;
+    case 7: sell_entries<T, L1, WIDE, 7>(val, col, base, lane, x, t, d); break;
+    }
+}
+
+// Row sum of slot r's row in CSR order.
+template <typename T, bool L1>
+__device__ __forceinline__ void sell_row(const SellView<T> &V, int r, const T *__restrict__ x,
+                                         T &t, T &d) {
+    const int4 h = __ldg(V.head + r / SELL_C);
+    if (h.y >= 0) sell_slice<T, L1, false>(V, h, r % SELL_C, x, t, d);
+    else sell_slice<T, L1, true>(V, h, r % SELL_C, x, t, d);
+}
+
+__global__ void __launch_bounds__(SELL_WIN, 8)
+k_l1_sell(int n, const __grid_constant__ SellView<float> V, const float *__restrict__ b,
           const float *__restrict__ x, float *__restrict__ xn, const float *__restrict__ omega) {
     const int r = blockIdx.x * SELL_WIN + threadIdx.x;
-    if (r >= npad) return;
-    const int i = srow[r];
-    if (i < 0) return;
-    float t = b[i], d = 0.f;
-    sell_row<true>(ptr[r / SELL_C] + r % SELL_C, slen[r], col, val, x, t, d);
+    const unsigned sl = __ldcs(V.slot + r);
+    const int i = blockIdx.x * SELL_WIN + (int)(sl & SELL_ROW);
+    if (i >= n) return;
+    float t = __ldcs(b + i), d = 0.f;
+    sell_row<float, true>(V, r, x, t, d);
     float xi = x[i];
     if (fabsf(d) > float(SMALLREAL)) xi += omega ? omega[i] * (t / d) : t / d;
     xn[i] = xi;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(SELL_WIN)
-k_spmv_sell(int npad, const int *__restrict__ ptr, const int *__restrict__ srow,
-            const int *__restrict__ slen, const int *__restrict__ col,
-            const float *__restrict__ val, const float *__restrict__ x,
-            const float *__restrict__ b, float *__restrict__ y, float alpha) {
+template <typename T, int MODE>
+__global__ void __launch_bounds__(SELL_WIN, 8)
+k_spmv_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ x,
+            const T *__restrict__ b, T *__restrict__ y, T alpha) {
     const int r = blockIdx.x * SELL_WIN + threadIdx.x;
-    if (r >= npad) return;
-    const int i = srow[r];
-    if (i < 0) return;
-    float t = 0.f, d = 0.f;
-    sell_row<false>(ptr[r / SELL_C] + r % SELL_C, slen[r], col, val, x, t, d);
+    const unsigned sl = __ldcs(V.slot + r);
+    const int i = blockIdx.x * SELL_WIN + (int)(sl & SELL_ROW);
+    if (i >= n) return;
+    const T bi = MODE == SPMV_RES ? __ldcs(b + i) : T(0);
+    T t = T(0), d = T(0);
+    sell_row<T, false>(V, r, x, t, d);
     if (MODE == SPMV_RES) {
-        y[i] = b[i] - t;
+        y[i] = bi - t;
     } else if (MODE == SPMV_AXPY) {
-        if (alpha == 1.f) y[i] += t;
-        else if (alpha == -1.f) y[i] -= t;
+        if (alpha == T(1)) y[i] += t;
+        else if (alpha == T(-1)) y[i] -= t;
         else y[i] += t * alpha;
     } else {
         y[i] = t;
@@ -142,68 +229,75 @@ k_spmv_sell(int npad, const int *__restrict__ ptr, const int *__restrict__ srow,
 
 int sell_pad_rows(int n) { return (n + SELL_WIN - 1) / SELL_WIN * SELL_WIN; }
 
-int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
+template <typename T>
+int sell_build(int n, const int *ia, const int *ja, const T *a, SellArrays<T> *out,
                cudaStream_t s) {
-    *out = SellArrays();
+    *out = SellArrays<T>();
     if (n <= 0) return SUCCESS;
-    const int npad = sell_pad_rows(n), nsl = npad / SELL_C;
-    int *w32 = nullptr, *tmp = nullptr;
-    unsigned long long *dtot = nullptr, htot = 0;
-    SellArrays S;
+    const int npad = sell_pad_rows(n), nsl = npad / SELL_C, win = npad / SELL_WIN;
+    int *cnt = nullptr, *ptr = nullptr, *tmp = nullptr;   // widths, pairs, lines; their sums
+    unsigned long long *dtot = nullptr, htot[3] = {0, 0, 0};
+    SellArrays<T> S;
     S.npad = npad;
     int rc = SUCCESS;
-    if ((rc = dalloc(&S.row, npad)) || (rc = dalloc(&S.len, npad)) ||
-        (rc = dalloc(&S.ptr, nsl + 1)) || (rc = dalloc(&w32, nsl)) ||
-        (rc = dalloc(&tmp, scan_tmp_size(nsl + 1))) || (rc = dalloc(&dtot, 1)))
-        goto fail;
-    if (cudaMemsetAsync(dtot, 0, sizeof(unsigned long long), s) != cudaSuccess) {
+    if ((rc = dalloc(&S.slot, npad)) || (rc = dalloc(&S.head, nsl)) ||
+        (rc = dalloc(&cnt, 3 * (size_t)nsl)) || (rc = dalloc(&ptr, 3 * ((size_t)nsl + 1))) ||
+        (rc = dalloc(&tmp, scan_tmp_size(nsl + 1))) || (rc = dalloc(&dtot, 3)))
+        goto done;
+    if (cudaMemsetAsync(dtot, 0, sizeof(htot), s) != cudaSuccess) {
         rc = ERROR_SOLVER_MISC;
-        goto fail;
+        goto done;
     }
-    k_sell_order<<<npad / SELL_WIN, SELL_WIN, 0, s>>>(n, ia, S.row, S.len, w32, dtot);
+    k_sell_order<<<win, SELL_WIN, 0, s>>>(n, ia, ja, S.slot, cnt, cnt + nsl, cnt + 2 * (size_t)nsl,
+                                          dtot);
     count_launch();
-    if (cudaMemcpyAsync(&htot, dtot, sizeof(htot), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    if (cudaMemcpyAsync(htot, dtot, sizeof(htot), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         rc = ERROR_SOLVER_MISC;
-        goto fail;
+        goto done;
     }
-    // the slice offsets are int: a level whose padded slices would not fit
-    // gets no copy (the bundles and lanes kernels serve it)
-    if (htot > (unsigned long long)(INT_MAX / 2)) goto fail;
-    if ((rc = scan_exclusive(w32, S.ptr, nsl, tmp, s))) goto fail;
-    if ((rc = dalloc(&S.col, htot > 0 ? htot : 1)) || (rc = dalloc(&S.val, htot > 0 ? htot : 1)))
-        goto fail;
-    k_sell_fill<<<grid_for(npad), 256, 0, s>>>(npad, S.ptr, S.row, S.len, ia, ja, a, S.col,
-                                               S.val);
+    // a level whose padded slices would not fit an int index, or whose rows a
+    // slot's length, gets no copy (the bundles and lanes kernels serve it)
+    if (htot[0] * SELL_C > (unsigned long long)(INT_MAX / 2)) goto done;
+    for (int q = 0; q < 3 && !rc; ++q)
+        rc = scan_exclusive(cnt + (size_t)q * nsl, ptr + q * ((size_t)nsl + 1), nsl, tmp, s);
+    if (rc || (rc = dalloc(&S.val, std::max(1ull, htot[0] * SELL_C))) ||
+        (rc = dalloc(&S.base, std::max(1ull, htot[1]))) ||
+        (rc = dalloc(&S.col, std::max(1ull, htot[2] * SELL_C))))
+        goto done;
+    k_sell_fill<T><<<win, SELL_WIN, 0, s>>>(ptr, ptr + nsl + 1, ptr + 2 * ((size_t)nsl + 1),
+                                            S.slot, ia, ja, a, S.head, S.col, S.base, S.val);
     count_launch();
-    HZB_LAUNCH_CHECK();
-    dfree(w32);
-    dfree(tmp);
-    dfree(dtot);
+    if (cudaGetLastError() != cudaSuccess) {
+        rc = ERROR_SOLVER_MISC;
+        goto done;
+    }
     *out = S;
-    return SUCCESS;
-fail:
-    dfree(w32);
+done:
+    dfree(cnt);
+    dfree(ptr);
     dfree(tmp);
     dfree(dtot);
-    S.release();
+    if (!out->npad) S.release();
     return rc;
 }
+template int sell_build<float>(int, const int *, const int *, const float *, SellArrays<float> *,
+                               cudaStream_t);
 
-void SellArrays::release() {
-    dfree(ptr);
-    dfree(row);
-    dfree(len);
+template <typename T>
+void SellArrays<T>::release() {
+    dfree(slot);
+    dfree(head);
+    dfree(base);
     dfree(col);
     dfree(val);
     npad = 0;
 }
+template void SellArrays<float>::release();
 
 int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
                   const float *omega, cudaStream_t s) {
-    const SellView &V = A.sell;
-    k_l1_sell<<<V.npad / SELL_WIN, SELL_WIN, 0, s>>>(V.npad, V.ptr, V.row, V.len, V.col, V.val,
-                                                     b, x, xn, omega);
+    k_l1_sell<<<A.sell.npad / SELL_WIN, SELL_WIN, 0, s>>>(A.n, A.sell, b, x, xn, omega);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
@@ -211,20 +305,16 @@ int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *x
 
 int sell_spmv(const DCsr<float> &A, int mode, const float *x, const float *b, float *y,
               float alpha, cudaStream_t s) {
-    const SellView &V = A.sell;
-    const int g = V.npad / SELL_WIN;
+    const int g = A.sell.npad / SELL_WIN;
     switch (mode) {
     case SPMV_RES:
-        k_spmv_sell<SPMV_RES><<<g, SELL_WIN, 0, s>>>(V.npad, V.ptr, V.row, V.len, V.col, V.val,
-                                                     x, b, y, alpha);
+        k_spmv_sell<float, SPMV_RES><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
         break;
     case SPMV_AXPY:
-        k_spmv_sell<SPMV_AXPY><<<g, SELL_WIN, 0, s>>>(V.npad, V.ptr, V.row, V.len, V.col, V.val,
-                                                      x, b, y, alpha);
+        k_spmv_sell<float, SPMV_AXPY><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
         break;
     default:
-        k_spmv_sell<SPMV_Y><<<g, SELL_WIN, 0, s>>>(V.npad, V.ptr, V.row, V.len, V.col, V.val, x,
-                                                   b, y, alpha);
+        k_spmv_sell<float, SPMV_Y><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
         break;
     }
     count_launch();

@@ -25,7 +25,7 @@ struct Level {
     int *ia32 = nullptr, *ja32 = nullptr;
     float *val32 = nullptr;
     bool own32 = false;
-    SellArrays sell32;                // sliced-ELL copy, when vec32 = SELL_LANES
+    SellArrays<float> sell32;                // sliced-ELL copy, when vec32 = SELL_LANES
     // level 0 of the mixed solve with stored exact zeros: the FP64 values of
     // the FP32 copy's pattern, for the outer Krylov loop's SpMV (a zero adds
     // nothing to a row sum, so its result is the full matrix's)

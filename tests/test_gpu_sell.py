@@ -43,3 +43,24 @@ def test_sell_matches_bundles_bitwise(monkeypatch, N, sigma):
     assert np.array_equal(x_s, x_b)
     A = sp.csr_matrix((val, ja, ia), shape=(len(b), len(b)))
     assert np.linalg.norm(b - A @ x_s) / np.linalg.norm(b) < 1e-8
+
+
+@pytest.mark.parametrize("n,far", [(4097, 0), (150001, 70000), (150016, 149000)])
+def test_sell_column_widths(monkeypatch, n, far):
+    """Slices whose columns at one position span more than 16 bits (rows that
+    couple over ``far`` beside rows that do not, forward beside backward) keep
+    32-bit columns, the others 16-bit ones; the last window is partly or fully filled
+    (n mod 256 = 1, 241 and 0), rows have odd and even lengths."""
+    A = sp.diags([np.full(n, 4.25), -np.ones(n - 1), -np.ones(n - 1)], [0, 1, -1]).tocsr()
+    if far:
+        i = np.arange(0, n - far, 97)
+        F = sp.coo_matrix((np.full(len(i), -0.5), (i, i + far)), shape=(n, n)).tocsr()
+        A = (A + F + F.T).tocsr()
+    A.sort_indices()
+    ia, ja, val = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    b = P.rhs_uniform(n, 5)
+    it_s, x_s, _ = mixed_solve(monkeypatch, "sell", ia, ja, val, b)
+    it_b, x_b, _ = mixed_solve(monkeypatch, "0", ia, ja, val, b)
+    assert it_s == it_b > 0
+    assert np.array_equal(x_s, x_b)
+    assert np.linalg.norm(b - A @ x_s) / np.linalg.norm(b) < 1e-8
