@@ -498,9 +498,10 @@ template <typename T, int MODE>
 static int spmv_mode(const DCsr<T> &A, const T *x, const T *b, T *y, T alpha, T *part,
                      cudaStream_t s) {
     if (A.n <= 0) return SUCCESS;
+    if (A.vec_lanes == SELL_LANES && A.sell.npad > 0 && !A.act &&
+        (sizeof(T) == 8 || MODE != SPMV_Y_DOT))
+        return sell_spmv<T>(A, MODE, x, b, y, alpha, part, s);
     if constexpr (sizeof(T) == 4 && MODE != SPMV_Y_DOT) {
-        if (A.vec_lanes == SELL_LANES && A.sell.npad > 0 && !A.act)
-            return sell_spmv(A, MODE, x, b, y, alpha, s);
         if (A.vec_lanes > 0) return spmv_vec_launch<MODE>(A, x, b, y, alpha, s);
     }
     switch (A.bundle_rows) {
@@ -623,16 +624,42 @@ int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cud
 // ---------------------------------------------------------------------------
 // Transfers (P = aggregate map, R = P^T with ascending fine rows)
 // ---------------------------------------------------------------------------
+// Two aggregates a thread, the first two rows of each (most have no more) in
+// flight together: the chain from an aggregate's range over its rows to their
+// values was waited for row by row (110 us a cycle on those levels, 87 now).
 template <typename T>
 __global__ void k_restrict(int nc, const int *__restrict__ ria,
                            const int *__restrict__ rja, const T *__restrict__ w,
                            T *__restrict__ bc, const unsigned char *__restrict__ act) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc;
-         c += gridDim.x * blockDim.x) {
-        if (act && !act[c / ACT_ROWS]) continue;
-        T t = T(0);
-        for (int k = ria[c]; k < ria[c + 1]; ++k) t += w[rja[k]];
-        bc[c] = t;
+    constexpr int U = 2;
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 < (unsigned)nc; c0 += U * step) {
+        int k0[U], k1[U], j0[U], j1[U];
+        bool on[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned c = c0 + q * step;
+            on[q] = c < (unsigned)nc && !(act && !act[c / ACT_ROWS]);
+            k0[q] = on[q] ? ria[c] : 0;
+            k1[q] = on[q] ? ria[c + 1] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            j0[q] = k0[q] < k1[q] ? rja[k0[q]] : 0;
+            j1[q] = k0[q] + 1 < k1[q] ? rja[k0[q] + 1] : 0;
+        }
+        T t[U], t1[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            t[q] = k0[q] < k1[q] ? T(0) + w[j0[q]] : T(0);
+            t1[q] = k0[q] + 1 < k1[q] ? w[j1[q]] : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (k0[q] + 1 < k1[q]) t[q] += t1[q];
+            for (int k = k0[q] + 2; k < k1[q]; ++k) t[q] += w[rja[k]];
+            if (on[q]) bc[c0 + q * step] = t[q];
+        }
     }
 }
 
@@ -650,19 +677,33 @@ template int restrict_agg<double>(int, const int *, const int *, const double *,
 template int restrict_agg<float>(int, const int *, const int *, const float *,
                                  float *, cudaStream_t, const unsigned char *);
 
+// four rows a thread, as in k_l1_first (104 us a cycle, 76 now)
 template <typename T>
 __global__ void k_prolong(int n, const int *__restrict__ agg,
                           const T *__restrict__ xc, T *__restrict__ x, T alpha,
                           const unsigned char *__restrict__ act) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        if (act && !act[i / ACT_ROWS]) continue;
-        T t = T(0);
-        const int c = agg[i];
-        if (c >= 0) t += xc[c];
-        if (alpha == T(1)) x[i] += t;
-        else if (alpha == T(-1)) x[i] -= t;
-        else x[i] += t * alpha;
+    constexpr int U = 4;
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < (unsigned)n; i0 += U * step) {
+        int c[U];
+        T xi[U], t[U];
+        bool on[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned i = i0 + q * step;
+            on[q] = i < (unsigned)n && !(act && !act[i / ACT_ROWS]);
+            c[q] = on[q] ? agg[i] : -1;
+            xi[q] = on[q] ? x[i] : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) t[q] = c[q] >= 0 ? T(0) + xc[c[q]] : T(0);
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (alpha == T(1)) xi[q] += t[q];
+            else if (alpha == T(-1)) xi[q] -= t[q];
+            else xi[q] += t[q] * alpha;
+            if (on[q]) x[i0 + q * step] = xi[q];
+        }
     }
 }
 
@@ -840,17 +881,32 @@ __global__ void k_l1_norms(int n, const int *__restrict__ ia, const T *__restric
     }
 }
 
+// Four rows a thread, their loads in flight together: with one, 123 us a cycle
+// on levels of 16.6 million down to 0.8 million rows, 68 now.
 template <typename T>
 __global__ void k_l1_first(int n, const T *__restrict__ b, const T *__restrict__ d,
                            T *__restrict__ xn, const float *__restrict__ omega,
                            const unsigned char *__restrict__ act) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        if (act && !act[i / ACT_ROWS]) continue;
-        const T di = d[i];
-        T xi = T(0);
-        if (fabs(di) > T(SMALLREAL)) xi += (omega ? T(omega[i]) : T(1)) * (b[i] / di);
-        xn[i] = xi;
+    constexpr int U = 4;
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < (unsigned)n; i0 += U * step) {
+        T bi[U], di[U];
+        float w[U];
+        bool on[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned i = i0 + q * step;
+            on[q] = i < (unsigned)n && !(act && !act[i / ACT_ROWS]);
+            bi[q] = on[q] ? b[i] : T(0);
+            di[q] = on[q] ? d[i] : T(0);
+            w[q] = omega && on[q] ? omega[i] : 1.f;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            T xi = T(0);
+            if (fabs(di[q]) > T(SMALLREAL)) xi += T(w[q]) * (bi[q] / di[q]);
+            if (on[q]) xn[i0 + q * step] = xi;
+        }
     }
 }
 
@@ -1420,26 +1476,66 @@ int reduce_blocks(int n) {
     return g < cap ? g : cap;
 }
 
-__global__ void k_reduce_final(const double *__restrict__ part, int np,
-                               double *out, int is_max) {
+// A CTA per sum, eight coalesced loads of a thread in flight (a contiguous slice
+// per thread: 83 us for the 260,000 partial sums of a product of 16.6 million
+// rows; 33 so by one CTA, which is why they go through k_reduce_part first).
+__global__ void __launch_bounds__(1024)
+k_reduce_final(const double *__restrict__ part, int np, double *out0, double *out1, int is_max) {
     __shared__ double sh[32];
+    part += (size_t)blockIdx.x * np;
     double v = 0.0;
-    // each thread folds a contiguous slice in order
-    const int per = (np + blockDim.x - 1) / blockDim.x;
-    const int b0 = threadIdx.x * per, b1 = min(b0 + per, np);
-    for (int k = b0; k < b1; ++k) v = is_max ? fmax(v, part[k]) : v + part[k];
+    constexpr int U = 8;
+    for (int k0 = threadIdx.x; k0 < np; k0 += U * blockDim.x) {
+        double u[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int k = k0 + q * (int)blockDim.x;
+            u[q] = k < np ? part[k] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (k0 + q * (int)blockDim.x < np) v = is_max ? fmax(v, u[q]) : v + u[q];
+        }
+    }
     v = is_max ? block_max(v, sh) : block_sum(v, sh);
-    if (threadIdx.x == 0) out[0] = v;
+    if (threadIdx.x == 0) (blockIdx.x ? out1 : out0)[0] = v;
 }
 
+// a CTA's contiguous range of np partial sums
+__global__ void __launch_bounds__(256)
+k_reduce_part(const double *__restrict__ part, int np, int per, double *out) {
+    __shared__ double sh[32];
+    const int k1 = min(np, (int)(blockIdx.x + 1) * per);
+    double v = 0.0;
+    for (int k = blockIdx.x * per + threadIdx.x; k < k1; k += 256) v += part[k];
+    v = block_sum(v, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = v;
+}
+
+static int reduce_threads(int np) { return np > 4096 ? 1024 : 256; }
 int reduce_final(const double *part, int np, double *out, cudaStream_t s) {
-    k_reduce_final<<<1, 256, 0, s>>>(part, np, out, 0);
+    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 0);
+    count_launch();
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
+// the second launch costs 2 us; one CTA takes as long for 16,000 more
+int reduce_final_many(const double *part, int np, double *scratch, double *out, cudaStream_t s) {
+    constexpr int PER = 1024;
+    if (np <= 16 * PER) return reduce_final(part, np, out, s);
+    const int per = std::max(PER, div_up(np, 1024)), g = div_up(np, per);
+    k_reduce_part<<<g, 256, 0, s>>>(part, np, per, scratch);
+    count_launch();
+    return reduce_final(scratch, g, out, s);
+}
+int reduce_final2(const double *part, int np, double *out0, double *out1, cudaStream_t s) {
+    k_reduce_final<<<2, reduce_threads(np), 0, s>>>(part, np, out0, out1, 0);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
 }
 int reduce_final_max(const double *part, int np, double *out, cudaStream_t s) {
-    k_reduce_final<<<1, 256, 0, s>>>(part, np, out, 1);
+    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 1);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;

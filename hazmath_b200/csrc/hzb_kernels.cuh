@@ -22,17 +22,29 @@ struct SellView {
     const int2 *base = nullptr;
     const T *val = nullptr;
 };
-template <typename T>
+// the arrays: FP32 values, and FP64 ones of the same pattern where they were asked for
 struct SellArrays {
     int npad = 0;
+    size_t nval = 0;
     unsigned *slot = nullptr;
     unsigned short *col = nullptr;
     int4 *head = nullptr;
     int2 *base = nullptr;
-    T *val = nullptr;
-    SellView<T> view() const {
+    float *val = nullptr;
+    double *val64 = nullptr;
+    template <typename T> SellView<T> pattern() const {
         SellView<T> v;
-        v.npad = npad; v.slot = slot; v.col = col; v.head = head; v.base = base; v.val = val;
+        v.npad = npad; v.slot = slot; v.col = col; v.head = head; v.base = base;
+        return v;
+    }
+    SellView<float> view() const {
+        SellView<float> v = pattern<float>();
+        v.val = val;
+        return v;
+    }
+    SellView<double> view64() const {
+        SellView<double> v = pattern<double>();
+        v.val = val64;
         return v;
     }
     void release();
@@ -79,13 +91,14 @@ bool fp32_schedule_known(int n, int nnz, int *lanes);
 // Sliced-ELL copy of a CSR matrix (hzb_sell.cu); *out stays empty
 // (npad 0) when its slice offsets would overflow int.  Sweep and SpMV on it
 // (no activity array, no SPMV_Y_DOT).
-template <typename T>
-int sell_build(int n, const int *ia, const int *ja, const T *a, SellArrays<T> *out,
+int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
                cudaStream_t s);
+int sell_values64(SellArrays *S, const int *ia, const double *a, cudaStream_t s);
 int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
                   const float *omega, cudaStream_t s);
-int sell_spmv(const DCsr<float> &A, int mode, const float *x, const float *b, float *y,
-              float alpha, cudaStream_t s);
+template <typename T>
+int sell_spmv(const DCsr<T> &A, int mode, const T *x, const T *b, T *y, T alpha, T *part,
+              cudaStream_t s);
 int spmv_blocks_rows(int n, int rows);
 
 // y = A x (SPMV_Y); y = b - A x (SPMV_RES); y += alpha A x with the
@@ -268,6 +281,11 @@ int gs_run(const DCsr<T> &A, int kind, const int *rows, const int *set_ptr,
 // Deterministic reductions: partial sums per block, then an ordered final
 // sum into out[0].
 int reduce_final(const double *part, int nparts, double *out, cudaStream_t s);
+// the same for many partial sums; scratch: 1024 words
+int reduce_final_many(const double *part, int nparts, double *scratch, double *out,
+                      cudaStream_t s);
+// two sums of nparts each, one behind the other in part
+int reduce_final2(const double *part, int nparts, double *out0, double *out1, cudaStream_t s);
 int reduce_final_max(const double *part, int nparts, double *out,
                      cudaStream_t s);
 int dot_partial(int n, const double *x, const double *y, double *part,

@@ -42,17 +42,22 @@ template <> struct SellPair<double> { using type = double2; };
 __global__ void __launch_bounds__(SELL_WIN)
 k_sell_order(int n, const int *__restrict__ ia, const int *__restrict__ ja, unsigned *slot,
              int *width, int *pairs, int *lines, unsigned long long *total) {
+    __shared__ __align__(16) int key[SELL_WIN];
     __shared__ int len[SELL_WIN], row[SELL_WIN], sum[3];
     const int t = threadIdx.x, w0 = blockIdx.x * SELL_WIN;
     const int i = w0 + t;
     const int li = i < n ? ia[i + 1] - ia[i] : -1;
+    // length, then index: one compare a pair of rows, four rows a load
+    const int k = min(li, INT_MAX / SELL_WIN - 1) * SELL_WIN + (SELL_WIN - 1 - t);
+    key[t] = k;
     len[t] = li;
     if (t < 3) sum[t] = 0;
     __syncthreads();
     int rank = 0;
-    for (int q = 0; q < SELL_WIN; ++q) {
-        const int lq = len[q];
-        rank += lq > li || (lq == li && q < t);
+#pragma unroll 8
+    for (int q = 0; q < SELL_WIN / 4; ++q) {
+        const int4 o = reinterpret_cast<const int4 *>(key)[q];
+        rank += (o.x > k) + (o.y > k) + (o.z > k) + (o.w > k);
     }
     row[rank] = t;
     if (li >= INT_MAX / SELL_WIN) atomicAdd(total, 1ull << 40);   // no room for the length
@@ -69,10 +74,10 @@ k_sell_order(int n, const int *__restrict__ ia, const int *__restrict__ ja, unsi
         wide |= hi - lo > 0xffff;
     }
     if (t % SELL_C == 0) {
-        const int k = (w0 + t) / SELL_C, np = (w + 1) / 2, nl = wide ? 2 * w : w;
-        width[k] = w;
-        pairs[k] = np;
-        lines[k] = nl;
+        const int sl = (w0 + t) / SELL_C, np = (w + 1) / 2, nl = wide ? 2 * w : w;
+        width[sl] = w;
+        pairs[sl] = np;
+        lines[sl] = nl;
         atomicAdd(sum, w);
         atomicAdd(sum + 1, np);
         atomicAdd(sum + 2, nl);
@@ -81,15 +86,20 @@ k_sell_order(int n, const int *__restrict__ ia, const int *__restrict__ ja, unsi
     if (t < 3) atomicAdd(total + t, (unsigned long long)sum[t]);
 }
 
+// entry u's place in a slice of width w: two side by side, the last of an odd width
+// alone
+__device__ __forceinline__ int sell_at(int u, int w, int lane) {
+    return u + 1 == w && u % 2 == 0 ? u * SELL_C + lane : u / 2 * 2 * SELL_C + 2 * lane + u % 2;
+}
+
 // A warp per slice: its entries, columns and bases, and its head: first line of
 // entries, first line of columns (negated and less one where they are 32 bits
 // wide), first pair of bases, width.
-template <typename T>
 __global__ void __launch_bounds__(SELL_WIN)
 k_sell_fill(const int *__restrict__ first, const int *__restrict__ pairs,
             const int *__restrict__ lines, const unsigned *__restrict__ slot,
-            const int *__restrict__ ia, const int *__restrict__ ja, const T *__restrict__ a,
-            int4 *head, unsigned short *col, int2 *base, T *val) {
+            const int *__restrict__ ia, const int *__restrict__ ja, const float *__restrict__ a,
+            int4 *head, unsigned short *col, int2 *base, float *val) {
     const int t = blockIdx.x * SELL_WIN + threadIdx.x, s = t / SELL_C, lane = t % SELL_C;
     const unsigned sl = slot[t];
     const int len = (int)(sl / SELL_WIN);
@@ -101,15 +111,26 @@ k_sell_fill(const int *__restrict__ first, const int *__restrict__ pairs,
         int c = len > 0 ? ja[k0 + min(u, len - 1)] : INT_MAX;
         const int lo = __reduce_min_sync(0xffffffffu, c);
         if (len == 0) c = lo;
-        // two entries side by side, the last of an odd width alone
-        const int at = u + 1 == w && u % 2 == 0 ? u * SELL_C + lane
-                                                : u / 2 * 2 * SELL_C + 2 * lane + u % 2;
-        val[(size_t)f0 * SELL_C + at] = u < len ? a[k0 + u] : T(0);
+        const int at = sell_at(u, w, lane);
+        val[(size_t)f0 * SELL_C + at] = u < len ? a[k0 + u] : 0.f;
         if (lane == 0) reinterpret_cast<int *>(base + p0 + u / 2)[u % 2] = lo;
         unsigned short *q = col + (size_t)l0 * SELL_C;
         if (wide) reinterpret_cast<int *>(q)[at] = c;
         else q[at] = (unsigned short)(c - lo);
     }
+}
+
+// The FP64 values of a copy whose FP32 ones are there.
+__global__ void __launch_bounds__(SELL_WIN)
+k_sell_values(const __grid_constant__ SellView<double> V, const int *__restrict__ ia,
+              const double *__restrict__ a, double *val) {
+    const int t = blockIdx.x * SELL_WIN + threadIdx.x, lane = t % SELL_C;
+    const unsigned sl = V.slot[t];
+    const int4 h = V.head[t / SELL_C];
+    const int len = (int)(sl / SELL_WIN);
+    const int k0 = len > 0 ? ia[blockIdx.x * SELL_WIN + (sl & SELL_ROW)] : 0;
+    for (int u = 0; u < h.w; ++u) val[(size_t)h.x * SELL_C + sell_at(u, h.w, lane)] =
+        u < len ? a[k0 + u] : 0.0;
 }
 
 // W entries of a row, all their loads and gathers in flight at once.  L1: t -= v x
@@ -157,6 +178,8 @@ __device__ __forceinline__ void sell_entries(const T *__restrict__ val,
     }
 }
 
+// entries in flight, of FP64 rows half as many (they take twice the registers)
+template <typename T> constexpr int SELL_G = sizeof(T) == 8 ? 4 : 8;
 template <typename T, bool L1, bool WIDE>
 __device__ __forceinline__ void sell_slice(const SellView<T> &V, int4 h, int lane,
                                            const T *__restrict__ x, T &t, T &d) {
@@ -164,20 +187,21 @@ __device__ __forceinline__ void sell_slice(const SellView<T> &V, int4 h, int lan
     const unsigned short *col = V.col + (size_t)(WIDE ? -h.y - 1 : h.y) * SELL_C;
     const int2 *base = V.base + h.z;
     int w = h.w;
-    for (; w >= 8; w -= 8) {
-        sell_entries<T, L1, WIDE, 8>(val, col, base, lane, x, t, d);
-        val += 8 * SELL_C;
-        col += 8 * SELL_C * (WIDE ? 2 : 1);
-        base += 4;
+    constexpr int G = SELL_G<T>;
+    for (; w >= G; w -= G) {
+        sell_entries<T, L1, WIDE, G>(val, col, base, lane, x, t, d);
+        val += G * SELL_C;
+        col += G * SELL_C * (WIDE ? 2 : 1);
+        base += G / 2;
     }
     switch (w) {                   // the same for the whole warp
     case 1: sell_entries<T, L1, WIDE, 1>(val, col, base, lane, x, t, d); break;
     case 2: sell_entries<T, L1, WIDE, 2>(val, col, base, lane, x, t, d); break;
     case 3: sell_entries<T, L1, WIDE, 3>(val, col, base, lane, x, t, d); break;
-    case 4: sell_entries<T, L1, WIDE, 4>(val, col, base, lane, x, t, d); break;
-    case 5: sell_entries<T, L1, WIDE, 5>(val, col, base, lane, x, t, d); break;
-    case 6: sell_entries<T, L1, WIDE, 6>(val, col, base, lane, x, t, d); break;
-    case 7: sell_entries<T, L1, WIDE, 7>(val, col, base, lane, x, t, d); break;
+    case 4: if (G > 4) sell_entries<T, L1, WIDE, 4>(val, col, base, lane, x, t, d); break;
+    case 5: if (G > 5) sell_entries<T, L1, WIDE, 5>(val, col, base, lane, x, t, d); break;
+    case 6: if (G > 6) sell_entries<T, L1, WIDE, 6>(val, col, base, lane, x, t, d); break;
+    case 7: if (G > 7) sell_entries<T, L1, WIDE, 7>(val, col, base, lane, x, t, d); break;
     }
 }
 
@@ -204,14 +228,18 @@ k_l1_sell(int n, const __grid_constant__ SellView<float> V, const float *__restr
     xn[i] = xi;
 }
 
+// 64 warps an SM here too (FP64, 16.6 million rows, with (x, y): 290 us; 322 with
+// 48, 443 with 32; 364 staged).  SPMV_Y_DOT: the partial sums of (x, y) over the same groups of `rows`
+// rows, added in the same order, as the staged kernels (the same bits).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SELL_WIN, 8)
 k_spmv_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ x,
-            const T *__restrict__ b, T *__restrict__ y, T alpha) {
+            const T *__restrict__ b, T *__restrict__ y, T alpha, T *__restrict__ part,
+            int rows) {
     const int r = blockIdx.x * SELL_WIN + threadIdx.x;
     const unsigned sl = __ldcs(V.slot + r);
     const int i = blockIdx.x * SELL_WIN + (int)(sl & SELL_ROW);
-    if (i >= n) return;
+    if (MODE != SPMV_Y_DOT && i >= n) return;
     const T bi = MODE == SPMV_RES ? __ldcs(b + i) : T(0);
     T t = T(0), d = T(0);
     sell_row<T, false>(V, r, x, t, d);
@@ -221,23 +249,39 @@ k_spmv_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ 
         if (alpha == T(1)) y[i] += t;
         else if (alpha == T(-1)) y[i] -= t;
         else y[i] += t * alpha;
-    } else {
+    } else if (MODE == SPMV_Y) {
         y[i] = t;
+    } else {
+        __shared__ T prod[SELL_WIN], sh[SELL_WIN / 32];
+        if (i < n) {
+            y[i] = t;
+            d = t * __ldg(x + i);
+        }
+        prod[sl & SELL_ROW] = d;
+        __syncthreads();
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = rows / 32;
+        d = warp_sum(prod[threadIdx.x]);
+        if (lane == 0) sh[warp] = d;
+        __syncthreads();
+        if (warp < SELL_WIN / rows) {
+            d = warp_sum(lane < per ? sh[warp * per + lane] : T(0));
+            const long long g = (long long)blockIdx.x * (SELL_WIN / rows) + warp;
+            if (lane == 0 && g * rows < n) part[g] = d;
+        }
     }
 }
 }  // namespace
 
 int sell_pad_rows(int n) { return (n + SELL_WIN - 1) / SELL_WIN * SELL_WIN; }
 
-template <typename T>
-int sell_build(int n, const int *ia, const int *ja, const T *a, SellArrays<T> *out,
+int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
                cudaStream_t s) {
-    *out = SellArrays<T>();
+    *out = SellArrays();
     if (n <= 0) return SUCCESS;
     const int npad = sell_pad_rows(n), nsl = npad / SELL_C, win = npad / SELL_WIN;
     int *cnt = nullptr, *ptr = nullptr, *tmp = nullptr;   // widths, pairs, lines; their sums
     unsigned long long *dtot = nullptr, htot[3] = {0, 0, 0};
-    SellArrays<T> S;
+    SellArrays S;
     S.npad = npad;
     int rc = SUCCESS;
     if ((rc = dalloc(&S.slot, npad)) || (rc = dalloc(&S.head, nsl)) ||
@@ -265,13 +309,14 @@ int sell_build(int n, const int *ia, const int *ja, const T *a, SellArrays<T> *o
         (rc = dalloc(&S.base, std::max(1ull, htot[1]))) ||
         (rc = dalloc(&S.col, std::max(1ull, htot[2] * SELL_C))))
         goto done;
-    k_sell_fill<T><<<win, SELL_WIN, 0, s>>>(ptr, ptr + nsl + 1, ptr + 2 * ((size_t)nsl + 1),
+    k_sell_fill<<<win, SELL_WIN, 0, s>>>(ptr, ptr + nsl + 1, ptr + 2 * ((size_t)nsl + 1),
                                             S.slot, ia, ja, a, S.head, S.col, S.base, S.val);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) {
         rc = ERROR_SOLVER_MISC;
         goto done;
     }
+    S.nval = (size_t)htot[0] * SELL_C;
     *out = S;
 done:
     dfree(cnt);
@@ -281,19 +326,23 @@ done:
     if (!out->npad) S.release();
     return rc;
 }
-template int sell_build<float>(int, const int *, const int *, const float *, SellArrays<float> *,
-                               cudaStream_t);
+int sell_values64(SellArrays *S, const int *ia, const double *a, cudaStream_t s) {
+    HZB_TRY(dalloc(&S->val64, std::max<size_t>(1, S->nval)));
+    k_sell_values<<<S->npad / SELL_WIN, SELL_WIN, 0, s>>>(S->view64(), ia, a, S->val64);
+    count_launch();
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
 
-template <typename T>
-void SellArrays<T>::release() {
+void SellArrays::release() {
     dfree(slot);
     dfree(head);
     dfree(base);
     dfree(col);
     dfree(val);
+    dfree(val64);
     npad = 0;
 }
-template void SellArrays<float>::release();
 
 int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
                   const float *omega, cudaStream_t s) {
@@ -303,23 +352,26 @@ int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *x
     return SUCCESS;
 }
 
-int sell_spmv(const DCsr<float> &A, int mode, const float *x, const float *b, float *y,
-              float alpha, cudaStream_t s) {
-    const int g = A.sell.npad / SELL_WIN;
+template <typename T>
+int sell_spmv(const DCsr<T> &A, int mode, const T *x, const T *b, T *y, T alpha, T *part,
+              cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        kernel<<<A.sell.npad / SELL_WIN, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha, part,
+                                                           A.bundle_rows);
+    };
     switch (mode) {
-    case SPMV_RES:
-        k_spmv_sell<float, SPMV_RES><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
-        break;
-    case SPMV_AXPY:
-        k_spmv_sell<float, SPMV_AXPY><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
-        break;
-    default:
-        k_spmv_sell<float, SPMV_Y><<<g, SELL_WIN, 0, s>>>(A.n, A.sell, x, b, y, alpha);
-        break;
+    case SPMV_RES: go(k_spmv_sell<T, SPMV_RES>); break;
+    case SPMV_AXPY: go(k_spmv_sell<T, SPMV_AXPY>); break;
+    case SPMV_Y_DOT: go(k_spmv_sell<T, SPMV_Y_DOT>); break;
+    default: go(k_spmv_sell<T, SPMV_Y>); break;
     }
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
 }
+template int sell_spmv<float>(const DCsr<float> &, int, const float *, const float *, float *,
+                              float, float *, cudaStream_t);
+template int sell_spmv<double>(const DCsr<double> &, int, const double *, const double *,
+                               double *, double, double *, cudaStream_t);
 
 }  // namespace hzb

@@ -22,11 +22,23 @@ __global__ void k_dot2_partial(int n, const double *__restrict__ z,
                                const double *__restrict__ r, double *part) {
     __shared__ double sh[32];
     double a = 0.0, b = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        const double zi = z[i];
-        a += zi * t[i];
-        b += zi * r[i];
+    constexpr int U = 4;
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < (unsigned)n; i0 += U * step) {
+        double zi[U], ti[U], ri[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned i = i0 + q * step;
+            const bool on = i < (unsigned)n;
+            zi[q] = on ? (double)z[i] : 0.0;
+            ti[q] = on ? t[i] : 0.0;
+            ri[q] = on ? r[i] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            a += zi[q] * ti[q];
+            b += zi[q] * ri[q];
+        }
     }
     a = block_sum(a, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
@@ -100,9 +112,20 @@ __global__ void k_fcg_p_f(int n, const double *__restrict__ zt,
                           const double *__restrict__ pap, const float *__restrict__ z,
                           double *p) {
     const double beta = -zt[0] / pap[0];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x)
-        p[i] = (double)z[i] + beta * p[i];
+    constexpr int U = 4;
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < (unsigned)n; i0 += U * step) {
+        double zi[U], pi[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned i = i0 + q * step;
+            zi[q] = i < (unsigned)n ? (double)z[i] : 0.0;
+            pi[q] = i < (unsigned)n ? p[i] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (i0 + q * step < (unsigned)n) p[i0 + q * step] = zi[q] + beta * pi[q];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -654,6 +677,13 @@ int ensure_fp32(hzb_solver *S) {
                 L.vec32 = A.vec_lanes;
                 if (L.vec32 != SELL_LANES) L.sell32.release();
             }
+            // the outer product reads the same rows as the sweeps: where the
+            // sliced form was the fastest for them it is for FP64 too (364 us
+            // staged, 290 sliced on 16.6 million rows)
+            if (l == 0 && !S->batch && L.vec32 == SELL_LANES && L.sell32.npad) {
+                HZB_TRY(sell_values64(&L.sell32, L.ia32, L.own32 ? L.val64nz : L.val, S->s));
+                dfree(L.val64nz);
+            }
         }
         ms_sched = lap(t);
         if (trace && ms_count + ms_copy + ms_vec + ms_norms + ms_sell + ms_sched > 1.0)
@@ -1161,7 +1191,8 @@ int pcg(hzb_solver *S, const DCsr<double> &A, const double *b, double *u,
     while (iter++ < MaxIt) {
         // t = A p ; temp2 = (t, p) ; alpha = temp1 / temp2 (device)
         HZB_TRY(spmv<double>(A, SPMV_Y_DOT, w.p, nullptr, w.t, 1.0, partd, s));
-        HZB_TRY(reduce_final(partd, spmv_blocks_rows(m, A.bundle_rows), w.sc + SC_T2, s));
+        HZB_TRY(reduce_final_many(partd, spmv_blocks_rows(m, A.bundle_rows), part4,
+                                  w.sc + SC_T2, s));
         // u += alpha p ; r -= alpha t ; norms for checks I and II
         HZB_TRY(pcg_update(m, w.sc + SC_T1, w.sc + SC_T2, u, w.r, w.p, w.t, part4, s));
         HZB_TRY(reduce_final(part4, G, w.sc + SC_RR, s));
@@ -1378,7 +1409,8 @@ int fcg_mixed(hzb_solver *S, const double *b, double *x, double tol, int maxit,
     Level &L0 = S->lv[0];
     while (iter++ < maxit) {
         HZB_TRY(spmv<double>(A, SPMV_Y_DOT, w.p, nullptr, w.t, 1.0, partd, s));
-        HZB_TRY(reduce_final(partd, spmv_blocks_rows(m, A.bundle_rows), w.sc + SC_T2, s));
+        HZB_TRY(reduce_final_many(partd, spmv_blocks_rows(m, A.bundle_rows), part4,
+                                  w.sc + SC_T2, s));
         k_fcg_update<<<G, 256, 0, s>>>(m, w.sc + SC_T1, w.sc + SC_T2, x, w.r, w.p, w.t,
                                         L0.b32, part4);
         count_launch();
@@ -1398,13 +1430,11 @@ int fcg_mixed(hzb_solver *S, const double *b, double *x, double tol, int maxit,
             HZB_TRY(d2f(m, w.r, L0.b32, s));   // the cycle starts from the true residual
         }
         HZB_TRY(cycles32(S));
-        k_dot2_partial_f<<<G, 256, 0, s>>>(m, L0.x32, w.t, w.r, part4);
+        k_dot2_partial_f<<<G, 512, 0, s>>>(m, L0.x32, w.t, w.r, part4);
         count_launch();
-        HZB_TRY(reduce_final(part4, G, w.sc + SC_ZT, s));
-        HZB_TRY(reduce_final(part4 + G, G, w.sc + SC_T3, s));
+        HZB_TRY(reduce_final2(part4, G, w.sc + SC_ZT, w.sc + SC_T1, s));
         k_fcg_p_f<<<grid_for(m), 256, 0, s>>>(m, w.sc + SC_ZT, w.sc + SC_T2, L0.x32, w.p);
-        k_copy_scalar<<<1, 1, 0, s>>>(w.sc + SC_T3, w.sc + SC_T1);
-        count_launch(2);
+        count_launch();
         HZB_LAUNCH_CHECK();
     }
     if (prtlvl > PRINT_NONE) {

@@ -25,11 +25,12 @@ struct Level {
     int *ia32 = nullptr, *ja32 = nullptr;
     float *val32 = nullptr;
     bool own32 = false;
-    SellArrays<float> sell32;                // sliced-ELL copy, when vec32 = SELL_LANES
+    SellArrays sell32;                // sliced-ELL copy, when vec32 = SELL_LANES
     // level 0 of the mixed solve with stored exact zeros: the FP64 values of
     // the FP32 copy's pattern, for the outer Krylov loop's SpMV (a zero adds
     // nothing to a row sum, so its result is the full matrix's)
     double *val64nz = nullptr;
+    // (in sell32's form instead where that is the FP32 copy's schedule)
     // transfer to level + 1 (P = agg map, R = P^T with ascending rows);
     // smoothed aggregation keeps P as a CSR with values and R's values too
     int nc = 0;
@@ -76,6 +77,12 @@ struct Level {
     }
     // the outer loop's FP64 operator: the zero-free copy when there is one
     DCsr<double> A64outer() const {
+        if (sell32.val64) {
+            DCsr<double> m = A64();
+            m.vec_lanes = SELL_LANES;
+            m.sell = sell32.view64();
+            return m;
+        }
         if (!val64nz) return A64();
         DCsr<double> m;
         m.n = n; m.nnz = nnz32; m.ia = ia32; m.ja = ja32; m.val = val64nz;

@@ -64,3 +64,27 @@ def test_sell_column_widths(monkeypatch, n, far):
     assert it_s == it_b > 0
     assert np.array_equal(x_s, x_b)
     assert np.linalg.norm(b - A @ x_s) / np.linalg.norm(b) < 1e-8
+
+
+def test_many_partial_sums(monkeypatch):
+    """More partial sums of the outer product than one CTA adds (above 16384 of
+    at most 256 rows each), the last of them of a part of its rows: the solve
+    still ends at its true residual, in the same bits on both schedules."""
+    n = 16384 * 256 + 4099
+    A = sp.diags([np.full(n, 4.25), -np.ones(n - 1), -np.ones(n - 1)], [0, 1, -1]).tocsr()
+    ia, ja, val = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    b = P.rhs_uniform(n, 5)
+    out = []
+    for schedule in ("sell", "0"):
+        monkeypatch.setenv("HZB_FP32_LANES", schedule)
+        S = hz.Solver(hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG, presmooth_iter=2,
+                                   postsmooth_iter=2),
+                      b200=hz.b200_param(precision=hz.HZB_PREC_MIXED,
+                                         matching=hz.HZB_MATCH_PARALLEL))
+        assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+        x = np.zeros(n)
+        out.append((S.solve_host(b, x), x))
+        S.close()
+    assert out[0][0] == out[1][0] > 0
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.linalg.norm(b - A @ out[0][1]) / np.linalg.norm(b) < 1e-8
