@@ -1480,7 +1480,8 @@ int reduce_blocks(int n) {
 // per thread: 83 us for the 260,000 partial sums of a product of 16.6 million
 // rows; 33 so by one CTA, which is why they go through k_reduce_part first).
 __global__ void __launch_bounds__(1024)
-k_reduce_final(const double *__restrict__ part, int np, double *out0, double *out1, int is_max) {
+k_reduce_final(const double *__restrict__ part, int np, double *out0, double *out1, int is_max,
+               double *h_out, const double *word, double *h_word) {
     __shared__ double sh[32];
     part += (size_t)blockIdx.x * np;
     double v = 0.0;
@@ -1498,7 +1499,13 @@ k_reduce_final(const double *__restrict__ part, int np, double *out0, double *ou
         }
     }
     v = is_max ? block_max(v, sh) : block_sum(v, sh);
-    if (threadIdx.x == 0) (blockIdx.x ? out1 : out0)[0] = v;
+    if (threadIdx.x == 0) {
+        (blockIdx.x ? out1 : out0)[0] = v;
+        if (h_out) {               // pinned host memory
+            *h_out = v;
+            *h_word = *word;
+        }
+    }
 }
 
 // a CTA's contiguous range of np partial sums
@@ -1514,7 +1521,8 @@ k_reduce_part(const double *__restrict__ part, int np, int per, double *out) {
 
 static int reduce_threads(int np) { return np > 4096 ? 1024 : 256; }
 int reduce_final(const double *part, int np, double *out, cudaStream_t s) {
-    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 0);
+    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 0, nullptr,
+                                                       nullptr, nullptr);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
@@ -1528,14 +1536,23 @@ int reduce_final_many(const double *part, int np, double *scratch, double *out, 
     count_launch();
     return reduce_final(scratch, g, out, s);
 }
+int reduce_final_host(const double *part, int np, double *out, double *h_out, const double *word,
+                      double *h_word, cudaStream_t s) {
+    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 0, h_out, word, h_word);
+    count_launch();
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
 int reduce_final2(const double *part, int np, double *out0, double *out1, cudaStream_t s) {
-    k_reduce_final<<<2, reduce_threads(np), 0, s>>>(part, np, out0, out1, 0);
+    k_reduce_final<<<2, reduce_threads(np), 0, s>>>(part, np, out0, out1, 0, nullptr,
+                                                       nullptr, nullptr);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
 }
 int reduce_final_max(const double *part, int np, double *out, cudaStream_t s) {
-    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 1);
+    k_reduce_final<<<1, reduce_threads(np), 0, s>>>(part, np, out, nullptr, 1, nullptr,
+                                                       nullptr, nullptr);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;

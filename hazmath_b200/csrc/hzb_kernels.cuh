@@ -281,6 +281,9 @@ int gs_run(const DCsr<T> &A, int kind, const int *rows, const int *set_ptr,
 // Deterministic reductions: partial sums per block, then an ordered final
 // sum into out[0].
 int reduce_final(const double *part, int nparts, double *out, cudaStream_t s);
+// the sum also to pinned host memory, with another device word
+int reduce_final_host(const double *part, int nparts, double *out, double *h_out,
+                      const double *word, double *h_word, cudaStream_t s);
 // the same for many partial sums; scratch: 1024 words
 int reduce_final_many(const double *part, int nparts, double *scratch, double *out,
                       cudaStream_t s);

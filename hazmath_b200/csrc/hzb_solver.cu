@@ -177,6 +177,7 @@ int KrylovWork::alloc(int nn, cudaStream_t st) {
     // on the stream the allocations were made on (the entry point's)
     HZB_CUDA(cudaMemsetAsync(sc, 0, SC_N * sizeof(double), st ? st : cur_stream()));
     if (!h_sc) HZB_CUDA(cudaMallocHost((void **)&h_sc, SC_N * sizeof(double)));
+    if (!ev) HZB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     return SUCCESS;
 }
 void KrylovWork::release_device() {
@@ -187,12 +188,12 @@ void KrylovWork::release() {
     release_device();
     if (h_sc) cudaFreeHost(h_sc);
     h_sc = nullptr;
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
 }
 
-static int fetch(hzb_solver *S, KrylovWork &w) {
-    HZB_CUDA(cudaMemcpyAsync(w.h_sc, w.sc, SC_N * sizeof(double),
-                             cudaMemcpyDeviceToHost, S->s));
-    HZB_CUDA(cudaStreamSynchronize(S->s));
+// the cycle's device waits, by the error word that came with the scalars
+static int waits_ok(hzb_solver *S, KrylovWork &w) {
     int e = 0;
     memcpy(&e, w.h_sc + SC_ERR, sizeof(int));
     if (e) {
@@ -201,6 +202,13 @@ static int fetch(hzb_solver *S, KrylovWork &w) {
         return ERROR_SOLVER_MISC;
     }
     return SUCCESS;
+}
+
+static int fetch(hzb_solver *S, KrylovWork &w) {
+    HZB_CUDA(cudaMemcpyAsync(w.h_sc, w.sc, SC_N * sizeof(double),
+                             cudaMemcpyDeviceToHost, S->s));
+    HZB_CUDA(cudaStreamSynchronize(S->s));
+    return waits_ok(S, w);
 }
 
 // the word the cycle's device waits raise (for paths that do not fetch the
@@ -1414,12 +1422,23 @@ int fcg_mixed(hzb_solver *S, const double *b, double *x, double tol, int maxit,
         k_fcg_update<<<G, 256, 0, s>>>(m, w.sc + SC_T1, w.sc + SC_T2, x, w.r, w.p, w.t,
                                         L0.b32, part4);
         count_launch();
-        HZB_TRY(reduce_final(part4, G, w.sc + SC_RR, s));
-        HZB_TRY(fetch(S, w));
+        // the residual's norm goes to the host by the kernel that adds it; while
+        // the host waits for it and decides, the cycle of the next step already
+        // runs, unless this step may be the last: a step seldom gains a digit (a
+        // wrong guess costs one cycle, and no result: the cycle writes nothing
+        // that a finished solve reads).  The gap between the steps was 20 us.
+        HZB_TRY(reduce_final_host(part4, G, w.sc + SC_RR, w.h_sc + SC_RR, w.sc + SC_ERR,
+                                  w.h_sc + SC_ERR, s));
+        HZB_CUDA(cudaEventRecord(w.ev, s));
+        const bool ahead = relres > 10 * tol;
+        if (ahead) HZB_TRY(cycles32(S));
+        HZB_CUDA(cudaEventSynchronize(w.ev));
+        HZB_TRY(waits_ok(S, w));
         absres = sqrt(w.h_sc[SC_RR]);
         relres = absres / normr0;
         print_info(prtlvl, STOP_REL_RES, iter, relres, absres, absres / absres0);
         absres0 = absres;
+        bool again = false;
         if (relres < tol) {
             // recompute the true FP64 residual before accepting
             HZB_TRY(spmv<double>(A, SPMV_RES, x, b, w.r, 1.0, nullptr, s));
@@ -1428,8 +1447,9 @@ int fcg_mixed(hzb_solver *S, const double *b, double *x, double tol, int maxit,
             relres = sqrt(w.h_sc[SC_X]) / normr0;
             if (relres < tol) break;
             HZB_TRY(d2f(m, w.r, L0.b32, s));   // the cycle starts from the true residual
+            again = true;
         }
-        HZB_TRY(cycles32(S));
+        if (!ahead || again) HZB_TRY(cycles32(S));
         k_dot2_partial_f<<<G, 512, 0, s>>>(m, L0.x32, w.t, w.r, part4);
         count_launch();
         HZB_TRY(reduce_final2(part4, G, w.sc + SC_ZT, w.sc + SC_T1, s));

@@ -111,6 +111,7 @@ struct KrylovWork {
     double *part = nullptr;   // 4 * reduce_blocks(n) + spmv_blocks(n)
     double *sc = nullptr;     // device scalars
     double *h_sc = nullptr;   // pinned host mirror
+    cudaEvent_t ev = nullptr; // when the scalars a step waits for are there
     int alloc(int n, cudaStream_t s = nullptr);   // scalars zeroed on s (or the current stream)
     void release_device();   // the device arrays (the pinned host mirror stays)
     void release();
