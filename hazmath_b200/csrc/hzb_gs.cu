@@ -18,17 +18,20 @@
 // anti-diagonal each touches a line of its own, and they fill the queue that
 // the shared loads of the computing warps go through), 0.6 with a set's copies
 // issued inside its barrier, 0.6 with a test per entry (200 instructions a set,
-// each waiting for the one before), 0.27 to 0.35 now.
+// each waiting for the one before), 0.27 to 0.35 with one set's loads behind the
+// other's, 0.18 to 0.23 now that parts of the CTA take the sets in turn.
 //   The row sum runs in CSR order from b_i with the diagonal skipped, each
 // value rounded as in gs_rows: the same bits.
 #include "hzb_solver.cuh"
 #include <algorithm>
+#include <type_traits>
 
 namespace hzb {
 
 namespace {
 
 constexpr int GS_ROWS = 256;           // a set's rows: one per computing thread
+constexpr int GS_TURNS = 3;            // parts of a CTA that take sets in turn
 constexpr int GS_SETS = 2048;          // sets of a schedule (their sizes lie in shared memory)
 constexpr int GS_BLOCK = 256;          // places per copy of x
 constexpr int GS_PAD = 8;              // set starts and slot pitches, in places
@@ -103,8 +106,16 @@ template <int Z>
 struct GsRow {
     unsigned c[Z / 2];              // two ring places each
     double v[Z];
-    __device__ __forceinline__ void load(const unsigned short *col, const double *val) {
-        if (Z % 4 == 0) {
+    // pairs of values `step` pairs apart
+    __device__ __forceinline__ void load(const unsigned short *col, const double *val,
+                                         int step = 1) {
+        if (Z == 8) {
+            const uint4 u = *reinterpret_cast<const uint4 *>(col);
+            c[0] = u.x;
+            c[1] = u.y;
+            c[2 % (Z / 2)] = u.z;
+            c[3 % (Z / 2)] = u.w;
+        } else if (Z % 4 == 0) {
 #pragma unroll
             for (int q = 0; q < Z / 4; ++q) {
                 const uint2 u = reinterpret_cast<const uint2 *>(col)[q];
@@ -117,26 +128,32 @@ struct GsRow {
         }
 #pragma unroll
         for (int q = 0; q < Z / 2; ++q) {
-            const double2 u = reinterpret_cast<const double2 *>(val)[q];
+            const double2 u = reinterpret_cast<const double2 *>(val)[q * step];
             v[2 * q] = u.x;
             v[2 * q + 1] = u.y;
         }
     }
-    __device__ __forceinline__ double sum(const double *ring, double acc) const {
-        double x[Z];
+    __device__ __forceinline__ void gather(const double *ring, double *x) const {
 #pragma unroll
         for (int q = 0; q < Z / 2; ++q) {
             x[2 * q] = ring[c[q] & 0xffffu];
             x[2 * q + 1] = ring[c[q] >> 16];
         }
+    }
+    __device__ __forceinline__ double finish(const double *x, double acc) const {
 #pragma unroll
         for (int q = 0; q < Z; ++q) acc -= v[q] * x[q];
         return acc;
     }
+    __device__ __forceinline__ double sum(const double *ring, double acc) const {
+        double x[Z];
+        gather(ring, x);
+        return finish(x, acc);
+    }
 };
 
-template <int KIND>
-__global__ void __launch_bounds__(GS_ROWS + 32, 1)
+template <int KIND, int UZ>
+__global__ void __launch_bounds__((UZ ? GS_TURNS : 1) * GS_ROWS + 32, 1)
 k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
     extern __shared__ __align__(16) unsigned char smem[];
     int4 *info = reinterpret_cast<int4 *>(smem);
@@ -147,7 +164,8 @@ k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
         reinterpret_cast<unsigned long long *>(stage0 + A.stages * stage_bytes);
     unsigned long long *empty = full + A.stages;
     __shared__ int s_dead;
-    const int t = threadIdx.x, ns = A.ns;
+    // threads that compute, and those of them on one set
+    const int ns = A.ns, t = threadIdx.x, all = blockDim.x - 32, nt = UZ ? all / GS_TURNS : all;
     for (int k = t; k < ns; k += blockDim.x) info[k] = A.info[k];
     if (t == 0) {
         s_dead = 0;
@@ -159,9 +177,9 @@ k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (t >= GS_ROWS) {
+    if (t >= all) {
         // groups of sets into their stages, and x as far as their rows reach
-        if (t > GS_ROWS) return;
+        if (t > all) return;
         int loaded = 0, to = 0, k = 0;  // places of x copied or on their way; the stage
         unsigned parity = 1;            // the first round finds every stage empty
         for (int s0 = 0; s0 < ns; s0 += A.group) {
@@ -192,73 +210,136 @@ k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
         }
         return;
     }
-    int k = 0, in_group = 0;            // the stage at hand, sets of it begun
-    unsigned parity = 0;
-    int e0 = 0, x0 = 0;                 // the group's first entry and place
-    const unsigned char *stage = stage0;
     const int val_bytes = A.E * 8, col_at = val_bytes + A.R * 16;
-    unsigned long long *release = nullptr;   // the stage that the next barrier frees
-    for (int s = 0; s < ns; ++s) {
-        const int4 I = info[s];
-        if (in_group == 0) {
-            bar_wait(full + k, parity, &s_dead, err);
-            x0 = I.x;
-            e0 = I.w;
-            stage = stage0 + k * stage_bytes;
+    auto store = [&](const int4 &I, int row, double acc, double dinv) {
+        if (row >= gs_rows(I)) return;
+        const int place = I.x + row, at = I.z + row;
+        double *px = ring + (at < A.ring ? at : at - A.ring);
+        if (KIND == 0) {
+            const double xn = acc * dinv;
+            *px = xn;
+            A.x[place] = xn;
+        } else if (place != A.skip_place && fabs(dinv) > double(SMALLREAL)) {
+            const double xn = KIND == 1 ? w * (acc / dinv) + (1 - w) * *px : acc / dinv;
+            *px = xn;
+            A.x[place] = xn;
         }
-        const int Z = gs_width(I);
-        const bool on = t < gs_rows(I);
-        const int at = on ? I.w - e0 + t * Z : 0;   // idle threads load the first row
-        const double *val = reinterpret_cast<const double *>(stage) + at;
-        const unsigned short *col = reinterpret_cast<const unsigned short *>(stage + col_at) + at;
-        const double2 bd = reinterpret_cast<const double2 *>(stage + val_bytes)[on ? I.x - x0 + t : 0];
+    };
+    if constexpr (UZ > 0) {
+        // Three parts of the CTA take the sets in turn: a part loads its next set
+        // (370 cycles) while the others finish one each (190, and 70 for the
+        // barrier), so that between two sets lie a barrier, the loads of x and
+        // the sums only.
+        const int turn = t / nt, row = t - turn * nt, warp0 = row & ~31;
+        int in = turn, k = 0;           // the set's place in its group, the group's stage
+        unsigned parity = 0;
+        auto place = [&]() {
+            while (in >= A.group) {
+                in -= A.group;
+                if (++k == A.stages) {
+                    k = 0;
+                    parity ^= 1u;
+                }
+            }
+        };
+        GsRow<UZ> r;
+        double2 bd = make_double2(0.0, 0.0);
+        int4 I = make_int4(0, 0, 0, 0);
+        auto fetch = [&](int s) {
+            I = info[s];
+            if (warp0 >= gs_rows(I)) return;
+            bar_wait(full + k, parity, &s_dead, err);
+            const int4 F = info[s - in];
+            const unsigned char *stage = stage0 + k * stage_bytes;
+            const int at = row < gs_rows(I) ? row : 0;   // idle threads load the first row
+            const double *val = reinterpret_cast<const double *>(stage) + (I.w - F.w);
+            const unsigned short *col =
+                reinterpret_cast<const unsigned short *>(stage + col_at) + (I.w - F.w);
+            r.load(col + at * UZ, val + 2 * at, gs_pitch(gs_rows(I)));
+            bd = reinterpret_cast<const double2 *>(stage + val_bytes)[I.x - F.x + at];
+        };
+        place();
+        if (turn < ns) fetch(turn);
+        for (int s = turn; s < ns; s += GS_TURNS) {
+            // the set before is complete, and its group when this set begins one
+            __syncwarp();
+            if (s) asm volatile("bar.sync %0, %1;" ::"r"(1 + turn), "r"(2 * nt) : "memory");
+            if (in == 0 && s && row == 0)
+                asm volatile("mbarrier.arrive.shared.b64 _, [%0];"
+                             ::"r"(smem_u32(empty + (k ? k : A.stages) - 1)) : "memory");
+            if (warp0 < gs_rows(I)) {
+                double x[UZ];
+                r.gather(ring, x);
+                store(I, row, r.finish(x, bd.x), bd.y);
+            }
+            // what this part wrote to the ring in a group comes before the copies
+            // that replace it
+            if (in + GS_TURNS >= A.group) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (s + 1 < ns)
+                asm volatile("bar.arrive %0, %1;" ::"r"(1 + (turn + 1) % GS_TURNS), "r"(2 * nt) : "memory");
+            in += GS_TURNS;
+            place();
+            if (s + GS_TURNS < ns) fetch(s + GS_TURNS);
+        }
+    } else {
+        int k = 0, in_group = 0;        // the stage at hand, sets of it begun
+        unsigned parity = 0;
+        int e0 = 0, x0 = 0;             // the group's first entry and place
+        const unsigned char *stage = stage0;
+        unsigned long long *release = nullptr;   // the stage that the next barrier frees
         // the previous set is complete, and its group when this set begins one
         auto barrier = [&]() {
-            asm volatile("bar.sync 1, %0;" ::"n"(GS_ROWS) : "memory");
+            asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
             if (release && t == 0)
                 asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(smem_u32(release))
                              : "memory");
         };
-        double acc;
-        switch (Z) {   // the same for every thread
-        case 0: barrier(); acc = bd.x; break;
-        case 2: { GsRow<2> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
-        case 4: { GsRow<4> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
-        case 6: { GsRow<6> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
-        case 8: { GsRow<8> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
-        default: {
-            barrier();
-            acc = bd.x;
-            for (int u = 0; u < Z; u += 2) {
-                GsRow<2> r;
-                r.load(col + u, val + u);
-                acc = r.sum(ring, acc);
+        for (int s = 0; s < ns; ++s) {
+            const int4 I = info[s];
+            if (in_group == 0) {
+                bar_wait(full + k, parity, &s_dead, err);
+                x0 = I.x;
+                e0 = I.w;
+                stage = stage0 + k * stage_bytes;
             }
-        }
-        }
-        release = nullptr;
-        if (on) {
-            const int place = I.x + t;
-            double *px = ring + (I.z + t < A.ring ? I.z + t : I.z + t - A.ring);
-            if (KIND == 0) {
-                const double xn = acc * bd.y;
-                *px = xn;
-                A.x[place] = xn;
-            } else if (place != A.skip_place && fabs(bd.y) > double(SMALLREAL)) {
-                const double xn = KIND == 1 ? w * (acc / bd.y) + (1 - w) * *px : acc / bd.y;
-                *px = xn;
-                A.x[place] = xn;
+            const int Z = gs_width(I);
+            const bool on = t < gs_rows(I);
+            const int at = on ? I.w - e0 + t * Z : 0;   // idle threads load the first row
+            const double *val = reinterpret_cast<const double *>(stage) + at;
+            const unsigned short *col =
+                reinterpret_cast<const unsigned short *>(stage + col_at) + at;
+            const double2 bd =
+                reinterpret_cast<const double2 *>(stage + val_bytes)[on ? I.x - x0 + t : 0];
+            double acc;
+            switch (Z) {   // the same for every thread
+            case 0: barrier(); acc = bd.x; break;
+            case 2: { GsRow<2> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+            case 4: { GsRow<4> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+            case 6: { GsRow<6> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+            case 8: { GsRow<8> r; r.load(col, val); barrier(); acc = r.sum(ring, bd.x); break; }
+            default: {
+                barrier();
+                acc = bd.x;
+                for (int u = 0; u < Z; u += 2) {
+                    GsRow<2> r;
+                    r.load(col + u, val + u);
+                    acc = r.sum(ring, acc);
+                }
             }
-        }
-        if (++in_group == A.group) {
-            // what this group wrote to the ring comes before the copies that
-            // replace it
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            in_group = 0;
-            release = empty + k;
-            if (++k == A.stages) {
-                k = 0;
-                parity ^= 1u;
+            }
+            release = nullptr;
+            store(I, t, acc, bd.y);
+            if (++in_group == A.group) {
+                // what this group wrote to the ring comes before the copies that
+                // replace it
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                in_group = 0;
+                release = empty + k;
+                if (++k == A.stages) {
+                    k = 0;
+                    parity ^= 1u;
+                }
             }
         }
     }
@@ -323,27 +404,33 @@ __global__ void k_gs_dist(int n, const int *__restrict__ ia, const int *__restri
 // one CTA per set: the entries row by row, zeros against the ring's zero place
 // behind a shorter row (subtracting +0.0 * 0.0 changes nothing)
 __global__ void __launch_bounds__(GS_ROWS)
-k_gs_fill(const int4 *__restrict__ info, int ring, const int *__restrict__ src,
+k_gs_fill(const int4 *__restrict__ info, int ring, int uniform, const int *__restrict__ src,
           const int *__restrict__ place, const int *__restrict__ ia, const int *__restrict__ ja,
           const double *__restrict__ a, unsigned short *col, double *val) {
     const int4 I = info[blockIdx.x];
     const int t = threadIdx.x, Z = gs_width(I);
     if (t >= gs_pitch(gs_rows(I))) return;
     const int i = t < gs_rows(I) ? src[I.x + t] : -1;
+    const int pitch = gs_pitch(gs_rows(I));
     col += I.w + t * Z;
-    val += I.w + t * Z;
+    val += I.w;
+    // pair q of row t: with one width for all sets side by side with the other
+    // rows' (a warp's loads are then free of conflicts), else with the row's own
+    auto at = [&](int u) {
+        return uniform ? (u / 2 * pitch + t) * 2 + u % 2 : t * Z + u;
+    };
     int u = 0;
     if (i >= 0)
         for (int k = ia[i]; k < ia[i + 1]; ++k) {
             const int j = ja[k];
             if (j == i) continue;
             col[u] = (unsigned short)(place[j] % ring);
-            val[u] = a[k];
+            val[at(u)] = a[k];
             ++u;
         }
     for (; u < Z; ++u) {
         col[u] = (unsigned short)ring;
-        val[u] = 0.0;
+        val[at(u)] = 0.0;
     }
 }
 
@@ -401,6 +488,16 @@ int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
         e = cudaMemcpyAsync(&dist, d_width + ns, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return done(false);
+    // Rows of up to 8 entries: one width for all sets, so that the next set's
+    // loads need no branch and run ahead of the barrier (0.35 us a set of a 2D
+    // level with each set its own width, 0.18 to 0.23 with the longest row's).
+    const int longest = *std::max_element(width.begin(), width.end());
+    const int uniform = longest <= 8 ? std::max(2, longest) : 0;
+    int max_rows = 0;
+    for (int k = 0; k < ns; ++k) {
+        if (uniform) width[k] = uniform;
+        max_rows = std::max(max_rows, sc->h_ptr[k + 1] - sc->h_ptr[k]);
+    }
     std::vector<int4> info(ns);
     long long ents = 0;
     for (int k = 0; k < ns; ++k) {
@@ -437,13 +534,15 @@ int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
         return done(false);
     e = cudaMemcpyAsync(G.info, info.data(), sizeof(int4) * ns, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        k_gs_fill<<<ns, GS_ROWS, 0, s>>>(G.info, ring, G.src, G.place, A.ia, A.ja, A.val,
+        k_gs_fill<<<ns, GS_ROWS, 0, s>>>(G.info, ring, uniform, G.src, G.place, A.ia, A.ja, A.val,
                                          G.col, G.val);
         count_launch();
         e = cudaMemcpyAsync(&G.last_place, G.place + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // and the host arrays above
     }
     G.ns = ns;
+    G.uniform = uniform;
+    G.threads = (max_rows + 31) / 32 * 32;
     G.group = group;
     G.E = E;
     G.R = R;
@@ -458,13 +557,26 @@ int gs_stream_sweep(const Schedule &sc, const double *d, const double *b, double
                     int kind, double w, int *err, cudaStream_t s) {
     const GsStream &G = sc.stream;
     const int skip_place = (kind & GS_SKIP_LAST) ? G.last_place : -1;   // SGS leaves row n - 1
-    auto kernel = (kind & 15) == 0 ? k_gs_stream<0> : (kind & 15) == 1 ? k_gs_stream<1> : k_gs_stream<2>;
+    auto of_kind = [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        switch (G.uniform) {
+        case 2: return k_gs_stream<K, 2>;
+        case 4: return k_gs_stream<K, 4>;
+        case 6: return k_gs_stream<K, 6>;
+        case 8: return k_gs_stream<K, 8>;
+        default: return k_gs_stream<K, 0>;
+        }
+    };
+    const int K = kind & 15;
+    auto kernel = K == 0   ? of_kind(std::integral_constant<int, 0>())
+                  : K == 1 ? of_kind(std::integral_constant<int, 1>())
+                           : of_kind(std::integral_constant<int, 2>());
     HZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)GS_SMEM));
     k_gs_in<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, b, d, x, G.bd, G.xp);
     const GsSweep A = {G.info, G.col, G.val, G.bd, G.xp, G.ns, G.group, G.E, G.R, G.stages,
                        G.ring, G.dist, G.places, skip_place};
-    kernel<<<1, GS_ROWS + 32, gs_smem(G.ns, G.E, G.R, G.ring, G.stages), s>>>(A, w, err);
+    kernel<<<1, G.threads * (G.uniform ? GS_TURNS : 1) + 32, gs_smem(G.ns, G.E, G.R, G.ring, G.stages), s>>>(A, w, err);
     k_gs_out<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, G.xp, x);
     count_launch(3);
     HZB_LAUNCH_CHECK();

@@ -85,6 +85,7 @@ int smoother_diagonals(const DCsr<double> &A, double *d_jac, double *d_gs_f,
 struct GsStream {
     int ns = 0, group = 0, E = 0, R = 0, ring = 0, stages = 0;   // stages 0: no stream
     int dist = 0, places = 0, last_place = 0;
+    int uniform = 0, threads = 0;                     // every set's width (0: its own); rows of the largest
     int4 *info = nullptr;
     int *src = nullptr, *place = nullptr;             // row of a place, place of a row
     unsigned short *col = nullptr;

@@ -267,3 +267,42 @@ def test_streamed_gauss_seidel_vs_oracle(port, name, sm, pre):
     x = dev(x0)
     assert hz.lib().hzb_smoother_device(sm, pre, 2, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
     assert np.array_equal(host(x), port.smooth(sm, pre, 2, ia, ja, val, b, x0, relax=1.15))
+
+
+def _stencil(N, ny, centre, side, corner):
+    """5- or 9-point stencil on N x ny points, row by row; ny = 1: a chain."""
+    ia, ja, val = [0], [], []
+    for i in range(N * ny):
+        y, x = divmod(i, N)
+        for dy in (-1, 0, 1):
+            for dx in (-1, 0, 1):
+                v = centre if dx == dy == 0 else corner * (1 + 0.1 * dx) if dx and dy else side
+                if v and 0 <= y + dy < ny and 0 <= x + dx < N:
+                    ja.append((y + dy) * N + x + dx)
+                    val.append(v)
+        ia.append(len(ja))
+    return np.array(ia, np.int32), np.array(ja, np.int32), np.array(val)
+
+
+GS_WIDTHS = {
+    "chain_2": lambda: _stencil(2, 1, 2.5, -1.0, 0.0),     # fewer sets than take turns
+    "chain_4": lambda: _stencil(4, 1, 2.5, -1.0, 0.0),
+    "chain_700": lambda: _stencil(700, 1, 2.5, -1.0, 0.0),  # 2 entries a row, sets of one row
+    "five_70": lambda: _stencil(70, 70, 4.5, -1.0, 0.0),   # 4
+    "seven_40": lambda: P.aniso2d_p1(40, 0.1, 0.5),        # 6
+    "nine_64": lambda: _stencil(64, 64, 9.0, -1.0, -0.5),  # 8
+}
+
+
+@pytest.mark.parametrize("name", sorted(GS_WIDTHS))
+@pytest.mark.parametrize("sm,pre", [(2, 1), (3, 1), (6, 0)])
+def test_streamed_gauss_seidel_row_widths(port, name, sm, pre):
+    """Schedules streamed with one width for all sets, for each width."""
+    ia, ja, val = GS_WIDTHS[name]()
+    n = len(ia) - 1
+    rng = np.random.default_rng(n + sm)
+    b, x0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    A = DevCSR(ia, ja, val)
+    x = dev(x0)
+    assert hz.lib().hzb_smoother_device(sm, pre, 3, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
+    assert np.array_equal(host(x), port.smooth(sm, pre, 3, ia, ja, val, b, x0, relax=1.15))
