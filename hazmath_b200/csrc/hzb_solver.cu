@@ -687,8 +687,10 @@ int ensure_fp32(hzb_solver *S) {
             }
             // the outer product reads the same rows as the sweeps: where the
             // sliced form was the fastest for them it is for FP64 too (364 us
-            // staged, 290 sliced on 16.6 million rows)
-            if (l == 0 && !S->batch && L.vec32 == SELL_LANES && L.sell32.npad) {
+            // staged, 290 sliced on 16.6 million rows); not where that would
+            // take a copy of the caller's values in place of the values
+            if (l == 0 && !S->batch && L.vec32 == SELL_LANES && L.sell32.npad &&
+                (L.own32 || L.own_A)) {
                 HZB_TRY(sell_values64(&L.sell32, L.ia32, L.own32 ? L.val64nz : L.val, S->s));
                 dfree(L.val64nz);
             }
