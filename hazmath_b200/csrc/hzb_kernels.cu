@@ -532,7 +532,7 @@ template int spmv<float>(const DCsr<float> &, int, const float *, const float *,
 // reuses them instead of timing the candidates again.
 namespace {
 std::mutex tune_mu;
-std::map<std::pair<int, int>, int> tune_bundle_rows, tune_fp32_lanes;
+std::map<std::pair<int, int>, int> tune_bundle_rows, tune_fp32_lanes, tune_sell64;
 bool tune_lookup(std::map<std::pair<int, int>, int> &m, int n, int nnz, int *v) {
     std::lock_guard<std::mutex> g(tune_mu);
     auto it = m.find({n, nnz});
@@ -579,6 +579,37 @@ int autotune_bundle(DCsr<double> &A, const double *x, double *y, cudaStream_t s)
     A.bundle_rows = best_rows;
     A.bundle_cap = best_cap;
     tune_store(tune_bundle_rows, A.n, A.nnz, best_rows);
+    return SUCCESS;
+}
+
+int sell64_known(int n, int nnz) {
+    int v = -1;
+    tune_lookup(tune_sell64, n, nnz, &v);
+    return v;
+}
+
+int autotune_sell64(const DCsr<double> &A, const double *b, const double *x, double *xn,
+                    bool *sliced, cudaStream_t s) {
+    cudaEvent_t e0, e1;
+    HZB_CUDA(cudaEventCreate(&e0));
+    HZB_CUDA(cudaEventCreate(&e1));
+    float ms[2] = {0.f, 0.f};
+    int rc = SUCCESS;
+    for (int q = 0; q < 2 && !rc; ++q) {
+        DCsr<double> B = A;
+        B.vec_lanes = q ? SELL_LANES : 0;
+        rc = l1_sweep<double>(B, b, x, xn, nullptr, s);   // warm
+        cudaEventRecord(e0, s);
+        for (int r = 0; r < 3 && !rc; ++r) rc = l1_sweep<double>(B, b, x, xn, nullptr, s);
+        cudaEventRecord(e1, s);
+        cudaEventSynchronize(e1);
+        cudaEventElapsedTime(&ms[q], e0, e1);
+    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    if (rc) return rc;
+    *sliced = ms[1] < ms[0];
+    tune_store(tune_sell64, A.n, A.nnz, *sliced ? 1 : 0);
     return SUCCESS;
 }
 
@@ -854,9 +885,9 @@ template <typename T>
 int l1_sweep(const DCsr<T> &A, const T *b, const T *x, T *xn,
              const float *omega, cudaStream_t s) {
     if (A.n <= 0) return SUCCESS;
+    if (A.vec_lanes == SELL_LANES && A.sell.npad > 0 && !A.act)
+        return sell_l1_sweep<T>(A, b, x, xn, omega, s);
     if constexpr (sizeof(T) == 4) {
-        if (A.vec_lanes == SELL_LANES && A.sell.npad > 0 && !A.act)
-            return sell_l1_sweep(A, b, x, xn, omega, s);
         if (A.vec_lanes > 0) return l1_vec_launch(A, b, x, xn, omega, s);
     }
     switch (A.bundle_rows) {
@@ -1725,7 +1756,11 @@ __global__ void k_nz_fill(int n, const int *__restrict__ ia, const int *__restri
          i += gridDim.x * blockDim.x) {
         int p = ia32[i];
         for (int k = ia[i]; k < ia[i + 1]; ++k)
-            if (a[k] != 0.0) { ja32[p] = ja[k]; a32[p] = (float)a[k]; ++p; }
+            if (a[k] != 0.0) {
+                ja32[p] = ja[k];
+                if (a32) a32[p] = (float)a[k];
+                ++p;
+            }
     }
 }
 int csr_nonzero_count(int n, const int *ia, const double *a, int *cnt, cudaStream_t s) {

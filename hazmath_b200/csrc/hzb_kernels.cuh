@@ -81,6 +81,11 @@ int bundle_capacity(int n, const int *ia, cudaStream_t s, int *cap);
 int bundle_capacity_rows(int n, int rows, const int *ia, cudaStream_t s, int *cap);
 // Picks the bundle size (64/128/256 rows) of A by timing its SpMV on x -> y.
 int autotune_bundle(DCsr<double> &A, const double *x, double *y, cudaStream_t s);
+// Whether A's sweep is faster from its sliced copy (A.sell) than staged, by timing;
+// an earlier answer for a level of this shape (-1: none).
+int autotune_sell64(const DCsr<double> &A, const double *b, const double *x, double *xn,
+                    bool *sliced, cudaStream_t s);
+int sell64_known(int n, int nnz);
 // Picks the FP32 schedule (staged bundles or 4/8/16 lanes per row) by timing
 // the l1-Jacobi sweep of A on b, x -> xn.
 int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cudaStream_t s);
@@ -89,13 +94,14 @@ int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cud
 bool fp32_schedule_known(int n, int nnz, int *lanes);
 
 // Sliced-ELL copy of a CSR matrix (hzb_sell.cu); *out stays empty
-// (npad 0) when its slice offsets would overflow int.  Sweep and SpMV on it
+// (npad 0) when its slice offsets would overflow int; a null: no FP32 values.  Sweep and SpMV on it
 // (no activity array, no SPMV_Y_DOT).
 int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
                cudaStream_t s);
 int sell_values64(SellArrays *S, const int *ia, const double *a, cudaStream_t s);
-int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
-                  const float *omega, cudaStream_t s);
+template <typename T>
+int sell_l1_sweep(const DCsr<T> &A, const T *b, const T *x, T *xn, const float *omega,
+                  cudaStream_t s);
 template <typename T>
 int sell_spmv(const DCsr<T> &A, int mode, const T *x, const T *b, T *y, T alpha, T *part,
               cudaStream_t s);

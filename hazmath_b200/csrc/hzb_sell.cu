@@ -112,7 +112,7 @@ k_sell_fill(const int *__restrict__ first, const int *__restrict__ pairs,
         const int lo = __reduce_min_sync(0xffffffffu, c);
         if (len == 0) c = lo;
         const int at = sell_at(u, w, lane);
-        val[(size_t)f0 * SELL_C + at] = u < len ? a[k0 + u] : 0.f;
+        if (val) val[(size_t)f0 * SELL_C + at] = u < len ? a[k0 + u] : 0.f;
         if (lane == 0) reinterpret_cast<int *>(base + p0 + u / 2)[u % 2] = lo;
         unsigned short *q = col + (size_t)l0 * SELL_C;
         if (wide) reinterpret_cast<int *>(q)[at] = c;
@@ -214,17 +214,18 @@ __device__ __forceinline__ void sell_row(const SellView<T> &V, int r, const T *_
     else sell_slice<T, L1, true>(V, h, r % SELL_C, x, t, d);
 }
 
+template <typename T>
 __global__ void __launch_bounds__(SELL_WIN, 8)
-k_l1_sell(int n, const __grid_constant__ SellView<float> V, const float *__restrict__ b,
-          const float *__restrict__ x, float *__restrict__ xn, const float *__restrict__ omega) {
+k_l1_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ b,
+          const T *__restrict__ x, T *__restrict__ xn, const float *__restrict__ omega) {
     const int r = blockIdx.x * SELL_WIN + threadIdx.x;
     const unsigned sl = __ldcs(V.slot + r);
     const int i = blockIdx.x * SELL_WIN + (int)(sl & SELL_ROW);
     if (i >= n) return;
-    float t = __ldcs(b + i), d = 0.f;
-    sell_row<float, true>(V, r, x, t, d);
-    float xi = x[i];
-    if (fabsf(d) > float(SMALLREAL)) xi += omega ? omega[i] * (t / d) : t / d;
+    T t = __ldcs(b + i), d = T(0);
+    sell_row<T, true>(V, r, x, t, d);
+    T xi = x[i];
+    if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[i]) * (t / d) : t / d;
     xn[i] = xi;
 }
 
@@ -305,7 +306,7 @@ int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *
     if (htot[0] * SELL_C > (unsigned long long)(INT_MAX / 2)) goto done;
     for (int q = 0; q < 3 && !rc; ++q)
         rc = scan_exclusive(cnt + (size_t)q * nsl, ptr + q * ((size_t)nsl + 1), nsl, tmp, s);
-    if (rc || (rc = dalloc(&S.val, std::max(1ull, htot[0] * SELL_C))) ||
+    if (rc || (a && (rc = dalloc(&S.val, std::max(1ull, htot[0] * SELL_C)))) ||
         (rc = dalloc(&S.base, std::max(1ull, htot[1]))) ||
         (rc = dalloc(&S.col, std::max(1ull, htot[2] * SELL_C))))
         goto done;
@@ -344,13 +345,18 @@ void SellArrays::release() {
     npad = 0;
 }
 
-int sell_l1_sweep(const DCsr<float> &A, const float *b, const float *x, float *xn,
-                  const float *omega, cudaStream_t s) {
-    k_l1_sell<<<A.sell.npad / SELL_WIN, SELL_WIN, 0, s>>>(A.n, A.sell, b, x, xn, omega);
+template <typename T>
+int sell_l1_sweep(const DCsr<T> &A, const T *b, const T *x, T *xn, const float *omega,
+                  cudaStream_t s) {
+    k_l1_sell<T><<<A.sell.npad / SELL_WIN, SELL_WIN, 0, s>>>(A.n, A.sell, b, x, xn, omega);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
 }
+template int sell_l1_sweep<float>(const DCsr<float> &, const float *, const float *, float *,
+                                  const float *, cudaStream_t);
+template int sell_l1_sweep<double>(const DCsr<double> &, const double *, const double *,
+                                   double *, const float *, cudaStream_t);
 
 template <typename T>
 int sell_spmv(const DCsr<T> &A, int mode, const T *x, const T *b, T *y, T alpha, T *part,

@@ -137,6 +137,7 @@ void Level::release() {
     dfree(val32);
     dfree(val64nz);
     sell32.release();
+    sell64.release();
     if (own32) { dfree(ia32); dfree(ja32); }
     ia32 = ja32 = nullptr;
     own32 = false;
@@ -713,6 +714,52 @@ int ensure_fp32(hzb_solver *S) {
 // ---------------------------------------------------------------------------
 // setup, amg_setup_unsmoothP_unsmoothR (amg_setup_ua.c:1228-1452)
 // ---------------------------------------------------------------------------
+// The sliced copy of a large level of an FP64 solve, where its sweep is faster:
+// rows in CSR order without the stored zeros, which add nothing, so the same bits.
+// Not of a matrix that stays in the caller's arrays.  Sweeps of the first three
+// coarse levels of a 127^3 system 40, 29 and 21 us staged, 26, 18 and 13 sliced.
+static int level_sliced64(hzb_solver *S, Level &L) {
+    if (!L.own_A || sell64_known(L.n, L.nnz) == 0) return SUCCESS;
+    cudaStream_t s = S->s;
+    int *cnt = nullptr, *ia = nullptr, *ja = nullptr, *tmp = nullptr, nz = 0;
+    double *val = nullptr;
+    int rc = SUCCESS;
+    if ((rc = dalloc(&cnt, L.n)) || (rc = dalloc(&ia, L.n + 1)) ||
+        (rc = dalloc(&tmp, scan_tmp_size(L.n + 1))) ||
+        (rc = csr_nonzero_count(L.n, L.ia, L.val, cnt, s)) ||
+        (rc = scan_exclusive(cnt, ia, L.n, tmp, s)))
+        goto done;
+    if (cudaMemcpyAsync(&nz, ia + L.n, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess) {
+        rc = ERROR_SOLVER_MISC;
+        goto done;
+    }
+    if (nz < L.nnz) {
+        if ((rc = dalloc(&ja, std::max(1, nz))) || (rc = dalloc(&val, std::max(1, nz))) ||
+            (rc = csr_nonzero_fill(L.n, L.ia, L.ja, L.val, ia, ja, nullptr, s)) ||
+            (rc = csr_nonzero_fill64(L.n, L.ia, L.val, ia, val, s)))
+            goto done;
+    }
+    if ((rc = sell_build(L.n, ia, val ? ja : L.ja, nullptr, &L.sell64, s)) || !L.sell64.npad ||
+        (rc = sell_values64(&L.sell64, ia, val ? val : L.val, s)))
+        goto done;
+    if (sell64_known(L.n, L.nnz) < 0) {
+        bool sliced = false;
+        if ((rc = vzero<double>(L.n, L.b, s)) ||
+            (rc = autotune_sell64(L.A64(), L.b, L.x, L.w, &sliced, s)))
+            goto done;
+        if (!sliced) L.sell64.release();
+    }
+done:
+    if (rc) L.sell64.release();
+    dfree(cnt);
+    dfree(ia);
+    dfree(tmp);
+    dfree(ja);
+    dfree(val);
+    return rc;
+}
+
 int level_smoother_data(hzb_solver *S, Level &L) {
     const int sm = S->amg.smoother;
     const bool gsf = smoother_needs_gs(sm);
@@ -974,6 +1021,9 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
             HZB_TRY(autotune_bundle(A, L.x, L.w, s));
             L.bundle_rows = A.bundle_rows;
             L.bundle_cap = A.bundle_cap;
+            if (S->amg.smoother == SMOOTHER_L1DIAG && S->bp.precision == HZB_PREC_FP64 &&
+                !batch && l < S->nl - 1 && L.nnz > SMALL_NNZ_64)
+                HZB_TRY(level_sliced64(S, L));
         }
     }
     // the merged kernels of the l1-Jacobi cycle's small levels read the norms

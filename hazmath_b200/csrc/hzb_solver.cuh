@@ -26,6 +26,9 @@ struct Level {
     float *val32 = nullptr;
     bool own32 = false;
     SellArrays sell32;                // sliced-ELL copy, when vec32 = SELL_LANES
+    // FP64 solves by the l1-Jacobi cycle, large levels: the matrix without its
+    // stored zeros (they add nothing to a row) in that form
+    SellArrays sell64;
     // level 0 of the mixed solve with stored exact zeros: the FP64 values of
     // the FP32 copy's pattern, for the outer Krylov loop's SpMV (a zero adds
     // nothing to a row sum, so its result is the full matrix's)
@@ -73,6 +76,10 @@ struct Level {
         m.n = n; m.nnz = nnz; m.ia = ia; m.ja = ja; m.val = val; m.bundle_cap = bundle_cap;
         m.bundle_rows = bundle_rows;
         m.act = act;
+        if (sell64.npad) {
+            m.vec_lanes = SELL_LANES;
+            m.sell = sell64.view64();
+        }
         return m;
     }
     // the outer loop's FP64 operator: the zero-free copy when there is one

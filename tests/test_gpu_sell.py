@@ -88,3 +88,29 @@ def test_many_partial_sums(monkeypatch):
     assert out[0][0] == out[1][0] > 0
     assert np.array_equal(out[0][1], out[1][1])
     assert np.linalg.norm(b - A @ out[0][1]) / np.linalg.norm(b) < 1e-8
+
+
+@pytest.mark.parametrize("N", [48, 64])
+def test_fp64_sliced_levels_bitwise(N):
+    """An FP64 solve whose large levels run from zero-free sliced copies: set up
+    from host arrays (level 0 too) and from device arrays (level 0 stays in the
+    caller's), the same iterates bit for bit."""
+    torch = pytest.importorskip("torch")
+    ia, ja, val = P.kuhn3d_p1(N, P.lognormal_field(N, 1.0, 8.0, 7))
+    b = P.rhs_uniform(len(ia) - 1, 8)
+    amg = hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG, presmooth_iter=2, postsmooth_iter=2)
+    par = hz.b200_param(precision=hz.HZB_PREC_FP64, matching=hz.HZB_MATCH_PARALLEL)
+    S = hz.Solver(amg, b200=par)
+    assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+    x = np.zeros(len(b))
+    it = S.solve_host(b, x)
+    S.close()
+    D = hz.Solver(amg, b200=par)
+    dia, dja, dval, db = (torch.from_numpy(np.ascontiguousarray(a)).cuda()
+                          for a in (ia, ja, val, b))
+    dx = torch.zeros_like(db)
+    assert D.setup_device(len(b), len(ja), dia.data_ptr(), dja.data_ptr(),
+                          dval.data_ptr()) == 0, hz.last_error()
+    assert D.solve_device(db.data_ptr(), dx.data_ptr()) == it > 0
+    D.close()
+    assert np.array_equal(x, dx.cpu().numpy())
