@@ -393,6 +393,10 @@ extern "C" INT hzb_time_kernel(hzb_solver *S, INT which, INT level, INT reps,
     // the FP32 kernels read the zero-free copy
     const double n = L.n, nnz = f32 ? L.nnz32 : L.nnz;
     double bytes = nnz * (vb + 4.0) + 4.0 * (n + 1);
+    // a sliced copy: 16-bit columns above a base per 32 entries, a word per row and
+    // 16 bytes per 32 rows
+    const SellArrays &sl = f32 ? L.sell32 : L.sell64;
+    if (sl.npad && which != HZB_K_GS64) bytes = sl.nval * (vb + 2.125) + 4.5 * n;
     switch (which) {
     case HZB_K_SPMV64: case HZB_K_SPMV32: bytes += 2 * vb * n; break;     // x, y
     case HZB_K_RES64: bytes += 3 * vb * n; break;                        // x, b, w

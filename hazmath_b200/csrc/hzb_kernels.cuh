@@ -58,10 +58,10 @@ struct DCsr {
     const T *val = nullptr;
     int bundle_cap = 0;   // max entries in any bundle of bundle_rows rows (0: none)
     int bundle_rows = 128;   // rows per CTA of the staged kernels: 64, 128 or 256
-    // FP32 only: lanes per row of the vector-CSR kernels (2..16), 0 for the
+    // lanes per row of the vector-CSR kernels (2..16, FP32 only), 0 for the
     // staged bundles, SELL_LANES for the sliced-ELL copy in `sell`.  A row's
     // partial sums are combined across its lanes, so the lanes kernels do
-    // not give the sequential CSR-order sum of the FP64 kernels.
+    // not give the sequential CSR-order sum of the others.
     int vec_lanes = 0;
     SellView<T> sell;
     // Optional activity of 256-row blocks (ACT_ROWS): kernels skip the rows
@@ -94,8 +94,9 @@ int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cud
 bool fp32_schedule_known(int n, int nnz, int *lanes);
 
 // Sliced-ELL copy of a CSR matrix (hzb_sell.cu); *out stays empty
-// (npad 0) when its slice offsets would overflow int; a null: no FP32 values.  Sweep and SpMV on it
-// (no activity array, no SPMV_Y_DOT).
+// (npad 0) when its slice offsets would overflow int; a null: no FP32 values.
+// FP64 values of the same pattern beside them.  Sweep and SpMV on it (no
+// activity array; SPMV_Y_DOT in FP64 only).
 int sell_build(int n, const int *ia, const int *ja, const float *a, SellArrays *out,
                cudaStream_t s);
 int sell_values64(SellArrays *S, const int *ia, const double *a, cudaStream_t s);
