@@ -22,6 +22,7 @@
 // other's, 0.18 to 0.23 now that parts of the CTA take the sets in turn.
 //   The row sum runs in CSR order from b_i with the diagonal skipped, each
 // value rounded as in gs_rows: the same bits.
+#include "hzb_gs_plan.h"
 #include "hzb_solver.cuh"
 #include <algorithm>
 #include <type_traits>
@@ -29,34 +30,6 @@
 namespace hzb {
 
 namespace {
-
-constexpr int GS_ROWS = 256;           // a set's rows: one per computing thread
-constexpr int GS_TURNS = 3;            // parts of a CTA that take sets in turn
-constexpr int GS_SETS = 2048;          // sets of a schedule (their sizes lie in shared memory)
-constexpr int GS_BLOCK = 256;          // places per copy of x
-constexpr int GS_PAD = 8;              // set starts and slot pitches, in places
-constexpr size_t GS_SMEM = 220 * 1024;
-
-// set s: first place (x), rows and entries per row (y; the latter even and in
-// the upper half), the first place's place in the ring (z), first entry (w); its
-// rows are rounded up to GS_PAD
-__host__ __device__ inline int gs_pitch(int rows) { return (rows + GS_PAD - 1) / GS_PAD * GS_PAD; }
-__host__ __device__ inline int gs_rows(int4 I) { return I.y & 0xffff; }
-__host__ __device__ inline int gs_width(int4 I) { return I.y >> 16; }
-// the places and entries behind a set
-__host__ __device__ inline int gs_end_place(int4 I) { return I.x + gs_pitch(gs_rows(I)); }
-__host__ __device__ inline int gs_end_entry(int4 I) {
-    return I.w + gs_width(I) * gs_pitch(gs_rows(I));
-}
-
-// one stage, a group of sets of E entries and R places: values, (b, d), columns
-__host__ __device__ inline size_t gs_stage(int E, int R) {
-    return (size_t)E * 8 + (size_t)R * 16 + (size_t)E * 2;
-}
-inline size_t gs_smem(int ns, int E, int R, int ring, int stages) {
-    return (size_t)ns * 16 + (size_t)(ring + 2) * 8 + (size_t)stages * gs_stage(E, R) +
-           (size_t)stages * 16;
-}
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);
@@ -452,16 +425,10 @@ int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
     G.release();
     const int n = A.n, ns = (int)sc->h_ptr.size() - 1;
     // sets of at most a row per thread throughout, and few enough of them
-    if (ns < 1 || ns > GS_SETS) return SUCCESS;
-    std::vector<int> start(ns), width(ns);
-    int places = 0;
-    for (int k = 0; k < ns; ++k) {
-        const int m = sc->h_ptr[k + 1] - sc->h_ptr[k];
-        if (m > GS_ROWS) return SUCCESS;
-        start[k] = places;
-        places += gs_pitch(m);
-    }
-    places = (places + GS_BLOCK - 1) / GS_BLOCK * GS_BLOCK;
+    std::vector<int> start;
+    const int places = gs_places(sc->h_ptr, &start);
+    if (!places) return SUCCESS;
+    std::vector<int> width(ns);
     int *d_start = nullptr, *d_width = nullptr, dist = 0;
     int rc = SUCCESS;
     cudaError_t e = cudaSuccess;
@@ -488,66 +455,29 @@ int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
         e = cudaMemcpyAsync(&dist, d_width + ns, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return done(false);
-    // Rows of up to 8 entries: one width for all sets, so that the next set's
-    // loads need no branch and run ahead of the barrier (0.35 us a set of a 2D
-    // level with each set its own width, 0.18 to 0.23 with the longest row's).
-    const int longest = *std::max_element(width.begin(), width.end());
-    const int uniform = longest <= 8 ? std::max(2, longest) : 0;
+    const GsPlan P = gs_plan(sc->h_ptr, start, places, width, dist);
+    if (!P.stages) return done(false);
     int max_rows = 0;
-    for (int k = 0; k < ns; ++k) {
-        if (uniform) width[k] = uniform;
-        max_rows = std::max(max_rows, sc->h_ptr[k + 1] - sc->h_ptr[k]);
-    }
-    std::vector<int4> info(ns);
-    long long ents = 0;
-    for (int k = 0; k < ns; ++k) {
-        const int m = sc->h_ptr[k + 1] - sc->h_ptr[k];
-        if (ents > (1LL << 30)) return done(false);
-        if (width[k] > 0x7fff) return done(false);
-        info[k] = int4{start[k], m | width[k] << 16, 0, (int)ents};
-        ents += (long long)width[k] * gs_pitch(m);
-    }
-    // Sets per stage and stages: large groups keep the copying warp ahead (it
-    // takes about 1 us a group), and the sets in flight have to cover the
-    // copies' latency (2 us, ten sets); the first choice that fits.  The ring
-    // spans the columns on both sides of the sets in flight.
-    static const int choice[][2] = {{8, 3}, {4, 4}, {4, 3}, {2, 6}, {2, 4}, {1, 8}, {1, 4}, {1, 3}, {1, 2}};
-    int ring = 0, stages = 0, group = 0, E = 0, R = 0;
-    for (const auto &c : choice) {
-        E = R = 0;
-        for (int k = 0; k < ns; k += c[0]) {
-            const int l = std::min(k + c[0], ns) - 1;
-            E = std::max(E, gs_end_entry(info[l]) - info[k].w);
-            R = std::max(R, gs_end_place(info[l]) - info[k].x);
-        }
-        const long long span = 2LL * dist + (long long)(c[1] + 1) * R + 2 * GS_BLOCK;
-        ring = (int)((std::min<long long>(span, places) + GS_BLOCK - 1) / GS_BLOCK * GS_BLOCK);
-        if (ring > 0xff00 || gs_smem(ns, E, R, ring, c[1]) > GS_SMEM) continue;
-        group = c[0];
-        stages = c[1];
-        break;
-    }
-    if (!stages) return done(false);
-    for (auto &I : info) I.z = I.x % ring;
-    if ((rc = dalloc(&G.info, ns)) || (rc = dalloc(&G.col, ents)) || (rc = dalloc(&G.val, ents)) ||
+    for (int k = 0; k < ns; ++k) max_rows = std::max(max_rows, sc->h_ptr[k + 1] - sc->h_ptr[k]);
+    if ((rc = dalloc(&G.info, ns)) || (rc = dalloc(&G.col, P.ents)) || (rc = dalloc(&G.val, P.ents)) ||
         (rc = dalloc(&G.bd, places)) || (rc = dalloc(&G.xp, places)))
         return done(false);
-    e = cudaMemcpyAsync(G.info, info.data(), sizeof(int4) * ns, cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(G.info, P.info.data(), sizeof(int4) * ns, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        k_gs_fill<<<ns, GS_ROWS, 0, s>>>(G.info, ring, uniform, G.src, G.place, A.ia, A.ja, A.val,
+        k_gs_fill<<<ns, GS_ROWS, 0, s>>>(G.info, P.ring, P.uniform, G.src, G.place, A.ia, A.ja, A.val,
                                          G.col, G.val);
         count_launch();
         e = cudaMemcpyAsync(&G.last_place, G.place + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // and the host arrays above
     }
     G.ns = ns;
-    G.uniform = uniform;
+    G.uniform = P.uniform;
     G.threads = (max_rows + 31) / 32 * 32;
-    G.group = group;
-    G.E = E;
-    G.R = R;
-    G.ring = ring;
-    G.stages = stages;
+    G.group = P.group;
+    G.E = P.E;
+    G.R = P.R;
+    G.ring = P.ring;
+    G.stages = P.stages;
     G.dist = dist;
     G.places = places;
     return done(true);

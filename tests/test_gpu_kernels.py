@@ -306,3 +306,35 @@ def test_streamed_gauss_seidel_row_widths(port, name, sm, pre):
     x = dev(x0)
     assert hz.lib().hzb_smoother_device(sm, pre, 3, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
     assert np.array_equal(host(x), port.smooth(sm, pre, 3, ia, ja, val, b, x0, relax=1.15))
+
+
+def _periodic(nx, ny, px, py):
+    """5-point matrix of a grid periodic in x or y, CSR rows ascending."""
+    import scipy.sparse as sp
+    def line(m, per):
+        d = sp.diags([np.full(m - 1, -1.0), np.full(m - 1, -1.0)], [-1, 1], format="lil")
+        if per:
+            d[0, m - 1] = d[m - 1, 0] = -0.75
+        return d.tocsr()
+    a = sp.kron(sp.eye(ny), line(nx, px)) + sp.kron(line(ny, py), sp.eye(nx)) * 1.25
+    a = (a + sp.eye(nx * ny) * 4.75).tocsr()
+    a.sort_indices()
+    return a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data
+
+
+# far couplings: the ring grows, and the choice of stages goes through the small
+# groups down to two stages of one set (from 153 points a side on), which the
+# single sequence takes
+@pytest.mark.parametrize("nx,ny,px,py", [
+    (100, 100, 0, 1), (127, 127, 1, 0), (137, 137, 0, 1), (145, 145, 1, 1), (151, 151, 1, 1),
+    (153, 153, 1, 0), (153, 153, 0, 1), (154, 154, 1, 1), (100, 242, 0, 1)])
+@pytest.mark.parametrize("sm,pre", [(2, 1), (2, 0), (6, 1)])
+def test_streamed_gauss_seidel_far_couplings(port, nx, ny, px, py, sm, pre):
+    ia, ja, val = _periodic(nx, ny, px, py)
+    n = len(ia) - 1
+    rng = np.random.default_rng(n + sm)
+    b, x0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    A = DevCSR(ia, ja, val)
+    x = dev(x0)
+    assert hz.lib().hzb_smoother_device(sm, pre, 2, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
+    assert np.array_equal(host(x), port.smooth(sm, pre, 2, ia, ja, val, b, x0, relax=1.15))
