@@ -6,6 +6,7 @@
 // rounded exactly as the reference's sequential C loops round it.
 #pragma once
 #include "hzb_common.cuh"
+#include "hzb_tally.h"
 
 namespace hzb {
 
@@ -228,39 +229,36 @@ __device__ __forceinline__ bool grid_step(unsigned *count, unsigned target, int 
     return grid_wait(count, target, err);
 }
 
-// The same with a vote:
-// *word counts arrivals in its lower half and arrivals with a true vote in its
-// upper half.  *any: somebody voted true in this crossing
-// (votes: the thread 0's count of true votes so far, 0 at the first).  Only
-// when nobody did may the CTAs leave the loop, so a CTA that reads the word
-// late cannot take a later crossing's votes for this one's.
-__device__ __forceinline__ bool grid_vote(unsigned long long *word, unsigned target, bool vote,
-                                          unsigned *votes, bool *any, int *err) {
-    __shared__ int s_go;
-    const int v = __syncthreads_or(vote);
+// The same with a count: *total is what all CTAs have counted in this crossing
+// and the ones before (one per thread that counts), the same for everyone.
+// words: two, zero at first; T: thread 0's.
+__device__ __forceinline__ bool grid_tally(unsigned long long *words, GridTally &T, bool counts,
+                                           unsigned *total, int *err) {
+    __shared__ unsigned s_total;
+    __shared__ int s_stop;
+    const unsigned mine = (unsigned)__syncthreads_count(counts);
     if (threadIdx.x == 0) {
-        int go = 1;
-        const unsigned long long one = v ? 0x100000001ull : 1ull;
-        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(one) : "memory");
-        unsigned long long w;
+        int bad = 0;
+        ++T.r;
+        unsigned long long w, *word = words + T.word();
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;"
+                     ::"l"(word), "l"(GridTally::arrival(mine)) : "memory");
         for (unsigned spin = 0;; ++spin) {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(word) : "memory");
-            if ((int)((unsigned)w - target) >= 0) break;
-            if ((spin & 63u) == 63u && *(volatile int *)err) { go = -1; break; }
+            if (T.complete(w, gridDim.x)) break;
+            if ((spin & 63u) == 63u && *(volatile int *)err) { bad = 1; break; }
             if (spin > GRID_SPIN_LIMIT) {
                 atomicExch(err, 1);
-                go = -1;
+                bad = 1;
                 break;
             }
         }
-        const unsigned now = (unsigned)(w >> 32);
-        if (go > 0 && now == *votes) go = 0;
-        *votes = now;
-        s_go = go;
+        s_total = T.total(w);
+        s_stop = bad;
     }
     __syncthreads();
-    *any = s_go > 0;
-    return s_go >= 0;
+    *total = s_total;
+    return !s_stop;
 }
 
 // consecutive level sets [first, last) of up to max_set rows each in one

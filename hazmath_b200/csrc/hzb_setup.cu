@@ -324,7 +324,7 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 // (167 ms for the 2,048,383 rows of the 128^3 log-normal system, 318 ms for
 // its hierarchy; 11.8 and 37 ms now).
 //
-// CLUSTER: the CTAs are one cluster of at most 8, whose barrier and votes (in
+// CLUSTER: the CTAs are one cluster of at most 8, whose barrier and counts (in
 // every member's shared memory) cost half as much.  Its window of 8192 rows
 // can lengthen the dependency chain, which holds with half of the rows in
 // play (16,256 rows of a 2D 5-point hierarchy: 0.7 ms against 0.9) but not on
@@ -338,11 +338,12 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
              unsigned long long *post, int *next, unsigned long long *bar, int *err) {
     const int lane = threadIdx.x & 31;
     constexpr int B = 4;             // candidates examined at a time
-    __shared__ int s_vote[2][HEM_CLUSTER];
+    __shared__ int s_count[2][HEM_CLUSTER];
     int u = -1, p0 = 0, p1 = 0;      // the row in play, its candidates left
     int pending = blockIdx.x * blockDim.x + threadIdx.x;   // enters next round
     bool more = true;                // rows may be left to take
-    unsigned votes = 0;
+    GridTally tally;
+    unsigned total = 0;              // rows decided
     const unsigned max_round = 3u * (unsigned)n + 16u;
     for (unsigned r = 1;; ++r) {
         const unsigned long long *prev = post + (size_t)((r - 1) & 1u) * n;
@@ -350,6 +351,7 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
         const unsigned long long mark = (unsigned long long)(0xffffffffu - r) << 32;
         const unsigned was = 0xffffffffu - (r - 1);
         const bool fresh = u < 0;
+        bool done = false;           // its row is decided in this round
         if (u < 0 && pending < n) {
             u = pending;
             p0 = ia[u];
@@ -362,7 +364,7 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             };
             const int su = __ldcg(state + u);
             const unsigned long long tu = __ldcg(prev + u);
-            bool done = su != -1;                  // an earlier row took it
+            done = su != -1;                       // an earlier row took it
             const bool mine = !fresh && threat(tu) == u;
             int best = -1;
             bool open = true;
@@ -407,21 +409,18 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
         int base = n;
         const int lead = __ffs(need) - 1;
         if (more && lane == lead) base = atomicAdd(next, __popc(need));
-        const bool vote = u >= 0 || more;
-        bool any;
         if (CLUSTER) {
             namespace cg = cooperative_groups;
             cg::cluster_group cl = cg::this_cluster();
-            const int v = __syncthreads_or(vote);
+            const int count = __syncthreads_count(done);
             if (threadIdx.x < gridDim.x)
-                *cl.map_shared_rank(&s_vote[r & 1u][blockIdx.x], threadIdx.x) = v;
+                *cl.map_shared_rank(&s_count[r & 1u][blockIdx.x], threadIdx.x) = count;
             cl.sync();
-            any = false;
-            for (unsigned q = 0; q < gridDim.x; ++q) any |= s_vote[r & 1u][q] != 0;
-        } else if (!grid_vote(bar, r * gridDim.x, vote, &votes, &any, err)) {
+            for (unsigned q = 0; q < gridDim.x; ++q) total += (unsigned)s_count[r & 1u][q];
+        } else if (!grid_tally(bar, tally, done, &total, err)) {
             return;
         }
-        if (!any) return;
+        if (total == (unsigned)n) return;
         if (need) {
             base = __shfl_sync(0xffffffffu, base, lead);
             pending = n;
@@ -534,8 +533,8 @@ __global__ void k_hem_final(int n, int *mask) {
 
 int hem_exact(int n, const int *nia, const int *nja, const double *nval,
               int *agg, int *nagg, int *work_n, cudaStream_t s) {
-    // out: aggregates, status | longest row | next row | barrier (2) | error
-    enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 6, O_N = 8 };
+    // out: aggregates, status | longest row | next row | barrier (4) | error
+    enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 8, O_N = 10 };
     int *out = nullptr;
     HZB_TRY(dalloc(&out, O_N));
     int h[O_N] = {0};
