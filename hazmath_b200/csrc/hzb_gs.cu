@@ -318,6 +318,13 @@ k_gs_stream(const __grid_constant__ GsSweep A, double w, int *err) {
     }
 }
 
+// Place of entry u of a set's row t: with one width for all sets its pairs lie
+// side by side with the other rows' (a warp's loads are then free of conflicts),
+// else with the row's own.
+__device__ __forceinline__ int gs_at(int uniform, int pitch, int Z, int t, int u) {
+    return uniform ? (u / 2 * pitch + t) * 2 + u % 2 : t * Z + u;
+}
+
 // vectors into the schedule's order (src: row of a place, -1 for padding)
 __global__ void k_gs_in(int places, const int *__restrict__ src, const double *__restrict__ b,
                         const double *__restrict__ d, const double *__restrict__ x, double2 *bd,
@@ -327,6 +334,42 @@ __global__ void k_gs_in(int places, const int *__restrict__ src, const double *_
         bd[q] = i >= 0 ? make_double2(b[i], d[i]) : make_double2(0.0, 0.0);
         xp[q] = i >= 0 ? x[i] : 0.0;
     }
+}
+// The same for a matrix in the caller's arrays, whose values are read as they
+// are: the rows' values go into the schedule's order too (a CTA per set).
+__global__ void __launch_bounds__(GS_ROWS)
+k_gs_in_values(int places, const int4 *__restrict__ info, int uniform,
+               const int *__restrict__ src, const double *__restrict__ b,
+               const double *__restrict__ d, const double *__restrict__ x,
+               const int *__restrict__ ia, const int *__restrict__ ja,
+               const double *__restrict__ a, double2 *bd, double *xp, double *val) {
+    const int4 I = info[blockIdx.x];
+    const int t = threadIdx.x, pitch = gs_pitch(gs_rows(I)), Z = gs_width(I);
+    if (t < pitch) {
+        constexpr int W = 8;        // entries in flight
+        const int i = src[I.x + t];
+        const int k0 = i >= 0 ? ia[i] : 0, k1 = i >= 0 ? ia[i + 1] : 0;
+        bd[I.x + t] = i >= 0 ? make_double2(b[i], d[i]) : make_double2(0.0, 0.0);
+        xp[I.x + t] = i >= 0 ? x[i] : 0.0;
+        int u = 0;
+        for (int kb = k0; kb < k1; kb += W) {
+            int c[W];
+            double v[W];
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+                c[q] = kb + q < k1 ? ja[kb + q] : i;
+                v[q] = kb + q < k1 ? a[kb + q] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < W; ++q)
+                if (c[q] != i) val[I.w + gs_at(uniform, pitch, Z, t, u++)] = v[q];
+        }
+    }
+    if (blockIdx.x == gridDim.x - 1)    // up to a whole block of places
+        for (int q = gs_end_place(I) + t; q < places; q += GS_ROWS) {
+            bd[q] = make_double2(0.0, 0.0);
+            xp[q] = 0.0;
+        }
 }
 __global__ void k_gs_out(int places, const int *__restrict__ src, const double *__restrict__ xp,
                          double *x) {
@@ -387,23 +430,18 @@ k_gs_fill(const int4 *__restrict__ info, int ring, int uniform, const int *__res
     const int pitch = gs_pitch(gs_rows(I));
     col += I.w + t * Z;
     val += I.w;
-    // pair q of row t: with one width for all sets side by side with the other
-    // rows' (a warp's loads are then free of conflicts), else with the row's own
-    auto at = [&](int u) {
-        return uniform ? (u / 2 * pitch + t) * 2 + u % 2 : t * Z + u;
-    };
     int u = 0;
     if (i >= 0)
         for (int k = ia[i]; k < ia[i + 1]; ++k) {
             const int j = ja[k];
             if (j == i) continue;
             col[u] = (unsigned short)(place[j] % ring);
-            val[at(u)] = a[k];
+            val[gs_at(uniform, pitch, Z, t, u)] = a[k];
             ++u;
         }
     for (; u < Z; ++u) {
         col[u] = (unsigned short)ring;
-        val[at(u)] = 0.0;
+        val[gs_at(uniform, pitch, Z, t, u)] = 0.0;
     }
 }
 
@@ -483,8 +521,8 @@ int gs_stream_build(const DCsr<double> &A, Schedule *sc, cudaStream_t s) {
     return done(true);
 }
 
-int gs_stream_sweep(const Schedule &sc, const double *d, const double *b, double *x,
-                    int kind, double w, int *err, cudaStream_t s) {
+int gs_stream_sweep(const Schedule &sc, const DCsr<double> *live, const double *d,
+                    const double *b, double *x, int kind, double w, int *err, cudaStream_t s) {
     const GsStream &G = sc.stream;
     const int skip_place = (kind & GS_SKIP_LAST) ? G.last_place : -1;   // SGS leaves row n - 1
     auto of_kind = [&](auto k) {
@@ -503,7 +541,11 @@ int gs_stream_sweep(const Schedule &sc, const double *d, const double *b, double
                            : of_kind(std::integral_constant<int, 2>());
     HZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)GS_SMEM));
-    k_gs_in<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, b, d, x, G.bd, G.xp);
+    if (live)
+        k_gs_in_values<<<G.ns, GS_ROWS, 0, s>>>(G.places, G.info, G.uniform, G.src, b, d, x,
+                                                live->ia, live->ja, live->val, G.bd, G.xp, G.val);
+    else
+        k_gs_in<<<grid_for(G.places), 256, 0, s>>>(G.places, G.src, b, d, x, G.bd, G.xp);
     const GsSweep A = {G.info, G.col, G.val, G.bd, G.xp, G.ns, G.group, G.E, G.R, G.stages,
                        G.ring, G.dist, G.places, skip_place};
     kernel<<<1, G.threads * (G.uniform ? GS_TURNS : 1) + 32, gs_smem(G.ns, G.E, G.R, G.ring, G.stages), s>>>(A, w, err);

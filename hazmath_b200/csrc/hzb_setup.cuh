@@ -106,10 +106,11 @@ struct Schedule {
 };
 // The stream of a schedule, for A's values (none when a set is too large), and
 // a sweep of it (kinds as gs_rows', x in place; err: raised if a copy never
-// arrives).
+// arrives).  live: the matrix when its values are the caller's, who may have
+// changed them since the build; they are taken over first.
 int gs_stream_build(const DCsr<double> &A, Schedule *sch, cudaStream_t s);
-int gs_stream_sweep(const Schedule &sch, const double *d, const double *b, double *x, int kind,
-                    double w, int *err, cudaStream_t s);
+int gs_stream_sweep(const Schedule &sch, const DCsr<double> *live, const double *d,
+                    const double *b, double *x, int kind, double w, int *err, cudaStream_t s);
 int gs_schedule(int n, const int *ia, const int *ja, int nnz,
                 Schedule *sch, cudaStream_t s);
 // The schedule of the opposite sweep: the sets in reverse order.  A row comes

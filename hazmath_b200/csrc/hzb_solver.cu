@@ -241,7 +241,7 @@ static int norm2sq(hzb_solver *S, KrylovWork &w, int n, const double *x, int slo
 // ---------------------------------------------------------------------------
 static int run_sets(hzb_solver *S, const DCsr<double> &A, const Schedule &sc,
                     int kind, const double *d, double w, const double *b,
-                    double *x, bool reverse) {
+                    double *x, bool reverse, bool own_A) {
     const int ns = (int)sc.h_ptr.size() - 1;
     // consecutive large sets go to one cooperative launch when the grid
     // barrier has its words (exact schedules) and a place to report to;
@@ -252,7 +252,7 @@ static int run_sets(hzb_solver *S, const DCsr<double> &A, const Schedule &sc,
     }();
     int *err = grid_ok ? wait_err(S) : nullptr;
     if (!reverse && sc.stream.stages && wait_err(S))
-        return gs_stream_sweep(sc, d, b, x, kind, w, wait_err(S), S->s);
+        return gs_stream_sweep(sc, own_A ? nullptr : &A, d, b, x, kind, w, wait_err(S), S->s);
     if (!reverse) {
         const size_t nr = sc.run_first.size();
         for (size_t q = 0; q < nr; ++q) {
@@ -294,8 +294,8 @@ static int gs_sweep(hzb_solver *S, Level &L, int kind, bool forward, double w) {
     const bool is_gs = (kind & 15) == 0;
     const double *d = is_gs ? (forward ? L.d_gs_f : L.d_gs_b)
                             : (forward ? L.d_sor_f : L.d_sor_b);
-    if (mc) return run_sets(S, A, L.col, kind, d, w, L.b, L.x, !forward);
-    return run_sets(S, A, forward ? L.fwd : L.bwd, kind, d, w, L.b, L.x, false);
+    if (mc) return run_sets(S, A, L.col, kind, d, w, L.b, L.x, !forward, L.own_A);
+    return run_sets(S, A, forward ? L.fwd : L.bwd, kind, d, w, L.b, L.x, false, L.own_A);
 }
 
 // one forward Gauss-Seidel sweep of level l as the cycle runs it (the level's
@@ -473,7 +473,12 @@ static int precond64_body(hzb_solver *S, const double *r, double *z,
     double *sb = L0.b, *sx = L0.x;
     L0.b = const_cast<double *>(r);
     L0.x = z;
-    int rc = vzero<double>(L0.n, z, S->s);
+    int rc = SUCCESS;
+    // a matrix in the caller's arrays is read as it is, its norms too (the zeroed
+    // vector lies between them and the kernels that start ahead of their turn)
+    if (!L0.own_A && small_first_level<double>(S, cyc, 0, true) == 0)
+        rc = l1_norms<double>(L0.A64(), L0.l1_64, S->s);
+    if (!rc) rc = vzero<double>(L0.n, z, S->s);
     for (int i = 0; rc == SUCCESS && i < cyc.maxit; ++i) rc = cycle64(S, cyc, 0, i == 0);
     L0.b = sb;
     L0.x = sx;

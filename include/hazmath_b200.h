@@ -481,7 +481,12 @@ typedef struct {
 
 INT  hzb_create(hzb_solver **s, const AMG_param *amg,
                 const linear_itsolver_param *it, const hzb_param *bp);
-/* setup from device arrays (int32 CSR, FP64 values) */
+/* setup from device arrays (int32 CSR, FP64 values).  They stay the caller's
+ * and have to be valid until the next setup or hzb_destroy.  A changed matrix
+ * needs a new setup: only level 0's FP64 residuals, products and sweeps read
+ * d_val as it is at the call; the hierarchy, the diagonals of the Jacobi,
+ * Gauss-Seidel and SOR sweeps, the coarsest inverse and all that the mixed
+ * precision stores are the setup's. */
 INT  hzb_setup_device(hzb_solver *s, INT n, INT nnz, const INT *d_ia,
                       const INT *d_ja, const REAL *d_val);
 /* setup from a host matrix (copied in) */

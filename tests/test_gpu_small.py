@@ -118,3 +118,46 @@ def test_fp32_small_levels_to_rounding(name, pre, post):
     assert np.abs(x - alpha * z[0]).max() <= tol * np.abs(alpha * z[0]).max()
     S.close()
     T.close()
+
+
+def _gs(A, pre, k, b, x):
+    x = dev(x)
+    assert hz.lib().hzb_smoother_device(hz.SMOOTHER_GS, pre, k, 1.0, *A.args(), ptr(dev(b)),
+                                        ptr(x)) == 0
+    return host(x)
+
+
+@pytest.mark.parametrize("smoother", [hz.SMOOTHER_L1DIAG, hz.SMOOTHER_GS])
+@pytest.mark.parametrize("make", [lambda: P.poisson2d_5pt(45), lambda: P.aniso2d_p1(50, 0.1, 0.5),
+                                  lambda: P.kuhn3d_p1(14, P.lognormal_field(14, 1.0, 4.0, 2))],
+                         ids=["2d_45", "aniso_50", "kuhn_14"])
+def test_values_changed_in_the_callers_array(smoother, make):
+    """A matrix in the caller's device arrays: level 0's sweeps and residual read
+    its values as they are at the call (only the hierarchy and the Gauss-Seidel
+    diagonals, which stay the same here, are the setup's)."""
+    ia, ja, val = make()
+    n = len(ia) - 1
+    A = DevCSR(ia, ja, val)
+    S = hz.Solver(hz.bench_amg(smoother=smoother, coarse_dof=n * 3 // 4))
+    assert S.setup_device(*A.args()) == 0
+    assert S.stats().num_levels == 2
+    agg = S.level(0)[3]
+    r = P.rhs_uniform(n, 5)
+    _precond(S, r)                       # captured with the first values
+    row = np.repeat(np.arange(n), np.diff(ia))
+    new = np.where(ja == row, val, val * np.random.default_rng(1).uniform(0.4, 0.9, len(ja)))
+    A.val.copy_(dev(new))
+    got = _precond(S, r)
+    sweep = _gs if smoother == hz.SMOOTHER_GS else lambda A, pre, k, b, x: _sweeps(A, k, b, x)
+    x = sweep(A, 1, 1, r, np.zeros(n))
+    t = dev(np.zeros(n))
+    assert hz.lib().hzb_dcsr_mxv_device(*A.args(), ptr(dev(x)), ptr(t)) == 0
+    w = r - host(t)
+    bc = np.zeros(S.stats().rows[1])
+    for i in range(n):
+        if agg[i] >= 0:
+            bc[agg[i]] += w[i]
+    xc = _cycle(S, 1, 1, 1, bc)
+    want = sweep(A, 0, 1, r, x + np.where(agg >= 0, xc[np.maximum(agg, 0)], 0.0))
+    assert np.array_equal(got, want)
+    S.close()
