@@ -723,8 +723,11 @@ int ensure_fp32(hzb_solver *S) {
 // rows in CSR order without the stored zeros, which add nothing, so the same bits.
 // Not of a matrix that stays in the caller's arrays.  Sweeps of the first three
 // coarse levels of a 127^3 system 40, 29 and 21 us staged, 26, 18 and 13 sliced.
+// HZB_FP64_SELL: 1 every such level, 0 none (the same results).
 static int level_sliced64(hzb_solver *S, Level &L) {
-    if (!L.own_A || sell64_known(L.n, L.nnz) == 0) return SUCCESS;
+    const char *force = getenv("HZB_FP64_SELL");
+    const int known = force && *force ? force[0] != '0' : sell64_known(L.n, L.nnz);
+    if (!L.own_A || known == 0) return SUCCESS;
     cudaStream_t s = S->s;
     int *cnt = nullptr, *ia = nullptr, *ja = nullptr, *tmp = nullptr, nz = 0;
     double *val = nullptr;
@@ -748,7 +751,7 @@ static int level_sliced64(hzb_solver *S, Level &L) {
     if ((rc = sell_build(L.n, ia, val ? ja : L.ja, nullptr, &L.sell64, s)) || !L.sell64.npad ||
         (rc = sell_values64(&L.sell64, ia, val ? val : L.val, s)))
         goto done;
-    if (sell64_known(L.n, L.nnz) < 0) {
+    if (known < 0) {
         bool sliced = false;
         if ((rc = vzero<double>(L.n, L.b, s)) ||
             (rc = autotune_sell64(L.A64(), L.b, L.x, L.w, &sliced, s)))

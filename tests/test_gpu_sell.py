@@ -114,3 +114,31 @@ def test_fp64_sliced_levels_bitwise(N):
     assert D.solve_device(db.data_ptr(), dx.data_ptr()) == it > 0
     D.close()
     assert np.array_equal(x, dx.cpu().numpy())
+
+
+@pytest.mark.parametrize("N", [48, 64])
+def test_fp64_sliced_and_staged_levels_bitwise(monkeypatch, N):
+    """The two forms of the FP64 cycle's large levels, each forced by
+    HZB_FP64_SELL (the bytes that hzb_time_kernel counts tell which one a level
+    has): the same iterates bit for bit."""
+    ia, ja, val = P.kuhn3d_p1(N, P.lognormal_field(N, 1.0, 8.0, 7))
+    b = P.rhs_uniform(len(ia) - 1, 8)
+    out = []
+    for form in ("1", "0"):
+        monkeypatch.setenv("HZB_FP64_SELL", form)
+        S = hz.Solver(hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG, presmooth_iter=2,
+                                   postsmooth_iter=2),
+                      b200=hz.b200_param(precision=hz.HZB_PREC_FP64,
+                                         matching=hz.HZB_MATCH_PARALLEL))
+        assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+        x = np.zeros(len(b))
+        it = S.solve_host(b, x)
+        st = S.stats()
+        large = [l for l in range(st.num_levels - 1) if st.nnz[l] > 1250000]
+        out.append((it, x, [S.time_kernel(hz.HZB_K_L1_64, l, 1)[1] for l in large]))
+        S.close()
+    (it_s, x_s, by_s), (it_b, x_b, by_b) = out
+    assert len(by_s) == len(by_b) >= (2 if N == 64 else 1)
+    assert all(s != t for s, t in zip(by_s, by_b))
+    assert it_s == it_b > 0
+    assert np.array_equal(x_s, x_b)
