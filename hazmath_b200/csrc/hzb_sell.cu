@@ -214,6 +214,27 @@ __device__ __forceinline__ void sell_row(const SellView<T> &V, int r, const T *_
     else sell_slice<T, L1, true>(V, h, r % SELL_C, x, t, d);
 }
 
+// The sum of slot r's row once more from t on, over its own entries only: a zero
+// that fills up a shorter row may meet an infinite or NaN x, and the row's own
+// result need not be NaN then.  For the rows whose sum came out NaN.
+template <typename T, bool L1>
+__device__ __forceinline__ T sell_row_own(const SellView<T> &V, int r, const T *__restrict__ x,
+                                          T t) {
+    const int len = (int)(__ldcg(V.slot + r) / SELL_WIN);
+    const int4 h = __ldcg(V.head + r / SELL_C);
+    const unsigned short *col = V.col + (size_t)(h.y < 0 ? -h.y - 1 : h.y) * SELL_C;
+#pragma unroll 1
+    for (int u = 0; u < len; ++u) {
+        const int at = sell_at(u, h.w, r % SELL_C);
+        const int2 b = V.base[h.z + u / 2];
+        const int c = h.y < 0 ? reinterpret_cast<const int *>(col)[at]
+                              : (u % 2 ? b.y : b.x) + (int)col[at];
+        const T p = V.val[(size_t)h.x * SELL_C + at] * x[c];
+        t = L1 ? t - p : t + p;
+    }
+    return t;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(SELL_WIN, 8)
 k_l1_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ b,
@@ -224,9 +245,16 @@ k_l1_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ b,
     if (i >= n) return;
     T t = __ldcs(b + i), d = T(0);
     sell_row<T, true>(V, r, x, t, d);
+    if (sizeof(T) == 8 && t != t) t = sell_row_own<T, true>(V, r, x, b[i]);
     T xi = x[i];
     if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[i]) * (t / d) : t / d;
     xn[i] = xi;
+    if (sizeof(T) == 4 && t != t) {
+        t = sell_row_own<T, true>(V, r, x, b[i]);
+        xi = x[i];
+        if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[i]) * (t / d) : t / d;
+        xn[i] = xi;
+    }
 }
 
 // 64 warps an SM here too (FP64, 16.6 million rows, with (x, y): 290 us; 322 with
@@ -244,6 +272,7 @@ k_spmv_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ 
     const T bi = MODE == SPMV_RES ? __ldcs(b + i) : T(0);
     T t = T(0), d = T(0);
     sell_row<T, false>(V, r, x, t, d);
+    if (t != t) t = sell_row_own<T, false>(V, r, x, T(0));
     if (MODE == SPMV_RES) {
         y[i] = bi - t;
     } else if (MODE == SPMV_AXPY) {

@@ -6,13 +6,15 @@ the mixed solve takes the same iterates bit for bit whichever of the two the
 levels run.  HZB_FP32_LANES forces the schedule of every level of at least
 4096 rows ("sell") or the bundles everywhere ("0").  The coarse levels of the
 Kuhn hierarchy have ragged rows (4 to ~30 entries), so the slices carry
-padding that the kernels must not read."""
+padding: zeros against the row's own last column, which must leave its sum as
+it is."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
 
 import hazmath_b200 as hz
 from hazmath_b200 import problems as P
+from gpu_util import dev, host, ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -142,3 +144,44 @@ def test_fp64_sliced_and_staged_levels_bitwise(monkeypatch, N):
     assert all(s != t for s, t in zip(by_s, by_b))
     assert it_s == it_b > 0
     assert np.array_equal(x_s, x_b)
+
+
+def test_infinite_x_beside_padding(monkeypatch):
+    """Rows shorter than their slice are filled up with zeros against a column of
+    their own: an infinite x there leaves their result what the row's own entries
+    make it (infinite, not NaN).  The rows of very different lengths below are
+    coupled too weakly to aggregate, so nothing but the sweeps reaches them; a
+    few have no entries but stored zeros, which the sliced copy drops."""
+    rng = np.random.default_rng(4)
+    ia, ja, val = P.kuhn3d_p1(48, P.lognormal_field(48, 1.0, 8.0, 7))
+    G = sp.csr_matrix((val, ja, ia))
+    m, k = len(ia) - 1, 1000
+    i = np.repeat(np.arange(k), rng.integers(0, 25, k))
+    j = rng.integers(0, k, len(i))
+    W = sp.coo_matrix((np.full(len(i), -1e-3), (i, j)), shape=(k, k)).tocsr()
+    W = W + W.T
+    W.setdiag(10.0)
+    A = sp.block_diag([G, W]).tocsr()
+    A.sort_indices()
+    ia, ja, val = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data.copy()
+    hit = m + np.arange(3, k, 7)
+    for q in range(m + 502, m + 520):   # the columns too: the matrix stays symmetric
+        if q not in hit:
+            val[ia[q]:ia[q + 1]] = 0.0
+            val[ja == q] = 0.0
+    r = P.rhs_uniform(m + k, 3)
+    r[hit] = np.inf
+    z = []
+    for form in ("1", "0"):
+        monkeypatch.setenv("HZB_FP64_SELL", form)
+        S = hz.Solver(hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG, strong_coupled=0.1),
+                      b200=hz.b200_param(precision=hz.HZB_PREC_FP64,
+                                         matching=hz.HZB_MATCH_PARALLEL))
+        assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+        d, o = dev(r), dev(np.zeros(m + k))
+        assert S.precond_device(ptr(d), ptr(o)) == 0, hz.last_error()
+        z.append(host(o))
+        S.close()
+    assert np.isfinite(z[1][:m]).all()
+    assert np.isinf(z[1][m:]).sum() > len(hit)       # the neighbours of the rows hit
+    assert np.array_equal(z[0], z[1], equal_nan=True)
