@@ -332,10 +332,27 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 // hence HEM_CLUSTER_ROWS.
 constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = 16384;
 
+// A chain is decided one row a round.  So every HEM_PACE rounds their pace is
+// looked at, and when the rows left would take longer at it than the walk below
+// takes for all of them (a round lasts as long as walk_rows of its rows), the
+// rounds stop and the walk starts over.  Of 2D and 3D hierarchies no level came
+// near it (at most 0.65 of the walk's time predicted, over 64 rounds; 32 rounds
+// are too few, a sweep front needs some tens to build up), of chains and strips
+// of up to 16 rows all were beyond it.
+//   Chains of 100,000 and 1,000,000 rows: 281 and 3045 ms in rounds, 6.6 and 61
+// with the walk; strips of 16 x 7,500 and 64 x 1,875: 22 and 6.0 in rounds, 7.8
+// and 6.0 so.  Up to HEM_WALK_SMALL rows the walk is the faster one anyway (2D,
+// 3D and anisotropic grids of 2,000 rows: 0.51 to 0.56 ms against 0.53 to 0.61;
+// of 4,000: 0.62 to 0.74 against 0.57 to 0.63).
+constexpr int HEM_WALK_SMALL = 2048;
+constexpr unsigned HEM_PACE = 64;
+constexpr int HEM_WALK_ROWS_GRID = 43, HEM_WALK_ROWS_CLUSTER = 20;   // 3.6 and 1.7 us a round
+
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HEM_BLOCK)
 k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, int *state,
-             unsigned long long *post, int *next, unsigned long long *bar, int *err) {
+             unsigned long long *post, int *next, unsigned long long *bar, int *err,
+             int walk_rows, int *stopped) {
     const int lane = threadIdx.x & 31;
     constexpr int B = 4;             // candidates examined at a time
     __shared__ int s_count[2][HEM_CLUSTER];
@@ -343,7 +360,7 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
     int pending = blockIdx.x * blockDim.x + threadIdx.x;   // enters next round
     bool more = true;                // rows may be left to take
     GridTally tally;
-    unsigned total = 0;              // rows decided
+    unsigned total = 0, paced = 0;   // rows decided, by now and at the last look
     const unsigned max_round = 3u * (unsigned)n + 16u;
     for (unsigned r = 1;; ++r) {
         const unsigned long long *prev = post + (size_t)((r - 1) & 1u) * n;
@@ -421,6 +438,14 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             return;
         }
         if (total == (unsigned)n) return;
+        if (walk_rows && r % HEM_PACE == 0) {
+            if ((long long)(n - (int)total) * HEM_PACE * walk_rows >
+                (long long)(total - paced) * n) {
+                if (blockIdx.x == 0 && threadIdx.x == 0) *stopped = 1;
+                return;
+            }
+            paced = total;
+        }
         if (need) {
             base = __shfl_sync(0xffffffffu, base, lead);
             pending = n;
@@ -431,6 +456,234 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             if (blockIdx.x == 0 && threadIdx.x == 0) *err = 1;
             return;
         }
+    }
+}
+
+// --- pass 1 as a walk ---------------------------------------------------------
+// For graphs whose rows can only be decided one after the other (a chain, a
+// narrow strip), where the rounds above give up: one CTA streams the ranked
+// lists through shared memory in tiles of 32 rows with cp.async, HEM_PIPE tiles
+// ahead of the tile it works on, so no global load latency sits on its critical
+// path (83 ns a row), and only looks for the first unmatched entry of a list.
+constexpr int HEM_RING_BITS = 1 << 20;                 // 128 KB of shared memory
+constexpr int HEM_RING_WORDS = HEM_RING_BITS / 32;
+constexpr int HEM_PIPE = 4;                 // tiles in flight ahead of the walk
+constexpr int HEM_TILE_CAP = 3072;          // staged candidates per tile
+// slots: the tiles in flight plus the one being walked
+constexpr int HEM_IA_SLOTS = 2 * HEM_PIPE + 2, HEM_IA_STRIDE = 36;
+constexpr int HEM_C_SLOTS = HEM_PIPE + 2;
+constexpr int HEM_MISC_WORDS = 32 * 2 + 32 + 2 * 32 + 2;   // info, Pm, picks, accepted
+constexpr size_t HEM_STAGED_SMEM =
+    (size_t)HEM_RING_WORDS * 4 + (size_t)HEM_C_SLOTS * HEM_TILE_CAP * 4 +
+    (size_t)HEM_IA_SLOTS * HEM_IA_STRIDE * 4 + (size_t)HEM_MISC_WORDS * 4;
+
+__global__ void k_graph_bandwidth(int n, const int *__restrict__ ia,
+                                  const int *__restrict__ ja, int *bw) {
+    __shared__ int sh[32];
+    int b = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += gridDim.x * blockDim.x)
+        for (int k = ia[i]; k < ia[i + 1]; ++k) b = max(b, abs(ja[k] - i));
+    b = block_max(b, sh);
+    if (threadIdx.x == 0) atomicMax(bw, b);
+}
+
+__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// The matched state of the vertices in play lives in a ring of shared memory:
+// one byte per vertex (BYTES, 2^17 vertices, plain stores) while the window
+// fits, else one bit per vertex (2^20 vertices, atomicOr).  Both rings take
+// 128 KB.  Ring size > 2 bw + 64: the 32 slots entering the window are
+// cleared when a tile begins (vertices >= r0 + bw cannot be matched before
+// tile r0 starts, and the slot's previous owner lies below r0 - bw).
+template <bool BYTES>
+struct HemRing {
+    static constexpr unsigned SIZE = BYTES ? (1u << 17) : (1u << 20);
+    static constexpr unsigned RM = SIZE - 1;
+    void *mem;
+    __device__ __forceinline__ bool get(int v) const {
+        const unsigned u = (unsigned)v & RM;
+        if (BYTES) return ((const volatile unsigned char *)mem)[u] != 0;
+        return (((const volatile unsigned *)mem)[u >> 5] >> (u & 31)) & 1u;
+    }
+    __device__ __forceinline__ void set(int v) {
+        const unsigned u = (unsigned)v & RM;
+        if (BYTES) ((volatile unsigned char *)mem)[u] = 1;
+        else atomicOr((unsigned *)mem + (u >> 5), 1u << (u & 31));
+    }
+    // vertices v0 .. v0 + 31, by the whole warp
+    __device__ __forceinline__ void clear32(int v0, int lane) {
+        if (BYTES) {
+            ((unsigned char *)mem)[((unsigned)v0 + lane) & RM] = 0;
+        } else {
+            const unsigned u = (unsigned)v0 & RM, sh = u & 31u, w0 = u >> 5;
+            unsigned *w = (unsigned *)mem;
+            if (lane == 0) w[w0] &= ~(0xffffffffu << sh);
+            if (lane == 1 && sh) w[(w0 + 1) & (SIZE / 32 - 1)] &= ~((1u << sh) - 1u);
+        }
+    }
+};
+
+// Two warps.  Warp 1 streams row pointers and ranked lists into shared
+// memory (cp.async, HEM_PIPE tiles ahead) and writes the pairs of finished
+// tiles to mask/cnt; warp 0 walks the tiles.  Within a tile of 32 rows every
+// row first takes its best candidate unmatched when the tile starts; rows are
+// then settled in order.  A row keeps that choice unless an earlier row of
+// the tile took it or matched the row's choice (vertices only ever become
+// matched, so the entries ranked above it stay ineligible); such a row scans
+// its list again.  For a row that keeps its choice the effect on the rows
+// after it is known in advance: the row it picks leaves the walk (rm) and the
+// rows that wanted the same vertex or this row go stale (st).
+template <bool BYTES>
+__global__ void __launch_bounds__(64)
+k_hem_pass1_staged(int n, int bw, const int *__restrict__ ia, const int *__restrict__ cand,
+                   int *mask, int *cnt, int *out) {
+    extern __shared__ unsigned hem_smem[];
+    HemRing<BYTES> ring{hem_smem};
+    int *cbuf = (int *)(hem_smem + HEM_RING_WORDS);
+    int *iabuf = cbuf + HEM_C_SLOTS * HEM_TILE_CAP;
+    uint2 *info = (uint2 *)(iabuf + HEM_IA_SLOTS * HEM_IA_STRIDE);
+    unsigned *pm = (unsigned *)(info + 32);
+    int *picks = (int *)(pm + 32);              // [2][32], by tile parity
+    unsigned *accepted = (unsigned *)(picks + 64);   // [2]
+    const int lane = threadIdx.x & 31;
+    const int ntiles = (n + 31) >> 5;
+
+    if (threadIdx.x >= 32) {   // ---- warp 1: staging and output
+        int nc = 0;
+        auto emit = [&](int u) {
+            const unsigned acc = accepted[u & 1];
+            if ((acc >> lane) & 1u) {
+                const int id = nc + __popc(acc & ((1u << lane) - 1u));
+                const int q = picks[(u & 1) * 32 + lane];
+                mask[(u << 5) + lane] = id;
+                mask[q] = id;
+                cnt[id] = 2;
+            }
+            nc += __popc(acc);
+        };
+        for (int j = -2 * HEM_PIPE; j < ntiles; ++j) {
+            if (j >= 2) emit(j - 2);
+            const int ui = j + 2 * HEM_PIPE;   // row pointers of tile j + 2 PIPE
+            if (ui < ntiles) {
+                const int r0 = ui << 5, rows = min(32, n - r0);
+                int *dst = iabuf + (ui % HEM_IA_SLOTS) * HEM_IA_STRIDE;
+                cp_async4(dst + lane, ia + r0 + min(lane, rows));
+                if (lane == 0) cp_async4(dst + 32, ia + r0 + rows);
+            }
+            cp_async_wait<HEM_PIPE - 1>();   // ia(j + PIPE) and cand(j) have landed
+            __syncwarp();
+            const int uc = j + HEM_PIPE;     // ranked lists of tile j + PIPE
+            if (uc >= 0 && uc < ntiles) {
+                const int *iu = iabuf + (uc % HEM_IA_SLOTS) * HEM_IA_STRIDE;
+                const int rows = min(32, n - (uc << 5));
+                const int e0 = iu[0], m = iu[rows] - e0;
+                if (m <= HEM_TILE_CAP) {
+                    int *dst = cbuf + (uc % HEM_C_SLOTS) * HEM_TILE_CAP;
+                    for (int e = lane; e < m; e += 32) cp_async4(dst + e, cand + e0 + e);
+                }
+            }
+            cp_async_commit();
+            if (j >= 0) __syncthreads();   // tile j is ready; tile j - 1 is walked
+        }
+        cp_async_wait<0>();
+        __syncthreads();                    // the last tile is walked
+        if (ntiles >= 2) emit(ntiles - 2);
+        if (ntiles >= 1) emit(ntiles - 1);
+        if (lane == 0) out[0] = nc;
+        return;
+    }
+
+    // ---- warp 0: the walk
+    for (int w = lane; w < HEM_RING_WORDS; w += 32) hem_smem[w] = 0u;
+    __syncthreads();
+    for (int t = 0; t < ntiles; ++t) {
+        const int r0 = t << 5, rows = min(32, n - r0);
+        ring.clear32(r0 + bw, lane);
+        __syncwarp();
+        const int *it = iabuf + (t % HEM_IA_SLOTS) * HEM_IA_STRIDE;
+        const int e0 = it[0];
+        const bool staged = it[rows] - e0 <= HEM_TILE_CAP;
+        const int *ct = staged ? cbuf + (t % HEM_C_SLOTS) * HEM_TILE_CAP : cand;
+        const int off = staged ? e0 : 0;
+        int *pk = picks + (t & 1) * 32;
+        // rows of the tile still unmatched and not isolated (pass 0)
+        const bool act = lane < rows && it[lane + 1] - it[lane] > 1 && !ring.get(r0 + lane);
+        unsigned todo = __ballot_sync(0xffffffffu, act);
+        int p = -1;
+        if (act) {
+            const int b1 = it[lane + 1];
+            for (int e = it[lane]; e < b1; e += 2) {
+                const int c0 = ct[e - off];
+                const int c1 = e + 1 < b1 ? ct[e + 1 - off] : -1;
+                const bool ok0 = c0 >= 0 && !ring.get(c0);
+                const bool ok1 = c1 >= 0 && !ring.get(c1);
+                if (ok0) { p = c0; break; }
+                if (ok1) { p = c1; break; }
+            }
+        }
+        const unsigned tl = (unsigned)(p - r0);   // < 32: the pick is a row of this tile
+        pm[lane] = 0u;
+        __syncwarp();
+        if (p >= 0 && tl < 32u) atomicOr(pm + tl, 1u << lane);
+        const unsigned same = __match_any_sync(0xffffffffu, p);
+        const unsigned has = __ballot_sync(0xffffffffu, p >= 0);
+        __syncwarp();
+        if (p >= 0) info[lane] = make_uint2(tl < 32u ? 1u << tl : 0u, same | pm[lane]);
+        else info[lane] = make_uint2(0u, 0u);
+        pk[lane] = p;
+        __syncwarp();
+        unsigned stale = 0u, done = 0u, racc = 0u, written = 0u;
+        while (todo) {
+            const int i = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            if ((stale >> i) & 1u) {
+                // the ring takes every pick of the tile so far, then row i scans again
+                const unsigned w = done & has & ~written;
+                if ((w >> lane) & 1u) { ring.set(r0 + lane); ring.set(p); }
+                written |= w;
+                __syncwarp();
+                const int b0 = it[i], b1 = it[i + 1];
+                int q = -1;
+                for (int e = b0; e < b1; e += 32) {
+                    const int c = e + lane < b1 ? ct[e + lane - off] : -1;
+                    const bool ok = c >= 0 && !ring.get(c);
+                    const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                    if (bal) {
+                        q = __shfl_sync(0xffffffffu, c, __ffs(bal) - 1);
+                        break;
+                    }
+                }
+                if (q >= 0) {
+                    if (lane == 0) { ring.set(r0 + i); ring.set(q); pk[i] = q; }
+                    racc |= 1u << i;
+                    const unsigned d = (unsigned)(q - r0);
+                    if (d < 32u) todo &= ~(1u << d);
+                    stale |= __ballot_sync(0xffffffffu, p == q || p == r0 + i);
+                }
+                __syncwarp();
+                continue;
+            }
+            const uint2 f = info[i];
+            done |= 1u << i;
+            todo &= ~f.x;
+            stale |= f.y;
+        }
+        const unsigned acc = (done & has) | racc;
+        const unsigned w = done & has & ~written;
+        if ((w >> lane) & 1u) { ring.set(r0 + lane); ring.set(p); }
+        if (lane == 0) accepted[t & 1] = acc;
+        __syncthreads();   // tile t walked; tile t + 1 staged
     }
 }
 
@@ -533,8 +786,9 @@ __global__ void k_hem_final(int n, int *mask) {
 
 int hem_exact(int n, const int *nia, const int *nja, const double *nval,
               int *agg, int *nagg, int *work_n, cudaStream_t s) {
-    // out: aggregates, status | longest row | next row | barrier (4) | error
-    enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 8, O_N = 10 };
+    // out: aggregates, status | longest row | next row | barrier (4) | error, stopped
+    enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 8, O_STOP = 9,
+           O_N = 10 };
     int *out = nullptr;
     HZB_TRY(dalloc(&out, O_N));
     int h[O_N] = {0};
@@ -549,74 +803,122 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
         e = cudaMemcpyAsync(&gnnz, nia + n, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { dfree(out); set_error(e, __FILE__, __LINE__); return ERROR_SOLVER_MISC; }
-    // 1: rounds over ranked lists; 4: one warp walks the rows, for rows longer
-    // than the ranking takes (its work grows with the square of a row's
-    // length).  HZB_HEM_PATH=4 names the walk for tests.
-    int path = h[O_LEN] <= HEM_RANK_MAXLEN ? 1 : 4;
-    if (const char *f = getenv("HZB_HEM_PATH"))
-        if (atoi(f) == 4) path = 4;
-    if (path == 1) {
-        int *cand = nullptr, *flag = nullptr, *pos = nullptr, *tmp = nullptr;
+    // Rounds over ranked lists, and the walk over them where the rounds' pace is
+    // too slow; a warp on the rows themselves for rows longer than the ranking
+    // takes (its work grows with the square of a row's length).  HZB_HEM_PATH
+    // names one for tests: 1 the rounds to their end, 2 the walk, 4 the warp.
+    int path = h[O_LEN] <= HEM_RANK_MAXLEN ? 0 : 4;
+    if (const char *f = getenv("HZB_HEM_PATH")) {
+        const int want = atoi(f);
+        if (want == 4 || (path == 0 && (want == 1 || want == 2))) path = want;
+    }
+    if (path == 0 && n <= HEM_WALK_SMALL) path = 2;
+    if (path != 4) {
+        int *cand = nullptr, *flag = nullptr, *pos = nullptr, *tmp = nullptr, m = 0;
         unsigned long long *post = nullptr;
+        int *cnt = work_n;
         if ((rc = dalloc(&cand, gnnz)) || (rc = dalloc(&post, (size_t)2 * n)) ||
             (rc = dalloc(&flag, n)) || (rc = dalloc(&pos, n + 1)) ||
             (rc = dalloc(&tmp, scan_tmp_size(n + 1)))) {
             dfree(cand); dfree(post); dfree(flag); dfree(pos); dfree(tmp); dfree(out);
             return rc;
         }
-        int *cnt = work_n;
-        k_hem_init<<<g, 256, 0, s>>>(n, nia, agg);
-        k_hem_rank<<<std::min(div_up(n, 8), 148 * 64), 256, 0, s>>>(n, nia, nja, nval, cand);
-        count_launch(2);
-        // all ones: older than any round's post
-        e = cudaMemsetAsync(post, 0xff, sizeof(unsigned long long) * 2 * n, s);
-        // one CTA per SM; a cluster of 1 to 8 on small levels
-        const bool cluster = n <= HEM_CLUSTER_ROWS;
-        int grid = std::min(sm_count(), div_up(n, HEM_BLOCK));
-        if (cluster) {
-            const int want = std::min(grid, HEM_CLUSTER);
-            for (grid = 1; grid < want;) grid *= 2;
-        }
-        const int first = grid * HEM_BLOCK;
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(out + O_NEXT, &first, sizeof(int), cudaMemcpyHostToDevice, s);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(HEM_BLOCK);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        if (cluster) {
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = grid;
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        } else {
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-        }
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia, (const int *)cand, agg, post,
-                                   out + O_NEXT, (unsigned long long *)(out + O_BAR),
-                                   out + O_ERR);
-        count_launch();
-        k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
-        rc = scan_exclusive(flag, pos, n, tmp, s);
-        int m = 0;
-        if (!rc) {
-            k_hem_number<<<g, 256, 0, s>>>(n, pos, agg, cnt);
-            cudaMemcpyAsync(out + O_NC, pos + n, sizeof(int), cudaMemcpyDeviceToDevice, s);
+        auto rank = [&]() {
+            k_hem_init<<<g, 256, 0, s>>>(n, nia, agg);
+            k_hem_rank<<<std::min(div_up(n, 8), 148 * 64), 256, 0, s>>>(n, nia, nja, nval, cand);
+            count_launch(2);
+        };
+        // the rows left over by pass 1, ascending, and how many (with out)
+        auto leftovers = [&]() -> int {
             k_flag_eq<<<g, 256, 0, s>>>(n, agg, -1, flag);
-            rc = scan_exclusive(flag, pos, n, tmp, s);
+            HZB_TRY(scan_exclusive(flag, pos, n, tmp, s));
+            // the ranked lists are done with (gnnz >= leftovers)
+            k_compact<<<g, 256, 0, s>>>(n, flag, pos, cand);
+            count_launch(2);
+            HZB_CUDA(cudaMemcpyAsync(&m, pos + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+            HZB_CUDA(cudaMemcpyAsync(h, out, O_N * sizeof(int), cudaMemcpyDeviceToHost, s));
+            HZB_CUDA(cudaStreamSynchronize(s));
+            return SUCCESS;
+        };
+        auto rounds = [&](bool may_stop) -> int {
+            rank();
+            // all ones: older than any round's post
+            HZB_CUDA(cudaMemsetAsync(post, 0xff, sizeof(unsigned long long) * 2 * n, s));
+            // one CTA per SM; a cluster of 1 to 8 on small levels
+            const bool cluster = n <= HEM_CLUSTER_ROWS;
+            int grid = std::min(sm_count(), div_up(n, HEM_BLOCK));
+            if (cluster) {
+                const int want = std::min(grid, HEM_CLUSTER);
+                for (grid = 1; grid < want;) grid *= 2;
+            }
+            const int first = grid * HEM_BLOCK;
+            HZB_CUDA(cudaMemsetAsync(out + O_BAR, 0, sizeof(int) * (O_N - O_BAR), s));
+            HZB_CUDA(cudaMemcpyAsync(out + O_NEXT, &first, sizeof(int), cudaMemcpyHostToDevice,
+                                     s));
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(HEM_BLOCK);
+            cfg.stream = s;
+            cudaLaunchAttribute attr[1];
+            if (cluster) {
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = grid;
+                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            } else {
+                attr[0].id = cudaLaunchAttributeCooperative;
+                attr[0].val.cooperative = 1;
+            }
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            HZB_CUDA(cudaLaunchKernelEx(
+                &cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia,
+                (const int *)cand, agg, post, out + O_NEXT, (unsigned long long *)(out + O_BAR),
+                out + O_ERR,
+                !may_stop ? 0 : cluster ? HEM_WALK_ROWS_CLUSTER : HEM_WALK_ROWS_GRID,
+                out + O_STOP));
+            k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
+            count_launch(2);
+            HZB_TRY(scan_exclusive(flag, pos, n, tmp, s));
+            k_hem_number<<<g, 256, 0, s>>>(n, pos, agg, cnt);
+            count_launch();
+            HZB_CUDA(cudaMemcpyAsync(out + O_NC, pos + n, sizeof(int), cudaMemcpyDeviceToDevice,
+                                     s));
+            return leftovers();
+        };
+        // *done: false when the graph reaches too far for the walk's ring
+        auto walk = [&](bool *done) -> int {
+            int bw = n - 1;
+            if (bw >= ((int)HemRing<true>::SIZE - 64) / 2) {
+                HZB_CUDA(cudaMemsetAsync(out + O_LEN, 0, sizeof(int), s));
+                k_graph_bandwidth<<<g, 256, 0, s>>>(n, nia, nja, out + O_LEN);
+                count_launch();
+                HZB_CUDA(cudaMemcpyAsync(&bw, out + O_LEN, sizeof(int), cudaMemcpyDeviceToHost,
+                                         s));
+                HZB_CUDA(cudaStreamSynchronize(s));
+            }
+            *done = bw < (HEM_RING_BITS - 64) / 2;
+            if (!*done) return SUCCESS;
+            rank();
+            auto kernel = bw < ((int)HemRing<true>::SIZE - 64) / 2 ? k_hem_pass1_staged<true>
+                                                                   : k_hem_pass1_staged<false>;
+            HZB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)HEM_STAGED_SMEM));
+            kernel<<<1, 64, HEM_STAGED_SMEM, s>>>(n, bw, nia, cand, agg, cnt, out);
+            count_launch();
+            return leftovers();
+        };
+        bool walked = false;
+        if (path == 2) rc = walk(&walked);
+        else rc = rounds(path == 0);
+        if (!rc && path == 0 && h[O_STOP]) {
+            rc = walk(&walked);
+            if (!rc && !walked) rc = rounds(false);
+        } else if (!rc && path == 2 && !walked) {
+            rc = rounds(false);
         }
-        if (!rc) {
-            int *list = cand;   // the ranked lists are done with (gnnz >= leftovers)
-            k_compact<<<g, 256, 0, s>>>(n, flag, pos, list);
-            count_launch(4);
-            cudaMemcpyAsync(&m, pos + n, sizeof(int), cudaMemcpyDeviceToHost, s);
-            cudaStreamSynchronize(s);
+        if (!rc && !h[O_ERR]) {
             if (m > 0) {
-                k_hem_pass2_list<<<1, 32, 0, s>>>(m, list, nia, nja, agg, cnt, out);
+                k_hem_pass2_list<<<1, 32, 0, s>>>(m, cand, nia, nja, agg, cnt, out);
                 count_launch();
             }
             k_hem_final<<<g, 256, 0, s>>>(n, agg);

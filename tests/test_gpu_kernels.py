@@ -5,6 +5,7 @@ import ctypes as C
 
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import hazmath_b200 as hz
 from hazmath_b200 import problems as P
@@ -310,7 +311,6 @@ def test_streamed_gauss_seidel_row_widths(port, name, sm, pre):
 
 def _periodic(nx, ny, px, py):
     """5-point matrix of a grid periodic in x or y, CSR rows ascending."""
-    import scipy.sparse as sp
     def line(m, per):
         d = sp.diags([np.full(m - 1, -1.0), np.full(m - 1, -1.0)], [-1, 1], format="lil")
         if per:
@@ -338,3 +338,51 @@ def test_streamed_gauss_seidel_far_couplings(port, nx, ny, px, py, sm, pre):
     x = dev(x0)
     assert hz.lib().hzb_smoother_device(sm, pre, 2, 1.15, *A.args(), ptr(dev(b)), ptr(x)) == 0
     assert np.array_equal(host(x), port.smooth(sm, pre, 2, ia, ja, val, b, x0, relax=1.15))
+
+
+def _strip(nx, ny, seed=None, periodic=False):
+    """5-point graph of nx x ny points (ny = 1: a chain), weights 1 or random."""
+    i = np.arange(nx * ny).reshape(ny, nx)
+    pairs = [(i[:, :-1], i[:, 1:]), (i[:-1], i[1:])]
+    if periodic:
+        pairs.append((i[:, :1], i[:, -1:]))
+    a = np.concatenate([p.ravel() for p, _ in pairs])
+    b = np.concatenate([q.ravel() for _, q in pairs])
+    w = np.ones(len(a)) if seed is None else np.random.default_rng(seed).uniform(0.5, 1.5, len(a))
+    n = nx * ny
+    A = sp.coo_matrix((-w, (a, b)), shape=(n, n)).tocsr()
+    A = (A + A.T + sp.eye(n) * 5.0).tocsr()
+    A.sort_indices()
+    return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+
+
+# rows that can only be decided one after the other: the rounds give way to the
+# walk (chains, strips of a few rows), or do not (wider ones); with couplings
+# beyond the byte ring (65,504 rows) and beyond the bit ring, where the rounds
+# go on to their end
+@pytest.mark.parametrize("nx,ny,kw", [
+    (500, 1, {}), (2001, 1, {"seed": 1}), (16384, 1, {}), (16385, 1, {}), (100000, 1, {"seed": 2}),
+    (2, 20000, {}), (4, 9000, {"seed": 3}), (16, 3000, {}), (64, 700, {}), (9000, 4, {}),
+    (70000, 1, {"periodic": True}), (530000, 1, {"periodic": True, "seed": 4})])
+def test_hem_chains_and_strips(port, nx, ny, kw):
+    ia, ja, val = _strip(nx, ny, **kw)
+    nc, agg = _hem(ia, ja, val, 0.0)
+    nc_o, agg_o = port.hem(ia, ja, val, 0.0)
+    assert nc == nc_o and np.array_equal(agg, agg_o)
+
+
+def test_hem_chain_no_slower_than_the_walk(monkeypatch):
+    """A chain of 100,000 rows, one decision after the other: 3 times the walk's
+    time at most (the rounds to their end take 20 times)."""
+    import time
+    ia, ja, val = _strip(100000, 1)
+    best = {}
+    for path in ("0", "2"):
+        monkeypatch.setenv("HZB_HEM_PATH", path)
+        _hem(ia, ja, val, 0.0)
+        best[path] = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            _hem(ia, ja, val, 0.0)
+            best[path] = min(best[path], time.perf_counter() - t)
+    assert best["0"] < 3 * best["2"]
