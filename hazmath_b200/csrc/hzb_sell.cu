@@ -214,25 +214,45 @@ __device__ __forceinline__ void sell_row(const SellView<T> &V, int r, const T *_
     else sell_slice<T, L1, true>(V, h, r % SELL_C, x, t, d);
 }
 
-// The sum of slot r's row once more from t on, over its own entries only: a zero
-// that fills up a shorter row may meet an infinite or NaN x, and the row's own
-// result need not be NaN then.  For the rows whose sum came out NaN.
+// The sums of this thread's row once more, t on from where it is, over the row's
+// own entries only: a zero that fills up a shorter row may meet an infinite or
+// NaN x, and the row's own result need not be NaN then.  For the rows whose sum
+// came out NaN.  Where it can be it is a call behind the store, the kernel's last
+// act, for which nothing is kept in registers: inline the FP64 sweep of 1.8
+// million rows took 53 to 55 us, so it takes 49.9 (49.7 without any of this).
 template <typename T, bool L1>
-__device__ __forceinline__ T sell_row_own(const SellView<T> &V, int r, const T *__restrict__ x,
-                                          T t) {
-    const int len = (int)(__ldcg(V.slot + r) / SELL_WIN);
+__device__ __forceinline__ void sell_row_own(const SellView<T> &V, const T *__restrict__ x, T &t,
+                                             T &d) {
+    const int r = blockIdx.x * SELL_WIN + threadIdx.x;
+    const unsigned sl = __ldcg(V.slot + r);
     const int4 h = __ldcg(V.head + r / SELL_C);
     const unsigned short *col = V.col + (size_t)(h.y < 0 ? -h.y - 1 : h.y) * SELL_C;
 #pragma unroll 1
-    for (int u = 0; u < len; ++u) {
+    for (int u = 0; u < (int)(sl / SELL_WIN); ++u) {
         const int at = sell_at(u, h.w, r % SELL_C);
         const int2 b = V.base[h.z + u / 2];
         const int c = h.y < 0 ? reinterpret_cast<const int *>(col)[at]
                               : (u % 2 ? b.y : b.x) + (int)col[at];
-        const T p = V.val[(size_t)h.x * SELL_C + at] * x[c];
-        t = L1 ? t - p : t + p;
+        const T v = V.val[(size_t)h.x * SELL_C + at];
+        if (L1) {
+            t -= v * x[c];
+            d += fabs(v);
+        } else {
+            t += v * x[c];
+        }
     }
-    return t;
+}
+
+// the sweep's row, from the start
+template <typename T>
+__device__ __noinline__ void l1_sell_again(const SellView<T> &V, const T *b, const T *x, T *xn,
+                                           const float *omega) {
+    const int k = blockIdx.x * SELL_WIN +
+                  (int)(__ldcg(V.slot + blockIdx.x * SELL_WIN + threadIdx.x) & SELL_ROW);
+    T t = b[k], d = T(0), xi = x[k];
+    sell_row_own<T, true>(V, x, t, d);
+    if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[k]) * (t / d) : t / d;
+    xn[k] = xi;
 }
 
 template <typename T>
@@ -245,16 +265,18 @@ k_l1_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ b,
     if (i >= n) return;
     T t = __ldcs(b + i), d = T(0);
     sell_row<T, true>(V, r, x, t, d);
-    if (sizeof(T) == 8 && t != t) t = sell_row_own<T, true>(V, r, x, b[i]);
     T xi = x[i];
     if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[i]) * (t / d) : t / d;
     xn[i] = xi;
-    if (sizeof(T) == 4 && t != t) {
-        t = sell_row_own<T, true>(V, r, x, b[i]);
-        xi = x[i];
-        if (fabs(d) > T(SMALLREAL)) xi += omega ? T(omega[i]) * (t / d) : t / d;
-        xn[i] = xi;
-    }
+    if (t != t) l1_sell_again<T>(V, b, x, xn, omega);
+}
+
+// the product's row, from the start: b_i - A x (RES) or A x
+template <typename T, bool RES>
+__device__ __noinline__ void spmv_sell_again(const SellView<T> &V, const T *x, T bi, T *yi) {
+    T t = T(0), d = T(0);
+    sell_row_own<T, false>(V, x, t, d);
+    *yi = RES ? bi - t : t;
 }
 
 // 64 warps an SM here too (FP64, 16.6 million rows, with (x, y): 290 us; 322 with
@@ -272,15 +294,20 @@ k_spmv_sell(int n, const __grid_constant__ SellView<T> V, const T *__restrict__ 
     const T bi = MODE == SPMV_RES ? __ldcs(b + i) : T(0);
     T t = T(0), d = T(0);
     sell_row<T, false>(V, r, x, t, d);
-    if (t != t) t = sell_row_own<T, false>(V, r, x, T(0));
+    if ((MODE == SPMV_AXPY || MODE == SPMV_Y_DOT) && t != t) {
+        t = T(0);
+        sell_row_own<T, false>(V, x, t, d);
+    }
     if (MODE == SPMV_RES) {
         y[i] = bi - t;
+        if (t != t) spmv_sell_again<T, true>(V, x, bi, y + i);
     } else if (MODE == SPMV_AXPY) {
         if (alpha == T(1)) y[i] += t;
         else if (alpha == T(-1)) y[i] -= t;
         else y[i] += t * alpha;
     } else if (MODE == SPMV_Y) {
         y[i] = t;
+        if (t != t) spmv_sell_again<T, false>(V, x, T(0), y + i);
     } else {
         __shared__ T prod[SELL_WIN], sh[SELL_WIN / 32];
         if (i < n) {
