@@ -212,3 +212,25 @@ def test_mixed_precision_kuhn():
     assert np.linalg.norm(x32 - x64) / np.linalg.norm(x64) < 1e-6
     S64.close()
     S32.close()
+
+
+def test_no_cycle_is_wasted_on_a_fast_solve():
+    """A mixed solve that gains several digits a step ends without a cycle beyond
+    the ones it uses: fewer launches than the same two steps with a third to come."""
+    ia, ja, val = P.kuhn3d_p1(24, P.lognormal_field(24, 1.0, 4.0, 3))
+    val = np.where(ja == np.repeat(np.arange(len(ia) - 1), np.diff(ia)), 11.0, 1.0) * val
+    b = P.rhs_uniform(len(ia) - 1, 1)
+    out = []
+    for tol, maxit in ((1e-8, 100), (1e-30, 2)):
+        it = hz.itsolver_param(linear_itsolver_type=hz.SOLVER_CG, linear_precond_type=hz.PREC_AMG,
+                               linear_tol=tol, linear_maxit=maxit, linear_stop_type=1)
+        S = hz.Solver(hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG, presmooth_iter=2,
+                                   postsmooth_iter=2), it,
+                      hz.b200_param(precision=hz.HZB_PREC_MIXED))
+        assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+        for _ in range(2):
+            S.solve_host(b, np.zeros(len(b)))
+        out.append((S.stats().iterations, S.stats().launches))
+        S.close()
+    assert out[0][0] == 2
+    assert out[0][1] < out[1][1] - 5      # a cycle is ten launches and more
