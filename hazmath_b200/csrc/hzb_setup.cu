@@ -325,12 +325,13 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 // its hierarchy; 11.8 and 37 ms now).
 //
 // CLUSTER: the CTAs are one cluster of at most 8, whose barrier and counts (in
-// every member's shared memory) cost half as much.  Its window of 8192 rows
-// can lengthen the dependency chain, which holds with half of the rows in
-// play (16,256 rows of a 2D 5-point hierarchy: 0.7 ms against 0.9) but not on
-// larger levels (32,512 rows: 584 rounds with 4096 in play, 254 with all),
-// hence HEM_CLUSTER_ROWS.
-constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = 16384;
+// every member's shared memory) cost less.  For levels whose rows are all in
+// play in it at once, 8192: there it takes 0.88 to 1.0 of the grid's time (2D,
+// 3D and anisotropic hierarchies, 2,400 to 8,192 rows; whole call 0.76 against
+// 0.69 ms at 4,096 rows of a 2D one).  With more rows its window lengthens the
+// dependency chain, and it takes 0.97 to 1.55 (9,600 rows 1.28 against 1.94
+// ms, 12,187 0.74 and 0.83, 16,256 1.33 and 2.06, 32,512 1.72 and 4.34).
+constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = HEM_BLOCK * HEM_CLUSTER;
 
 // A chain is decided one row a round.  So every HEM_PACE rounds their pace is
 // looked at, and when the rows left would take longer at it than the walk below

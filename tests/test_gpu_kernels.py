@@ -386,3 +386,15 @@ def test_hem_chain_no_slower_than_the_walk(monkeypatch):
             _hem(ia, ja, val, 0.0)
             best[path] = min(best[path], time.perf_counter() - t)
     assert best["0"] < 3 * best["2"]
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 32), (683, 3), (64, 128), (2731, 3), (128, 128)])
+def test_hem_rounds_of_cluster_and_grid(port, monkeypatch, nx, ny):
+    """Both sides of the sizes where the walk, the cluster and the grid take over
+    (2048 and 8192 rows), the rounds to their end too."""
+    ia, ja, val = _strip(nx, ny, seed=5)
+    nc_o, agg_o = port.hem(ia, ja, val, 0.0)
+    for path in ("0", "1"):
+        monkeypatch.setenv("HZB_HEM_PATH", path)
+        nc, agg = _hem(ia, ja, val, 0.0)
+        assert nc == nc_o and np.array_equal(agg, agg_o)
