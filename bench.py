@@ -811,8 +811,8 @@ def run_single(args, rank, world, local, dist):
                          "bytes_per_launch": l1_by, "ms_per_launch": l1_ms,
                          "traffic": TRAFFIC_PER_BYTE["l1_32"] * l1_by,
                          "traffic_source": "ncu DRAM bytes per algorithmic byte of the "
-                         "sliced-ELL sweep (level 0 of the 160^3 instance), times this "
-                         "launch's bytes"},
+                         "sliced-ELL sweep (level 0 of the 160^3 instance: reads as "
+                         "measured, the whole result as written), times this launch's bytes"},
             "solve_roofline": {"bound": "hbm", "bytes": solve_by,
                                "seconds": solve_ml, "achieved": solve_by / solve_ml / 1e9,
                                "peak": peak, "unit": "GB/s",
@@ -1116,12 +1116,14 @@ def parity_vs_fixture(name, st, iters):
 # DRAM bytes (read + written) per algorithmic byte of one launch, measured by
 # ncu over the bytes hzb_time_kernel counts: the FP32 l1-Jacobi sweep in the
 # sliced-ELL schedule the autotuner picks on the fine levels (level 0 of the
-# 160^3 instance of the family: 222.5 MB read and 5.6 MB written, the rest of
-# the result staying in L2, for 238,075,584 algorithmic bytes), and the drop-in's
+# 160^3 instance of the family, 4,019,679 rows and 238,075,584 algorithmic bytes:
+# 222.5 MB read, and the whole result counted as written, 4 bytes a row -- of the
+# one captured launch 5.6 of its 16.1 MB had left L2, but the 256^3 sweeps'
+# results, 66 MB each, leave it before they are read again), and the drop-in's
 # FP64 SpMV on level 0 of the 128^3 case.  The 256^3 launches run the same
 # kernels over more entries, and their traffic is this ratio times their
 # algorithmic bytes.
-TRAFFIC_PER_BYTE = {"l1_32": (222512896 + 5590784) / 238075583.5,
+TRAFFIC_PER_BYTE = {"l1_32": (222512896 + 4 * 4019679) / 238075583.5,
                     "spmv64": 404.52e6 / 405049716.0}
 
 

@@ -103,3 +103,11 @@ def test_clock_samples_after_mark():
     late = bench.Clocks.summary(rows, datetime.datetime(2027, 1, 1))
     assert late["samples"] == 3 and late["sm_mhz"] == 1905.0
     assert bench.Clocks.summary([], mark)["sm_mhz"] is None
+
+
+def test_traffic_is_no_less_than_what_a_launch_moves():
+    """The sweep's DRAM bytes per algorithmic byte count its whole result: a
+    capture of one launch ends while part of it is still in L2."""
+    sys.path.insert(0, ROOT)
+    import bench
+    assert 1.0 <= bench.TRAFFIC_PER_BYTE["l1_32"] < 1.02
