@@ -255,6 +255,13 @@ __global__ void k_longest_row(int n, const int *__restrict__ ia, int *longest) {
     if (threadIdx.x == 0) atomicMax(longest, len);
 }
 
+int longest_row(int n, const int *ia, int *longest, cudaStream_t s) {
+    k_longest_row<<<grid_for(n), 256, 0, s>>>(n, ia, longest);
+    count_launch();
+    HZB_LAUNCH_CHECK();
+    return SUCCESS;
+}
+
 __global__ void k_hem_init(int n, const int *__restrict__ ia, int *state) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
          k += gridDim.x * blockDim.x)

@@ -9,6 +9,8 @@ namespace hzb {
 
 // out[0..n] = exclusive scan of in[0..n), out[n] = total.  tmp: >= scan_tmp(n)
 int scan_tmp_size(int n);
+// *longest (zeroed): the most entries of a row
+int longest_row(int n, const int *ia, int *longest, cudaStream_t s);
 int scan_exclusive(const int *in, int *out, int n, int *tmp, cudaStream_t s);
 
 // strength graph Neigh (construct_strongly_coupled, amg_setup_ua.c:375-455);

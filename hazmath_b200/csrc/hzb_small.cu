@@ -252,7 +252,9 @@ struct SmallData;
 template <>
 struct SmallData<float> {
     static constexpr int LPR = 4, B = 4;
-    static bool fits(const Level &L) { return L.n <= SMALL_ROWS_32; }
+    static bool fits(const Level &L) {
+        return L.n <= SMALL_ROWS_32 && L.largest_agg <= SMALL_AGG;
+    }
     static const int *ia(const Level &L) { return L.ia32; }
     static const int *ja(const Level &L) { return L.ja32; }
     static const float *val(const Level &L) { return L.val32; }
@@ -265,7 +267,10 @@ struct SmallData<float> {
 template <>
 struct SmallData<double> {
     static constexpr int LPR = 1, B = 8;
-    static bool fits(const Level &L) { return L.nnz <= SMALL_NNZ_64; }
+    static bool fits(const Level &L) {
+        return L.nnz <= SMALL_NNZ_64 && (long long)SMALL_ROW_64 * L.n >= L.nnz &&
+               L.largest_agg <= SMALL_AGG;
+    }
     static const int *ia(const Level &L) { return L.ia; }
     static const int *ja(const Level &L) { return L.ja; }
     static const double *val(const Level &L) { return L.val; }

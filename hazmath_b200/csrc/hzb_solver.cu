@@ -1048,12 +1048,29 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
         HZB_TRY(S->kwc.alloc(S->lv[S->nl - 1].n, s));
     if (S->bp.precision == HZB_PREC_MIXED) HZB_TRY(ensure_fp32(S));
     trace.mark("fp32");
+    // the sizes of the aggregates, for the rule of the merged kernels
+    int largest[MAX_AMG_LVL] = {0}, *d_largest = nullptr;
+    if (!batch) {
+        HZB_TRY(dalloc(&d_largest, MAX_AMG_LVL));
+        rc = cudaMemsetAsync(d_largest, 0, sizeof(largest), s) == cudaSuccess ? SUCCESS
+                                                                             : ERROR_SOLVER_MISC;
+        for (int l = 0; l < std::min<int>(S->nl - 1, MAX_AMG_LVL) && !rc; ++l)
+            if (S->lv[l].ria && !S->lv[l].sa && S->lv[l].n <= SMALL_NNZ_64)
+                rc = longest_row(S->lv[l].nc, S->lv[l].ria, d_largest + l, s);
+        if (!rc && cudaMemcpyAsync(largest, d_largest, sizeof(largest), cudaMemcpyDeviceToHost,
+                                   s) != cudaSuccess)
+            rc = ERROR_SOLVER_MISC;
+        dfree(d_largest);
+        HZB_TRY(rc);
+    }
     HZB_CUDA(cudaEventRecord(S->e1, s));
     HZB_CUDA(cudaEventSynchronize(S->e1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, S->e0, S->e1);
     S->st.setup_seconds = ms * 1e-3;
     S->st.num_levels = S->nl;
+    for (int l = 0; l < std::min<int>(S->nl - 1, MAX_AMG_LVL); ++l)
+        if (largest[l]) S->lv[l].largest_agg = largest[l];
     for (int l = 0; l < S->nl && l < MAX_AMG_LVL; ++l) {
         S->st.rows[l] = S->lv[l].n;
         S->st.nnz[l] = S->lv[l].nnz;

@@ -61,6 +61,7 @@ struct Level {
     float *d_gs32 = nullptr;
     float *l1_32 = nullptr;           // l1 row norms for the FP32 first sweep
     double *l1_64 = nullptr;          // the FP64 cycle's, on small levels
+    int largest_agg = 1 << 30;        // fine rows of a row of the next level, at most
     Schedule fwd, bwd, col;
     // coarsest level with the direct solver: the transposed matrix the
     // reference factors (and leaves in mgl[nl-1].A)
@@ -210,7 +211,16 @@ int cycle32(hzb_solver *S, const AMG_param &cyc, bool level0_zero);
 // entries in, the 64^3 solve takes 8.45 and 9.05 ms; with 0.5 and 1.1 million
 // the 400^2 one 6.4 and 5.9).  Above, the bundles and the sliced ELL copy
 // stream their rows better.
+//   And while what one thread (FP64) or four lanes (FP32) do one after the other
+// stays short.  The fine rows of a coarse row: up to SMALL_AGG, which heavy edge
+// matching and 2D VMB aggregates keep to (gains of 1.03 to 1.5 in a solve), HEC
+// and 3D VMB ones do not (sizes of 13 to 314: 0.07 to 1.08 of the speed of the
+// separate kernels, 0.77 where 1096 rows joined one aggregate).  The entries of
+// a row, in FP64: SMALL_ROW_64 in the mean (27-point levels of 24 to 34: 0.95 to
+// 1.00, random graphs of 75 to 430 in the coarsest levels 0.80 to 0.96; FP32 1.2
+// to 1.7 on the same).
 constexpr int SMALL_ROWS_32 = 262144, SMALL_NNZ_64 = 1250000;
+constexpr int SMALL_AGG = 12, SMALL_ROW_64 = 24;
 template <typename T>
 int small_first_level(const hzb_solver *S, const AMG_param &cyc, int l0, bool zero);
 template <typename T>

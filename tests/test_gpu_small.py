@@ -161,3 +161,51 @@ def test_values_changed_in_the_callers_array(smoother, make):
     want = sweep(A, 0, 1, r, x + np.where(agg >= 0, xc[np.maximum(agg, 0)], 0.0))
     assert np.array_equal(got, want)
     S.close()
+
+
+def _random_graph(n, deg, seed):
+    rng = np.random.default_rng(seed)
+    i, j = rng.integers(0, n, n * deg // 2), rng.integers(0, n, n * deg // 2)
+    A = sp.coo_matrix((-rng.uniform(0.5, 1.5, len(i)), (i, j)), shape=(n, n)).tocsr()
+    A = A + A.T
+    A.setdiag(0)
+    A.eliminate_zeros()
+    A = (A + sp.diags(1.01 * -np.asarray(A.sum(1)).ravel() + 0.1)).tocsr()
+    A.sort_indices()
+    return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+
+
+# aggregates and rows on both sides of the merged kernels' rule
+@pytest.mark.parametrize("agg", [hz.HEM, hz.HEC, hz.VMB])
+@pytest.mark.parametrize("make", [lambda: P.poisson2d_5pt(90), lambda: _random_graph(5000, 8, 1),
+                                  lambda: _random_graph(5000, 22, 2),
+                                  lambda: _random_graph(5000, 40, 3)],
+                         ids=["2d_90", "random_8", "random_22", "random_40"])
+def test_fp64_cycle_by_aggregates_bit_exact(agg, make):
+    ia, ja, val = make()
+    r = P.rhs_uniform(len(ia) - 1, 5)
+    S = hz.Solver(_amg(1, 2, coarse_dof=600, aggregation_type=agg))
+    assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+    assert S.stats().num_levels >= 2
+    assert np.array_equal(_precond(S, r), _cycle(S, 0, 1, 2, r))
+    S.close()
+
+
+@pytest.mark.parametrize("precision", [hz.HZB_PREC_FP64, hz.HZB_PREC_MIXED])
+def test_large_aggregates_keep_the_separate_kernels(precision):
+    """HEC aggregates of hundreds of long rows: an iteration takes no more than 3
+    times one with pairs on the same matrix (merged, where a thread takes an
+    aggregate's rows one after the other, 15 times)."""
+    ia, ja, val = _random_graph(20000, 60, 1)
+    b = P.rhs_uniform(len(ia) - 1, 5)
+    t = {}
+    for agg in (hz.HEC, hz.HEM):
+        S = hz.Solver(_amg(2, 2, aggregation_type=agg), None, hz.b200_param(precision=precision))
+        assert S.setup_host(ia, ja, val) == 0, hz.last_error()
+        t[agg] = []
+        for _ in range(4):
+            assert S.solve_host(b, np.zeros(len(b))) > 0
+            st = S.stats()
+            t[agg].append(st.solve_seconds / st.iterations)
+        S.close()
+    assert min(t[hz.HEC]) < 3 * min(t[hz.HEM])
