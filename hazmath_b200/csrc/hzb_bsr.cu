@@ -880,7 +880,8 @@ forward:
         HZB_TRY(bsr_smoothing(S, L, cyc, true));
         bsr_residual(L, E.b, E.x, E.w, s);
         Level &Cn = H.lv[l + 1].s;
-        HZB_TRY(restrict_agg<double>(E.nc, E.ria, E.rja, E.w, Cn.b, s));
+        HZB_TRY(restrict_agg<double>(E.nc, E.ria, E.rja, E.w, Cn.b, s, nullptr,
+                                     S->amg.aggregation_type == VMB));
         ++l;
         HZB_TRY(vzero<double>(Cn.n, Cn.x, s));
     }

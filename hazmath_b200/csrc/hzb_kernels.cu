@@ -658,10 +658,23 @@ int autotune_fp32(DCsr<float> &A, const float *b, const float *x, float *xn, cud
 // Two aggregates a thread, the first two rows of each (most have no more) in
 // flight together: the chain from an aggregate's range over its rows to their
 // values was waited for row by row (110 us a cycle on those levels, 87 now).
-template <typename T>
+// LARGE: an aggregate a thread, row by row in a plain loop, whose loads the
+// compiler batches: for hierarchies with aggregates of a dozen rows and more
+// (HEC on 60^3 points: 645 us a solve, 906 by pairs; batches of 4 and 8 behind
+// the pair between 640 and 1010, with the pairs' levels up to 1 % slower).
+template <typename T, bool LARGE>
 __global__ void k_restrict(int nc, const int *__restrict__ ria,
                            const int *__restrict__ rja, const T *__restrict__ w,
                            T *__restrict__ bc, const unsigned char *__restrict__ act) {
+    if constexpr (LARGE) {
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+            if (act && !act[c / ACT_ROWS]) continue;
+            T t = T(0);
+            for (int k = ria[c]; k < ria[c + 1]; ++k) t += w[rja[k]];
+            bc[c] = t;
+        }
+        return;
+    }
     constexpr int U = 2;
     const unsigned step = gridDim.x * blockDim.x;
     for (unsigned c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 < (unsigned)nc; c0 += U * step) {
@@ -696,17 +709,18 @@ __global__ void k_restrict(int nc, const int *__restrict__ ria,
 
 template <typename T>
 int restrict_agg(int nc, const int *ria, const int *rja, const T *w, T *bc,
-                 cudaStream_t s, const unsigned char *act_c) {
+                 cudaStream_t s, const unsigned char *act_c, bool large) {
     if (nc <= 0) return SUCCESS;
-    k_restrict<T><<<grid_for(nc), 256, 0, s>>>(nc, ria, rja, w, bc, act_c);
+    if (large) k_restrict<T, true><<<grid_for(nc), 256, 0, s>>>(nc, ria, rja, w, bc, act_c);
+    else k_restrict<T, false><<<grid_for(nc), 256, 0, s>>>(nc, ria, rja, w, bc, act_c);
     count_launch();
     HZB_LAUNCH_CHECK();
     return SUCCESS;
 }
 template int restrict_agg<double>(int, const int *, const int *, const double *,
-                                  double *, cudaStream_t, const unsigned char *);
+                                  double *, cudaStream_t, const unsigned char *, bool);
 template int restrict_agg<float>(int, const int *, const int *, const float *,
-                                 float *, cudaStream_t, const unsigned char *);
+                                 float *, cudaStream_t, const unsigned char *, bool);
 
 // four rows a thread, as in k_l1_first (104 us a cycle, 76 now)
 template <typename T>

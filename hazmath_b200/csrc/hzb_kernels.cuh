@@ -120,7 +120,7 @@ int spmv_blocks(int n);
 // b_c[c] = sum over R row c of w (R rows list fine indices ascending).
 template <typename T>
 int restrict_agg(int nc, const int *ria, const int *rja, const T *w, T *bc,
-                 cudaStream_t s, const unsigned char *act_c = nullptr);
+                 cudaStream_t s, const unsigned char *act_c = nullptr, bool large = false);
 // x_i (+/-)= alpha * x_c[agg_i] as dcsr_aAxpy_agg does for unit P.
 template <typename T>
 int prolong_agg(int n, const int *agg, const T *xc, T *x, T alpha,

@@ -380,7 +380,8 @@ static bool smoother_needs_gs(int sm) {
 int restrict_level(hzb_solver *S, int l, const double *w, double *bc) {
     const Level &L = S->lv[l];
     if (L.sa) return spmv<double>(L.R64(), SPMV_Y, w, nullptr, bc, 1.0, nullptr, S->s);
-    return restrict_agg<double>(L.nc, L.ria, L.rja, w, bc, S->s);
+    return restrict_agg<double>(L.nc, L.ria, L.rja, w, bc, S->s, nullptr,
+                                L.largest_agg > SMALL_AGG);
 }
 
 int prolong_level(hzb_solver *S, int l, const double *xc, double *x, double alpha) {
@@ -550,7 +551,8 @@ int cycle32(hzb_solver *S, const AMG_param &cyc, bool level0_zero) {
             HZB_TRY(smooth32(S, l, true, cyc, l > 0 || level0_zero));
             HZB_TRY(spmv<float>(L.A32(), SPMV_RES, L.x32, L.b32, L.w32, 1.0f, nullptr, S->s));
             if (l + 1 < small)
-                HZB_TRY(restrict_agg<float>(L.nc, L.ria, L.rja, L.w32, S->lv[l + 1].b32, S->s));
+                HZB_TRY(restrict_agg<float>(L.nc, L.ria, L.rja, L.w32, S->lv[l + 1].b32, S->s,
+                                            nullptr, L.largest_agg > SMALL_AGG));
         }
         HZB_TRY(small_levels<float>(S, small, 0, cyc));
         for (int l = small - 1; l >= 0; --l) {
@@ -573,7 +575,7 @@ forward:
         zero[l] = false;
         HZB_TRY(spmv<float>(L.A32(), SPMV_RES, L.x32, L.b32, L.w32, 1.0f, nullptr, S->s));
         HZB_TRY(restrict_agg<float>(L.nc, L.ria, L.rja, L.w32, S->lv[l + 1].b32, S->s,
-                                    S->lv[l + 1].act));
+                                    S->lv[l + 1].act, L.largest_agg > SMALL_AGG));
         ++l;
         if (l < nl - 1) zero[l] = true;   // x_l = 0, folded into its first sweep
     }
@@ -1048,21 +1050,16 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
         HZB_TRY(S->kwc.alloc(S->lv[S->nl - 1].n, s));
     if (S->bp.precision == HZB_PREC_MIXED) HZB_TRY(ensure_fp32(S));
     trace.mark("fp32");
-    // the sizes of the aggregates, for the rule of the merged kernels
-    int largest[MAX_AMG_LVL] = {0}, *d_largest = nullptr;
-    if (!batch) {
-        HZB_TRY(dalloc(&d_largest, MAX_AMG_LVL));
-        rc = cudaMemsetAsync(d_largest, 0, sizeof(largest), s) == cudaSuccess ? SUCCESS
-                                                                             : ERROR_SOLVER_MISC;
-        for (int l = 0; l < std::min<int>(S->nl - 1, MAX_AMG_LVL) && !rc; ++l)
-            if (S->lv[l].ria && !S->lv[l].sa && S->lv[l].n <= SMALL_NNZ_64)
-                rc = longest_row(S->lv[l].nc, S->lv[l].ria, d_largest + l, s);
-        if (!rc && cudaMemcpyAsync(largest, d_largest, sizeof(largest), cudaMemcpyDeviceToHost,
-                                   s) != cudaSuccess)
-            rc = ERROR_SOLVER_MISC;
-        dfree(d_largest);
-        HZB_TRY(rc);
-    }
+    // the sizes of the aggregates, for the rules of the merged kernels and the
+    // restriction: counted in the solve's scalars (zero until then), read with the
+    // synchronisation below
+    const size_t largest_bytes = MAX_AMG_LVL * sizeof(int);
+    static_assert(MAX_AMG_LVL * sizeof(int) <= SC_ERR * sizeof(double), "scalars too few");
+    for (int l = 0; l < std::min<int>(S->nl - 1, MAX_AMG_LVL); ++l)
+        if (S->lv[l].ria && !S->lv[l].sa)
+            HZB_TRY(longest_row(S->lv[l].nc, S->lv[l].ria, (int *)S->kw.sc + l, s));
+    HZB_CUDA(cudaMemcpyAsync(S->kw.h_sc, S->kw.sc, largest_bytes, cudaMemcpyDeviceToHost, s));
+    HZB_CUDA(cudaMemsetAsync(S->kw.sc, 0, largest_bytes, s));
     HZB_CUDA(cudaEventRecord(S->e1, s));
     HZB_CUDA(cudaEventSynchronize(S->e1));
     float ms = 0.f;
@@ -1070,7 +1067,7 @@ int setup(hzb_solver *S, int n, int nnz, const int *d_ia, const int *d_ja,
     S->st.setup_seconds = ms * 1e-3;
     S->st.num_levels = S->nl;
     for (int l = 0; l < std::min<int>(S->nl - 1, MAX_AMG_LVL); ++l)
-        if (largest[l]) S->lv[l].largest_agg = largest[l];
+        if (const int largest = ((const int *)S->kw.h_sc)[l]) S->lv[l].largest_agg = largest;
     for (int l = 0; l < S->nl && l < MAX_AMG_LVL; ++l) {
         S->st.rows[l] = S->lv[l].n;
         S->st.nnz[l] = S->lv[l].nnz;
