@@ -1362,39 +1362,68 @@ k_rap_rows(int nc, const int *__restrict__ ria, const int *__restrict__ rja,
     }
 }
 
-// Rows with a bound above RAP_CAP2, a thread each, slots in scratch at off[c]
-__global__ void k_rap_build_big(int nc, const int *__restrict__ ria,
-                                const int *__restrict__ rja, const int *__restrict__ ia,
-                                const int *__restrict__ ja, const double *__restrict__ a,
-                                const int *__restrict__ agg, const int *__restrict__ off,
-                                const int *__restrict__ list, int nlist, int *scol, double *sval,
-                                int *rowcnt) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nlist;
-         t += gridDim.x * blockDim.x) {
+// Rows with a bound above RAP_CAP2, a warp each, slots in scratch at off[c]: the
+// entries one by one in order, each column looked for by all lanes.  (A thread a
+// row, a list of nothing but long rows took 1074 ms where 941 had been spread
+// over all rows' warps: HEC aggregates of a random graph of 60 entries a row;
+// 43 now.)
+__global__ void __launch_bounds__(128)
+k_rap_build_big(const int *__restrict__ ria, const int *__restrict__ rja,
+                const int *__restrict__ ia, const int *__restrict__ ja,
+                const double *__restrict__ a, const int *__restrict__ agg,
+                const int *__restrict__ off, const int *__restrict__ list, int nlist, int *scol,
+                double *sval, int *rowcnt) {
+    constexpr int B = 4;            // places that a lane looks at together
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nlist; t += warps) {
         const int c = list[t];
         int *cols = scol + off[c];
         double *vals = sval + off[c];
         int cnt = 1;
-        cols[0] = c;
-        vals[0] = 0.0;
+        if (lane == 0) {
+            cols[0] = c;
+            vals[0] = 0.0;
+        }
+        __syncwarp();
         for (int q = ria[c]; q < ria[c + 1]; ++q) {
-            const int i = rja[q];
-            for (int k = ia[i]; k < ia[i + 1]; ++k) {
-                const int cc = agg[ja[k]];
-                if (cc < 0) continue;
-                int pos = -1;
-                for (int u = 0; u < cnt; ++u)
-                    if (cols[u] == cc) { pos = u; break; }
-                if (pos >= 0) {
-                    vals[pos] += a[k];
-                } else {
-                    cols[cnt] = cc;
-                    vals[cnt] = a[k];
-                    ++cnt;
+            const int k1 = ia[rja[q] + 1];
+            for (int kb = ia[rja[q]]; kb < k1; kb += 32) {
+                const int mine = kb + lane < k1 ? agg[ja[kb + lane]] : -1;
+                const double v = kb + lane < k1 ? a[kb + lane] : 0.0;
+                for (int j = 0; j < min(32, k1 - kb); ++j) {
+                    const int cc = __shfl_sync(FULL, mine, j);
+                    const double x = __shfl_sync(FULL, v, j);
+                    if (cc < 0) continue;
+                    int pos = -1;
+                    for (int u0 = 0; u0 < cnt && pos < 0; u0 += 32 * B) {
+                        int at[B];
+#pragma unroll
+                        for (int w = 0; w < B; ++w) {
+                            const int u = u0 + 32 * w + lane;
+                            at[w] = u < cnt ? cols[u] : -1;
+                        }
+#pragma unroll
+                        for (int w = 0; w < B; ++w) {
+                            const unsigned hit = __ballot_sync(FULL, at[w] == cc);
+                            if (hit) pos = u0 + 32 * w + __ffs(hit) - 1;
+                        }
+                    }
+                    if (lane == 0) {
+                        if (pos >= 0) {
+                            vals[pos] += x;
+                        } else {
+                            cols[cnt] = cc;
+                            vals[cnt] = x;
+                        }
+                    }
+                    if (pos < 0) ++cnt;
+                    __syncwarp();
                 }
             }
         }
-        rowcnt[c] = cnt;
+        if (lane == 0) rowcnt[c] = cnt;
     }
 }
 // and their rows copied to the product, a warp each
@@ -1453,7 +1482,7 @@ int rap_agg(const DCsr<double> &A, int nc, const int *agg, const int *ria,
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
     if (h[2]) {
-        // rows of thousands of entries: bounds, scratch and a thread per row
+        // rows of thousands of entries: bounds, scratch and a warp per row
         int total = 0;
         if ((rc = dalloc(&ub, nc))) goto fail;
         if ((rc = dalloc(&off, nc + 1))) goto fail;
@@ -1465,9 +1494,8 @@ int rap_agg(const DCsr<double> &A, int nc, const int *agg, const int *ria,
         if (e != cudaSuccess) { set_error(e, __FILE__, __LINE__); rc = ERROR_SOLVER_MISC; goto fail; }
         if ((rc = dalloc(&scol, total))) goto fail;
         if ((rc = dalloc(&sval, total))) goto fail;
-        k_rap_build_big<<<grid_for(h[2], 128), 128, 0, s>>>(
-            nc, ria, rja, A.ia, A.ja, A.val, agg, off, list + (size_t)2 * nc, h[2], scol, sval,
-            rowcnt);
+        k_rap_build_big<<<grid_for(32LL * h[2], 128), 128, 0, s>>>(
+            ria, rja, A.ia, A.ja, A.val, agg, off, list + (size_t)2 * nc, h[2], scol, sval, rowcnt);
         count_launch();
         if ((rc = scan_exclusive(rowcnt, cia, nc, tmp, s))) goto fail;
         e = cudaMemcpyAsync(&h[3], cia + nc, sizeof(int), cudaMemcpyDeviceToHost, s);
