@@ -11,6 +11,7 @@ import hashlib
 
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import hazmath_b200 as hz
 from hazmath_b200 import problems as P
@@ -176,5 +177,32 @@ def test_bsr_precond_block_sizes_vs_oracle(port, nb, N, smoother):
     assert S.setup_bsr_host(nb, ia, ja, val) == 0, hz.last_error()
     z = S.bsr_precond_host(r)
     assert np.array_equal(z, S.bsr_precond_host(r))
+    S.close()
+    np.testing.assert_allclose(z, z_o, rtol=0, atol=ZTOL * np.abs(z_o).max())
+
+
+@pytest.mark.parametrize("nb", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("nx,ny", [(700, 1), (3, 300), (40, 9)])
+def test_bsr_small_level_sets_vs_oracle(port, nb, nx, ny):
+    """Level sets that one CTA of a warp or a few takes at a time: a block chain
+    (a row a set), narrow strips."""
+    i = np.arange(nx * ny).reshape(ny, nx)
+    a = np.r_[i[:, :-1].ravel(), i[:-1].ravel()]
+    b = np.r_[i[:, 1:].ravel(), i[1:].ravel()]
+    n = nx * ny
+    A = sp.coo_matrix((-np.ones(len(a)), (a, b)), shape=(n, n)).tocsr()
+    A = (A + A.T + sp.eye(n) * 4.2).tocsr()
+    A.sort_indices()
+    B = 2.0 * np.eye(nb) + 0.3 / nb * np.add.outer(np.arange(nb), np.arange(nb)) / nb
+    P.BLOCK_COUPLING.setdefault(nb, B)
+    ia, ja, val = P.block_system(A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data,
+                                 nb, 60 + nb)
+    r = P.rhs_uniform(n * nb, 7)
+    port.bsr_hierarchy(nb, ia, ja, val, coarse_dof=60)
+    z_o = port.bsr_precond(r, cycle_type=1, smoother=hz.SMOOTHER_GS, presmooth_iter=1)
+    S = hz.Solver(hz.bench_amg(coarse_dof=60, coarse_solver=0, smoother=hz.SMOOTHER_GS),
+                  itparam("pcg"))
+    assert S.setup_bsr_host(nb, ia, ja, val) == 0, hz.last_error()
+    z = S.bsr_precond_host(r)
     S.close()
     np.testing.assert_allclose(z, z_o, rtol=0, atol=ZTOL * np.abs(z_o).max())
