@@ -340,27 +340,28 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 // ms, 12,187 0.74 and 0.83, 16,256 1.33 and 2.06, 32,512 1.72 and 4.34).
 constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = HEM_BLOCK * HEM_CLUSTER;
 
-// A chain is decided one row a round.  So every HEM_PACE rounds their pace is
-// looked at, and when the rows left would take longer at it than the walk below
-// takes for all of them (a round lasts as long as walk_rows of its rows), the
-// rounds stop and the walk starts over.  Of 2D and 3D hierarchies no level came
-// near it (at most 0.65 of the walk's time predicted, over 64 rounds; 32 rounds
-// are too few, a sweep front needs some tens to build up), of chains and strips
-// of up to 16 rows all were beyond it.
-//   Chains of 100,000 and 1,000,000 rows: 281 and 3045 ms in rounds, 6.6 and 61
-// with the walk; strips of 16 x 7,500 and 64 x 1,875: 22 and 6.0 in rounds, 7.8
-// and 6.0 so.  Up to HEM_WALK_SMALL rows the walk is the faster one anyway (2D,
-// 3D and anisotropic grids of 2,000 rows: 0.51 to 0.56 ms against 0.53 to 0.61;
-// of 4,000: 0.62 to 0.74 against 0.57 to 0.63).
-constexpr int HEM_WALK_SMALL = 2048;
-constexpr unsigned HEM_PACE = 64;
-constexpr int HEM_WALK_ROWS_GRID = 43, HEM_WALK_ROWS_CLUSTER = 20;   // 3.6 and 1.7 us a round
+// A chain is decided one row a round.  So every HEM_PACE rounds the rows decided
+// in them are looked at, and the rounds stop for the walk below, which starts
+// over, when at this pace, and with it growing on as it did since the window
+// before, they would not be through in the walk's time for all rows (a round
+// lasts as long as HEM_WALK_ROWS of them: 4 to 5 us against 60 to 82 ns).  The
+// growth counts: on 2D levels a front builds up for hundreds of rounds, and by
+// the pace alone those gave up (500,000 rows: 30 ms instead of 16).  Over 150
+// levels of 2D, anisotropic, 3D and strip hierarchies no stop cost more than the
+// rounds to their end (sum 245 ms; 284 in rounds, 232 with the better of the two
+// each time).  Chains of 100,000 and 1,000,000 rows: 281 and 3045 ms in rounds,
+// 6.6 and 61 so; strips of 16 x 7,500 points 22 and 7.8.
+//   Up to HEM_WALK_SMALL rows the walk goes first: 0.30 to 0.55 ms a call where
+// the rounds take 0.34 to 2.2 (2D 0.69 and 0.40, log-normal 3D 0.87 and 0.48,
+// constant 3D 0.34 and 0.41, all of about 3,900 rows).
+constexpr unsigned HEM_PACE = 32;
+constexpr int HEM_WALK_ROWS = 43, HEM_WALK_SMALL = 4096;
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HEM_BLOCK)
 k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, int *state,
              unsigned long long *post, int *next, unsigned long long *bar, int *err,
-             int walk_rows, int *stopped) {
+             int may_stop, int *stopped) {
     const int lane = threadIdx.x & 31;
     constexpr int B = 4;             // candidates examined at a time
     __shared__ int s_count[2][HEM_CLUSTER];
@@ -369,6 +370,7 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
     bool more = true;                // rows may be left to take
     GridTally tally;
     unsigned total = 0, paced = 0;   // rows decided, by now and at the last look
+    float pace = 0.f;                // in the window before that
     const unsigned max_round = 3u * (unsigned)n + 16u;
     for (unsigned r = 1;; ++r) {
         const unsigned long long *prev = post + (size_t)((r - 1) & 1u) * n;
@@ -446,12 +448,15 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             return;
         }
         if (total == (unsigned)n) return;
-        if (walk_rows && r % HEM_PACE == 0) {
-            if ((long long)(n - (int)total) * HEM_PACE * walk_rows >
-                (long long)(total - paced) * n) {
+        if (may_stop && r % HEM_PACE == 0) {
+            // the same for every CTA: only the common count goes in
+            const float d = (float)(total - paced), w = (float)n / (HEM_WALK_ROWS * HEM_PACE);
+            if (r > HEM_PACE &&
+                d * w + 0.5f * fmaxf(0.f, d - pace) * w * w < (float)(n - (int)total)) {
                 if (blockIdx.x == 0 && threadIdx.x == 0) *stopped = 1;
                 return;
             }
+            pace = d;
             paced = total;
         }
         if (need) {
@@ -881,9 +886,7 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             HZB_CUDA(cudaLaunchKernelEx(
                 &cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia,
                 (const int *)cand, agg, post, out + O_NEXT, (unsigned long long *)(out + O_BAR),
-                out + O_ERR,
-                !may_stop ? 0 : cluster ? HEM_WALK_ROWS_CLUSTER : HEM_WALK_ROWS_GRID,
-                out + O_STOP));
+                out + O_ERR, (int)may_stop, out + O_STOP));
             k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
             count_launch(2);
             HZB_TRY(scan_exclusive(flag, pos, n, tmp, s));

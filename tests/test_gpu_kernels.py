@@ -388,13 +388,36 @@ def test_hem_chain_no_slower_than_the_walk(monkeypatch):
     assert best["0"] < 3 * best["2"]
 
 
-@pytest.mark.parametrize("nx,ny", [(64, 32), (683, 3), (64, 128), (2731, 3), (128, 128)])
+@pytest.mark.parametrize("nx,ny", [(64, 64), (4097, 1), (64, 128), (2731, 3), (128, 128)])
 def test_hem_rounds_of_cluster_and_grid(port, monkeypatch, nx, ny):
     """Both sides of the sizes where the walk, the cluster and the grid take over
-    (2048 and 8192 rows), the rounds to their end too."""
+    (4096 and 8192 rows), the rounds to their end too."""
     ia, ja, val = _strip(nx, ny, seed=5)
     nc_o, agg_o = port.hem(ia, ja, val, 0.0)
     for path in ("0", "1"):
         monkeypatch.setenv("HZB_HEM_PATH", path)
         nc, agg = _hem(ia, ja, val, 0.0)
         assert nc == nc_o and np.array_equal(agg, agg_o)
+
+
+def test_hem_rounds_are_not_given_up_on_a_growing_front(monkeypatch):
+    """The first coarse level of a 2D grid of 600^2 points, whose sweep front
+    builds up for hundreds of rounds: no more than 1.3 times the rounds to their
+    end (given up by the pace of the first rounds alone, 2.3 times)."""
+    import time
+    ia, ja, val = P.aniso2d_p1(600, 1.0, 0.0)
+    S = hz.Solver(hz.bench_amg(smoother=hz.SMOOTHER_L1DIAG))
+    assert S.setup_host(ia, ja, val) == 0
+    A = DevCSR(*S.level(1)[:3])
+    S.close()
+    agg, nc = dev(np.zeros(A.n, np.int32)), C.c_int()
+    best = {}
+    for path in ("0", "1"):
+        monkeypatch.setenv("HZB_HEM_PATH", path)
+        times = []
+        for _ in range(4):
+            t = time.perf_counter()
+            assert hz.lib().hzb_aggregation_hem_device(*A.args(), 0.0, ptr(agg), C.byref(nc)) == 0
+            times.append(time.perf_counter() - t)
+        best[path] = min(times)
+    assert best["0"] < 1.3 * best["1"]
