@@ -1214,7 +1214,7 @@ def run_bsr(args, rank, world, local, dist):
             "setup_s": statistics.mean(setup_s), "solve_s": statistics.mean(solve_s),
             "dof_per_s": n / statistics.mean(solve_s),
             "roofline": {"bound": "hbm", "kernel": "level-0 ascending block Gauss-Seidel "
-                         "sweep (k_bsr_gs_set<3> / k_bsr_gs_run<3> over the level sets)",
+                         "sweep (k_bsr_gs_sets_grid<3> / k_bsr_gs_cluster<3> over the level sets)",
                          "achieved": gs_gbs, "peak": peak, "unit": "GB/s",
                          "frac": gs_gbs / peak, "peak_kind": peak_kind,
                          "bytes_per_launch": gs_by, "ms_per_launch": gs_ms, "traffic": None},

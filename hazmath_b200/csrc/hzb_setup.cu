@@ -326,10 +326,10 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 // its candidates.  The smallest undecided row is always decided within three
 // rounds, so the loop ends.
 //
-// Bound by the latency of a round (row state, previous posts, barrier: 3 to
-// 4 us over the grid), not by bytes: a walk of one CTA took 83 ns per row
-// (167 ms for the 2,048,383 rows of the 128^3 log-normal system, 318 ms for
-// its hierarchy; 11.8 and 37 ms now).
+// Bound by the latency of a round (row state, previous posts, barrier: 4 to 5
+// us), not by bytes: a walk of one CTA takes 60 to 83 ns per row (167 ms for the
+// 2,048,383 rows of the 128^3 log-normal system, 318 ms for its hierarchy; 11.8
+// and 30 ms in rounds).
 //
 // CLUSTER: the CTAs are one cluster of at most 8, whose barrier and counts (in
 // every member's shared memory) cost less.  For levels whose rows are all in

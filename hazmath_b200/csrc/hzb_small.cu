@@ -1,8 +1,9 @@
 // hzb_small.cu -- the l1-Jacobi V-cycle on its small levels.
 //
-// Below some ten thousand rows a level lies in L2, and a kernel lasts as long
-// as its launch (about 1 us between the nodes of a graph) and its chain of
-// dependent loads: row pointers, columns, x, at 0.3 to 0.4 us each.  So here
+// A small level (SMALL_ROWS_32, SMALL_NNZ_64: some hundred thousand rows) lies in
+// L2, and a kernel lasts as long as its launch and its chain of dependent loads:
+// row pointers, columns, x, at 0.3 to 0.4 us each (2.4 us a node of the graph in
+// all on the smallest).  So here
 // work is merged where a row's result is all the next step needs of it: the
 // residual is formed for the fine rows of a coarse row and summed at once,
 // with the coarse level's first sweep from x = 0 (b_i / d_i) behind it, and
