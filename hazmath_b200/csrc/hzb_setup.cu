@@ -356,12 +356,16 @@ constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = HEM_BLOCK * 
 // constant 3D 0.34 and 0.41, all of about 3,900 rows).
 constexpr unsigned HEM_PACE = 32;
 constexpr int HEM_WALK_ROWS = 43, HEM_WALK_SMALL = 4096;
+// A graph that reaches too far for the walk's ring (524,000 rows) goes on in
+// rounds, unless one warp on the rows themselves, 1 us each, is the faster one at
+// that (a periodic chain of 600,000 rows: 0.6 s, 1.8 in rounds).
+constexpr int HEM_WARP_ROWS = 4;
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HEM_BLOCK)
 k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, int *state,
              unsigned long long *post, int *next, unsigned long long *bar, int *err,
-             int may_stop, int *stopped) {
+             int walk_rows, int *stopped) {
     const int lane = threadIdx.x & 31;
     constexpr int B = 4;             // candidates examined at a time
     __shared__ int s_count[2][HEM_CLUSTER];
@@ -448,9 +452,9 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             return;
         }
         if (total == (unsigned)n) return;
-        if (may_stop && r % HEM_PACE == 0) {
+        if (walk_rows && r % HEM_PACE == 0) {
             // the same for every CTA: only the common count goes in
-            const float d = (float)(total - paced), w = (float)n / (HEM_WALK_ROWS * HEM_PACE);
+            const float d = (float)(total - paced), w = (float)n / (walk_rows * HEM_PACE);
             if (r > HEM_PACE &&
                 d * w + 0.5f * fmaxf(0.f, d - pace) * w * w < (float)(n - (int)total)) {
                 if (blockIdx.x == 0 && threadIdx.x == 0) *stopped = 1;
@@ -853,7 +857,7 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             HZB_CUDA(cudaStreamSynchronize(s));
             return SUCCESS;
         };
-        auto rounds = [&](bool may_stop) -> int {
+        auto rounds = [&](int walk_rows) -> int {
             rank();
             // all ones: older than any round's post
             HZB_CUDA(cudaMemsetAsync(post, 0xff, sizeof(unsigned long long) * 2 * n, s));
@@ -886,7 +890,7 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             HZB_CUDA(cudaLaunchKernelEx(
                 &cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia,
                 (const int *)cand, agg, post, out + O_NEXT, (unsigned long long *)(out + O_BAR),
-                out + O_ERR, (int)may_stop, out + O_STOP));
+                out + O_ERR, walk_rows, out + O_STOP));
             k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
             count_launch(2);
             HZB_TRY(scan_exclusive(flag, pos, n, tmp, s));
@@ -919,15 +923,13 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             return leftovers();
         };
         bool walked = false;
-        if (path == 2) rc = walk(&walked);
-        else rc = rounds(path == 0);
-        if (!rc && path == 0 && h[O_STOP]) {
+        if (path != 2) rc = rounds(path == 0 ? HEM_WALK_ROWS : 0);
+        if (!rc && (path == 2 || h[O_STOP])) {
             rc = walk(&walked);
-            if (!rc && !walked) rc = rounds(false);
-        } else if (!rc && path == 2 && !walked) {
-            rc = rounds(false);
+            if (!rc && !walked) rc = rounds(HEM_WARP_ROWS);
+            if (!rc && !walked && h[O_STOP]) path = 4;
         }
-        if (!rc && !h[O_ERR]) {
+        if (!rc && !h[O_ERR] && path != 4) {
             if (m > 0) {
                 k_hem_pass2_list<<<1, 32, 0, s>>>(m, cand, nia, nja, agg, cnt, out);
                 count_launch();
@@ -936,7 +938,8 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             count_launch();
         }
         dfree(cand); dfree(post); dfree(flag); dfree(pos); dfree(tmp);
-    } else {   // the whole state in global memory
+    }
+    if (!rc && path == 4) {   // the whole state in global memory
         k_hem_seq<<<1, 32, 0, s>>>(n, nia, nja, nval, agg, work_n, out);
         count_launch();
     }
