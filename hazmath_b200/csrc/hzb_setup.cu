@@ -341,31 +341,37 @@ __global__ void k_hem_rank(int n, const int *__restrict__ ia, const int *__restr
 constexpr int HEM_BLOCK = 1024, HEM_CLUSTER = 8, HEM_CLUSTER_ROWS = HEM_BLOCK * HEM_CLUSTER;
 
 // A chain is decided one row a round.  So every HEM_PACE rounds the rows decided
-// in them are looked at, and the rounds stop for the walk below, which starts
+// in them and the time they took are looked at (the first CTA's, for all; either
+// way gives the same map), and the rounds stop for the walk below, which starts
 // over, when at this pace, and with it growing on as it did since the window
-// before, they would not be through in the walk's time for all rows (a round
-// lasts as long as HEM_WALK_ROWS of them: 4 to 5 us against 60 to 82 ns).  The
-// growth counts: on 2D levels a front builds up for hundreds of rounds, and by
-// the pace alone those gave up (500,000 rows: 30 ms instead of 16).  Over 150
-// levels of 2D, anisotropic, 3D and strip hierarchies no stop cost more than the
-// rounds to their end (sum 245 ms; 284 in rounds, 232 with the better of the two
-// each time).  Chains of 100,000 and 1,000,000 rows: 281 and 3045 ms in rounds,
-// 6.6 and 61 so; strips of 16 x 7,500 points 22 and 7.8.
+// before, they would not be through in the walk's time for all rows, hem_walk_ns
+// each.  The growth counts: on 2D levels a front builds up for hundreds of rounds,
+// and by the pace alone those gave up (500,000 rows: 30 ms instead of 16).  The
+// time counts: a round of 4 to 5 us takes 12 to 21 when long rows crowd into a
+// narrow band.  Over 150 levels of 2D, anisotropic, 3D and strip hierarchies
+// 254 ms (288 in rounds, 651 as walks).  Chains of 100,000 and
+// 1,000,000 rows: 281 and 3045 ms in rounds, 6.6 and 61 so; strips of 16 x 7,500
+// points 22 and 7.8; 200,000 rows of 30 entries within 300 columns 55 and 19.5.
 //   Up to HEM_WALK_SMALL rows the walk goes first: 0.30 to 0.55 ms a call where
 // the rounds take 0.34 to 2.2 (2D 0.69 and 0.40, log-normal 3D 0.87 and 0.48,
-// constant 3D 0.34 and 0.41, all of about 3,900 rows).
+// constant 3D 0.34 and 0.41, all of about 3,900 rows), and in proportion to the
+// rows' length above 25 entries (random graphs of 8,000 rows with 50 entries 2.0
+// and 2.2 ms, with 200 3.1 and 8.3; of 16,000 with 100 4.4 and 4.5).
 constexpr unsigned HEM_PACE = 32;
-constexpr int HEM_WALK_ROWS = 43, HEM_WALK_SMALL = 4096;
+constexpr int HEM_WALK_SMALL = 4096, HEM_WALK_ROW = 25;
+// the walk takes 60 to 80 ns a row of 5 to 15 entries, 85 to 180 of 30, 220 to 440
+// of 100; a third more here, so that it is clearly the faster one
+inline float hem_walk_ns(int n, int nnz) { return 85.f + 1.5f * (float)nnz / (float)n; }
 // A graph that reaches too far for the walk's ring (524,000 rows) goes on in
 // rounds, unless one warp on the rows themselves, 1 us each, is the faster one at
 // that (a periodic chain of 600,000 rows: 0.6 s, 1.8 in rounds).
-constexpr int HEM_WARP_ROWS = 4;
+constexpr float HEM_WARP_NS = 1300.f;
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HEM_BLOCK)
 k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, int *state,
              unsigned long long *post, int *next, unsigned long long *bar, int *err,
-             int walk_rows, int *stopped) {
+             float walk_ns, int *stopped, unsigned *window_ns) {
     const int lane = threadIdx.x & 31;
     constexpr int B = 4;             // candidates examined at a time
     __shared__ int s_count[2][HEM_CLUSTER];
@@ -375,6 +381,7 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
     GridTally tally;
     unsigned total = 0, paced = 0;   // rows decided, by now and at the last look
     float pace = 0.f;                // in the window before that
+    unsigned long long clock = 0;    // of the first CTA's first thread
     const unsigned max_round = 3u * (unsigned)n + 16u;
     for (unsigned r = 1;; ++r) {
         const unsigned long long *prev = post + (size_t)((r - 1) & 1u) * n;
@@ -435,6 +442,12 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             if (!done) atomicMin(cur + u, mark | (unsigned)u);
             if (done) u = -1;
         }
+        if (walk_ns > 0.f && r % HEM_PACE == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+            __stcg(window_ns, (unsigned)min(now - clock, 0xffffffffull));
+            clock = now;
+        }
         // rows for the threads without one, ascending
         const unsigned need = __ballot_sync(0xffffffffu, u < 0);
         int base = n;
@@ -452,9 +465,10 @@ k_hem_rounds(int n, const int *__restrict__ ia, const int *__restrict__ cand, in
             return;
         }
         if (total == (unsigned)n) return;
-        if (walk_rows && r % HEM_PACE == 0) {
-            // the same for every CTA: only the common count goes in
-            const float d = (float)(total - paced), w = (float)n / (walk_rows * HEM_PACE);
+        if (walk_ns > 0.f && r % HEM_PACE == 0) {
+            // the same for every CTA: only the common count and time go in
+            const float d = (float)(total - paced);
+            const float w = (float)n * walk_ns / fmaxf(1.f, (float)__ldcg(window_ns));
             if (r > HEM_PACE &&
                 d * w + 0.5f * fmaxf(0.f, d - pace) * w * w < (float)(n - (int)total)) {
                 if (blockIdx.x == 0 && threadIdx.x == 0) *stopped = 1;
@@ -803,9 +817,10 @@ __global__ void k_hem_final(int n, int *mask) {
 
 int hem_exact(int n, const int *nia, const int *nja, const double *nval,
               int *agg, int *nagg, int *work_n, cudaStream_t s) {
-    // out: aggregates, status | longest row | next row | barrier (4) | error, stopped
+    // out: aggregates, status | longest row | next row | barrier (4) | error, stopped,
+    // a window's time
     enum { O_NC = 0, O_STATUS = 1, O_LEN = 2, O_NEXT = 3, O_BAR = 4, O_ERR = 8, O_STOP = 9,
-           O_N = 10 };
+           O_NS = 10, O_N = 12 };
     int *out = nullptr;
     HZB_TRY(dalloc(&out, O_N));
     int h[O_N] = {0};
@@ -829,7 +844,9 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
         const int want = atoi(f);
         if (want == 4 || (path == 0 && (want == 1 || want == 2))) path = want;
     }
-    if (path == 0 && n <= HEM_WALK_SMALL) path = 2;
+    if (path == 0 &&
+        n <= (long long)HEM_WALK_SMALL * std::max<long long>(HEM_WALK_ROW, gnnz / n) / HEM_WALK_ROW)
+        path = 2;
     if (path != 4) {
         int *cand = nullptr, *flag = nullptr, *pos = nullptr, *tmp = nullptr, m = 0;
         unsigned long long *post = nullptr;
@@ -857,7 +874,7 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             HZB_CUDA(cudaStreamSynchronize(s));
             return SUCCESS;
         };
-        auto rounds = [&](int walk_rows) -> int {
+        auto rounds = [&](float walk_ns) -> int {
             rank();
             // all ones: older than any round's post
             HZB_CUDA(cudaMemsetAsync(post, 0xff, sizeof(unsigned long long) * 2 * n, s));
@@ -890,7 +907,7 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             HZB_CUDA(cudaLaunchKernelEx(
                 &cfg, cluster ? k_hem_rounds<true> : k_hem_rounds<false>, n, nia,
                 (const int *)cand, agg, post, out + O_NEXT, (unsigned long long *)(out + O_BAR),
-                out + O_ERR, walk_rows, out + O_STOP));
+                out + O_ERR, walk_ns, out + O_STOP, (unsigned *)(out + O_NS)));
             k_hem_visitors<<<g, 256, 0, s>>>(n, agg, flag);
             count_launch(2);
             HZB_TRY(scan_exclusive(flag, pos, n, tmp, s));
@@ -923,10 +940,10 @@ int hem_exact(int n, const int *nia, const int *nja, const double *nval,
             return leftovers();
         };
         bool walked = false;
-        if (path != 2) rc = rounds(path == 0 ? HEM_WALK_ROWS : 0);
+        if (path != 2) rc = rounds(path == 0 ? hem_walk_ns(n, gnnz) : 0.f);
         if (!rc && (path == 2 || h[O_STOP])) {
             rc = walk(&walked);
-            if (!rc && !walked) rc = rounds(HEM_WARP_ROWS);
+            if (!rc && !walked) rc = rounds(HEM_WARP_NS);
             if (!rc && !walked && h[O_STOP]) path = 4;
         }
         if (!rc && !h[O_ERR] && path != 4) {
